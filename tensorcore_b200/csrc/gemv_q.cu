@@ -31,9 +31,8 @@
 #include <cstdlib>
 
 namespace tcb {
-cudaError_t init_tc_kernels(int smem_optin);
-cudaError_t launch_gemv_q4_tc(const GemvQArgs& a, const LaunchEnv& env, cudaStream_t stream,
-                              const char** name);
+cudaError_t init_gemm_q_tc_kernels(int smem_optin);
+cudaError_t launch_gemm_q_tc(const GemvQArgs& a, const LaunchEnv& env, cudaStream_t stream);
 cudaError_t init_decode_kernel(int smem_optin);
 namespace {
 
@@ -574,7 +573,7 @@ cudaError_t set_smem(K kernel, int bytes) {
 }  // namespace
 
 cudaError_t init_gemv_kernels(int smem_optin) {
-    cudaError_t e = init_tc_kernels(smem_optin);
+    cudaError_t e = init_gemm_q_tc_kernels(smem_optin);
     if (e == cudaSuccess) e = init_gemm_tc_kernel(smem_optin);
     if (e != cudaSuccess) return e;
     e = init_decode_kernel(smem_optin);
@@ -602,19 +601,48 @@ cudaError_t launch_gemv_q(const GemvQArgs& a, const LaunchEnv& env, cudaStream_t
     const size_t xsz = a.x_f32 ? 4 : 2, ysz = a.y_f32 ? 4 : 2;
     const bool fuse = a.gamma != nullptr;
 
-    // Batched decode: the tcgen05 kernel reads the weights once for up to 32 activation rows.
-    // It rounds dequantised weights to fp16, which only the fp16-activation bound allows.
-    const bool want_tc = env.variant == VARIANT_TC ||
-                         (env.variant == VARIANT_AUTO && batched_tc_rows(a.M, a.N, a.K));
-    // The fused RMSNorm form takes it too, behind a pass that normalises the rows into the stream's
-    // scratch as fp16 (one more rounding, inside the same bound).
-    const size_t slab_rows = a.M < 32 ? a.M : 32;
-    const size_t norm_need = slab_rows * static_cast<size_t>(a.K) * 2 + slab_rows * 4;
-    const bool fuse_tc = fuse && a.norm_scratch && a.norm_scratch_bytes >= norm_need && a.K % 256 == 0;
-    // Prefill-sized calls: the weights are dequantised once into the stream's scratch (fp16, the same
-    // rounding as the kernel below applies on the fly) and multiplied on the tensor cores as a GEMM
-    // with B transposed; Q8_0 too.  fp16 activations and results only (the rounding of the weights is
-    // inside their bound, not inside the fp32 one).
+    // Five rows or more (tc_rows): the tcgen05 kernel dequantises the weights on their way to the tensor
+    // cores and reads them once per 256 rows.  It rounds dequantised weights to fp16, which only the
+    // fp16-activation bound allows.  The fused RMSNorm form takes it too, behind a pass that normalises
+    // the rows into the stream's scratch as fp16 (one more rounding, inside the same bound); rows that
+    // are not 16-byte aligned are copied there.
+    if (!a.x_f32 && a.K % 256 == 0 && (env.variant == VARIANT_TC ? a.fmt == FMT_Q4_0 : env.variant == VARIANT_AUTO && tc_rows(a))) {
+        const bool copy = !fuse && (reinterpret_cast<uintptr_t>(a.X) & 15u) != 0;
+        const size_t row_bytes = static_cast<size_t>(a.K) * 2 + 4;      // a row and its 1/rms
+        size_t slab = static_cast<size_t>(a.M);
+        if (fuse || copy) slab = a.norm_scratch ? a.norm_scratch_bytes / row_bytes : 0;
+        if (slab > static_cast<size_t>(a.M)) slab = static_cast<size_t>(a.M);
+        bool done = slab > 0;
+        for (int m0 = 0; done && m0 < a.M && err == cudaSuccess; m0 += static_cast<int>(slab)) {
+            GemvQArgs s = a;
+            s.M = a.M - m0 < static_cast<int>(slab) ? a.M - m0 : static_cast<int>(slab);
+            s.X = static_cast<const uint8_t*>(a.X) + static_cast<size_t>(m0) * a.K * xsz;
+            s.Y = static_cast<uint8_t*>(a.Y) + static_cast<size_t>(m0) * a.N * ysz;
+            if (fuse) {
+                float* rstd = reinterpret_cast<float*>(static_cast<uint8_t*>(a.norm_scratch) + slab * static_cast<size_t>(a.K) * 2);
+                err = launch_norm_forward(s.X, a.gamma, nullptr, a.norm_scratch, nullptr, rstd, s.M, a.K, a.eps, stream);
+                ++count;
+            } else if (copy) {
+                err = cudaMemcpyAsync(a.norm_scratch, s.X, static_cast<size_t>(s.M) * a.K * 2, cudaMemcpyDeviceToDevice, stream);
+            }
+            if (err != cudaSuccess) break;
+            if (fuse || copy) { s.X = a.norm_scratch; s.gamma = nullptr; }
+            const cudaError_t te = launch_gemm_q_tc(s, env, stream);
+            if (te == cudaErrorNotSupported && m0 == 0) { done = false; count = 0; (void)cudaGetLastError(); break; }
+            err = te;
+            ++count;
+        }
+        if (done) {
+            if (launches) *launches += count;
+            if (name) *name = a.M >= gemm_min_rows(a.fmt) && !a.y_f32
+                                  ? (a.fmt == FMT_Q4_0 ? "q4_0_dequant_gemm_tcgen05_sm100" : "q8_0_dequant_gemm_tcgen05_sm100")
+                                  : "q4_0_gemv_tcgen05_sm100";
+            return err;
+        }
+    }
+    // Prefill-sized calls whose K is no multiple of 256: the weights are dequantised once into the
+    // stream's scratch (fp16, the same rounding as above) and multiplied on the tensor cores as a GEMM
+    // with B transposed.
     if (env.variant == VARIANT_AUTO && a.M >= gemm_min_rows(a.fmt) && !a.x_f32 && !a.y_f32 && a.dequant_scratch &&
         a.dequant_scratch_bytes >= static_cast<size_t>(a.N) * a.K * 2 && a.K % 32 == 0 &&
         (!fuse || (a.norm_scratch && a.norm_scratch_bytes >= static_cast<size_t>(a.M) * a.K * 2 + static_cast<size_t>(a.M) * 4))) {
@@ -638,33 +666,6 @@ cudaError_t launch_gemv_q(const GemvQArgs& a, const LaunchEnv& env, cudaStream_t
         }
         if (e != cudaErrorNotSupported) return e;
         (void)cudaGetLastError();
-    }
-    if (want_tc && a.fmt == FMT_Q4_0 && !a.x_f32 && (!fuse || fuse_tc)) {
-        bool done = true;
-        for (int m0 = 0; m0 < a.M; m0 += 32) {
-            GemvQArgs s = a;
-            s.M = (a.M - m0) < 32 ? (a.M - m0) : 32;
-            s.X = static_cast<const uint8_t*>(a.X) + static_cast<size_t>(m0) * a.K * xsz;
-            s.Y = static_cast<uint8_t*>(a.Y) + static_cast<size_t>(m0) * a.N * ysz;
-            if (fuse) {
-                float* rstd = reinterpret_cast<float*>(static_cast<uint8_t*>(a.norm_scratch) + slab_rows * static_cast<size_t>(a.K) * 2);
-                const cudaError_t ne = launch_norm_forward(s.X, a.gamma, nullptr, a.norm_scratch, nullptr, rstd, s.M, a.K,
-                                                           a.eps, stream);
-                if (ne != cudaSuccess) { err = ne; break; }
-                ++count;
-                s.X = a.norm_scratch;
-                s.gamma = nullptr;
-            }
-            const cudaError_t te = launch_gemv_q4_tc(s, env, stream, &used);
-            if (te == cudaErrorNotSupported && m0 == 0) { done = false; break; }
-            if (te != cudaSuccess) { err = te; break; }
-            ++count;
-        }
-        if (done) {
-            if (launches) *launches += count;
-            if (name) *name = used;
-            return err;
-        }
     }
 
     // Up to kMaxMB activation rows per pass on the integer dot-product kernels.

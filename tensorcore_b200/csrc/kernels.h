@@ -34,32 +34,32 @@ struct GemvQArgs {
     int fmt = 0, M = 0, N = 0, K = 0;
     bool x_f32 = false, y_f32 = false;
     float eps = 0.f;
-    // scratch of the stream the call runs on, for the batched fused form (batched_tc_rows, fp16): room for
-    // min(M, 32) normalised rows of K halves and as many floats; without it that form takes the
-    // integer dot-product kernels, four rows per pass
+    // scratch of the stream the call runs on, for the batched fused form (tc_rows, fp16): room for some of
+    // the M normalised rows of K halves and as many floats (the call goes through them in slabs of what
+    // fits); without it that form takes the integer dot-product kernels, four rows per pass
     void* norm_scratch = nullptr;
     size_t norm_scratch_bytes = 0;
-    // scratch of the stream for prefill-sized calls (gemm_min_rows activation rows or more, fp16 in and
-    // out): room for the weights as fp16, N * K halves; with it they are dequantised once and multiplied
-    // on the tensor cores instead of streamed once per 32 (Q4_0) or 4 (Q8_0) rows
+    // scratch of the stream for prefill-sized calls whose K is no multiple of 256 (gemm_min_rows activation
+    // rows or more, fp16 in and out): room for the weights as fp16, N * K halves; with it they are
+    // dequantised once and multiplied on the tensor cores instead of streamed once per four rows
     void* dequant_scratch = nullptr;
     size_t dequant_scratch_bytes = 0;
 };
-// Measured back to back on a stream over rotating weight copies.  Q4_0 14336 x 4096: the batched
-// kernel takes 32 rows a pass, 64 rows 44 us, 80 rows 63 us, against 64 us this way whatever the row
-// count.  Q8_0 has no batched tensor-core kernel and streams the blocks once per 4 rows: 14336 x 4096
-// 8 / 12 / 16 / 32 rows 53 / 80 / 105 / 210 us against 66 - 78 us this way; 4096 x 4096 24 / 35 / 46 /
-// 90 against 31; 28672 x 8192 155 / 232 / 308 / 615 against 243 - on every shape measured the fourth
-// pass (13 rows) is where this way wins.
+// From how many activation rows a call with fp16 activations and results counts as prefill-sized: Q8_0 calls
+// then take the tcgen05 kernel (fp16-rounded weights) instead of the integer kernels (four rows a pass),
+// and calls whose K is no multiple of 256 are dequantised once and multiplied as a GEMM.  Q8_0 14336 x 4096 on the integer
+// kernels: 8 / 12 / 16 / 32 rows 53 / 80 / 105 / 210 us; the tcgen05 kernel takes 20 us for any of them,
+// but its results carry the rounding of the weights, which these row counts did not have.
 inline int gemm_min_rows(int fmt) { return fmt == 0 ? 96 : 13; }
-// Whether a Q4_0 call with fp16 activations of M rows goes to the batched tcgen05 kernel by default.
-// Five rows or more always; four rows where the matrix is large enough that two passes' worth of
-// integer dot products cost more than the tensor-core kernel's fixed part (measured back to back on
-// a stream, M = 4: 14336 x 4096 21.3 -> 17.8 us, 4096 x 14336 28.6 -> 20.9, 8192 x 8192 23.4 -> 18.7,
-// 28672 x 8192 59.2 -> 51.5, 1024 x 8192 14.1 -> 10.7, 32000 x 4096 32.0 -> 28.8; 4096 x 4096 stays
-// on the dot-product kernel, 9.6 against 11.0 us; at three rows the two are level or the
-// dot-product kernel wins).
+// Whether a Q4_0 call with fp16 activations of M rows goes to the tcgen05 kernel by default.  Five rows or
+// more always; four rows where the matrix is large enough that the integer dot products cost more than
+// the tensor-core kernel's fixed part (M = 4 back to back: 14336 x 4096 21.3 us on the integer kernel;
+// 4096 x 4096 9.6).  Fewer rows stay on the integer kernels, which do not round the weights.
 inline bool batched_tc_rows(int M, int N, int K) { return M >= 5 || (M == 4 && (K >= 8192 || N > 4096)); }
+// Whether a call with fp16 activations and K % 256 == 0 goes to the tcgen05 kernel by default.
+inline bool tc_rows(const GemvQArgs& a) {
+    return a.fmt == 0 ? batched_tc_rows(a.M, a.N, a.K) : a.M >= gemm_min_rows(1) && !a.y_f32;
+}
 
 struct DenseNormGemvArgs {
     const void* X = nullptr;      // [M,K] fp16

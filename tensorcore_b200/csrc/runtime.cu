@@ -232,15 +232,16 @@ void dense_scratch_for(tc_context* ctx, cudaStream_t st, tcb::DenseNormGemvArgs*
 // plain fp16 activations).
 // Whether the call is prefill-sized: its weights are dequantised once and multiplied as a GEMM.
 bool dequant_gemm_wanted(const tcb::GemvQArgs& a) {
-    return a.M >= tcb::gemm_min_rows(a.fmt) && !a.x_f32 && !a.y_f32 && a.K % 32 == 0 &&
+    return a.M >= tcb::gemm_min_rows(a.fmt) && !a.x_f32 && !a.y_f32 && a.K % 256 != 0 && a.K % 32 == 0 &&
            static_cast<size_t>(a.N) * a.K * 2 <= (static_cast<size_t>(3) << 29);      // at most 1.5 GB of scratch
 }
 size_t norm_scratch_need(const tcb::GemvQArgs& a) {
-    if (!a.gamma || a.x_f32) return 0;
-    if (dequant_gemm_wanted(a)) return static_cast<size_t>(a.M) * a.K * 2 + static_cast<size_t>(a.M) * 4;
-    if (a.fmt != 0 || !tcb::batched_tc_rows(a.M, a.N, a.K) || a.K % 256 != 0) return 0;
-    const size_t rows = a.M < 32 ? a.M : 32;
-    return rows * static_cast<size_t>(a.K) * 2 + rows * 4;
+    if (a.x_f32) return 0;
+    if (dequant_gemm_wanted(a)) return a.gamma ? static_cast<size_t>(a.M) * a.K * 2 + static_cast<size_t>(a.M) * 4 : 0;
+    if (a.K % 256 != 0 || !tcb::tc_rows(a)) return 0;
+    if (!a.gamma && (reinterpret_cast<uintptr_t>(a.X) & 15u) == 0) return 0;
+    const size_t rows = a.M < 2048 ? a.M : 2048;      // larger calls go through the scratch in slabs
+    return rows * (static_cast<size_t>(a.K) * 2 + 4);
 }
 void norm_scratch_for(cudaStream_t st, size_t need, tcb::GemvQArgs* a) {
     if (need == 0) return;

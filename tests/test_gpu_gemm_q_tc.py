@@ -1,0 +1,86 @@
+"""GPU: the tcgen05 kernel that dequantises Q4_0 / Q8_0 weights on their way to the tensor cores, at the
+edges of its tiles: every accumulator layout (16, 32, 64, 128 and 256 columns, several column tiles),
+row counts around the 128-row tile, one group of K and uneven splits of K, unaligned activations.
+
+Bar against a 64-bit dequantise-and-dot: a dequantised weight is rounded to fp16 once (relative error at
+most 2^-11, 2^-11 / sqrt(3) rms, independent between products, so the same relative to the result) and an
+fp16 result once more: sqrt(2) * 2^-11 / sqrt(3) = 4.0e-4, and 2.82e-4 without the second; the margin
+of a tenth is for small samples."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROUND = 2.0 ** -11 / np.sqrt(3.0)
+
+
+def data(oracle, fmt, M, N, K):
+    rng = np.random.default_rng(M * 31 + N * 7 + K + fmt)
+    W = (rng.standard_normal((N, K)) * 0.02).astype(np.float32).astype(np.float16)
+    X = rng.standard_normal((M, K)).astype(np.float16)
+    return X, oracle.quantize_weights(W, fmt)
+
+
+@pytest.mark.parametrize("fmt,M,N,K", [
+    (0, 5, 128, 256), (0, 16, 129, 512), (0, 17, 127, 768), (0, 32, 1000, 2304), (0, 33, 260, 1024), (0, 48, 128, 1280),
+    (0, 64, 640, 2816), (0, 65, 130, 512), (0, 128, 257, 1536), (0, 129, 384, 768), (0, 256, 128, 2048),
+    (0, 257, 200, 512), (0, 300, 19000, 256), (0, 520, 136, 1024),
+    (1, 13, 128, 256), (1, 16, 1000, 4096), (1, 32, 129, 768), (1, 64, 260, 2560), (1, 80, 127, 1024),
+    (1, 128, 512, 1536), (1, 200, 130, 512), (1, 256, 300, 2304), (1, 513, 128, 768)])
+def test_tile_edges_against_64_bit(tc, ctx, oracle, fmt, M, N, K):
+    X, Wq = data(oracle, fmt, M, N, K)
+    want = oracle.dequant_dot_f64(X.astype(np.float64), Wq, fmt, N)
+    with ctx.buffer_from_array(X) as bx, ctx.buffer_from_array(Wq) as bw, ctx.buffer(M * N * 4) as by:
+        ctx.gemv_quantized(bx, bw, by, fmt, M, N, K)
+        assert "tcgen05" in tc.cuda_last_kernel_name()
+        got = by.to_numpy((M, N), np.float16).astype(np.float64)
+        assert oracle.scaled_rms(got, want) <= 1.1 * np.sqrt(2.0) * ROUND
+        if fmt == 0:                                          # fp32 results
+            tc.gemv_quantized_ex(ctx, bx, bw, by, fmt, M, N, K, "f16", "f32", None)
+            got32 = by.to_numpy((M, N), np.float32).astype(np.float64)
+            assert oracle.scaled_rms(got32, want) <= 1.1 * ROUND
+            assert np.array_equal(got32.astype(np.float32).astype(np.float16), got.astype(np.float16))
+    assert tc.take_device_error(ctx) == 0
+
+
+@pytest.mark.parametrize("fmt,M", [(0, 8), (0, 40), (1, 20)])
+def test_activations_at_any_even_address(tc, ctx, oracle, fmt, M):
+    """Rows that start 2, 8 or 14 bytes past a 16-byte boundary give the same bits as aligned ones."""
+    N, K = 300, 1024
+    X, Wq = data(oracle, fmt, M, N, K)
+    outs = []
+    for off in (0, 2, 8, 14):
+        with ctx.buffer(X.nbytes + 16) as bx, ctx.buffer_from_array(Wq) as bw, ctx.buffer(M * N * 2) as by:
+            bx.upload(X, off)
+            tc.raw_gemv_quantized(ctx, bx.device_ptr() + off, bw.device_ptr(), by.device_ptr(), fmt, M, N, K)
+            import torch
+            torch.cuda.synchronize()
+            assert "tcgen05" in tc.cuda_last_kernel_name()
+            outs.append(by.to_numpy((M, N), np.float16))
+    assert all(np.array_equal(outs[0], o) for o in outs[1:])
+
+
+def test_non_finite_weights_scales_and_activations(tc, ctx, oracle):
+    """An infinite activation makes the results of its row non-finite, an infinite scale those of its
+    weight row; nothing else changes."""
+    M, N, K = 16, 256, 512
+    X, Wq = data(oracle, 0, M, N, K)
+    with ctx.buffer(M * K * 2) as bx, ctx.buffer(Wq.nbytes) as bw, ctx.buffer(M * N * 2) as by:
+        def call(x, w):
+            bx.upload(x)
+            bw.upload(w)
+            ctx.gemv_quantized(bx, bw, by, 0, M, N, K)
+            return by.to_numpy((M, N), np.float16)
+        base = call(X, Wq)
+        X2 = X.copy()
+        X2[3, 77] = np.inf
+        got = call(X2, Wq)
+        assert not np.isfinite(got[3]).any()
+        keep = np.arange(M) != 3
+        assert np.array_equal(got[keep], base[keep])
+        W2 = Wq.copy().reshape(N, K // 32, 18)
+        W2[5, 2, :2] = np.array([np.inf], np.float16).view(np.uint8)
+        got = call(X, W2.reshape(Wq.shape))
+        assert not np.isfinite(got[:, 5]).any()
+        keep = np.arange(N) != 5
+        assert np.array_equal(got[:, keep], base[:, keep])
