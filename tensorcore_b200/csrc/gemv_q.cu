@@ -620,7 +620,7 @@ cudaError_t launch_gemv_q(const GemvQArgs& a, const LaunchEnv& env, cudaStream_t
             s.Y = static_cast<uint8_t*>(a.Y) + static_cast<size_t>(m0) * a.N * ysz;
             if (fuse) {
                 float* rstd = reinterpret_cast<float*>(static_cast<uint8_t*>(a.norm_scratch) + slab * static_cast<size_t>(a.K) * 2);
-                err = launch_norm_forward(s.X, a.gamma, nullptr, a.norm_scratch, nullptr, rstd, s.M, a.K, a.eps, stream);
+                err = launch_norm_forward(s.X, a.gamma, nullptr, a.norm_scratch, nullptr, rstd, s.M, a.K, a.eps, stream, env.pdl);
                 ++count;
             } else if (copy) {
                 err = cudaMemcpyAsync(a.norm_scratch, s.X, static_cast<size_t>(s.M) * a.K * 2, cudaMemcpyDeviceToDevice, stream);

@@ -232,7 +232,8 @@ cudaError_t launch_gemv_q4_decode_static(const GemvQArgs* ops, int n_ops, const 
 // --- the small operations between the GEMVs of a decode step (step_ops.cu); fp16 data --------
 cudaError_t launch_norm_forward(const void* X, const void* gamma, const void* beta /* null = RMSNorm */,
                                 void* Y, float* mean_out /* may be null */, float* rstd_out, int N, int D,
-                                float eps, cudaStream_t stream);
+                                float eps, cudaStream_t stream,
+                                bool pdl = false /* may start while the kernel before it runs */);
 cudaError_t launch_swiglu(const void* gate, const void* up, void* out, int n, cudaStream_t stream);
 cudaError_t launch_rope(void* X, const float* cos_t, const float* sin_t, int batch, int heads, int seq,
                         int head_dim, cudaStream_t stream);

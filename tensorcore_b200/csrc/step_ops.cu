@@ -60,6 +60,84 @@ __global__ void __launch_bounds__(256) norm_forward_kernel(const __half* X, cons
     }
 }
 
+// The same for rows of a multiple of 8 elements at 16-byte aligned addresses: the row stays in registers
+// (V 16-byte vectors per thread), so it is read once, with every load in flight at a time.  What bounds a
+// call is latency - one round trip, two block sums, one store - not bytes.  In front of the batched
+// quantized GEMV (512 rows of 4096) the pass and its launch took 10.8 us as the scalar kernel above.
+template <int V>
+__global__ void __launch_bounds__(256) norm_forward_vec_kernel(const uint4* X, const uint4* gamma, const uint4* beta, uint4* Y,
+                                                               float* mean_out, float* rstd_out, int D, float eps) {
+    __shared__ double scratch[8];
+    // The next kernel's prologue may start; then wait for the one before (launched with programmatic
+    // serialization when it is part of a chain, else this returns at once).
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int tid = threadIdx.x, vecs = D >> 3;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const uint4* xr = X + static_cast<size_t>(blockIdx.x) * vecs;
+    uint4* yr = Y + static_cast<size_t>(blockIdx.x) * vecs;
+    uint4 x[V], g[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        const int c = tid + 256 * i;
+        x[i] = g[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (c < vecs) { x[i] = xr[c]; g[i] = gamma[c]; }
+    }
+    auto pair = [](const uint4& v, int t) {
+        return __half22float2(reinterpret_cast<const __half2*>(&v)[t]);
+    };
+    float mean = 0.f;
+    if (beta != nullptr) {
+        double s = 0.0;
+#pragma unroll
+        for (int i = 0; i < V; ++i)
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const float2 f = pair(x[i], t);
+                s += static_cast<double>(f.x) + static_cast<double>(f.y);
+            }
+        mean = static_cast<float>(block_sum_d(s, scratch) / D);
+    }
+    double sq = 0.0;
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        if (tid + 256 * i >= vecs) break;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const float2 f = pair(x[i], t);
+            const double a = __fsub_rn(f.x, mean), b = __fsub_rn(f.y, mean);
+            sq += a * a;
+            sq += b * b;
+        }
+    }
+    const float rstd = 1.0f / sqrtf(static_cast<float>(block_sum_d(sq, scratch) / D) + eps);
+    if (tid == 0) {
+        rstd_out[blockIdx.x] = rstd;
+        if (mean_out) mean_out[blockIdx.x] = mean;
+    }
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        const int c = tid + 256 * i;
+        if (c >= vecs) break;
+        uint4 out, b4 = make_uint4(0u, 0u, 0u, 0u);
+        if (beta != nullptr) b4 = beta[c];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const float2 xv = pair(x[i], t), gv = pair(g[i], t);
+            float2 y;
+            if (beta != nullptr) {
+                const float2 bv = pair(b4, t);
+                y.x = __fadd_rn(__fmul_rn(__fmul_rn(__fsub_rn(xv.x, mean), rstd), gv.x), bv.x);
+                y.y = __fadd_rn(__fmul_rn(__fmul_rn(__fsub_rn(xv.y, mean), rstd), gv.y), bv.y);
+            } else {
+                y.x = __fmul_rn(__fmul_rn(xv.x, rstd), gv.x);
+                y.y = __fmul_rn(__fmul_rn(xv.y, rstd), gv.y);
+            }
+            reinterpret_cast<__half2*>(&out)[t] = __floats2half2_rn(y.x, y.y);
+        }
+        yr[c] = out;
+    }
+}
+
 // out = silu(gate) * up, silu(x) = x / (1 + exp(-x)) with the reference's tail clamps.
 __global__ void swiglu_kernel(const __half* gate, const __half* up, __half* out, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -106,11 +184,29 @@ __global__ void __launch_bounds__(128) gemm_f16_rows_kernel(const __half* A, con
 }  // namespace
 
 cudaError_t launch_norm_forward(const void* X, const void* gamma, const void* beta, void* Y, float* mean_out,
-                                float* rstd_out, int N, int D, float eps, cudaStream_t stream) {
-    norm_forward_kernel<<<N, 256, 0, stream>>>(static_cast<const __half*>(X), static_cast<const __half*>(gamma),
-                                               static_cast<const __half*>(beta), static_cast<__half*>(Y), mean_out,
-                                               rstd_out, D, eps);
-    return cudaGetLastError();
+                                float* rstd_out, int N, int D, float eps, cudaStream_t stream, bool pdl) {
+    const uintptr_t all = reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(gamma) |
+                          reinterpret_cast<uintptr_t>(beta) | reinterpret_cast<uintptr_t>(Y);
+    if (D % 8 != 0 || (all & 15u) != 0 || D > 8 * 256 * 8) {
+        norm_forward_kernel<<<N, 256, 0, stream>>>(static_cast<const __half*>(X), static_cast<const __half*>(gamma),
+                                                   static_cast<const __half*>(beta), static_cast<__half*>(Y),
+                                                   mean_out, rstd_out, D, eps);
+        return cudaGetLastError();
+    }
+    const int v = (D / 8 + 255) / 256;
+    auto* kernel = v <= 1 ? norm_forward_vec_kernel<1> : v <= 2 ? norm_forward_vec_kernel<2> : v <= 4 ? norm_forward_vec_kernel<4>
+                                                                                                  : norm_forward_vec_kernel<8>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(N));
+    cfg.blockDim = dim3(256);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<const uint4*>(X), static_cast<const uint4*>(gamma),
+                              static_cast<const uint4*>(beta), static_cast<uint4*>(Y), mean_out, rstd_out, D, eps);
 }
 
 cudaError_t launch_swiglu(const void* gate, const void* up, void* out, int n, cudaStream_t stream) {
