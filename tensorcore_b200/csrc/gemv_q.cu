@@ -33,6 +33,8 @@
 namespace tcb {
 cudaError_t init_gemm_q_tc_kernels(int smem_optin);
 cudaError_t launch_gemm_q_tc(const GemvQArgs& a, const LaunchEnv& env, cudaStream_t stream);
+cudaError_t init_gemv_q_rows_kernels(int smem_optin);
+cudaError_t launch_gemv_q_rows(const GemvQArgs& a, const LaunchEnv& env, cudaStream_t stream);
 cudaError_t init_decode_kernel(int smem_optin);
 namespace {
 
@@ -575,6 +577,7 @@ cudaError_t set_smem(K kernel, int bytes) {
 cudaError_t init_gemv_kernels(int smem_optin) {
     cudaError_t e = init_gemm_q_tc_kernels(smem_optin);
     if (e == cudaSuccess) e = init_gemm_tc_kernel(smem_optin);
+    if (e == cudaSuccess) e = init_gemv_q_rows_kernels(smem_optin);
     if (e != cudaSuccess) return e;
     e = init_decode_kernel(smem_optin);
     if (e != cudaSuccess) return e;
@@ -669,8 +672,9 @@ cudaError_t launch_gemv_q(const GemvQArgs& a, const LaunchEnv& env, cudaStream_t
     }
 
     // Up to kMaxMB activation rows per pass on the integer dot-product kernels.
-    for (int m0 = 0; m0 < a.M && err == cudaSuccess; m0 += kMaxMB) {
-        const int mb = (a.M - m0) < kMaxMB ? (a.M - m0) : kMaxMB;
+    int mb = 0;
+    for (int m0 = 0; m0 < a.M && err == cudaSuccess; m0 += mb) {
+        mb = (a.M - m0) < kMaxMB ? (a.M - m0) : kMaxMB;
         GemvQArgs s = a;
         s.X = static_cast<const uint8_t*>(a.X) + static_cast<size_t>(m0) * a.K * xsz;
         s.Y = static_cast<uint8_t*>(a.Y) + static_cast<size_t>(m0) * a.N * ysz;
@@ -696,6 +700,21 @@ cudaError_t launch_gemv_q(const GemvQArgs& a, const LaunchEnv& env, cudaStream_t
                                     : launch_stream_mb<FMT_Q8_0>(mb, pl, stream, env.pdl);
             used = a.fmt == FMT_Q4_0 ? "q4_0_gemv_stream_sm100" : "q8_0_gemv_stream_sm100";
         } else {
+            // Rows no tiled or bulk copy can describe: a lane per block, as many rows as fit shared memory;
+            // weights at an odd address or very long rows take the byte-wise kernel.
+            cudaError_t re = cudaErrorNotSupported;
+            for (;; mb = (mb + 1) / 2) {
+                s.M = mb;
+                re = launch_gemv_q_rows(s, env, stream);
+                if (re != cudaErrorNotSupported || mb == 1) break;
+            }
+            if (re != cudaErrorNotSupported) {
+                err = re;
+                used = a.fmt == FMT_Q4_0 ? "q4_0_gemv_generic_rows_sm100" : "q8_0_gemv_generic_rows_sm100";
+                ++count;
+                continue;
+            }
+            (void)cudaGetLastError();
             GenericParams g;
             g.W = s.W; g.X = s.X; g.Y = s.Y; g.gamma = s.gamma;
             g.M = mb; g.N = s.N; g.K = s.K; g.nb = s.K / 32;

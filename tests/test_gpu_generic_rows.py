@@ -1,0 +1,48 @@
+"""GPU: the kernel for quantized rows that no tiled copy can describe (K not a multiple of 256, weights at
+any even address), at the edges of its blocks-per-lane and rows-per-warp split.
+
+fp32 activations and results stay fp32 arithmetic: a sum of K products in fp32 differs from the 64-bit one
+by about sqrt(K) * 2^-24 relative to its terms, below 2e-6 scaled RMS for K up to 9000."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("fmt", [0, 1])
+@pytest.mark.parametrize("M,N,K", [(1, 1, 32), (2, 3, 96), (3, 5, 1056), (4, 37, 992), (1, 601, 4128), (3, 1187, 2080),
+                                   (4, 150, 8352), (6, 40, 544), (4, 20, 20512)])
+def test_fp32_rows_against_64_bit(tc, ctx, oracle, fmt, M, N, K):
+    rng = np.random.default_rng(M * 31 + N * 7 + K + fmt)
+    Wq = oracle.quantize_weights((rng.standard_normal((N, K)) * 0.02).astype(np.float16), fmt)
+    X = rng.standard_normal((M, K)).astype(np.float32)
+    g = (1 + 0.1 * rng.standard_normal(K)).astype(np.float32)
+    want = oracle.dequant_dot_f64(X.astype(np.float64), Wq, fmt, N)
+    x64 = X.astype(np.float64)
+    xn = x64 / np.sqrt((x64 * x64).mean(axis=1, keepdims=True) + 1e-5) * g
+    wantf = oracle.dequant_dot_f64(xn, Wq, fmt, N)
+    with ctx.buffer_from_array(X) as bx, ctx.buffer_from_array(Wq) as bw, ctx.buffer_from_array(g) as bg, \
+            ctx.buffer(M * N * 4) as by:
+        tc.gemv_quantized_ex(ctx, bx, bw, by, fmt, M, N, K, "f32", "f32", None)
+        assert "generic" in tc.cuda_last_kernel_name()
+        assert oracle.scaled_rms(by.to_numpy((M, N), np.float32).astype(np.float64), want) <= 2e-6
+        tc.fused_rmsnorm_gemv_quantized_ex(ctx, bx, bg, bw, by, fmt, M, N, K, 1e-5, "f32", "f32", None)
+        assert oracle.scaled_rms(by.to_numpy((M, N), np.float32).astype(np.float64), wantf) <= 2e-6
+
+
+@pytest.mark.parametrize("fmt", [0, 1])
+@pytest.mark.parametrize("w_off,x_off", [(2, 0), (4, 2), (6, 6), (8, 10), (1, 0), (14, 14)])
+def test_any_weight_and_activation_address(tc, ctx, oracle, fmt, w_off, x_off):
+    """Same bits wherever the operands lie, up to fp32 summation order."""
+    import torch
+    M, N, K = 3, 70, 1120
+    rng = np.random.default_rng(w_off + 100 * x_off + fmt)
+    Wq = oracle.quantize_weights((rng.standard_normal((N, K)) * 0.02).astype(np.float16), fmt)
+    X = rng.standard_normal((M, K)).astype(np.float16)
+    want = oracle.dequant_dot_f64(X.astype(np.float64), Wq, fmt, N)
+    with ctx.buffer(X.nbytes + 16) as bx, ctx.buffer(Wq.nbytes + 16) as bw, ctx.buffer(M * N * 4) as by:
+        bx.upload(X, x_off)
+        bw.upload(Wq, w_off)
+        tc.raw_gemv_quantized(ctx, bx.device_ptr() + x_off, bw.device_ptr() + w_off, by.device_ptr(), fmt, M, N, K, "f16", "f32")
+        torch.cuda.synchronize()
+        assert oracle.scaled_rms(by.to_numpy((M, N), np.float32).astype(np.float64), want) <= 2e-6
