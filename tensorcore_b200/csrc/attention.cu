@@ -1,27 +1,20 @@
-// Scaled-dot-product attention forward for decode: few query rows against a long K/V cache.
+// Scaled-dot-product attention forward.
 //
 // Interface replaced: tc_attention_forward (include/tensorcore/attention.h:24-60; arithmetic of
 // lib/ops/attention_cpu.cpp:131-277): fp16 Q [B,H,Sq,D], K/V [B,Hkv,Sk,D], O [B,H,Sq,D], optional
 // fp32 LSE [B,H,Sq]; softmax in fp32; causal mask (key index > query index), sliding window
 // (query - key > window), ALiBi (score -= slope * (query - key)), grouped-query heads.
 //
-// One query row is a streaming pass over its head's K and V (2 * Sk * D * 2 bytes): HBM-bound.
-//   * The query heads that share a K/V head (grouped-query attention) are handled by ONE CTA, so
-//     the cache is read once per K/V head, not once per query head.
-//   * A row's keys are cut into chunks so that about eight CTAs per SM are in flight (a decode step
-//     has only B * Hkv * Sq groups); every CTA keeps an online-softmax state per query head (running
-//     maximum m, denominator l, unnormalised output o[D]) for its chunk.
-//   * head_dim 128 (attention_decode128_kernel): every load is a coalesced 512-byte piece of the
-//     cache, 16 lanes per key; see the kernel.
-//   * Other head_dims (attention_decode_kernel): a lane takes a key for the scores (D / 8
-//     independent 16-byte loads, the query rows in shared memory), then the lanes switch to a
-//     slice of D each and walk the step's 32 value rows, eight row loads in flight at a time, the
-//     probabilities broadcast by shuffle.
-// The warps of a CTA are merged through shared memory; with one chunk the CTA writes O (and LSE)
-// itself, otherwise it leaves (m, l, o) in scratch and a second small kernel merges the chunks.
-// head_dim 64 is compiled with fixed trip counts; any other head_dim <= 128 takes a generic
-// instance of the same code.  No tensor cores: with one to a few query rows the work is a
-// matrix-vector product.
+//   * head_dim 64 and 128 at 16-byte aligned addresses: attention_mma_kernel, one kernel for a decode step
+//     and a prefill block, on the tensor cores; see there.
+//   * Other head_dims and addresses: attention_decode_kernel, a streaming pass per query row on the CUDA
+//     cores.  A lane takes a key for the scores (the query rows in shared memory), then the lanes
+//     switch to a slice of D each and walk the step's 32 value rows, eight row loads in flight at a
+//     time, the probabilities broadcast by shuffle; two query heads that share a K/V head go together.
+//   * A row's keys are cut into chunks when there are too few CTAs otherwise.  A CTA keeps an
+//     online-softmax state (running maximum m, denominator l, unnormalised output o[D]) for its chunk;
+//     with one chunk it writes O (and LSE) itself, else it leaves (m, l, o) in scratch and a second
+//     small kernel merges the chunks.
 #include "kernels.h"
 
 #include <cuda_fp16.h>
@@ -46,6 +39,7 @@ struct AttnParams {
     int chunks, keys_per_chunk;
     float scale;
     int causal, window;
+    int vec;              // Q, K and V are 16-byte aligned
 };
 
 __device__ __forceinline__ float warp_max(float v) {
@@ -57,18 +51,17 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
-// DC: head_dim when it is 64 or 128 (fixed trip counts), 0 for the generic instance.  G: query heads
-// per CTA.
-template <int DC, int G>
+// Any head_dim up to 128.  G: query heads per CTA.
+template <int G>
 __global__ void __launch_bounds__(kAttnWarps * 32) attention_decode_kernel(const AttnParams p) {
     // the merge kernel that follows may be set up now; it waits for this grid before it reads anything
     asm volatile("griddepcontrol.launch_dependents;");
-    constexpr int kPer = DC ? DC / 32 : kAttnMaxD / 32;      // output elements per lane
+    constexpr int kPer = kAttnMaxD / 32;                     // output elements per lane
     __shared__ float q_s[G][kAttnMaxD];
     __shared__ float o_s[kAttnWarps][G][kAttnMaxD];
     __shared__ float m_s[kAttnWarps][G], l_s[kAttnWarps][G];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int D = DC ? DC : p.D;
+    const int D = p.D;
     // blockIdx.x = ((b * heads_per_grid) + hg) * Sq + i, where hg counts groups of G query heads
     const int groups = p.Hq / G;
     const int i = blockIdx.x % p.Sq, bg = blockIdx.x / p.Sq, hg = bg % groups, b = bg / groups;
@@ -89,7 +82,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_decode_kernel(const
 
     // this lane's slice of the output: `per` consecutive elements when D is a multiple of 32 (one
     // vector load per value row), else elements lane, lane + 32, ...
-    const int per = (D & 31) == 0 ? D >> 5 : 0;
+    const int per = (D & 31) == 0 && p.vec ? D >> 5 : 0;
     auto elem = [&](int t) { return per ? lane * per + t : lane + 32 * t; };
     float o[G][kPer];
     float m[G], l[G];
@@ -110,24 +103,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_decode_kernel(const
             float acc[G];
 #pragma unroll
             for (int g = 0; g < G; ++g) acc[g] = 0.f;
-            if (DC) {
-                uint4 raw[DC ? DC / 8 : 1];
-#pragma unroll
-                for (int c = 0; c < DC / 8; ++c) raw[c] = __ldg(reinterpret_cast<const uint4*>(kr) + c);   // all in flight
-#pragma unroll
-                for (int c = 0; c < DC / 8; ++c) {
-                    const __half2* h2 = reinterpret_cast<const __half2*>(&raw[c]);
-#pragma unroll
-                    for (int t = 0; t < 4; ++t) {
-                        const float2 f = __half22float2(h2[t]);
-#pragma unroll
-                        for (int g = 0; g < G; ++g) {
-                            acc[g] = fmaf(q_s[g][8 * c + 2 * t], f.x, acc[g]);
-                            acc[g] = fmaf(q_s[g][8 * c + 2 * t + 1], f.y, acc[g]);
-                        }
-                    }
-                }
-            } else {
+            {
                 for (int d = 0; d < D; ++d) {
                     const float kv = __half2float(kr[d]);
 #pragma unroll
@@ -168,12 +144,12 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_decode_kernel(const
             for (int r = 0; r < kRows; ++r) {
                 const int c = c0 + r;
                 const __half* vr = Vh + static_cast<size_t>(j0 + (c < n ? c : n - 1)) * D;
-                if (DC == 128 || (!DC && per == 4)) {
+                if (per == 4) {
                     const uint2 raw = __ldg(reinterpret_cast<const uint2*>(vr + 4 * lane));
                     const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&raw.x));
                     const float2 bq = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
                     v[r][0] = a.x; v[r][1] = a.y; v[r][2] = bq.x; v[r][3] = bq.y;
-                } else if (DC == 64 || (!DC && per == 2)) {
+                } else if (per == 2) {
                     const float2 a = __half22float2(*reinterpret_cast<const __half2*>(vr + 2 * lane));
                     v[r][0] = a.x; v[r][1] = a.y;
                 } else {
@@ -232,184 +208,275 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_decode_kernel(const
     }
 }
 
-// Fast kernel for head_dim 128: every load is a coalesced 512-byte piece of the cache.
+// ---------------------------------------------------------------------------------------
+// Matrix kernel, head_dim 64 and 128: scores and outputs on the tensor cores (mma.sync m16n8k16).
 //
-// K (and V) of a head are contiguous [Sk][128] fp16: 32 keys are 8 KB, which a warp reads with
-// 16 instructions of 32 x 16 bytes.  Instruction c brings keys 2c (lanes 0-15) and 2c + 1 (lanes
-// 16-31); a lane holds eight consecutive elements of its key - always elements 8 * (lane % 16)
-// .. + 7, so its slice of every query row sits in registers.  A key's score is the sum of its 16
-// lanes' partial dot products (four shuffles, after which all 16 lanes know it), so the half-warp
-// that loads value row 2c (+1) already has that key's probability: no broadcast.  A lane
-// accumulates its eight output elements over the keys of its half; the two halves are added at
-// the end.  G query heads that share the K/V head are processed together (G <= 4).
-// The kernel is bound by how many warps an SM keeps in flight (a step is a chain of round trips and
-// shuffles), so the one- and two-head instances are held to 96 / 128 registers for five / four CTAs
-// per SM at the price of a few spilled words (32 heads x 4096 keys: 36.9 -> 30.8 us; batch 8 x 2048
-// keys: 99.5 -> 83.9 us); the four-head instance was slower that way (233 registers, two CTAs).
-template <int G>
-__global__ void __launch_bounds__(kAttnWarps * 32, G == 1 ? 5 : (G == 2 ? 4 : 1)) attention_decode128_kernel(const AttnParams p) {
+// The rows of a tile are the (query, head) pairs that share a K/V head, head fastest: the eight or
+// fewer heads of a grouped-query decode step are one 16-row tile and read the cache once; a prefill
+// block is cut into 64-row tiles.  K and V arrive in steps of 64 keys through a ring in shared memory
+// (cp.async, 16-byte pieces, piece index XORed with the row so that ldmatrix is conflict-free).
+//   SPLIT_KEYS (16 rows or fewer): all four warps hold the same rows and take 16 keys of a step each,
+//     with softmax states of their own that are merged at the end.
+//   else: a warp owns 16 of the 64 rows and takes all 64 keys.
+// The scores' products are exact and summed in fp32.  The probabilities stay fp32: for the product with V
+// each is split into an fp16 value and the fp16 remainder (22 bits of it), which costs a third
+// more MMAs and keeps the result as close to a 64-bit one as fp32 multiply-adds had it.
+// A decode step is bound by the cache stream, a prefill block by the tensor pipe and the chain of a
+// step (scores, maximum, exponentials, outputs); two CTAs per SM overlap their chains.
+// ---------------------------------------------------------------------------------------
+constexpr int kStepKeys = 64;
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldmatrix4_trans(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t pack_h2(float a, float b) {
+    const __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+// What the fp16 pair `h` leaves of (a, b), as fp16.
+__device__ __forceinline__ uint32_t rest_h2(uint32_t h, float a, float b) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
+    return pack_h2(a - f.x, b - f.y);
+}
+
+template <int D> struct MmaShape {
+    static constexpr int kStages = D == 128 ? 3 : 4;
+    static constexpr int kStageBytes = 2 * kStepKeys * D * 2;
+    static constexpr int kSmem = kStages * kStageBytes;
+};
+
+template <int D, bool SPLIT_KEYS>
+__global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const AttnParams p) {
     asm volatile("griddepcontrol.launch_dependents;");
-    constexpr int D = 128;
-    __shared__ float o_s[kAttnWarps][G][D];
-    __shared__ float m_s[kAttnWarps][G], l_s[kAttnWarps][G];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int hl = lane & 15, half = lane >> 4;
-    const int groups = p.Hq / G;
-    const int i = blockIdx.x % p.Sq, bg = blockIdx.x / p.Sq, hg = bg % groups, b = bg / groups;
-    const int h0 = hg * G;
-    const int hkv = h0 / (p.Hq / p.Hkv);
+    using S = MmaShape<D>;
+    constexpr int kTileRows = SPLIT_KEYS ? 16 : 64;
+    constexpr int kKeys = SPLIT_KEYS ? 16 : 64;           // keys of a step this warp takes
+    constexpr int kNT = kKeys / 8, kPieces = D / 8;
+    extern __shared__ __align__(128) uint8_t smem[];
+    const uint32_t ring = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, tq = lane & 3;
+    const int G = p.Hq / p.Hkv, R = p.Sq * G;
+    const int heads = p.B * p.Hkv, bk = blockIdx.x % heads;
+    const int row_tiles = (R + kTileRows - 1) / kTileRows;
+    const int tile0 = (row_tiles - 1 - static_cast<int>(blockIdx.x / heads)) * kTileRows;   // long causal tiles first
+    const int b = bk / p.Hkv, hkv = bk % p.Hkv;
     const int chunk = blockIdx.y;
-    const __half* Kh = p.K + (static_cast<size_t>(b) * p.Hkv + hkv) * p.Sk * D;
-    const __half* Vh = p.V + (static_cast<size_t>(b) * p.Hkv + hkv) * p.Sk * D;
-    float q[G][8], slope[G];
+    const __half* Kh = p.K + static_cast<size_t>(bk) * p.Sk * D;
+    const __half* Vh = p.V + static_cast<size_t>(bk) * p.Sk * D;
+
+    // this thread's two rows, their queries, and the fragments of the query matrix
+    const int r_lo = tile0 + (SPLIT_KEYS ? 0 : warp * 16) + gq;
+    int qi[2];
+    float slope[2];
+    size_t row_at[2];
+    bool live[2];
+    uint32_t qf[D / 16][4];
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(p.Q + ((static_cast<size_t>(b) * p.Hq + h0 + g) * p.Sq + i) * D + 8 * hl);
-        const __half2* h2 = reinterpret_cast<const __half2*>(&raw);
+    for (int e = 0; e < 2; ++e) {
+        const int r = r_lo + 8 * e;
+        live[e] = r < R;
+        const int rr = live[e] ? r : R - 1;
+        qi[e] = rr / G;
+        const int h = hkv * G + (rr - qi[e] * G);
+        row_at[e] = (static_cast<size_t>(b) * p.Hq + h) * p.Sq + qi[e];
+        slope[e] = p.slopes ? p.slopes[h] : 0.f;
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(p.Q + row_at[e] * D) + tq;
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            const float2 f = __half22float2(h2[t]);
-            q[g][2 * t] = f.x * p.scale;         // the scale folded into the query
-            q[g][2 * t + 1] = f.y * p.scale;
+        for (int k = 0; k < D / 16; ++k) {
+            qf[k][e] = src[8 * k];
+            qf[k][2 + e] = src[8 * k + 4];
         }
-        slope[g] = p.slopes ? p.slopes[h0 + g] : 0.f;
     }
-    const int k0 = chunk * p.keys_per_chunk, k1 = min(p.Sk, k0 + p.keys_per_chunk);
-    float o[G][8], m[G], l[G];
+    // keys any row of the tile can see, in whole steps from the chunk's start
+    const int r_last = min(R, tile0 + kTileRows) - 1;
+    const int i_min = tile0 / G, i_max = r_last / G;
+    int k0 = chunk * p.keys_per_chunk, k1 = min(p.Sk, k0 + p.keys_per_chunk);
+    if (p.causal) k1 = min(k1, i_max + 1);
+    if (p.window > 0 && i_min - p.window > k0) k0 += (i_min - p.window - k0) / kStepKeys * kStepKeys;
+    const int steps = k1 > k0 ? (k1 - k0 + kStepKeys - 1) / kStepKeys : 0;
+
+    auto fetch = [&](int st) {
+        if (st < steps) {
+            const int base = k0 + st * kStepKeys;
+            const uint32_t dst = ring + (st % S::kStages) * S::kStageBytes;
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-        m[g] = -INFINITY;
-        l[g] = 0.f;
-#pragma unroll
-        for (int t = 0; t < 8; ++t) o[g][t] = 0.f;
-    }
-    for (int j0 = k0 + warp * 32; j0 < k1; j0 += kAttnWarps * 32) {
-        // scores of the step's 32 keys: s[g][c] belongs to key j0 + 2c + half
-        float s[G][16];
-#pragma unroll
-        for (int hb = 0; hb < 2; ++hb) {          // two batches of eight loads: 32 registers of raw keys
-            uint4 raw[8];
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const int j = j0 + 2 * (8 * hb + c) + half;
-                raw[c] = j < k1 ? __ldg(reinterpret_cast<const uint4*>(Kh + static_cast<size_t>(j) * D) + hl)
-                                : make_uint4(0u, 0u, 0u, 0u);
-            }
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const __half2* h2 = reinterpret_cast<const __half2*>(&raw[c]);
-                float kf[8];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    const float2 f = __half22float2(h2[t]);
-                    kf[2 * t] = f.x; kf[2 * t + 1] = f.y;
-                }
-#pragma unroll
-                for (int g = 0; g < G; ++g) {
-                    float acc = 0.f;
-#pragma unroll
-                    for (int t = 0; t < 8; ++t) acc = fmaf(q[g][t], kf[t], acc);
-                    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-                    acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-                    acc += __shfl_xor_sync(0xffffffffu, acc, 4);
-                    acc += __shfl_xor_sync(0xffffffffu, acc, 8);
-                    const int j = j0 + 2 * (8 * hb + c) + half;
-                    float sc = acc;
-                    if (j >= k1) sc = -INFINITY;
-                    if (p.causal && j > i) sc = -INFINITY;
-                    if (p.window > 0 && i - j > p.window) sc = -INFINITY;
-                    if (p.slopes) sc -= slope[g] * static_cast<float>(i - j);
-                    s[g][8 * hb + c] = sc;
-                }
+            for (int u = 0; u < kStepKeys * kPieces / (kAttnWarps * 32); ++u) {
+                const int e = tid + u * kAttnWarps * 32, key = e / kPieces, piece = e % kPieces;
+                const bool in = base + key < k1;
+                const size_t at = static_cast<size_t>(in ? base + key : k0) * D + piece * 8;
+                const uint32_t off = static_cast<uint32_t>(key * D * 2 + ((piece ^ (key & 7)) * 16));
+                cp_async16(dst + off, Kh + at, in);
+                cp_async16(dst + kStepKeys * D * 2 + off, Vh + at, in);
             }
         }
-        bool any = false;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
 #pragma unroll
-        for (int g = 0; g < G; ++g) {
-            float mx = s[g][0];
+    for (int st = 0; st < S::kStages - 1; ++st) fetch(st);
+
+    float o[D / 8][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
 #pragma unroll
-            for (int c = 1; c < 16; ++c) mx = fmaxf(mx, s[g][c]);
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));       // the other half's keys
-            const float m_new = fmaxf(m[g], mx);
-            if (m_new > -INFINITY) {
-                const float keep = m[g] > -INFINITY ? __expf(m[g] - m_new) : 0.f;
-                float sum = 0.f;
+    for (int n = 0; n < D / 8; ++n)
 #pragma unroll
-                for (int c = 0; c < 16; ++c) {
-                    s[g][c] = s[g][c] > -INFINITY ? __expf(s[g][c] - m_new) : 0.f;    // now the probability
-                    sum += s[g][c];
+        for (int e = 0; e < 4; ++e) o[n][e] = 0.f;
+    const int mi = lane >> 3, ml = lane & 7;               // ldmatrix: which 8x8 matrix, which of its rows
+
+    for (int st = 0; st < steps; ++st) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(S::kStages - 2) : "memory");
+        __syncthreads();                                   // the step has landed; everyone is done with the one before
+        fetch(st + S::kStages - 1);
+        const uint32_t ks = ring + (st % S::kStages) * S::kStageBytes, vs = ks + kStepKeys * D * 2;
+        const int kw = SPLIT_KEYS ? warp * 16 : 0, jb = k0 + st * kStepKeys + kw;   // this warp's first key
+
+        float s[kNT][4];
+#pragma unroll
+        for (int n = 0; n < kNT; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[n][e] = 0.f;
+#pragma unroll
+        for (int k = 0; k < D / 16; ++k)
+#pragma unroll
+            for (int n = 0; n < kNT; n += 2) {
+                const int key = kw + n * 8 + (mi >> 1) * 8 + ml, piece = 2 * k + (mi & 1);
+                uint32_t bf[4];
+                ldmatrix4(bf, ks + static_cast<uint32_t>(key * D * 2 + ((piece ^ ml) * 16)));
+                mma_16816(s[n], qf[k], bf[0], bf[1]);
+                mma_16816(s[n + 1], qf[k], bf[2], bf[3]);
+            }
+        const bool masked = jb + kKeys > k1 || (p.causal && jb + kKeys - 1 > i_min) || p.window > 0 || p.slopes != nullptr;
+        float mx[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+        for (int n = 0; n < kNT; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                float sc = s[n][e] * p.scale;
+                if (masked) {
+                    const int j = jb + n * 8 + 2 * tq + (e & 1), i = qi[e >> 1];
+                    if (j >= k1 || (p.causal && j > i) || (p.window > 0 && i - j > p.window)) sc = -INFINITY;
+                    if (p.slopes) sc -= slope[e >> 1] * static_cast<float>(i - j);
                 }
-                sum += __shfl_xor_sync(0xffffffffu, sum, 16);
-                l[g] = l[g] * keep + sum;
+                s[n][e] = sc;
+                mx[e >> 1] = fmaxf(mx[e >> 1], sc);
+            }
+        float ref[2];
 #pragma unroll
-                for (int t = 0; t < 8; ++t) o[g][t] *= keep;
-                m[g] = m_new;
-                any = true;
+        for (int e = 0; e < 2; ++e) {
+            mx[e] = fmaxf(mx[e], __shfl_xor_sync(0xffffffffu, mx[e], 1));
+            mx[e] = fmaxf(mx[e], __shfl_xor_sync(0xffffffffu, mx[e], 2));
+            const float m_new = fmaxf(m[e], mx[e]);
+            ref[e] = m_new > -INFINITY ? m_new : 0.f;      // a row that sees no key so far keeps zero sums
+            const float keep = m[e] > -INFINITY ? __expf(m[e] - ref[e]) : 0.f;
+            m[e] = m_new;
+            l[e] *= keep;
+#pragma unroll
+            for (int n = 0; n < D / 8; ++n) { o[n][2 * e] *= keep; o[n][2 * e + 1] *= keep; }
+        }
+#pragma unroll
+        for (int n = 0; n < kNT; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                s[n][e] = s[n][e] > -INFINITY ? __expf(s[n][e] - ref[e >> 1]) : 0.f;     // now the probability
+                l[e >> 1] += s[n][e];
+            }
+#pragma unroll
+        for (int k = 0; k < kKeys / 16; ++k) {
+            uint32_t hi[4], lo[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {                  // (rows lo, hi) x (keys 0-7, 8-15)
+                const float a = s[2 * k + (q >> 1)][2 * (q & 1)], c = s[2 * k + (q >> 1)][2 * (q & 1) + 1];
+                hi[q] = pack_h2(a, c);
+                lo[q] = rest_h2(hi[q], a, c);
+            }
+#pragma unroll
+            for (int n = 0; n < D / 8; n += 2) {
+                const int key = kw + k * 16 + (mi & 1) * 8 + ml, piece = n + (mi >> 1);
+                uint32_t bf[4];
+                ldmatrix4_trans(bf, vs + static_cast<uint32_t>(key * D * 2 + ((piece ^ ml) * 16)));
+                mma_16816(o[n], hi, bf[0], bf[1]);
+                mma_16816(o[n + 1], hi, bf[2], bf[3]);
+                mma_16816(o[n], lo, bf[0], bf[1]);
+                mma_16816(o[n + 1], lo, bf[2], bf[3]);
+            }
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        l[e] += __shfl_xor_sync(0xffffffffu, l[e], 1);
+        l[e] += __shfl_xor_sync(0xffffffffu, l[e], 2);
+    }
+
+    if constexpr (!SPLIT_KEYS) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            if (!live[e]) continue;
+            if (p.chunks == 1) {
+                const float inv = l[e] != 0.f ? 1.0f / l[e] : 0.f;
+                uint32_t* dst = reinterpret_cast<uint32_t*>(p.O + row_at[e] * D) + tq;
+#pragma unroll
+                for (int n = 0; n < D / 8; ++n) dst[4 * n] = pack_h2(o[n][2 * e] * inv, o[n][2 * e + 1] * inv);
+                if (tq == 0 && p.LSE) p.LSE[row_at[e]] = m[e] + logf(fmaxf(l[e], 1e-30f));
             } else {
+                float* dst = p.part + (row_at[e] * p.chunks + chunk) * (D + 2);
 #pragma unroll
-                for (int c = 0; c < 16; ++c) s[g][c] = 0.f;
+                for (int n = 0; n < D / 8; ++n)
+                    *reinterpret_cast<float2*>(dst + 2 + 8 * n + 2 * tq) = make_float2(o[n][2 * e], o[n][2 * e + 1]);
+                if (tq == 0) { dst[0] = m[e]; dst[1] = l[e]; }
             }
         }
-        if (!any) continue;                                   // warp-uniform
+    } else {
+        // merge the warps' states through the ring, which everybody has finished reading
+        float* o_s = reinterpret_cast<float*>(smem);                     // [warp][16][D]
+        float* ml_s = o_s + kAttnWarps * 16 * D;                         // [warp][16][2]
+        __syncthreads();
 #pragma unroll
-        for (int hb = 0; hb < 2; ++hb) {
-            uint4 raw[8];
+        for (int e = 0; e < 2; ++e) {
+            const int r = gq + 8 * e;
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const int j = j0 + 2 * (8 * hb + c) + half;
-                raw[c] = j < k1 ? __ldg(reinterpret_cast<const uint4*>(Vh + static_cast<size_t>(j) * D) + hl)
-                                : make_uint4(0u, 0u, 0u, 0u);
-            }
+            for (int n = 0; n < D / 8; ++n)
+                *reinterpret_cast<float2*>(o_s + (warp * 16 + r) * D + 8 * n + 2 * tq) = make_float2(o[n][2 * e], o[n][2 * e + 1]);
+            if (tq == 0) { ml_s[(warp * 16 + r) * 2] = m[e]; ml_s[(warp * 16 + r) * 2 + 1] = l[e]; }
+        }
+        __syncthreads();
+        const int rows = min(16, R - tile0);
+        for (int t = tid; t < rows * D; t += kAttnWarps * 32) {
+            const int r = t / D, d = t - r * D;
+            float mm = -INFINITY;
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const __half2* h2 = reinterpret_cast<const __half2*>(&raw[c]);
-                float vf[8];
+            for (int w = 0; w < kAttnWarps; ++w) mm = fmaxf(mm, ml_s[(w * 16 + r) * 2]);
+            float ll = 0.f, acc = 0.f;
 #pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    const float2 f = __half22float2(h2[t]);
-                    vf[2 * t] = f.x; vf[2 * t + 1] = f.y;
+            for (int w = 0; w < kAttnWarps; ++w) {
+                const float mw = ml_s[(w * 16 + r) * 2];
+                if (mw > -INFINITY) {
+                    const float f = __expf(mw - mm);
+                    ll += ml_s[(w * 16 + r) * 2 + 1] * f;
+                    acc += o_s[(w * 16 + r) * D + d] * f;
                 }
-#pragma unroll
-                for (int g = 0; g < G; ++g) {
-                    const float pc = s[g][8 * hb + c];
-#pragma unroll
-                    for (int t = 0; t < 8; ++t) o[g][t] = fmaf(pc, vf[t], o[g][t]);
-                }
             }
-        }
-    }
-    // the two halves of the warp hold the same output slice over different keys
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-#pragma unroll
-        for (int t = 0; t < 8; ++t) o[g][t] += __shfl_xor_sync(0xffffffffu, o[g][t], 16);
-        if (lane == 0) { m_s[warp][g] = m[g]; l_s[warp][g] = l[g]; }
-        if (half == 0) {
-#pragma unroll
-            for (int t = 0; t < 8; ++t) o_s[warp][g][8 * hl + t] = o[g][t];
-        }
-    }
-    __syncthreads();
-    for (int t = tid; t < G * D; t += blockDim.x) {
-        const int g = t / D, d = t - g * D;
-        float mm = -INFINITY;
-        for (int w = 0; w < kAttnWarps; ++w) mm = fmaxf(mm, m_s[w][g]);
-        float ll = 0.f, acc = 0.f;
-        for (int w = 0; w < kAttnWarps; ++w) {
-            if (m_s[w][g] > -INFINITY) {
-                const float e = __expf(m_s[w][g] - mm);
-                ll += l_s[w][g] * e;
-                acc += o_s[w][g][d] * e;
+            const int i = (tile0 + r) / G, h = hkv * G + (tile0 + r) % G;
+            const size_t row = (static_cast<size_t>(b) * p.Hq + h) * p.Sq + i;
+            if (p.chunks == 1) {
+                p.O[row * D + d] = __float2half_rn(ll != 0.f ? acc / ll : 0.f);
+                if (d == 0 && p.LSE) p.LSE[row] = mm + logf(fmaxf(ll, 1e-30f));
+            } else {
+                float* dst = p.part + (row * p.chunks + chunk) * (D + 2);
+                dst[2 + d] = acc;
+                if (d == 0) { dst[0] = mm; dst[1] = ll; }
             }
-        }
-        const size_t row = (static_cast<size_t>(b) * p.Hq + h0 + g) * p.Sq + i;
-        if (p.chunks == 1) {
-            p.O[row * D + d] = __float2half_rn(ll != 0.f ? acc / ll : 0.f);
-            if (d == 0 && p.LSE) p.LSE[row] = mm + logf(fmaxf(ll, 1e-30f));
-        } else {
-            float* dst = p.part + (row * p.chunks + chunk) * (D + 2);
-            dst[2 + d] = acc;
-            if (d == 0) { dst[0] = mm; dst[1] = ll; }
         }
     }
 }
@@ -451,38 +518,82 @@ __global__ void __launch_bounds__(128) attention_merge_kernel(const AttnParams p
     if (tid == 0 && p.LSE) p.LSE[row] = mm + logf(fmaxf(ll, 1e-30f));
 }
 
-template <int DC>
-cudaError_t launch_group(int group, dim3 grid, cudaStream_t stream, const AttnParams& p) {
-    switch (group) {
-        case 1: attention_decode_kernel<DC, 1><<<grid, kAttnWarps * 32, 0, stream>>>(p); break;
-        case 2: attention_decode_kernel<DC, 2><<<grid, kAttnWarps * 32, 0, stream>>>(p); break;
-        case 4: attention_decode_kernel<DC, 4><<<grid, kAttnWarps * 32, 0, stream>>>(p); break;
-        default: return cudaErrorNotSupported;
-    }
-    return cudaGetLastError();
-}
-
-// Query heads one CTA takes together: two of those that share a K/V head (the other pairs of the same
-// K/V head run in other CTAs and find the cache in L2).  Four at a time was measured slower (64 heads on
-// 8 K/V heads x 8192 keys: 47.3 against 41.3 us): the four-head instance needs 233 registers, two CTAs
-// per SM; one at a time re-reads the cache eight times (73.5 us).
+// Query heads one CTA of the vector kernel takes together: two of those that share a K/V head (the
+// other pairs of the same K/V head run in other CTAs and find the cache in L2).
 int attention_group(int Hq, int Hkv) {
     const int per = Hq / Hkv;
     return per % 2 == 0 ? 2 : 1;
 }
 
+bool matrix_head_dim(int D) { return D == 64 || D == 128; }
+
+// How a row's keys are cut: chunks of keys_per_chunk keys.
+void attention_chunks(int B, int Hq, int Hkv, int Sq, int Sk, int D, int sm_count, int* chunks, int* keys_per_chunk) {
+    const int sms = sm_count > 0 ? sm_count : 148;
+    if (!matrix_head_dim(D)) {
+        // Enough CTAs for eight per SM, chunks of at least 128 keys (one step of 32 keys per warp): a
+        // step is a few dependent round trips to memory, so the bandwidth comes from many warps in
+        // flight, not from long chunks.
+        const long long ctas = static_cast<long long>(B) * (Hq / attention_group(Hq, Hkv)) * Sq;
+        int c = static_cast<int>((8LL * sms + ctas - 1) / ctas);
+        const int most = (Sk + 127) / 128;
+        if (c > most) c = most;
+        if (c > kMergeMaxChunks) c = kMergeMaxChunks;
+        if (c < 1) c = 1;
+        *chunks = c;
+        *keys_per_chunk = (Sk + c - 1) / c;
+        return;
+    }
+    // Matrix kernel: the number of chunks whose waves of CTAs (two per SM) take the fewest steps of 64 keys,
+    // a CTA's start and end counted as two steps and the merge launch as three.
+    const long long R = static_cast<long long>(Sq) * (Hq / Hkv);
+    const long long tiles = R <= 16 ? 1 : (R + 63) / 64;
+    const long long ctas = static_cast<long long>(B) * Hkv * tiles, slots = 2LL * sms;
+    const int steps = (Sk + kStepKeys - 1) / kStepKeys;
+    int best = 1;
+    double best_cost = 0.0;
+    for (int c = 1; c <= steps && c <= kMergeMaxChunks; ++c) {
+        const int per = (steps + c - 1) / c;
+        const double cost = static_cast<double>((ctas * c + slots - 1) / slots) * (per + 2.0) + (c > 1 ? 3.0 + 0.05 * c : 0.0);
+        if (c == 1 || cost < best_cost) { best = c; best_cost = cost; }
+    }
+    const int per = (steps + best - 1) / best;
+    *keys_per_chunk = per * kStepKeys;
+    *chunks = (steps + per - 1) / per;
+}
+
+template <int D>
+cudaError_t launch_matrix(const AttnParams& p, cudaStream_t stream) {
+    const long long R = static_cast<long long>(p.Sq) * (p.Hq / p.Hkv);
+    const bool split = R <= 16;
+    const long long x = static_cast<long long>(p.B) * p.Hkv * (split ? 1 : (R + 63) / 64);
+    if (R > 0x7fffffffLL || x > 0x7fffffffLL) return cudaErrorNotSupported;
+    const dim3 grid(static_cast<unsigned>(x), static_cast<unsigned>(p.chunks));
+    auto* kernel = split ? attention_mma_kernel<D, true> : attention_mma_kernel<D, false>;
+    kernel<<<grid, kAttnWarps * 32, MmaShape<D>::kSmem, stream>>>(p);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_vector(dim3 grid, cudaStream_t stream, const AttnParams& p) {
+    if (p.group == 2) attention_decode_kernel<2><<<grid, kAttnWarps * 32, 0, stream>>>(p);
+    else attention_decode_kernel<1><<<grid, kAttnWarps * 32, 0, stream>>>(p);
+    return cudaGetLastError();
+}
+
 }  // namespace
 
+cudaError_t init_attention_kernels() {
+    const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(attention_mma_kernel<128, true>, a, MmaShape<128>::kSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_mma_kernel<128, false>, a, MmaShape<128>::kSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_mma_kernel<64, true>, a, MmaShape<64>::kSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_mma_kernel<64, false>, a, MmaShape<64>::kSmem);
+    return e;
+}
+
 size_t attention_scratch_floats(int B, int Hq, int Hkv, int Sq, int Sk, int D, int sm_count, int* chunks_out) {
-    // Enough CTAs for eight per SM, chunks of at least 128 keys (one step of 32 keys per warp): a
-    // step is a few dependent round trips to memory, so the bandwidth comes from many warps in
-    // flight, not from long chunks.
-    const long long ctas = static_cast<long long>(B) * (Hq / attention_group(Hq, Hkv)) * Sq;
-    int chunks = static_cast<int>((8LL * sm_count + ctas - 1) / ctas);
-    const int most = (Sk + 127) / 128;
-    if (chunks > most) chunks = most;
-    if (chunks < 1) chunks = 1;
-    if (chunks > kMergeMaxChunks) chunks = kMergeMaxChunks;
+    int chunks = 1, per = Sk;
+    attention_chunks(B, Hq, Hkv, Sq, Sk, D, sm_count, &chunks, &per);
     if (chunks_out) *chunks_out = chunks;
     const size_t rows = static_cast<size_t>(B) * Hq * Sq;
     return chunks > 1 ? rows * chunks * (D + 2) : 0;
@@ -501,28 +612,19 @@ cudaError_t launch_attention_forward(const void* Q, const void* K, const void* V
     p.O = static_cast<__half*>(O); p.LSE = LSE; p.part = scratch; p.slopes = slopes_dev;
     p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.Sq = Sq; p.Sk = Sk; p.D = D;
     p.group = attention_group(Hq, Hkv);
-    int chunks = 1;
-    (void)attention_scratch_floats(B, Hq, Hkv, Sq, Sk, D, sm_count, &chunks);
-    if (chunks > 1 && !scratch) chunks = 1;
-    p.chunks = chunks;
-    p.keys_per_chunk = (Sk + chunks - 1) / chunks;
+    attention_chunks(B, Hq, Hkv, Sq, Sk, D, sm_count, &p.chunks, &p.keys_per_chunk);
+    if (p.chunks > 1 && !scratch) { p.chunks = 1; p.keys_per_chunk = Sk; }
     p.scale = scale; p.causal = causal ? 1 : 0; p.window = window;
-    const dim3 grid(static_cast<unsigned>(rows / p.group), static_cast<unsigned>(chunks));
-    cudaError_t e;
-    const bool aligned = ((reinterpret_cast<uintptr_t>(Q) | reinterpret_cast<uintptr_t>(K) | reinterpret_cast<uintptr_t>(V)) & 15u) == 0;
-    if (D == 128 && aligned) {
-        switch (p.group) {
-            case 4: attention_decode128_kernel<4><<<grid, kAttnWarps * 32, 0, stream>>>(p); break;
-            case 2: attention_decode128_kernel<2><<<grid, kAttnWarps * 32, 0, stream>>>(p); break;
-            default: attention_decode128_kernel<1><<<grid, kAttnWarps * 32, 0, stream>>>(p); break;
-        }
-        e = cudaGetLastError();
-    } else {
-        e = D == 64 ? launch_group<64>(p.group, grid, stream, p) : launch_group<0>(p.group, grid, stream, p);
-    }
+    const uintptr_t at = reinterpret_cast<uintptr_t>(Q) | reinterpret_cast<uintptr_t>(K) | reinterpret_cast<uintptr_t>(V);
+    p.vec = (at & 15u) == 0;
+    cudaError_t e = cudaErrorNotSupported;
+    if (matrix_head_dim(D) && p.vec && (reinterpret_cast<uintptr_t>(O) & 3u) == 0)
+        e = D == 128 ? launch_matrix<128>(p, stream) : launch_matrix<64>(p, stream);
+    if (e == cudaErrorNotSupported)
+        e = launch_vector(dim3(static_cast<unsigned>(rows / p.group), static_cast<unsigned>(p.chunks)), stream, p);
     if (e != cudaSuccess) return e;
     if (launches) *launches += 1;
-    if (chunks > 1) {
+    if (p.chunks > 1) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(static_cast<unsigned>(rows));
         cfg.blockDim = dim3(128);

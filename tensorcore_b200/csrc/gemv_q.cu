@@ -578,6 +578,7 @@ cudaError_t init_gemv_kernels(int smem_optin) {
     cudaError_t e = init_gemm_q_tc_kernels(smem_optin);
     if (e == cudaSuccess) e = init_gemm_tc_kernel(smem_optin);
     if (e == cudaSuccess) e = init_gemv_q_rows_kernels(smem_optin);
+    if (e == cudaSuccess) e = init_attention_kernels();
     if (e != cudaSuccess) return e;
     e = init_decode_kernel(smem_optin);
     if (e != cudaSuccess) return e;

@@ -249,7 +249,8 @@ cudaError_t launch_gemm_f16_tc(const void* A, const void* B, void* C, int M, int
                                bool transpose_b, float alpha, float beta, const LaunchEnv& env, cudaStream_t stream,
                                bool bf16 = false, bool transpose_a = false);
 
-// --- attention forward for decode (attention.cu); fp16 data, fp32 softmax ----------------------------
+// --- attention forward (attention.cu); fp16 data, fp32 softmax ----------------------------
+cudaError_t init_attention_kernels();
 // Floats of scratch the launch needs, and into how many key chunks it will cut a row (1 = no scratch).
 size_t attention_scratch_floats(int B, int Hq, int Hkv, int Sq, int Sk, int D, int sm_count, int* chunks_out);
 // cudaErrorNotSupported: head_dim above 128.  slopes_dev: ALiBi slopes on the device, or null.

@@ -1,0 +1,84 @@
+"""GPU: the matrix attention kernel (head_dim 64 and 128) at the edges of its row tiles (16 and 64 rows of
+(query, head) pairs), key steps (64) and key chunks, with every mask.
+
+Bar against 64-bit softmax attention: the one rounding is the fp16 result, 2^-11 relative at most
+(2^-11 / sqrt(3) = 2.82e-4 scaled RMS; a twentieth on top for the fp32 sums and small samples); the
+log-sum-exp is an fp32 number: half a unit in the last place of its scores (up to 500 with ALiBi), 2^-23
+relative with the sum's own rounding, and 1e-5."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def exact(Q, K, V, causal, window, slopes):
+    B, H, Sq, D = Q.shape
+    Hkv, Sk = K.shape[1], K.shape[2]
+    q, k, v = (t.astype(np.float64) for t in (Q, K, V))
+    k, v = np.repeat(k, H // Hkv, axis=1), np.repeat(v, H // Hkv, axis=1)
+    s = q @ k.transpose(0, 1, 3, 2) / np.sqrt(D)
+    i, j = np.arange(Sq)[:, None], np.arange(Sk)[None, :]
+    if slopes is not None:
+        s = s - np.asarray(slopes, np.float64)[None, :, None, None] * (i - j)
+    hide = np.zeros((Sq, Sk), bool)
+    if causal:
+        hide |= j > i
+    if window > 0:
+        hide |= i - j > window
+    s = np.where(hide, -np.inf, s)
+    m = s.max(axis=-1, keepdims=True)
+    p = np.exp(s - np.where(np.isfinite(m), m, 0.0))
+    l = p.sum(axis=-1, keepdims=True)
+    o = np.where(l > 0, p / np.where(l > 0, l, 1.0), 0.0) @ v
+    with np.errstate(divide="ignore"):
+        return o, (m + np.log(l))[..., 0]
+
+
+@pytest.mark.parametrize("B,H,Hkv,Sq,Sk,D,causal,window,alibi", [
+    (1, 1, 1, 1, 1, 128, False, 0, False), (2, 8, 1, 1, 63, 64, False, 0, False), (1, 16, 2, 2, 65, 128, False, 0, False),
+    (1, 17, 1, 1, 200, 64, False, 0, True), (3, 4, 4, 16, 16, 64, True, 0, False), (1, 4, 4, 17, 17, 128, True, 0, False),
+    (1, 8, 2, 64, 64, 128, True, 0, False), (2, 6, 2, 43, 129, 64, True, 0, True), (1, 8, 4, 200, 200, 128, True, 50, False),
+    (1, 2, 2, 130, 70, 128, True, 0, False), (1, 2, 2, 300, 300, 64, False, 20, False), (1, 4, 1, 96, 1000, 128, False, 0, True),
+    (1, 2, 2, 150, 40, 64, False, 30, False)])
+def test_against_64_bit(tc, ctx, B, H, Hkv, Sq, Sk, D, causal, window, alibi):
+    rng = np.random.default_rng(Sq * 31 + Sk + D)
+    Q = rng.standard_normal((B, H, Sq, D)).astype(np.float16)
+    K = rng.standard_normal((B, Hkv, Sk, D)).astype(np.float16)
+    V = rng.standard_normal((B, Hkv, Sk, D)).astype(np.float16)
+    slopes = [2.0 ** -(1 + h % 8) for h in range(H)] if alibi else None
+    want, lse = exact(Q, K, V, causal, window, slopes)
+    bufs = [ctx.buffer_from_array(t) for t in (Q, K, V)] + [ctx.buffer(Q.nbytes), ctx.buffer(B * H * Sq * 4)]
+    tc.attention_forward(ctx, *bufs[:4], B, H, Sq, Sk, D, LSE=bufs[4], causal=causal, kv_heads=Hkv, window_size=window,
+                         alibi_slopes=slopes)
+    got = bufs[3].to_numpy(Q.shape, np.float16).astype(np.float64)
+    got_lse = bufs[4].to_numpy((B, H, Sq), np.float32).astype(np.float64)
+    for b in bufs:
+        b.close()
+    rms = np.sqrt(((got - want) ** 2).mean() / (want ** 2).mean())
+    assert rms <= 1.05 * 2.0 ** -11 / np.sqrt(3.0)
+    assert np.abs(got - want).max() <= 2.0 ** -11 * np.abs(want).max() + 1e-5
+    seen = np.isfinite(lse)
+    assert np.array_equal(seen, np.isfinite(got_lse)) and (np.abs(got_lse[seen] - lse[seen]) <= 1e-5 + 2.0 ** -23 * np.abs(lse[seen])).all()
+    assert tc.take_device_error(ctx) == 0
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_unaligned_cache_takes_the_vector_kernel(tc, ctx, D):
+    """A cache 2 bytes past a 16-byte boundary gives the same results."""
+    B, H, Hkv, Sq, Sk = 1, 4, 2, 3, 150
+    rng = np.random.default_rng(D)
+    Q = rng.standard_normal((B, H, Sq, D)).astype(np.float16)
+    K = rng.standard_normal((B, Hkv, Sk, D)).astype(np.float16)
+    V = rng.standard_normal((B, Hkv, Sk, D)).astype(np.float16)
+    want, _ = exact(Q, K, V, True, 0, None)
+    bq, bo = ctx.buffer_from_array(Q), ctx.buffer(Q.nbytes)
+    hold = [ctx.buffer(K.nbytes + 16) for _ in range(2)]
+    views = []
+    for h, t in zip(hold, (K, V)):
+        h.upload(t, 2)
+        views.append(ctx.buffer_from_ptr(h.device_ptr() + 2, t.nbytes))
+    tc.attention_forward(ctx, bq, views[0], views[1], bo, B, H, Sq, Sk, D, causal=True, kv_heads=Hkv)
+    got = bo.to_numpy(Q.shape, np.float16).astype(np.float64)
+    for b in [bq, bo] + views + hold:
+        b.close()
+    assert np.abs(got - want).max() <= 2.0 ** -11 * np.abs(want).max() + 1e-5
