@@ -40,12 +40,14 @@ constexpr int kMaxStages = 12;   // the ring is as deep as shared memory allows,
 constexpr int kAStage = kBM * kBK * 2;
 constexpr int kGemmThreads = 6 * 32;          // producer, MMA issuer, four epilogue warps
 constexpr int kGemmBarBytes = 1024;
+constexpr uint32_t kGemmTmemCols = 512;      // two accumulators of up to 256 columns
 constexpr uint32_t kSwizzle128 = 2;           // layout type of the shared-memory descriptor
 
 struct GemmParams {
     __half* C;
     uint32_t* err;
     int M, N, K, ldc;
+    int bn;            // columns of a tile: multiple of 16 (of 64 when B is MN-major), at most 256
     float alpha, beta;
     int b_kmajor;      // B was given transposed ([N][K])
     int a_mnmajor;     // A was given transposed ([K][M])
@@ -75,10 +77,21 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint
     return smem_desc_kmajor(saddr, lbo, sbo) | (static_cast<uint64_t>(layout) << 61);
 }
 
-template <int BN>
+// Whole-warp bounded wait that leaves the warp converged.
+__device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+    if (__all_sync(0xffffffffu, bar_try_wait(bar, parity))) return true;
+    const long long t0 = clock64();
+    for (;;) {
+        if (__all_sync(0xffffffffu, bar_try_wait(bar, parity))) return true;
+        const bool stop = *abort_flag || clock64() - t0 > 2000000000LL;
+        if (__any_sync(0xffffffffu, stop)) return false;
+    }
+}
+
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap bmap) {
-    constexpr int kBStage = BN * kBK * 2;
+    const int BN = p.bn;
+    const int kBStage = BN * kBK * 2;
     extern __shared__ __align__(1024) uint8_t smem[];
     GemmBars* bars = reinterpret_cast<GemmBars*>(smem);
     volatile int* abort_flag = &bars->abort_flag;
@@ -86,7 +99,10 @@ gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap,
     const int stages = p.stages;
     const uint32_t a_stage = p.a_stage;
     uint8_t* b_ring = a_ring + stages * a_stage;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // The warp number by shuffle and one elected lane inside warp-uniform control flow around every copy, MMA
+    // and commit, so that the compiler has their operands as uniform values: under `lane == 0` an MMA took
+    // 70 to 112 clocks to issue, as long as the tensor core works on a 256-wide one.
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int ksteps = (p.K + kBK - 1) / kBK;
     // Tiles of C, numbered column-block-major (the CTAs running at the same time share a block of B's
     // columns and walk down A); CTA c takes tiles c, c + gridDim.x, ...
@@ -102,7 +118,7 @@ gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap,
         prefetch_tensormap(&amap);
         prefetch_tensormap(&bmap);
     }
-    if (warp == 1) tmem_alloc(&bars->tmem_base, 2 * BN);     // two accumulators: a tile's epilogue overlaps the next tile's MMAs
+    if (warp == 1) tmem_alloc(&bars->tmem_base, kGemmTmemCols);     // two accumulators: a tile's epilogue overlaps the next tile's MMAs
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -110,13 +126,13 @@ gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap,
     bool failed = false;
 
     if (warp == 0) {
-        if (lane == 0) {
-            int issued = 0, s = 0;
-            uint32_t par = 0;
-            for (int t = blockIdx.x; t < n_tiles && !failed; t += gridDim.x) {
-                const int m0 = (t % tiles_m) * kBM, n0 = (t / tiles_m) * BN;
-                for (int ks = 0; ks < ksteps; ++ks, ++issued, s = (s + 1 == stages ? 0 : s + 1), par ^= (s == 0 ? 1u : 0u)) {
-                    if (!bar_wait(&bars->empty[s], par ^ 1u, abort_flag)) { failed = true; break; }
+        int issued = 0, s = 0;
+        uint32_t par = 0;
+        for (int t = blockIdx.x; t < n_tiles && !failed; t += gridDim.x) {
+            const int m0 = (t % tiles_m) * kBM, n0 = (t / tiles_m) * BN;
+            for (int ks = 0; ks < ksteps; ++ks) {
+                if (!wait_all(&bars->empty[s], par ^ 1u, abort_flag)) { failed = true; break; }
+                if (elect_one()) {
                     bar_expect_tx(&bars->full[s], p.a_tx + kBStage);
                     if (p.a_mnmajor) {       // [K][M]: two boxes of 64 m x 64 k, like B as given
                         tensor_load_2d(a_ring + s * a_stage, &amap, m0, ks * kBK, &bars->full[s]);
@@ -127,53 +143,59 @@ gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap,
                     if (p.b_kmajor) {
                         tensor_load_2d(b_ring + s * kBStage, &bmap, ks * kBK, n0, &bars->full[s]);
                     } else {
-#pragma unroll
                         for (int c = 0; c < BN / 64; ++c)
                             tensor_load_2d(b_ring + s * kBStage + c * 8192, &bmap, n0 + 64 * c, ks * kBK, &bars->full[s]);
                     }
                 }
-            }
-            if (failed || *abort_flag) {
-                // Let copies already in flight land before the CTA's shared memory is released.
-                const int first = issued > stages ? issued - stages : 0;
-                for (int c = first; c < issued; ++c)
-                    bar_wait(&bars->full[c % stages], static_cast<uint32_t>(c / stages) & 1u, nullptr, 100000000LL);
+                __syncwarp();
+                ++issued;
+                if (++s == stages) { s = 0; par ^= 1u; }
             }
         }
+        if (failed || *abort_flag) {
+            // Let copies already in flight land before the CTA's shared memory is released.
+            const int first = issued > stages ? issued - stages : 0;
+            for (int c = first; c < issued; ++c)
+                bar_wait(&bars->full[c % stages], static_cast<uint32_t>(c / stages) & 1u, nullptr, 100000000LL);
+        }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // bit 16: B is MN-major; bits 7-9 and 10-12: operand formats (0 binary16, 1 bfloat16)
-            const uint32_t idesc = idesc_f16_f32(kBM, BN) | (p.b_kmajor ? 0u : (1u << 16)) | (p.a_mnmajor ? (1u << 15) : 0u) |
-                                   (p.bf16 ? ((1u << 7) | (1u << 10)) : 0u);
-            int it = 0, s = 0;
-            uint32_t par = 0;
-            for (int t = blockIdx.x; t < n_tiles && !failed; t += gridDim.x, ++it) {
-                const int acc = it & 1;
-                // the accumulator's previous tile (two tiles ago) has been read out
-                if (!bar_wait(&bars->acc_empty[acc], (static_cast<uint32_t>(it >> 1) & 1u) ^ 1u, abort_flag)) { failed = true; break; }
+        // bit 16: B is MN-major; bits 7-9 and 10-12: operand formats (0 binary16, 1 bfloat16)
+        const uint32_t idesc = idesc_f16_f32(kBM, BN) | (p.b_kmajor ? 0u : (1u << 16)) | (p.a_mnmajor ? (1u << 15) : 0u) |
+                               (p.bf16 ? ((1u << 7) | (1u << 10)) : 0u);
+        // descriptor strides, and how far a K step of 16 moves along (in the descriptor's 16-byte units)
+        const uint64_t a_form = p.a_mnmajor ? smem_desc(0, 8192u, 1024u, kSwizzle128) : smem_desc(0, 16u, 1024u, kSwizzle128);
+        const uint64_t b_form = p.b_kmajor ? smem_desc(0, 16u, 1024u, kSwizzle128) : smem_desc(0, 8192u, 1024u, kSwizzle128);
+        const uint32_t a_step = p.a_mnmajor ? 128u : 2u, b_step = p.b_kmajor ? 2u : 128u;
+        int it = 0, s = 0;
+        uint32_t par = 0;
+        for (int t = blockIdx.x; t < n_tiles && !failed; t += gridDim.x, ++it) {
+            const int acc = it & 1;
+            // the accumulator's previous tile (two tiles ago) has been read out
+            if (!wait_all(&bars->acc_empty[acc], (static_cast<uint32_t>(it >> 1) & 1u) ^ 1u, abort_flag)) { failed = true; break; }
+            tc_fence_after_sync();
+            const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
+            for (int ks = 0; ks < ksteps; ++ks) {
+                if (!wait_all(&bars->full[s], par, abort_flag)) { failed = true; break; }
                 tc_fence_after_sync();
-                const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
-                for (int ks = 0; ks < ksteps; ++ks, s = (s + 1 == stages ? 0 : s + 1), par ^= (s == 0 ? 1u : 0u)) {
-                    if (!bar_wait(&bars->full[s], par, abort_flag)) { failed = true; break; }
-                    tc_fence_after_sync();
-                    const uint32_t a_addr = s_u32(a_ring + s * a_stage), b_addr = s_u32(b_ring + s * kBStage);
+                const uint64_t adesc = a_form | ((s_u32(a_ring + s * a_stage) >> 4) & 0x3FFFu);
+                const uint64_t bdesc = b_form | ((s_u32(b_ring + s * kBStage) >> 4) & 0x3FFFu);
+                if (elect_one()) {
 #pragma unroll
-                    for (int j = 0; j < kBK / 16; ++j) {
-                        const uint64_t adesc = p.a_mnmajor ? smem_desc(a_addr + j * 2048, 8192u, 1024u, kSwizzle128)
-                                                           : smem_desc(a_addr + j * 32, 16u, 1024u, kSwizzle128);
-                        const uint64_t bdesc = p.b_kmajor ? smem_desc(b_addr + j * 32, 16u, 1024u, kSwizzle128)
-                                                          : smem_desc(b_addr + j * 2048, 8192u, 1024u, kSwizzle128);
-                        mma_f16_ss(d_tmem, adesc, bdesc, idesc, (ks > 0 || j > 0) ? 1u : 0u);
-                    }
+                    for (int j = 0; j < kBK / 16; ++j)
+                        mma_f16_ss(d_tmem, adesc + static_cast<uint64_t>(j * a_step), bdesc + static_cast<uint64_t>(j * b_step), idesc,
+                                   (ks > 0 || j > 0) ? 1u : 0u);
                     mma_commit(&bars->empty[s]);
+                    if (ks + 1 == ksteps) mma_commit(&bars->acc_full[acc]);
                 }
-                if (!failed) mma_commit(&bars->acc_full[acc]);
+                __syncwarp();
+                if (++s == stages) { s = 0; par ^= 1u; }
             }
-            if (failed || *abort_flag) {
-                // every MMA issued so far has completed before the tensor memory is released
-                mma_commit(&bars->drain);
-                bar_wait(&bars->drain, 0, nullptr, 100000000LL);
-            }
+        }
+        if (failed || *abort_flag) {
+            // every MMA issued so far has completed before the tensor memory is released
+            if (elect_one()) mma_commit(&bars->drain);
+            __syncwarp();
+            bar_wait(&bars->drain, 0, nullptr, 100000000LL);
         }
     }
     if (failed) {
@@ -250,7 +272,7 @@ gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap,
     __syncthreads();
     if (warp == 1) {
         tc_fence_after_sync();
-        tmem_dealloc(tmem_base, 2 * BN);
+        tmem_dealloc(tmem_base, kGemmTmemCols);
     }
 }
 
@@ -279,10 +301,10 @@ bool encode_rows_sw128(CUtensorMap* map, const void* base, uint64_t rows, uint64
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN>
 cudaError_t launch_tile(const GemmParams& p, const void* A, const void* B, int lda, int ldb, bool transpose_b,
                         const LaunchEnv& env, cudaStream_t stream) {
     const bool transpose_a = p.a_mnmajor != 0;
+    const int BN = p.bn;
     CUtensorMap amap, bmap;
     // A decode batch or a short prefill block has far fewer than 128 rows: copying only those (2 KB
     // instead of 16 KB a stage at 16 rows) leaves the SM's copy bandwidth to B, which is what such a
@@ -307,16 +329,14 @@ cudaError_t launch_tile(const GemmParams& p, const void* A, const void* B, int l
     const long tiles = static_cast<long>((p.N + BN - 1) / BN) * ((p.M + kBM - 1) / kBM);
     const long sms = env.sm_count > 0 ? env.sm_count : 148;
     const dim3 grid(static_cast<unsigned>(tiles < sms ? tiles : sms));     // one CTA per SM walks the tiles
-    gemm_f16_tc_kernel<BN><<<grid, kGemmThreads, smem, stream>>>(q, amap, bmap);
+    gemm_f16_tc_kernel<<<grid, kGemmThreads, smem, stream>>>(q, amap, bmap);
     return cudaGetLastError();
 }
 
 }  // namespace
 
 cudaError_t init_gemm_tc_kernel(int smem_optin) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_f16_tc_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(gemm_f16_tc_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin);
+    return cudaFuncSetAttribute(gemm_f16_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin);
 }
 
 // cudaErrorNotSupported when the operands are outside what the tiled copies can describe: the leading
@@ -334,13 +354,22 @@ cudaError_t launch_gemm_f16_tc(const void* A, const void* B, void* C, int M, int
     p.b_kmajor = transpose_b ? 1 : 0;
     p.bf16 = bf16 ? 1 : 0;
     p.a_mnmajor = transpose_a ? 1 : 0;
-    // 256-wide tiles halve the re-reads of A and the number of MMA instructions; measured faster than 128-wide
-    // ones whenever N fills them (4096^3: 1119 against 769 TFLOP/s; 512 x 11008 x 4096: 629 against 523).
+    // Tile width: the one whose rounds of tiles over the SMs take least, by a model of a 64-wide K step: four
+    // MMAs of N / 2 clocks each, but at least 54 (the measured floor of an MMA with both operands in shared
+    // memory), and the stage's bytes at 45 per clock; the last tile's read-out is not hidden.  512 x 11008 x
+    // 4096 takes 160-wide tiles (two rounds) instead of two rounds of 256-wide ones of which the second
+    // is nearly empty.  B as given is laid out in pieces of 64 columns.
     const long sms = env.sm_count > 0 ? env.sm_count : 148;
-    const long tiles256 = static_cast<long>((M + kBM - 1) / kBM) * ((N + 255) / 256);
-    const bool wide = N >= 256 && tiles256 >= sms;      // few rows of A: narrower tiles spread over more SMs
-    return wide ? launch_tile<256>(p, A, B, lda, ldb, transpose_b, env, stream)
-                : launch_tile<128>(p, A, B, lda, ldb, transpose_b, env, stream);
+    const long tiles_m = (M + kBM - 1) / kBM, ksteps = (K + kBK - 1) / kBK;
+    const long a_bytes = (transpose_a || M >= kBM ? kBM : ((M + 7) & ~7)) * kBK * 2L;
+    double best = 0.0;
+    for (int bn = 256; bn >= 64; bn -= transpose_b ? 16 : 64) {
+        const long tiles = tiles_m * ((N + bn - 1) / bn);
+        const double mma = 4.0 * (bn > 108 ? bn / 2.0 : 54.0), copy = (a_bytes + bn * kBK * 2L) / 45.0;
+        const double cost = static_cast<double>((tiles + sms - 1) / sms) * ksteps * (mma > copy ? mma : copy) + 1000.0 + 8.0 * bn;
+        if (best == 0.0 || cost < best) { best = cost; p.bn = bn; }
+    }
+    return launch_tile(p, A, B, lda, ldb, transpose_b, env, stream);
 }
 
 }  // namespace tcb

@@ -1,0 +1,33 @@
+"""GPU: tc_gemm on the tensor cores over tile widths: shapes that take narrow, odd and 256-wide tiles, both
+forms of both operands.  One rounding of the result: fp16 2^-11 / sqrt(3) = 2.82e-4 scaled RMS, bf16
+2^-8 / sqrt(3) = 2.26e-3; a twentieth on top for the fp32 sums and small samples."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,N,K", [(8, 72, 64), (5, 4096, 136), (128, 2368, 192), (130, 9480, 72), (512, 11008, 128), (300, 1000, 520),
+                                   (1024, 4800, 64)])
+@pytest.mark.parametrize("ta,tb", [(False, True), (False, False), (True, True)])
+@pytest.mark.parametrize("dtype", ["f16", "bf16"])
+def test_widths_against_64_bit(tc, ctx, M, N, K, ta, tb, dtype):
+    import torch
+    if ta and M % 8:
+        pytest.skip("a transposed A has rows of M elements, which the tiled copies need in multiples of 8")
+    dt = torch.float16 if dtype == "f16" else torch.bfloat16
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M + N + K)
+    A = torch.randn((K, M) if ta else (M, K), generator=g, device="cuda").to(dt)
+    B = torch.randn((N, K) if tb else (K, N), generator=g, device="cuda").to(dt)
+    C = torch.full((M, N), float("nan"), device="cuda", dtype=dt)
+    bufs = [ctx.buffer_from_ptr(t.data_ptr(), t.numel() * 2) for t in (A, B, C)]
+    torch.cuda.synchronize()
+    tc.gemm(ctx, *bufs, M, N, K, dtype=dtype, transpose_a=ta, transpose_b=tb)
+    assert tc.cuda_last_kernel_name() == "gemm_f16_tcgen05_sm100"
+    want = (A.double().t() if ta else A.double()) @ (B.double().t() if tb else B.double())
+    err = ((C.double() - want).square().mean() / want.square().mean()).sqrt().item()
+    for b in bufs:
+        b.close()
+    assert err <= 1.05 * (2.0 ** -11 if dtype == "f16" else 2.0 ** -8) / np.sqrt(3.0)
+    assert tc.take_device_error(ctx) == 0
