@@ -6,6 +6,7 @@
 // for every activation row (lib/ops/quantized_cpu.cpp:193-228).  Here the packed weights are read
 // once per tile of up to 256 activation rows and never exist as fp16 in memory:
 //
+//   * Up to four matrices that share their activations (q, k and v; gate and up) are one launch.
 //   * A CTA owns 128 weight rows x NB activation rows (NB = 16 .. 256, the MMA's N) and a K range; a
 //     cluster of up to 8 CTAs shares a tile along K when there are fewer tiles than SMs.  The unit of
 //     work is one group of 8 blocks (256 weights) of the 128 rows: a single tiled TMA copy of 128 rows
@@ -59,15 +60,18 @@ constexpr int kMmaWarp = kDqWarps + 2;     // four issuers
 constexpr int kThreads = (kDqWarps + 2 + 4) * 32;
 constexpr int kMaxRing = 12;
 constexpr int kMaxSlots = 4;
+constexpr int kMaxMats = 4;                // matrices that share their activations in one launch
 constexpr int kSub = 64;                   // weights per row and A slot
 constexpr uint32_t kTmemCols = 512;
 constexpr int kBarBytes = 1024;
 constexpr uint32_t kSwizzle128 = 2;        // descriptor layout type
 
 struct QtcParams {
-    void* Y;
+    void* Y[kMaxMats];
+    int N[kMaxMats];
+    int tile0[kMaxMats];   // first row tile of each matrix (INT_MAX past the last)
     uint32_t* err;
-    int M, N;
+    int M;
     int y_f32;
     int nb;            // MMA N extent: multiple of 16, <= 256
     int groups;        // K / 256
@@ -78,6 +82,8 @@ struct QtcParams {
     int x_stages;      // per issuer
     int off_raw, off_x;
 };
+
+struct QtcMaps { CUtensorMap w[kMaxMats], x; };
 
 struct Bars {
     uint64_t raw_full[kMaxRing], raw_empty[kMaxRing];
@@ -181,7 +187,7 @@ struct Pos {                                // position in a ring
 // K slices per activation stage.  With one or two issuers two warpgroups keep up with the MMAs.
 template <int FMT, int I, int SLOTS, int XK>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_q_tc_kernel(const QtcParams p, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap) {
+gemm_q_tc_kernel(const QtcParams p, const __grid_constant__ QtcMaps maps) {
     using F = QFmt<FMT>;
     constexpr int kRawBytes = kRows * F::kGroup;
     constexpr int kActive = I == 4 ? 4 : 2;          // warpgroups that dequantise
@@ -199,15 +205,22 @@ gemm_q_tc_kernel(const QtcParams p, const __grid_constant__ CUtensorMap wmap, co
     const int crank = split > 1 ? static_cast<int>(cluster_ctarank()) : 0;
     const int g0 = p.groups * crank / split;
     const int n_units = p.groups * (crank + 1) / split - g0;
-    const int row0 = (tile / p.col_tiles) * kRows;
+    const int rt = tile / p.col_tiles;
+    int mat = 0, N = p.N[0], first_tile = 0;
+    void* Y = p.Y[0];
+#pragma unroll
+    for (int i = 1; i < kMaxMats; ++i)
+        if (rt >= p.tile0[i]) { mat = i; N = p.N[i]; Y = p.Y[i]; first_tile = p.tile0[i]; }
+    const CUtensorMap* wmap = &maps.w[mat];
+    const int row0 = (rt - first_tile) * kRows;
     const int m0 = (tile % p.col_tiles) * nb;
     uint8_t* raw_ring = smem + p.off_raw;
     uint8_t* x_ring = smem + p.off_x;
     const int x_bytes = nb * 128 * XK;
 
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    if (tid == kRawWarp * 32) prefetch_tensormap(&wmap);
-    if (tid == kXWarp * 32) prefetch_tensormap(&xmap);
+    if (tid == kRawWarp * 32) prefetch_tensormap(wmap);
+    if (tid == kXWarp * 32) prefetch_tensormap(&maps.x);
     if (tid == 0) {
         for (int i = 0; i < kMaxRing; ++i) {
             bar_init(&bars->raw_full[i], 1);
@@ -280,7 +293,7 @@ gemm_q_tc_kernel(const QtcParams p, const __grid_constant__ CUtensorMap wmap, co
                 if (!wait_all(&bars->raw_empty[st], ring.ph ^ 1u, abort_flag)) { failed = true; break; }
                 if (elect_one()) {
                     bar_expect_tx(&bars->raw_full[st], kRawBytes);
-                    tensor_load_2d(raw_ring + st * kRawBytes, &wmap, (g0 + r + j) * (F::kGroup / F::kElem), row0, &bars->raw_full[st]);
+                    tensor_load_2d(raw_ring + st * kRawBytes, wmap, (g0 + r + j) * (F::kGroup / F::kElem), row0, &bars->raw_full[st]);
                     sent[st] += 1;
                 }
                 __syncwarp();
@@ -306,7 +319,7 @@ gemm_q_tc_kernel(const QtcParams p, const __grid_constant__ CUtensorMap wmap, co
                     if (!wait_all(&bars->x_empty[st], ring.ph ^ 1u, abort_flag)) { failed = true; break; }
                     if (elect_one()) {
                         bar_expect_tx(&bars->x_full[st], x_bytes);
-                        tensor_load_3d(x_ring + st * x_bytes, &xmap, 0, m0, (g0 + r + j) * 4 + s, &bars->x_full[st]);
+                        tensor_load_3d(x_ring + st * x_bytes, &maps.x, 0, m0, (g0 + r + j) * 4 + s, &bars->x_full[st]);
                         sent[kMaxRing + st] += 1;
                     }
                     __syncwarp();
@@ -393,13 +406,13 @@ gemm_q_tc_kernel(const QtcParams p, const __grid_constant__ CUtensorMap wmap, co
                 if (split > 1) {
 #pragma unroll
                     for (int e = 0; e < 16; ++e) red[(c0 + e) * kRows + r] = f[e];
-                } else if (row < p.N) {
+                } else if (row < N) {
 #pragma unroll
                     for (int e = 0; e < 16; ++e) {
                         if (c0 + e >= m_end) break;
-                        const size_t o = static_cast<size_t>(m0 + c0 + e) * p.N + row;
-                        if (p.y_f32) static_cast<float*>(p.Y)[o] = f[e];
-                        else static_cast<__half*>(p.Y)[o] = __float2half_rn(f[e]);
+                        const size_t o = static_cast<size_t>(m0 + c0 + e) * N + row;
+                        if (p.y_f32) static_cast<float*>(Y)[o] = f[e];
+                        else static_cast<__half*>(Y)[o] = __float2half_rn(f[e]);
                     }
                 }
             }
@@ -418,13 +431,13 @@ gemm_q_tc_kernel(const QtcParams p, const __grid_constant__ CUtensorMap wmap, co
             for (int e = tid; e < m_end * rows_c; e += kThreads) {
                 const int m = e / rows_c, r = r_lo + e % rows_c;
                 const int row = row0 + r;
-                if (row >= p.N) continue;
+                if (row >= N) continue;
                 float acc = 0.f;
                 for (int c = 0; c < split; ++c)
                     acc += ld_cluster_f32(red_addr + static_cast<uint32_t>(m * kRows + r) * 4u, c);
-                const size_t o = static_cast<size_t>(m0 + m) * p.N + row;
-                if (p.y_f32) static_cast<float*>(p.Y)[o] = acc;
-                else static_cast<__half*>(p.Y)[o] = __float2half_rn(acc);
+                const size_t o = static_cast<size_t>(m0 + m) * N + row;
+                if (p.y_f32) static_cast<float*>(Y)[o] = acc;
+                else static_cast<__half*>(Y)[o] = __float2half_rn(acc);
             }
         }
         cluster_sync_all();   // peers may still be reading this CTA's partials
@@ -462,7 +475,7 @@ int max_active_clusters(int size, int smem) {
     return n > 0 ? n : 0;
 }
 
-using QtcKernel = void (*)(const QtcParams, const CUtensorMap, const CUtensorMap);
+using QtcKernel = void (*)(const QtcParams, const QtcMaps);
 struct QtcVariant { int max_nb, issuers, active, xk; QtcKernel kernel[2]; };
 const QtcVariant kVariants[] = {
     {16, 4, 4, 4, {gemm_q_tc_kernel<FMT_Q4_0, 4, 3, 4>, gemm_q_tc_kernel<FMT_Q8_0, 4, 3, 4>}},
@@ -483,25 +496,36 @@ cudaError_t init_gemm_q_tc_kernels(int smem_optin) {
     return cudaSuccess;
 }
 
-// cudaErrorNotSupported when the operation is outside this kernel's domain.
-cudaError_t launch_gemm_q_tc(const GemvQArgs& a, const LaunchEnv& env, cudaStream_t stream) {
-    if (a.x_f32 || a.gamma != nullptr || (a.fmt != FMT_Q4_0 && a.fmt != FMT_Q8_0)) return cudaErrorNotSupported;
-    if (a.M < 1 || a.K <= 0 || a.K % 256 != 0 || a.N <= 0) return cudaErrorNotSupported;
-    if ((reinterpret_cast<uintptr_t>(a.W) & 15u) || (reinterpret_cast<uintptr_t>(a.X) & 15u)) return cudaErrorNotSupported;
-
+// Up to kMaxMats products of the same activation rows in one launch: ops[1 ..] differ from ops[0] in W, Y and N
+// only.  cudaErrorNotSupported when the operation is outside this kernel's domain.
+cudaError_t launch_gemm_q_tc(const GemvQArgs* ops, int n_ops, const LaunchEnv& env, cudaStream_t stream) {
+    if (n_ops < 1 || n_ops > kMaxMats) return cudaErrorNotSupported;
+    const GemvQArgs& a = ops[0];
     QtcParams p{};
-    p.Y = a.Y;
     p.err = env.err_word;
-    p.M = a.M; p.N = a.N;
+    p.M = a.M;
     p.y_f32 = a.y_f32 ? 1 : 0;
     p.groups = a.K / 256;
     // Activation rows in as few equal tiles of at most 256 as there can be.
     p.col_tiles = (a.M + 255) / 256;
     p.nb = ((a.M + p.col_tiles - 1) / p.col_tiles + 15) & ~15;
+    long long row_tiles = 0;
+    for (int i = 0; i < kMaxMats; ++i) {
+        p.tile0[i] = 0x7fffffff;
+        if (i >= n_ops) continue;
+        const GemvQArgs& o = ops[i];
+        if (o.x_f32 || o.gamma != nullptr || (o.fmt != FMT_Q4_0 && o.fmt != FMT_Q8_0) || o.M < 1 || o.K <= 0 || o.K % 256 != 0 || o.N <= 0 ||
+            (reinterpret_cast<uintptr_t>(o.W) & 15u) || (reinterpret_cast<uintptr_t>(o.X) & 15u))
+            return cudaErrorNotSupported;
+        p.tile0[i] = static_cast<int>(row_tiles);
+        p.Y[i] = o.Y;
+        p.N[i] = o.N;
+        row_tiles += (o.N + kRows - 1) / kRows;
+    }
     const QtcVariant* v = kVariants;
     while (v->max_nb < p.nb) ++v;
     const int raw_bytes = kRows * (a.fmt == FMT_Q4_0 ? 144 : 272), x_bytes = p.nb * 128 * v->xk;
-    const long long tiles_ll = static_cast<long long>((a.N + kRows - 1) / kRows) * p.col_tiles;
+    const long long tiles_ll = row_tiles * p.col_tiles;
     if (tiles_ll > 0x0fffffff) return cudaErrorNotSupported;
     const int tiles = static_cast<int>(tiles_ll);
 
@@ -532,11 +556,13 @@ cudaError_t launch_gemm_q_tc(const GemvQArgs& a, const LaunchEnv& env, cudaStrea
     p.split = split;
     const int smem_all = split > 1 && p.off_x + red_bytes > smem ? p.off_x + red_bytes : smem;
 
-    CUtensorMap wmap, xmap;
+    QtcMaps maps;
     const int gb = a.fmt == FMT_Q4_0 ? 144 : 272;
-    if (!encode_bytes_2d(&wmap, a.W, a.N, static_cast<uint64_t>(p.groups) * gb, gb, kRows, a.fmt == FMT_Q4_0 ? 1 : 4))
-        return cudaErrorNotSupported;
-    if (!encode_f16_slices_sw128(&xmap, a.X, a.M, a.K, p.nb, v->xk)) return cudaErrorNotSupported;
+    for (int i = 0; i < n_ops; ++i)
+        if (!encode_bytes_2d(&maps.w[i], ops[i].W, ops[i].N, static_cast<uint64_t>(p.groups) * gb, gb, kRows, a.fmt == FMT_Q4_0 ? 1 : 4))
+            return cudaErrorNotSupported;
+    for (int i = n_ops; i < kMaxMats; ++i) maps.w[i] = maps.w[0];
+    if (!encode_f16_slices_sw128(&maps.x, a.X, a.M, a.K, p.nb, v->xk)) return cudaErrorNotSupported;
 
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(tiles) * split);
@@ -558,7 +584,7 @@ cudaError_t launch_gemm_q_tc(const GemvQArgs& a, const LaunchEnv& env, cudaStrea
         attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
         ++cfg.numAttrs;
     }
-    return cudaLaunchKernelEx(&cfg, v->kernel[a.fmt == FMT_Q4_0 ? 0 : 1], p, wmap, xmap);
+    return cudaLaunchKernelEx(&cfg, v->kernel[a.fmt == FMT_Q4_0 ? 0 : 1], p, maps);
 }
 
 }  // namespace tcb

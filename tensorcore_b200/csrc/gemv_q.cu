@@ -32,7 +32,7 @@
 
 namespace tcb {
 cudaError_t init_gemm_q_tc_kernels(int smem_optin);
-cudaError_t launch_gemm_q_tc(const GemvQArgs& a, const LaunchEnv& env, cudaStream_t stream);
+cudaError_t launch_gemm_q_tc(const GemvQArgs* ops, int n_ops, const LaunchEnv& env, cudaStream_t stream);
 cudaError_t init_gemv_q_rows_kernels(int smem_optin);
 cudaError_t launch_gemv_q_rows(const GemvQArgs& a, const LaunchEnv& env, cudaStream_t stream);
 cudaError_t init_decode_kernel(int smem_optin);
@@ -597,6 +597,76 @@ cudaError_t init_gemv_kernels(int smem_optin) {
     return e;
 }
 
+static bool wants_tc(const GemvQArgs& a, const LaunchEnv& env) {
+    return !a.x_f32 && a.K % 256 == 0 && (env.variant == VARIANT_TC ? a.fmt == FMT_Q4_0 : env.variant == VARIANT_AUTO && tc_rows(a));
+}
+
+bool gemv_q_groupable(const GemvQArgs* ops, int n, const GemvQArgs& b, const LaunchEnv& env) {
+    const GemvQArgs& a = ops[0];
+    if (n >= 4 || !wants_tc(a, env) || !wants_tc(b, env)) return false;
+    if (a.fmt != b.fmt || a.M != b.M || a.K != b.K || a.X != b.X || a.gamma != b.gamma || a.eps != b.eps || a.y_f32 != b.y_f32)
+        return false;
+    const size_t wb = static_cast<size_t>(a.K / 32) * (a.fmt == FMT_Q4_0 ? 18 : 34), ysz = a.y_f32 ? 4 : 2;
+    auto apart = [](const void* p, size_t np, const void* q, size_t nq) {
+        const uintptr_t x = reinterpret_cast<uintptr_t>(p), y = reinterpret_cast<uintptr_t>(q);
+        return x + np <= y || y + nq <= x;
+    };
+    auto ybytes = [&](const GemvQArgs& o) { return static_cast<size_t>(o.M) * o.N * ysz; };
+    auto inputs_apart = [&](const GemvQArgs& y, const GemvQArgs& w) {      // y's result against what the launch reads
+        return apart(y.Y, ybytes(y), w.W, w.N * wb) && apart(y.Y, ybytes(y), a.X, static_cast<size_t>(a.M) * a.K * 2) &&
+               (!a.gamma || apart(y.Y, ybytes(y), a.gamma, static_cast<size_t>(a.K) * 2));
+    };
+    for (int i = 0; i < n; ++i)
+        if (!inputs_apart(ops[i], b) || !inputs_apart(b, ops[i]) || !apart(ops[i].Y, ybytes(ops[i]), b.Y, ybytes(b))) return false;
+    return true;
+}
+
+// Products of five rows or more (tc_rows): the tcgen05 kernel dequantises the weights on their way to the
+// tensor cores and reads them once per 256 rows.  It rounds dequantised weights to fp16, which only the
+// fp16-activation bound allows.  The fused RMSNorm form takes it too, behind a pass that normalises the
+// rows into the stream's scratch as fp16 (one more rounding, inside the same bound) - once for all
+// products of a group; rows that are not 16-byte aligned are copied there.
+cudaError_t launch_gemv_q_group(const GemvQArgs* ops, int n, const LaunchEnv& env, cudaStream_t stream, int* launches,
+                                const char** name) {
+    const GemvQArgs& a = ops[0];
+    const bool fuse = a.gamma != nullptr, copy = !fuse && (reinterpret_cast<uintptr_t>(a.X) & 15u) != 0;
+    const size_t row_bytes = static_cast<size_t>(a.K) * 2 + 4;      // a row and its 1/rms
+    size_t slab = static_cast<size_t>(a.M);
+    if (fuse || copy) slab = a.norm_scratch ? a.norm_scratch_bytes / row_bytes : 0;
+    if (slab > static_cast<size_t>(a.M)) slab = static_cast<size_t>(a.M);
+    if (slab == 0) return cudaErrorNotSupported;
+    int count = 0;
+    for (int m0 = 0; m0 < a.M; m0 += static_cast<int>(slab)) {
+        GemvQArgs s[4];
+        const int rows = a.M - m0 < static_cast<int>(slab) ? a.M - m0 : static_cast<int>(slab);
+        const void* x = static_cast<const uint8_t*>(a.X) + static_cast<size_t>(m0) * a.K * 2;
+        cudaError_t e = cudaSuccess;
+        if (fuse) {
+            float* rstd = reinterpret_cast<float*>(static_cast<uint8_t*>(a.norm_scratch) + slab * static_cast<size_t>(a.K) * 2);
+            e = launch_norm_forward(x, a.gamma, nullptr, a.norm_scratch, nullptr, rstd, rows, a.K, a.eps, stream, env.pdl);
+            ++count;
+        } else if (copy) {
+            e = cudaMemcpyAsync(a.norm_scratch, x, static_cast<size_t>(rows) * a.K * 2, cudaMemcpyDeviceToDevice, stream);
+        }
+        if (e != cudaSuccess) return e;
+        for (int i = 0; i < n; ++i) {
+            s[i] = ops[i];
+            s[i].M = rows;
+            s[i].gamma = nullptr;
+            s[i].X = fuse || copy ? a.norm_scratch : x;
+            s[i].Y = static_cast<uint8_t*>(ops[i].Y) + static_cast<size_t>(m0) * ops[i].N * (a.y_f32 ? 4 : 2);
+        }
+        e = launch_gemm_q_tc(s, n, env, stream);
+        if (e != cudaSuccess) return e;      // cudaErrorNotSupported only on the first slab: the others differ in rows alone
+        ++count;
+    }
+    if (launches) *launches += count;
+    if (name) *name = a.M >= gemm_min_rows(a.fmt) && !a.y_f32
+                          ? (a.fmt == FMT_Q4_0 ? "q4_0_dequant_gemm_tcgen05_sm100" : "q8_0_dequant_gemm_tcgen05_sm100")
+                          : "q4_0_gemv_tcgen05_sm100";
+    return cudaSuccess;
+}
+
 cudaError_t launch_gemv_q(const GemvQArgs& a, const LaunchEnv& env, cudaStream_t stream,
                           int* launches, const char** name) {
     int count = 0;
@@ -605,44 +675,10 @@ cudaError_t launch_gemv_q(const GemvQArgs& a, const LaunchEnv& env, cudaStream_t
     const size_t xsz = a.x_f32 ? 4 : 2, ysz = a.y_f32 ? 4 : 2;
     const bool fuse = a.gamma != nullptr;
 
-    // Five rows or more (tc_rows): the tcgen05 kernel dequantises the weights on their way to the tensor
-    // cores and reads them once per 256 rows.  It rounds dequantised weights to fp16, which only the
-    // fp16-activation bound allows.  The fused RMSNorm form takes it too, behind a pass that normalises
-    // the rows into the stream's scratch as fp16 (one more rounding, inside the same bound); rows that
-    // are not 16-byte aligned are copied there.
-    if (!a.x_f32 && a.K % 256 == 0 && (env.variant == VARIANT_TC ? a.fmt == FMT_Q4_0 : env.variant == VARIANT_AUTO && tc_rows(a))) {
-        const bool copy = !fuse && (reinterpret_cast<uintptr_t>(a.X) & 15u) != 0;
-        const size_t row_bytes = static_cast<size_t>(a.K) * 2 + 4;      // a row and its 1/rms
-        size_t slab = static_cast<size_t>(a.M);
-        if (fuse || copy) slab = a.norm_scratch ? a.norm_scratch_bytes / row_bytes : 0;
-        if (slab > static_cast<size_t>(a.M)) slab = static_cast<size_t>(a.M);
-        bool done = slab > 0;
-        for (int m0 = 0; done && m0 < a.M && err == cudaSuccess; m0 += static_cast<int>(slab)) {
-            GemvQArgs s = a;
-            s.M = a.M - m0 < static_cast<int>(slab) ? a.M - m0 : static_cast<int>(slab);
-            s.X = static_cast<const uint8_t*>(a.X) + static_cast<size_t>(m0) * a.K * xsz;
-            s.Y = static_cast<uint8_t*>(a.Y) + static_cast<size_t>(m0) * a.N * ysz;
-            if (fuse) {
-                float* rstd = reinterpret_cast<float*>(static_cast<uint8_t*>(a.norm_scratch) + slab * static_cast<size_t>(a.K) * 2);
-                err = launch_norm_forward(s.X, a.gamma, nullptr, a.norm_scratch, nullptr, rstd, s.M, a.K, a.eps, stream, env.pdl);
-                ++count;
-            } else if (copy) {
-                err = cudaMemcpyAsync(a.norm_scratch, s.X, static_cast<size_t>(s.M) * a.K * 2, cudaMemcpyDeviceToDevice, stream);
-            }
-            if (err != cudaSuccess) break;
-            if (fuse || copy) { s.X = a.norm_scratch; s.gamma = nullptr; }
-            const cudaError_t te = launch_gemm_q_tc(s, env, stream);
-            if (te == cudaErrorNotSupported && m0 == 0) { done = false; count = 0; (void)cudaGetLastError(); break; }
-            err = te;
-            ++count;
-        }
-        if (done) {
-            if (launches) *launches += count;
-            if (name) *name = a.M >= gemm_min_rows(a.fmt) && !a.y_f32
-                                  ? (a.fmt == FMT_Q4_0 ? "q4_0_dequant_gemm_tcgen05_sm100" : "q8_0_dequant_gemm_tcgen05_sm100")
-                                  : "q4_0_gemv_tcgen05_sm100";
-            return err;
-        }
+    if (wants_tc(a, env)) {
+        const cudaError_t te = launch_gemv_q_group(&a, 1, env, stream, launches, name);
+        if (te != cudaErrorNotSupported) return te;
+        (void)cudaGetLastError();
     }
     // Prefill-sized calls whose K is no multiple of 256: the weights are dequantised once into the
     // stream's scratch (fp16, the same rounding as above) and multiplied on the tensor cores as a GEMM

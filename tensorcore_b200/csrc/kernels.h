@@ -159,6 +159,12 @@ cudaError_t launch_quantize(const void* W_f16, void* W_quant, int fmt, int N, in
                             const char** name);
 cudaError_t launch_gemv_q(const GemvQArgs& a, const LaunchEnv& env, cudaStream_t stream,
                           int* launches, const char** name);
+// Whether b may run in one launch with ops[0 .. n-1]: the same activations (and norm) and options, the tcgen05
+// kernel's domain, and no result that another of them reads or writes.
+bool gemv_q_groupable(const GemvQArgs* ops, int n, const GemvQArgs& b, const LaunchEnv& env);
+// The products of such a group, at most four.  cudaErrorNotSupported: launch them one by one.
+cudaError_t launch_gemv_q_group(const GemvQArgs* ops, int n, const LaunchEnv& env, cudaStream_t stream,
+                                int* launches, const char** name);
 cudaError_t launch_dense_norm_gemv(const DenseNormGemvArgs& a, const LaunchEnv& env,
                                    cudaStream_t stream, int* launches, const char** name);
 

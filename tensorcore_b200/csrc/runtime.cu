@@ -796,6 +796,31 @@ cudaError_t launch_recorded(tc_context* ctx, const RecordedOp& op, cudaStream_t 
     return tcb::launch_gemv_q(op.a, env, st, launches, name);
 }
 
+// The operations of a list in order; neighbours that share their activations (q, k and v; gate and up) run as
+// one launch where their kernel can take several matrices.
+cudaError_t launch_list(tc_context* ctx, const std::vector<RecordedOp>& list, cudaStream_t st, int* launches, const char** name) {
+    cudaError_t e = cudaSuccess;
+    for (size_t i = 0; i < list.size() && e == cudaSuccess;) {
+        const LaunchEnv env = make_env(ctx, i > 0);
+        tcb::GemvQArgs group[4];
+        int n = 0;
+        group[n++] = list[i].a;
+        while (i + n < list.size() && tcb::gemv_q_groupable(group, n, list[i + n].a, env)) {
+            group[n] = list[i + n].a;
+            ++n;
+        }
+        if (n > 1) {
+            e = tcb::launch_gemv_q_group(group, n, env, st, launches, name);
+            if (e == cudaSuccess) { i += n; continue; }
+            if (e != cudaErrorNotSupported) break;
+            (void)cudaGetLastError();
+        }
+        e = launch_recorded(ctx, list[i], st, i > 0, launches, name);
+        ++i;
+    }
+    return e;
+}
+
 constexpr int kMegaMaxOps = 1024;
 constexpr size_t kMegaFlagBytes = 256;
 
@@ -1001,8 +1026,7 @@ tc_status_t submit_pending(tc_stream* s) {
             if (e == cudaSuccess) {
                 cudaError_t le = cudaSuccess;
                 int k = 0;
-                for (size_t i = 0; i < s->pending.size() && le == cudaSuccess; ++i)
-                    le = launch_recorded(ctx, s->pending[i], s->s, i > 0, &k, &name);
+                le = launch_list(ctx, s->pending, s->s, &k, &name);
                 e = cudaStreamEndCapture(s->s, &graph);
                 if (le != cudaSuccess) e = le;
                 if (e == cudaSuccess && graph) {
@@ -1029,10 +1053,7 @@ tc_status_t submit_pending(tc_stream* s) {
             if (!done) { drop_graphs(s); }
         }
     }
-    if (!done) {
-        for (size_t i = 0; i < s->pending.size() && e == cudaSuccess; ++i)
-            e = launch_recorded(ctx, s->pending[i], s->s, i > 0, &launches, &name);
-    }
+    if (!done && e == cudaSuccess) e = launch_list(ctx, s->pending, s->s, &launches, &name);
     if (e == cudaSuccess && any_staged) {
         for (RecordedOp& op : s->pending)
             if (e == cudaSuccess) e = finish_output(op.Y, op.y_bytes, s->s);

@@ -84,3 +84,53 @@ def test_non_finite_weights_scales_and_activations(tc, ctx, oracle):
         assert not np.isfinite(got[:, 5]).any()
         keep = np.arange(N) != 5
         assert np.array_equal(got[:, keep], base[:, keep])
+
+
+@pytest.mark.parametrize("fmt,M", [(0, 5), (0, 33), (1, 16), (0, 130)])
+def test_products_that_share_their_activations_run_as_one_launch(tc, ctx, oracle, fmt, M):
+    """q, k and v of a layer (different row counts), recorded with the norm fused: one pass over the rows and
+    one product launch a submission, whether launched directly or replayed from a graph."""
+    K, Ns = 512, (384, 130, 127)
+    X, _ = data(oracle, fmt, M, 64, K)
+    g = (1 + 0.1 * np.random.default_rng(3).standard_normal(K)).astype(np.float16)
+    ws = [data(oracle, fmt, M + i, n, K)[1] for i, n in enumerate(Ns)]
+    want = [oracle.fused_rmsnorm_gemv_quantized_f32(X.astype(np.float32), g.astype(np.float32), w, fmt, n) for w, n in zip(ws, Ns)]
+    bx, bg = ctx.buffer_from_array(X), ctx.buffer_from_array(g)
+    bw, by = [ctx.buffer_from_array(w) for w in ws], [ctx.buffer(M * n * 2) for n in Ns]
+    s = ctx.stream()
+    for _ in range(4):
+        before = tc.launch_count()
+        for w, y, n in zip(bw, by, Ns):
+            tc.fused_rmsnorm_gemv_quantized_ex(ctx, bx, bg, w, y, fmt, M, n, K, 1e-5, "f16", "f16", s)
+        s.sync()
+        assert tc.launch_count() - before == 2
+        for y, n, v in zip(by, Ns, want):
+            # three roundings to fp16: weights, normalised rows, result
+            assert oracle.scaled_rms(y.to_numpy((M, n), np.float16), v) <= 1.1 * np.sqrt(3.0) * ROUND
+    s.close()
+    for b in [bx, bg] + bw + by:
+        b.close()
+
+
+def test_dependent_products_do_not_share_a_launch(tc, ctx, oracle):
+    """A recorded product that writes what a neighbour reads or writes keeps its place: the second product
+    overwrites the activations of both, the third overwrites the first one's result."""
+    M, K = 8, 512
+    X, w1 = data(oracle, 0, M, K, K)
+    _, w2 = data(oracle, 0, M + 1, K, K)
+    bx, b1, b2, by = ctx.buffer_from_array(X), ctx.buffer_from_array(w1), ctx.buffer_from_array(w2), ctx.buffer(M * K * 2)
+    s = ctx.stream()
+    ctx.gemv_quantized_async(bx, b1, by, 0, M, K, K, s)      # y = W1 x
+    ctx.gemv_quantized_async(bx, b2, bx, 0, M, K, K, s)      # x is overwritten after that (its value is not looked at: in place)
+    s.sync()
+    y1 = by.to_numpy((M, K), np.float16)
+    assert oracle.scaled_rms(y1.astype(np.float64), oracle.dequant_dot_f64(X.astype(np.float64), w1, 0, K)) <= 5e-4
+    bx.upload(X)
+    ctx.gemv_quantized_async(bx, b1, by, 0, M, K, K, s)
+    ctx.gemv_quantized_async(bx, b2, by, 0, M, K, K, s)      # the same result buffer: the later product's values stay
+    s.sync()
+    y2 = by.to_numpy((M, K), np.float16)
+    assert oracle.scaled_rms(y2.astype(np.float64), oracle.dequant_dot_f64(X.astype(np.float64), w2, 0, K)) <= 5e-4
+    s.close()
+    for b in (bx, b1, b2, by):
+        b.close()
