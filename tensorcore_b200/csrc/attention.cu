@@ -5,8 +5,8 @@
 // fp32 LSE [B,H,Sq]; softmax in fp32; causal mask (key index > query index), sliding window
 // (query - key > window), ALiBi (score -= slope * (query - key)), grouped-query heads.
 //
-//   * head_dim 64 and 128 at 16-byte aligned addresses: attention_mma_kernel, one kernel for a decode step
-//     and a prefill block, on the tensor cores; see there.
+//   * head_dim 64 and 128 at 16-byte aligned addresses: tensor cores, attention_mma_kernel below for a decode
+//     step (up to 64 query rows per K/V head) and attention_tc.cu for a prefill block.
 //   * Other head_dims and addresses: attention_decode_kernel, a streaming pass per query row on the CUDA
 //     cores.  A lane takes a key for the scores (the query rows in shared memory), then the lanes
 //     switch to a slice of D each and walk the step's 32 value rows, eight row loads in flight at a
@@ -25,22 +25,6 @@ namespace {
 
 constexpr int kAttnWarps = 4;
 constexpr int kAttnMaxD = 128;
-
-struct AttnParams {
-    const __half* Q;
-    const __half* K;
-    const __half* V;
-    __half* O;
-    float* LSE;           // may be null
-    float* part;          // [rows][chunks][D + 2] when chunks > 1
-    const float* slopes;  // device copy of the ALiBi slopes, or null
-    int B, Hq, Hkv, Sq, Sk, D;
-    int group;            // query heads a CTA handles together (attention_group)
-    int chunks, keys_per_chunk;
-    float scale;
-    int causal, window;
-    int vec;              // Q, K and V are 16-byte aligned
-};
 
 __device__ __forceinline__ float warp_max(float v) {
     for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -211,9 +195,9 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_decode_kernel(const
 // ---------------------------------------------------------------------------------------
 // Matrix kernel, head_dim 64 and 128: scores and outputs on the tensor cores (mma.sync m16n8k16).
 //
-// The rows of a tile are the (query, head) pairs that share a K/V head, head fastest: the eight or
-// fewer heads of a grouped-query decode step are one 16-row tile and read the cache once; a prefill
-// block is cut into 64-row tiles.  K and V arrive in steps of 64 keys through a ring in shared memory
+// For decode steps and a few query rows: up to 64 (query, head) pairs that share a K/V head, head fastest,
+// are one tile, so the heads of a grouped-query decode step read the cache once (more rows take
+// attention_tc.cu).  K and V arrive in steps of 64 keys through a ring in shared memory
 // (cp.async, 16-byte pieces, piece index XORed with the row so that ldmatrix is conflict-free).
 //   SPLIT_KEYS (16 rows or fewer): all four warps hold the same rows and take 16 keys of a step each,
 //     with softmax states of their own that are merged at the end.
@@ -221,10 +205,12 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_decode_kernel(const
 // The scores' products are exact and summed in fp32.  The probabilities stay fp32: for the product with V
 // each is split into an fp16 value and the fp16 remainder (22 bits of it), which costs a third
 // more MMAs and keeps the result as close to a 64-bit one as fp32 multiply-adds had it.
-// A decode step is bound by the cache stream, a prefill block by the tensor pipe and the chain of a
-// step (scores, maximum, exponentials, outputs); two CTAs per SM overlap their chains.
+// A decode step is bound by the cache stream; two CTAs per SM overlap the chains of their steps (scores,
+// maximum, exponentials, outputs).  Eight sequences, 32 heads on 8 K/V heads x 4096 keys: 31 us (4.3 TB/s),
+// 85 us as a streaming pass of CUDA-core dot products per two heads.
 // ---------------------------------------------------------------------------------------
 constexpr int kStepKeys = 64;
+constexpr int kMmaRows = 64;           // rows (query, head) of a K/V head up to which this kernel is used
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
@@ -241,6 +227,12 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4],
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// exp(x), results below the normal range as zero.
+__device__ __forceinline__ float exp_of(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f));
+    return y;
 }
 __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
     const __half2 h = __floats2half2_rn(a, b);
@@ -270,8 +262,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, tq = lane & 3;
     const int G = p.Hq / p.Hkv, R = p.Sq * G;
     const int heads = p.B * p.Hkv, bk = blockIdx.x % heads;
-    const int row_tiles = (R + kTileRows - 1) / kTileRows;
-    const int tile0 = (row_tiles - 1 - static_cast<int>(blockIdx.x / heads)) * kTileRows;   // long causal tiles first
+    constexpr int tile0 = 0;
     const int b = bk / p.Hkv, hkv = bk % p.Hkv;
     const int chunk = blockIdx.y;
     const __half* Kh = p.K + static_cast<size_t>(bk) * p.Sk * D;
@@ -357,19 +348,34 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const
                 mma_16816(s[n + 1], qf[k], bf[2], bf[3]);
             }
         const bool masked = jb + kKeys > k1 || (p.causal && jb + kKeys - 1 > i_min) || p.window > 0 || p.slopes != nullptr;
+        // straight-line selects: a branch per element costs more than the arithmetic; a NaN score counts as masked
         float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
         for (int n = 0; n < kNT; ++n)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                float sc = s[n][e] * p.scale;
-                if (masked) {
-                    const int j = jb + n * 8 + 2 * tq + (e & 1), i = qi[e >> 1];
-                    if (j >= k1 || (p.causal && j > i) || (p.window > 0 && i - j > p.window)) sc = -INFINITY;
-                    if (p.slopes) sc -= slope[e >> 1] * static_cast<float>(i - j);
+            for (int e = 0; e < 4; ++e) s[n][e] *= p.scale;
+        if (p.slopes) {
+#pragma unroll
+            for (int n = 0; n < kNT; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s[n][e] -= slope[e >> 1] * static_cast<float>(qi[e >> 1] - (jb + n * 8 + 2 * tq + (e & 1)));
+        }
+        if (masked) {
+#pragma unroll
+            for (int n = 0; n < kNT; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int i = qi[e >> 1], j = n * 8 + 2 * tq + (e & 1);
+                    const int hi = (p.causal ? min(k1, i + 1) : k1) - jb, lo = p.window > 0 ? i - p.window - jb : 0;
+                    s[n][e] = j < hi && j >= lo ? s[n][e] : -INFINITY;
                 }
-                s[n][e] = sc;
-                mx[e >> 1] = fmaxf(mx[e >> 1], sc);
+        }
+#pragma unroll
+        for (int n = 0; n < kNT; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                s[n][e] = fmaxf(s[n][e], -INFINITY);
+                mx[e >> 1] = fmaxf(mx[e >> 1], s[n][e]);
             }
         float ref[2];
 #pragma unroll
@@ -378,7 +384,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const
             mx[e] = fmaxf(mx[e], __shfl_xor_sync(0xffffffffu, mx[e], 2));
             const float m_new = fmaxf(m[e], mx[e]);
             ref[e] = m_new > -INFINITY ? m_new : 0.f;      // a row that sees no key so far keeps zero sums
-            const float keep = m[e] > -INFINITY ? __expf(m[e] - ref[e]) : 0.f;
+            const float keep = exp_of(m[e] - ref[e]);
             m[e] = m_new;
             l[e] *= keep;
 #pragma unroll
@@ -388,7 +394,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const
         for (int n = 0; n < kNT; ++n)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                s[n][e] = s[n][e] > -INFINITY ? __expf(s[n][e] - ref[e >> 1]) : 0.f;     // now the probability
+                s[n][e] = exp_of(s[n][e] - ref[e >> 1]);       // now the probability
                 l[e >> 1] += s[n][e];
             }
 #pragma unroll
@@ -544,12 +550,13 @@ void attention_chunks(int B, int Hq, int Hkv, int Sq, int Sk, int D, int sm_coun
         *keys_per_chunk = (Sk + c - 1) / c;
         return;
     }
-    // Matrix kernel: the number of chunks whose waves of CTAs (two per SM) take the fewest steps of 64 keys,
-    // a CTA's start and end counted as two steps and the merge launch as three.
+    // Matrix kernels: the number of chunks whose waves of CTAs (two per SM; one of the prefill kernel) take the
+    // fewest key steps, a CTA's start and end counted as two steps and the merge launch as three.
     const long long R = static_cast<long long>(Sq) * (Hq / Hkv);
-    const long long tiles = R <= 16 ? 1 : (R + 63) / 64;
-    const long long ctas = static_cast<long long>(B) * Hkv * tiles, slots = 2LL * sms;
-    const int steps = (Sk + kStepKeys - 1) / kStepKeys;
+    const bool prefill = R > kMmaRows;            // 128-row tiles, one CTA per SM, steps of 128 keys
+    const long long tiles = R <= 16 ? 1 : (prefill ? (R + 127) / 128 : 1);
+    const long long ctas = static_cast<long long>(B) * Hkv * tiles, slots = prefill ? sms : 2LL * sms;
+    const int step_keys = prefill ? 128 : kStepKeys, steps = (Sk + step_keys - 1) / step_keys;
     int best = 1;
     double best_cost = 0.0;
     for (int c = 1; c <= steps && c <= kMergeMaxChunks; ++c) {
@@ -558,16 +565,17 @@ void attention_chunks(int B, int Hq, int Hkv, int Sq, int Sk, int D, int sm_coun
         if (c == 1 || cost < best_cost) { best = c; best_cost = cost; }
     }
     const int per = (steps + best - 1) / best;
-    *keys_per_chunk = per * kStepKeys;
+    *keys_per_chunk = per * step_keys;
     *chunks = (steps + per - 1) / per;
 }
 
 template <int D>
 cudaError_t launch_matrix(const AttnParams& p, cudaStream_t stream) {
     const long long R = static_cast<long long>(p.Sq) * (p.Hq / p.Hkv);
+    if (R > kMmaRows) return launch_attention_prefill(p, stream);
     const bool split = R <= 16;
-    const long long x = static_cast<long long>(p.B) * p.Hkv * (split ? 1 : (R + 63) / 64);
-    if (R > 0x7fffffffLL || x > 0x7fffffffLL) return cudaErrorNotSupported;
+    const long long x = static_cast<long long>(p.B) * p.Hkv;
+    if (x > 0x7fffffffLL) return cudaErrorNotSupported;
     const dim3 grid(static_cast<unsigned>(x), static_cast<unsigned>(p.chunks));
     auto* kernel = split ? attention_mma_kernel<D, true> : attention_mma_kernel<D, false>;
     kernel<<<grid, kAttnWarps * 32, MmaShape<D>::kSmem, stream>>>(p);
@@ -588,7 +596,7 @@ cudaError_t init_attention_kernels() {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_mma_kernel<128, false>, a, MmaShape<128>::kSmem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_mma_kernel<64, true>, a, MmaShape<64>::kSmem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_mma_kernel<64, false>, a, MmaShape<64>::kSmem);
-    return e;
+    return e == cudaSuccess ? init_attention_prefill_kernels() : e;
 }
 
 size_t attention_scratch_floats(int B, int Hq, int Hkv, int Sq, int Sk, int D, int sm_count, int* chunks_out) {
@@ -602,7 +610,7 @@ size_t attention_scratch_floats(int B, int Hq, int Hkv, int Sq, int Sk, int D, i
 cudaError_t launch_attention_forward(const void* Q, const void* K, const void* V, void* O, float* LSE,
                                      float* scratch, const float* slopes_dev, int B, int Hq, int Hkv, int Sq,
                                      int Sk, int D, float scale, bool causal, int window, int sm_count,
-                                     cudaStream_t stream, int* launches) {
+                                     cudaStream_t stream, int* launches, uint32_t* err_word) {
     if (D <= 0 || D > kAttnMaxD) return cudaErrorNotSupported;
     const long long rows_ll = static_cast<long long>(B) * Hq * Sq;
     if (rows_ll <= 0 || rows_ll > 0x7fffffffLL) return cudaErrorNotSupported;
@@ -617,8 +625,9 @@ cudaError_t launch_attention_forward(const void* Q, const void* K, const void* V
     p.scale = scale; p.causal = causal ? 1 : 0; p.window = window;
     const uintptr_t at = reinterpret_cast<uintptr_t>(Q) | reinterpret_cast<uintptr_t>(K) | reinterpret_cast<uintptr_t>(V);
     p.vec = (at & 15u) == 0;
+    p.err = err_word;
     cudaError_t e = cudaErrorNotSupported;
-    if (matrix_head_dim(D) && p.vec && (reinterpret_cast<uintptr_t>(O) & 3u) == 0)
+    if (matrix_head_dim(D) && p.vec && (reinterpret_cast<uintptr_t>(O) & 15u) == 0)
         e = D == 128 ? launch_matrix<128>(p, stream) : launch_matrix<64>(p, stream);
     if (e == cudaErrorNotSupported)
         e = launch_vector(dim3(static_cast<unsigned>(rows / p.group), static_cast<unsigned>(p.chunks)), stream, p);

@@ -2,6 +2,7 @@
 // Everything here works on raw device pointers; handle validation happens above.
 #pragma once
 
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -257,13 +258,32 @@ cudaError_t launch_gemm_f16_tc(const void* A, const void* B, void* C, int M, int
 
 // --- attention forward (attention.cu); fp16 data, fp32 softmax ----------------------------
 cudaError_t init_attention_kernels();
+struct AttnParams {
+    const __half* Q;
+    const __half* K;
+    const __half* V;
+    __half* O;
+    float* LSE;           // may be null
+    float* part;          // [rows][chunks][D + 2] when chunks > 1
+    const float* slopes;  // device copy of the ALiBi slopes, or null
+    int B, Hq, Hkv, Sq, Sk, D;
+    int group;            // query heads a CTA handles together (attention_group)
+    int chunks, keys_per_chunk;
+    float scale;
+    int causal, window;
+    int vec;              // Q, K and V are 16-byte aligned
+    uint32_t* err;        // device-visible word for an error bit, or null
+};
+// The tcgen05 kernel for prefill blocks (attention_tc.cu): head_dim 64 or 128, all addresses 16-byte aligned.
+cudaError_t init_attention_prefill_kernels();
+cudaError_t launch_attention_prefill(const AttnParams& p, cudaStream_t stream);
 // Floats of scratch the launch needs, and into how many key chunks it will cut a row (1 = no scratch).
 size_t attention_scratch_floats(int B, int Hq, int Hkv, int Sq, int Sk, int D, int sm_count, int* chunks_out);
 // cudaErrorNotSupported: head_dim above 128.  slopes_dev: ALiBi slopes on the device, or null.
 cudaError_t launch_attention_forward(const void* Q, const void* K, const void* V, void* O, float* LSE,
                                      float* scratch, const float* slopes_dev, int B, int Hq, int Hkv, int Sq,
                                      int Sk, int D, float scale, bool causal, int window, int sm_count,
-                                     cudaStream_t stream, int* launches);
+                                     cudaStream_t stream, int* launches, uint32_t* err_word);
 
 // --- collectives over NCCL (dist_nccl.cpp); return 0, or -1 bad arguments, -2 NCCL not found,
 // -3 rendezvous failed, -4 NCCL / CUDA error ----------------------------------------------------

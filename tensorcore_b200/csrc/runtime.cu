@@ -1592,7 +1592,7 @@ extern "C" tc_status_t tc_attention_forward(tc_context* ctx, const tc_attention_
         return tcb::launch_attention_forward(Q->dptr, K->dptr, V->dptr, O->dptr,
                                              LSE ? static_cast<float*>(LSE->dptr) : nullptr,
                                              chunks > 1 ? ctx->attn_scratch : nullptr, slopes_dev, B, Hq, Hkv, Sq, Sk,
-                                             D, scale, d->causal, d->window_size, ctx->sm_count, s0, &launched);
+                                             D, scale, d->causal, d->window_size, ctx->sm_count, s0, &launched, ctx->err_dev);
     });
     if (launched > 1) g_launches.fetch_add(static_cast<uint64_t>(launched - 1));
     return st;
@@ -1635,7 +1635,7 @@ extern "C" tc_status_t tcx_raw_attention_forward(tc_context* ctx, const tc_atten
     const cudaError_t e = tcb::launch_attention_forward(Q, K, V, O, static_cast<float*>(LSE),
                                                         chunks > 1 ? ctx->attn_scratch : nullptr, nullptr, d->batch,
                                                         d->heads, Hkv, d->seq_q, d->seq_kv, d->head_dim, scale, d->causal,
-                                                        d->window_size, ctx->sm_count, st, &launched);
+                                                        d->window_size, ctx->sm_count, st, &launched, ctx->err_dev);
     g_launches.fetch_add(static_cast<uint64_t>(launched));
     t_last_kernel = "attention_decode_sm100";
     return record("tcx_raw_attention_forward", from_cuda(e, TC_ERR_DISPATCH));
