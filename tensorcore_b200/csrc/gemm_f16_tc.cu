@@ -3,10 +3,13 @@
 // dequantised weights use (include/tensorcore/gemm.h:16-58; arithmetic lib/ops/gemm_cpu.cpp:544-568,
 // which adds the products in k order; here the tensor core's order, same fp32 accumulation).
 //
-//   * One CTA per SM walks the 128 x BN tiles of C (BN = 128 or 256), each over the whole K, 64 at a
-//     time, through a ring of four stages (16 KB of A + BN * 128 bytes of B each) that keeps running
-//     across tiles; two accumulators in tensor memory, so that one tile is read out and stored while
-//     the next one's MMAs run.
+//   * One CTA per SM walks the tiles of C (128 or 256 rows x 64 to 256 columns), each over the whole K, 64
+//     at a time, through a ring of stages that keeps running across tiles; two sets of accumulators in
+//     tensor memory where they fit, so that one tile is read out and stored while the next one's MMAs
+//     run.  What bounds it is shared-memory bandwidth: a K step of a 256 x 160 tile writes 52 KB and its
+//     MMAs read 72 KB (B once per 128 rows), 970 clocks at 128 bytes each against 640 of tensor work;
+//     1030 measured.  512 x 11008 x 4096: 128-row tiles 47 us, 256-row tiles 41 us; 4096^3 110 and
+//     100 us.  With few rows of A a K step takes 590 clocks of waits and issue, whatever the tile.
 //   * Operands reach shared memory by tiled TMA copies of 128-byte rows written with the 128-byte
 //     swizzle, the layout the MMA's shared-memory descriptors read directly:
 //       - A ([M][K]) and a transposed B ([N][K]) are K-major: a box of 64 k x 128 (or BN) rows;
@@ -37,8 +40,7 @@ using namespace sm100;
 
 constexpr int kBM = 128, kBK = 64;
 constexpr int kMaxStages = 12;   // the ring is as deep as shared memory allows, up to this
-constexpr int kAStage = kBM * kBK * 2;
-constexpr int kGemmThreads = 6 * 32;          // producer, MMA issuer, four epilogue warps
+constexpr int kGemmThreads = 10 * 32;         // producer, MMA issuer, four epilogue warps per 128 rows of the tile
 constexpr int kGemmBarBytes = 1024;
 constexpr uint32_t kGemmTmemCols = 512;      // two accumulators of up to 256 columns
 constexpr uint32_t kSwizzle128 = 2;           // layout type of the shared-memory descriptor
@@ -47,6 +49,8 @@ struct GemmParams {
     __half* C;
     uint32_t* err;
     int M, N, K, ldc;
+    int mt;            // rows of a tile in units of 128: 1 or 2
+    int accs;          // accumulator sets: 2 where tensor memory has room
     int bn;            // columns of a tile: multiple of 16 (of 64 when B is MN-major), at most 256
     float alpha, beta;
     int b_kmajor;      // B was given transposed ([N][K])
@@ -90,7 +94,7 @@ __device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, volatil
 
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap bmap) {
-    const int BN = p.bn;
+    const int BN = p.bn, MT = p.mt, tile_rows = kBM * MT;
     const int kBStage = BN * kBK * 2;
     extern __shared__ __align__(1024) uint8_t smem[];
     GemmBars* bars = reinterpret_cast<GemmBars*>(smem);
@@ -106,12 +110,12 @@ gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap,
     const int ksteps = (p.K + kBK - 1) / kBK;
     // Tiles of C, numbered column-block-major (the CTAs running at the same time share a block of B's
     // columns and walk down A); CTA c takes tiles c, c + gridDim.x, ...
-    const int tiles_m = (p.M + kBM - 1) / kBM, tiles_n = (p.N + BN - 1) / BN;
+    const int tiles_m = (p.M + tile_rows - 1) / tile_rows, tiles_n = (p.N + BN - 1) / BN;
     const int n_tiles = tiles_m * tiles_n;
 
     if (tid == 0) {
         for (int i = 0; i < stages; ++i) { bar_init(&bars->full[i], 1); bar_init(&bars->empty[i], 1); }
-        for (int i = 0; i < 2; ++i) { bar_init(&bars->acc_full[i], 1); bar_init(&bars->acc_empty[i], 4); }
+        for (int i = 0; i < 2; ++i) { bar_init(&bars->acc_full[i], 1); bar_init(&bars->acc_empty[i], 4 * p.mt); }
         bar_init(&bars->drain, 1);
         bars->abort_flag = 0;
         fence_barrier_init();
@@ -129,14 +133,14 @@ gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap,
         int issued = 0, s = 0;
         uint32_t par = 0;
         for (int t = blockIdx.x; t < n_tiles && !failed; t += gridDim.x) {
-            const int m0 = (t % tiles_m) * kBM, n0 = (t / tiles_m) * BN;
+            const int m0 = (t % tiles_m) * tile_rows, n0 = (t / tiles_m) * BN;
             for (int ks = 0; ks < ksteps; ++ks) {
                 if (!wait_all(&bars->empty[s], par ^ 1u, abort_flag)) { failed = true; break; }
                 if (elect_one()) {
                     bar_expect_tx(&bars->full[s], p.a_tx + kBStage);
-                    if (p.a_mnmajor) {       // [K][M]: two boxes of 64 m x 64 k, like B as given
-                        tensor_load_2d(a_ring + s * a_stage, &amap, m0, ks * kBK, &bars->full[s]);
-                        tensor_load_2d(a_ring + s * a_stage + 8192, &amap, m0 + 64, ks * kBK, &bars->full[s]);
+                    if (p.a_mnmajor) {       // [K][M]: boxes of 64 m x 64 k, like B as given
+                        for (int c = 0; c < 2 * MT; ++c)
+                            tensor_load_2d(a_ring + s * a_stage + c * 8192, &amap, m0 + 64 * c, ks * kBK, &bars->full[s]);
                     } else {
                         tensor_load_2d(a_ring + s * a_stage, &amap, ks * kBK, m0, &bars->full[s]);
                     }
@@ -166,14 +170,14 @@ gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap,
         const uint64_t a_form = p.a_mnmajor ? smem_desc(0, 8192u, 1024u, kSwizzle128) : smem_desc(0, 16u, 1024u, kSwizzle128);
         const uint64_t b_form = p.b_kmajor ? smem_desc(0, 16u, 1024u, kSwizzle128) : smem_desc(0, 8192u, 1024u, kSwizzle128);
         const uint32_t a_step = p.a_mnmajor ? 128u : 2u, b_step = p.b_kmajor ? 2u : 128u;
-        int it = 0, s = 0;
+        int s = 0;
         uint32_t par = 0;
-        for (int t = blockIdx.x; t < n_tiles && !failed; t += gridDim.x, ++it) {
-            const int acc = it & 1;
-            // the accumulator's previous tile (two tiles ago) has been read out
-            if (!wait_all(&bars->acc_empty[acc], (static_cast<uint32_t>(it >> 1) & 1u) ^ 1u, abort_flag)) { failed = true; break; }
+        uint32_t acc_par = 0;
+        for (int t = blockIdx.x, acc = 0; t < n_tiles && !failed; t += gridDim.x) {
+            // the accumulator's previous tile has been read out
+            if (!wait_all(&bars->acc_empty[acc], acc_par ^ 1u, abort_flag)) { failed = true; break; }
             tc_fence_after_sync();
-            const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
+            const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * MT * BN);
             for (int ks = 0; ks < ksteps; ++ks) {
                 if (!wait_all(&bars->full[s], par, abort_flag)) { failed = true; break; }
                 tc_fence_after_sync();
@@ -181,15 +185,20 @@ gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap,
                 const uint64_t bdesc = b_form | ((s_u32(b_ring + s * kBStage) >> 4) & 0x3FFFu);
                 if (elect_one()) {
 #pragma unroll
-                    for (int j = 0; j < kBK / 16; ++j)
-                        mma_f16_ss(d_tmem, adesc + static_cast<uint64_t>(j * a_step), bdesc + static_cast<uint64_t>(j * b_step), idesc,
-                                   (ks > 0 || j > 0) ? 1u : 0u);
+                    for (int j = 0; j < kBK / 16; ++j) {
+                        const uint64_t bd = bdesc + static_cast<uint64_t>(j * b_step);
+                        const uint32_t add = (ks > 0 || j > 0) ? 1u : 0u;
+                        mma_f16_ss(d_tmem, adesc + static_cast<uint64_t>(j * a_step), bd, idesc, add);
+                        // the second 128 rows: 16 KB further on in either layout
+                        if (MT == 2) mma_f16_ss(d_tmem + BN, adesc + static_cast<uint64_t>(1024u + j * a_step), bd, idesc, add);
+                    }
                     mma_commit(&bars->empty[s]);
                     if (ks + 1 == ksteps) mma_commit(&bars->acc_full[acc]);
                 }
                 __syncwarp();
                 if (++s == stages) { s = 0; par ^= 1u; }
             }
+            if (++acc == p.accs) { acc = 0; acc_par ^= 1u; }
         }
         if (failed || *abort_flag) {
             // every MMA issued so far has completed before the tensor memory is released
@@ -204,15 +213,15 @@ gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap,
     }
     __syncwarp();
 
-    if (warp >= 2) {
+    if (warp >= 2 && warp < 2 + 4 * MT) {
         const int quad = warp & 3;                          // the TMEM lanes this warp may read
+        const int half = warp >= 6 ? 1 : 0;                 // which 128 rows of the tile
         const bool vec = (p.ldc % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15u) == 0) && p.beta == 0.f;
-        int it = 0;
-        for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, ++it) {
-            const int m0 = (t % tiles_m) * kBM, n0 = (t / tiles_m) * BN;
-            const int acc = it & 1;
+        uint32_t acc_par = 0;
+        for (int t = blockIdx.x, acc = 0; t < n_tiles; t += gridDim.x) {
+            const int m0 = (t % tiles_m) * tile_rows + half * kBM, n0 = (t / tiles_m) * BN;
             const int row = m0 + quad * 32 + lane;
-            const bool ok = bar_wait_warp(&bars->acc_full[acc], static_cast<uint32_t>(it >> 1) & 1u, abort_flag) &&
+            const bool ok = bar_wait_warp(&bars->acc_full[acc], acc_par, abort_flag) &&
                             __all_sync(0xffffffffu, !*abort_flag);
             if (!ok) {
                 if (lane == 0 && !*abort_flag) {
@@ -222,7 +231,7 @@ gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap,
                 break;
             }
             tc_fence_after_sync();
-            const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(acc * BN);
+            const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>((acc * MT + half) * BN);
 #pragma unroll 1
             for (int c0 = 0; c0 < BN; c0 += 16) {
                 uint32_t v[16];
@@ -266,6 +275,7 @@ gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap,
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) bar_arrive(&bars->acc_empty[acc]);
+            if (++acc == p.accs) { acc = 0; acc_par ^= 1u; }
         }
     }
     tc_fence_before_sync();
@@ -309,9 +319,10 @@ cudaError_t launch_tile(const GemmParams& p, const void* A, const void* B, int l
     // A decode batch or a short prefill block has far fewer than 128 rows: copying only those (2 KB
     // instead of 16 KB a stage at 16 rows) leaves the SM's copy bandwidth to B, which is what such a
     // call streams.
-    const int a_rows = (!transpose_a && p.M < kBM) ? ((p.M + 7) & ~7) : kBM;
+    const int tile_rows = kBM * p.mt;
+    const int a_rows = (!transpose_a && p.M < tile_rows) ? ((p.M + 7) & ~7) : tile_rows;
     GemmParams q = p;
-    q.a_tx = transpose_a ? static_cast<uint32_t>(kAStage) : static_cast<uint32_t>(a_rows) * kBK * 2u;
+    q.a_tx = static_cast<uint32_t>(a_rows) * kBK * 2u;
     q.a_stage = q.a_tx;     // a multiple of 1024: a_rows is a multiple of 8 rows of 128 bytes
     const int stage_bytes = static_cast<int>(q.a_stage) + BN * kBK * 2;
     q.stages = (env.smem_optin - kGemmBarBytes) / stage_bytes;
@@ -326,10 +337,10 @@ cudaError_t launch_tile(const GemmParams& p, const void* A, const void* B, int l
         ? encode_rows_sw128(&bmap, B, static_cast<uint64_t>(p.N), static_cast<uint64_t>(p.K), static_cast<uint64_t>(ldb), BN)
         : encode_rows_sw128(&bmap, B, static_cast<uint64_t>(p.K), static_cast<uint64_t>(p.N), static_cast<uint64_t>(ldb), kBK);
     if (!okb) return cudaErrorNotSupported;
-    const long tiles = static_cast<long>((p.N + BN - 1) / BN) * ((p.M + kBM - 1) / kBM);
+    const long tiles = static_cast<long>((p.N + BN - 1) / BN) * ((p.M + tile_rows - 1) / tile_rows);
     const long sms = env.sm_count > 0 ? env.sm_count : 148;
     const dim3 grid(static_cast<unsigned>(tiles < sms ? tiles : sms));     // one CTA per SM walks the tiles
-    gemm_f16_tc_kernel<<<grid, kGemmThreads, smem, stream>>>(q, amap, bmap);
+    gemm_f16_tc_kernel<<<grid, (2 + 4 * p.mt) * 32, smem, stream>>>(q, amap, bmap);
     return cudaGetLastError();
 }
 
@@ -354,20 +365,27 @@ cudaError_t launch_gemm_f16_tc(const void* A, const void* B, void* C, int M, int
     p.b_kmajor = transpose_b ? 1 : 0;
     p.bf16 = bf16 ? 1 : 0;
     p.a_mnmajor = transpose_a ? 1 : 0;
-    // Tile width: the one whose rounds of tiles over the SMs take least, by a model of a 64-wide K step: four
-    // MMAs of N / 2 clocks each, but at least 54 (the measured floor of an MMA with both operands in shared
-    // memory), and the stage's bytes at 45 per clock; the last tile's read-out is not hidden.  512 x 11008 x
-    // 4096 takes 160-wide tiles (two rounds) instead of two rounds of 256-wide ones of which the second
-    // is nearly empty.  B as given is laid out in pieces of 64 columns.
+    // Tile: the one whose rounds over the SMs take least, by a model of a 64-wide K step: four MMAs of N / 2 clocks
+    // per 128 rows, each at least 54 (the measured floor with both operands in shared memory), or the
+    // shared-memory traffic - the stage's bytes written once, A read once and B once per 128 rows - at 110
+    // bytes per clock (measured between 105 and 123 over widths of 64 to 256).  256 rows need less
+    // traffic per flop; their two accumulators leave room for a second set only up to 128 columns, so a
+    // tile's read-out is not hidden beyond that.  B as given is laid out in pieces of 64 columns.
     const long sms = env.sm_count > 0 ? env.sm_count : 148;
-    const long tiles_m = (M + kBM - 1) / kBM, ksteps = (K + kBK - 1) / kBK;
-    const long a_bytes = (transpose_a || M >= kBM ? kBM : ((M + 7) & ~7)) * kBK * 2L;
+    const long ksteps = (K + kBK - 1) / kBK;
     double best = 0.0;
-    for (int bn = 256; bn >= 64; bn -= transpose_b ? 16 : 64) {
-        const long tiles = tiles_m * ((N + bn - 1) / bn);
-        const double mma = 4.0 * (bn > 108 ? bn / 2.0 : 54.0), copy = (a_bytes + bn * kBK * 2L) / 45.0;
-        const double cost = static_cast<double>((tiles + sms - 1) / sms) * ksteps * (mma > copy ? mma : copy) + 1000.0 + 8.0 * bn;
-        if (best == 0.0 || cost < best) { best = cost; p.bn = bn; }
+    for (int mt = 1; mt <= (M > kBM ? 2 : 1); ++mt) {
+        const long rows = kBM * mt, tiles_m = (M + rows - 1) / rows;
+        const long a_bytes = (transpose_a || M >= rows ? rows : ((M + 7) & ~7)) * kBK * 2L;
+        for (int bn = 256; bn >= 64; bn -= transpose_b ? 16 : 64) {
+            const long tiles = tiles_m * ((N + bn - 1) / bn), rounds = (tiles + sms - 1) / sms;
+            const int accs = 2 * mt * bn <= static_cast<int>(kGemmTmemCols) ? 2 : 1;
+            const double mma = 4.0 * mt * (bn > 108 ? bn / 2.0 : 54.0), traffic = (a_bytes + bn * kBK * 2L + mt * (kBM + bn) * kBK * 2L) / 110.0;
+            const double read_out = 1000.0 + 8.0 * bn;
+            const double cost = static_cast<double>(rounds) * (ksteps * (mma > traffic ? mma : traffic) + (accs == 1 ? read_out : 0.0)) +
+                                (accs == 1 ? 0.0 : read_out);
+            if (best == 0.0 || cost < best) { best = cost; p.bn = bn; p.mt = mt; p.accs = accs; }
+        }
     }
     return launch_tile(p, A, B, lda, ldb, transpose_b, env, stream);
 }
