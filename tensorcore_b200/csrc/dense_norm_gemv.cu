@@ -6,9 +6,8 @@
 // once, 2 bytes per weight.
 //
 // Main kernel (dense_norm_gemv_split_kernel): W is cut into tiles of 256 columns (512-byte row
-// segments: a warp copies one, 16 bytes per lane) by a K range chosen so that there are about
-// four tiles per SM - the hardware spreads them evenly, and three CTAs per SM keep 144 KB of
-// copies in flight.  A CTA starts the asynchronous copies of its first stages (cp.async into a
+// segments: a warp copies one, 16 bytes per lane) by a K range chosen so that the tiles fill whole
+// waves of three CTAs per SM, which keep 144 KB of copies in flight.  A CTA starts the asynchronous copies of its first stages (cp.async into a
 // four-stage ring in shared memory; a thread reads back exactly the pieces it copied, so the
 // ring needs no barrier), works out the row statistics meanwhile (K values from L2; cheaper than
 // a separate kernel and an fp16 round trip), normalises its K range into shared memory, streams
@@ -186,11 +185,48 @@ __global__ void __launch_bounds__(kDThreads) dense_norm_gemv_kernel(const DenseP
 }
 
 // Statistics of row m for the split kernel: mean (LayerNorm) and 1/std or 1/rms, the reference's
-// arithmetic (double-precision sums, lib/ops/training_cpu.cpp:799-935).
+// arithmetic (double-precision sums, lib/ops/training_cpu.cpp:799-935).  Every tile pays for this before
+// its first product, so the row comes in 16-byte pieces where it can (all loads of a thread in flight;
+// up to 8192 elements are kept in registers between the two passes of a LayerNorm).
 __device__ void row_stats(const DenseParams& p, int m, double* scratch, float& mean, float& rstd) {
+    constexpr int kKeep = 4;
     const int tid = threadIdx.x, K = p.K;
     const __half* xr = p.X + static_cast<size_t>(m) * K;
     mean = 0.f;
+    if (K % 8 == 0 && K <= kKeep * 8 * kDThreads && (reinterpret_cast<uintptr_t>(p.X) & 15u) == 0) {
+        uint4 v[kKeep];
+#pragma unroll
+        for (int i = 0; i < kKeep; ++i) {
+            v[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (tid + kDThreads * i < K / 8) v[i] = __ldg(reinterpret_cast<const uint4*>(xr) + tid + kDThreads * i);
+        }
+        auto pair = [&](int i, int t) { return __half22float2(reinterpret_cast<const __half2*>(&v[i])[t]); };
+        if (p.beta != nullptr) {
+            double s = 0.0;
+#pragma unroll
+            for (int i = 0; i < kKeep; ++i)
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    const float2 f = pair(i, t);
+                    s += static_cast<double>(f.x) + static_cast<double>(f.y);
+                }
+            mean = static_cast<float>(dblock_sum(s, scratch) / K);
+        }
+        double ss = 0.0;
+#pragma unroll
+        for (int i = 0; i < kKeep; ++i) {
+            if (tid + kDThreads * i >= K / 8) break;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const float2 f = pair(i, t);
+                const double a = __fsub_rn(f.x, mean), b = __fsub_rn(f.y, mean);
+                ss += a * a;
+                ss += b * b;
+            }
+        }
+        rstd = 1.0f / sqrtf(static_cast<float>(dblock_sum(ss, scratch) / K) + p.eps);
+        return;
+    }
     if (p.beta != nullptr) {
         double s = 0.0;
         for (int k = tid; k < K; k += kDThreads) s += static_cast<double>(__half2float(xr[k]));
@@ -431,14 +467,18 @@ cudaError_t launch_dense_split(const SplitParams& sp, int strips, int smem_optin
 
 // Tiles of the split kernel for one launch of up to kDMaxMB rows.
 void dense_split_shape(int N, int K, int sm_count, int* strips, int* chunks, int* kc) {
-    // about four tiles per SM (three CTAs are resident per SM; more, shorter tiles measured slower:
-    // every tile pays for the row statistics and for a fence before its ticket), K ranges of whole
-    // ring stages
+    // The number of K ranges whose waves of tiles take least: three CTAs are resident per SM, and a tile costs
+    // its rows and about 96 rows' time for the row statistics and the fence before its ticket.  4096 x 11008:
+    // ten ranges, one wave of 430 tiles (four tiles per SM before: 602 tiles, a third of a wave left over).
     const int st = (N + kSplitCols - 1) / kSplitCols;
-    int ch = (4 * sm_count + st - 1) / st;
     const int most = (K + 2 * kStageRows - 1) / (2 * kStageRows);
-    if (ch > most) ch = most;
-    if (ch < 1) ch = 1;
+    int ch = 1;
+    double best = 0.0;
+    for (int c = 1; c <= most && c <= 256; ++c) {
+        const double waves = static_cast<double>((static_cast<long long>(st) * c + 3 * sm_count - 1) / (3 * sm_count));
+        const double cost = waves * (static_cast<double>(K) / c + 96.0);
+        if (best == 0.0 || cost < best) { best = cost; ch = c; }
+    }
     int rows = (K + ch - 1) / ch;
     rows = (rows + kStageRows - 1) / kStageRows * kStageRows;
     *strips = st;
