@@ -15,7 +15,8 @@
 // units are dealt to 16 warps, and the partial sums of a row are added in block order: deterministic.
 // HBM-bound in principle; what it reaches is set by how many units a warp gets (one to three).
 // 5003 x 4128 Q8_0, three fp32 rows: 283 us before (a warp per row, byte loads, activations from L1 for
-// every weight).
+// every weight); 14.8 us before a unit's blocks were fetched while the activations are staged and the unit
+// before it is computed, 14.1 us with that.
 #include "gemv_common.cuh"
 
 namespace tcb {
@@ -89,6 +90,26 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_q_rows_kernel(const Rows
     float* part = reinterpret_cast<float*>(smem + p.off_part);  // [chunks][max_rows][MB]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     pdl_launch_dependents();
+    const int r0 = static_cast<int>(static_cast<long long>(p.N) * blockIdx.x / gridDim.x);
+    const int r1 = static_cast<int>(static_cast<long long>(p.N) * (blockIdx.x + 1) / gridDim.x);
+    const int groups = (r1 - r0 + kGroupRows - 1) / kGroupRows, units = groups * p.chunks;
+    const size_t row_bytes = static_cast<size_t>(p.nb) * kBlock;
+    // Blocks of this warp's next unit, on their way while the activations are staged or a unit is computed.
+    RowBlock<FMT> blk[kGroupRows];
+    int off[kGroupRows];
+    auto fetch = [&](int u) {
+        const int g = u % groups, c = u / groups, b = c * p.cb + lane;
+        const bool active = u < units && lane < p.cb && b < p.nb;
+#pragma unroll
+        for (int r = 0; r < kGroupRows; ++r) {
+            int row = r0 + g * kGroupRows + r;
+            if (row >= r1) row = r1 - 1;                        // its result is not stored
+            const uint8_t* at = p.W + static_cast<size_t>(row) * row_bytes + static_cast<size_t>(active ? b : 0) * kBlock;
+            off[r] = static_cast<int>(reinterpret_cast<uintptr_t>(at) & 7u);
+            blk[r].load(at, active);
+        }
+    };
+    fetch(warp);
     pdl_wait();
 
     auto load4 = [&](const void* src, size_t at) {
@@ -131,25 +152,11 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_q_rows_kernel(const Rows
     }
     __syncthreads();
 
-    const int r0 = static_cast<int>(static_cast<long long>(p.N) * blockIdx.x / gridDim.x);
-    const int r1 = static_cast<int>(static_cast<long long>(p.N) * (blockIdx.x + 1) / gridDim.x);
-    const int groups = (r1 - r0 + kGroupRows - 1) / kGroupRows;
-    const size_t row_bytes = static_cast<size_t>(p.nb) * kBlock;
-    for (int u = warp; u < groups * p.chunks; u += kRowsWarps) {
+    for (int u = warp; u < units; u += kRowsWarps) {
         const int g = u % groups, c = u / groups;
         const int b = c * p.cb + lane;
         const bool active = lane < p.cb && b < p.nb;
         const int bx = active ? b : 0;
-        RowBlock<FMT> blk[kGroupRows];
-        int off[kGroupRows];
-#pragma unroll
-        for (int r = 0; r < kGroupRows; ++r) {
-            int row = r0 + g * kGroupRows + r;
-            if (row >= r1) row = r1 - 1;                        // its result is not stored
-            const uint8_t* at = p.W + static_cast<size_t>(row) * row_bytes + static_cast<size_t>(bx) * kBlock;
-            off[r] = static_cast<int>(reinterpret_cast<uintptr_t>(at) & 7u);
-            blk[r].load(at, active);
-        }
         uint32_t q[kGroupRows][RowBlock<FMT>::kQ];
         float d[kGroupRows], acc[kGroupRows][MB];
 #pragma unroll
@@ -158,6 +165,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_q_rows_kernel(const Rows
 #pragma unroll
             for (int m = 0; m < MB; ++m) acc[r][m] = 0.f;
         }
+        if (u + kRowsWarps < units) fetch(u + kRowsWarps);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             float4 x[MB];
