@@ -399,10 +399,28 @@ void teardown_device(tc_context* ctx) {
     ctx->err_dev = nullptr;
 }
 
-uint64_t fnv1a(uint64_t h, const void* data, size_t n) {
+// Hash of n bytes, eight at a time (each step is a bijection of the state; the shift brings high bits down).
+uint64_t hash_bytes(uint64_t h, const void* data, size_t n) {
     const uint8_t* p = static_cast<const uint8_t*>(data);
-    for (size_t i = 0; i < n; ++i) { h ^= p[i]; h *= 1099511628211ull; }
+    for (; n > 0;) {
+        uint64_t w = 0;
+        const size_t k = n < 8 ? n : 8;
+        std::memcpy(&w, p, k);
+        h = (h ^ w) * 1099511628211ull;
+        h ^= h >> 32;
+        p += k;
+        n -= k;
+    }
     return h;
+}
+// Signature of a recorded list under a kernel variant.
+uint64_t list_signature(const std::vector<RecordedOp>& list, int variant) {
+    uint64_t h = 1469598103934665603ull;
+    for (const RecordedOp& op : list) {
+        h = hash_bytes(h, &op.kind, sizeof(op.kind));
+        h = hash_bytes(h, &op.a, sizeof(op.a));
+    }
+    return hash_bytes(h, &variant, sizeof(variant));
 }
 
 }  // namespace
@@ -962,7 +980,6 @@ tc_status_t submit_pending(tc_stream* s) {
     if (s->pending.empty()) return TC_OK;
     bind_device(ctx);
     bool any_staged = false;
-    uint64_t sig = 1469598103934665603ull;
     tcb::GemvQArgs scratch_of;          // the stream's scratch for normalised rows, sized for the widest operation
     {
         size_t need = 0, dq = 0;
@@ -989,12 +1006,7 @@ tc_status_t submit_pending(tc_stream* s) {
         tc_buffer* bufs[4] = {op.X, op.W, op.Y, op.gamma};
         for (tc_buffer* b : bufs)
             if (b && staged(b)) any_staged = true;
-        sig = fnv1a(sig, &op.kind, sizeof(op.kind));
-        sig = fnv1a(sig, &op.a, sizeof(op.a));
     }
-    const int variant = g_variant.load();
-    sig = fnv1a(sig, &variant, sizeof(variant));
-
     cudaError_t e = cudaSuccess;
     // Host-visible inputs first (staging copies or prefetch hints), outside any graph.
     for (RecordedOp& op : s->pending) {
@@ -1015,7 +1027,9 @@ tc_status_t submit_pending(tc_stream* s) {
         else (void)cudaGetLastError();
     }
     if (!done && e == cudaSuccess && ctx->graphs && !any_staged && s->pending.size() > 1) {
-        CachedGraph& cg = s->cache[sig];
+        // Only lists that are replayed as graphs are hashed: byte by byte and for every list, the 225 operations of
+        // a 7B token took longer to hash than to record.
+        CachedGraph& cg = s->cache[list_signature(s->pending, g_variant.load())];
         if (cg.exec) {
             e = cudaGraphLaunch(cg.exec, s->s);
             launches = cg.kernels;
