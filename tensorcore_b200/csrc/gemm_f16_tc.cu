@@ -9,7 +9,8 @@
 //     run.  What bounds it is shared-memory bandwidth: a K step of a 256 x 160 tile writes 52 KB and its
 //     MMAs read 72 KB (B once per 128 rows), 970 clocks at 128 bytes each against 640 of tensor work;
 //     1030 measured.  512 x 11008 x 4096: 128-row tiles 47 us, 256-row tiles 41 us; 4096^3 110 and
-//     100 us.  With few rows of A a K step takes 590 clocks of waits and issue, whatever the tile.
+//     100 us.  With few rows of A the waits and the issue of a K step are the bound, so a stage then holds
+//     several.
 //   * Operands reach shared memory by tiled TMA copies of 128-byte rows written with the 128-byte
 //     swizzle, the layout the MMA's shared-memory descriptors read directly:
 //       - A ([M][K]) and a transposed B ([N][K]) are K-major: a box of 64 k x 128 (or BN) rows;
@@ -28,6 +29,7 @@
 // bounded: it sets the error word and lets the kernel end.
 #include "kernels.h"
 #include "sm100_prims.cuh"
+#include "tensor_map.h"
 
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -92,10 +94,13 @@ __device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, volatil
     }
 }
 
+// KS: 64-wide K slices per stage.
+template <int KS>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap bmap) {
     const int BN = p.bn, MT = p.mt, tile_rows = kBM * MT;
-    const int kBStage = BN * kBK * 2;
+    const int kBSlice = BN * kBK * 2, kBStage = KS * kBSlice;
+    const uint32_t a_slice = p.a_stage / KS;
     extern __shared__ __align__(1024) uint8_t smem[];
     GemmBars* bars = reinterpret_cast<GemmBars*>(smem);
     volatile int* abort_flag = &bars->abort_flag;
@@ -107,7 +112,7 @@ gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap,
     // and commit, so that the compiler has their operands as uniform values: under `lane == 0` an MMA took
     // 70 to 112 clocks to issue, as long as the tensor core works on a 256-wide one.
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-    const int ksteps = (p.K + kBK - 1) / kBK;
+    const int ksteps = (p.K + kBK * KS - 1) / (kBK * KS);
     // Tiles of C, numbered column-block-major (the CTAs running at the same time share a block of B's
     // columns and walk down A); CTA c takes tiles c, c + gridDim.x, ...
     const int tiles_m = (p.M + tile_rows - 1) / tile_rows, tiles_n = (p.N + BN - 1) / BN;
@@ -138,17 +143,23 @@ gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap,
                 if (!wait_all(&bars->empty[s], par ^ 1u, abort_flag)) { failed = true; break; }
                 if (elect_one()) {
                     bar_expect_tx(&bars->full[s], p.a_tx + kBStage);
-                    if (p.a_mnmajor) {       // [K][M]: boxes of 64 m x 64 k, like B as given
+                    // K-major operands: a box is KS slices of 64 k of all rows; MN-major ones ([K][M], B as given): boxes
+                    // of 64 m (n) x KS * 64 k
+                    if (p.a_mnmajor) {
                         for (int c = 0; c < 2 * MT; ++c)
-                            tensor_load_2d(a_ring + s * a_stage + c * 8192, &amap, m0 + 64 * c, ks * kBK, &bars->full[s]);
+                            tensor_load_2d(a_ring + s * a_stage + c * KS * 8192, &amap, m0 + 64 * c, ks * KS * kBK, &bars->full[s]);
+                    } else if (KS > 1) {
+                        tensor_load_3d(a_ring + s * a_stage, &amap, 0, m0, ks * KS, &bars->full[s]);
                     } else {
                         tensor_load_2d(a_ring + s * a_stage, &amap, ks * kBK, m0, &bars->full[s]);
                     }
-                    if (p.b_kmajor) {
-                        tensor_load_2d(b_ring + s * kBStage, &bmap, ks * kBK, n0, &bars->full[s]);
-                    } else {
+                    if (!p.b_kmajor) {
                         for (int c = 0; c < BN / 64; ++c)
-                            tensor_load_2d(b_ring + s * kBStage + c * 8192, &bmap, n0 + 64 * c, ks * kBK, &bars->full[s]);
+                            tensor_load_2d(b_ring + s * kBStage + c * KS * 8192, &bmap, n0 + 64 * c, ks * KS * kBK, &bars->full[s]);
+                    } else if (KS > 1) {
+                        tensor_load_3d(b_ring + s * kBStage, &bmap, 0, n0, ks * KS, &bars->full[s]);
+                    } else {
+                        tensor_load_2d(b_ring + s * kBStage, &bmap, ks * kBK, n0, &bars->full[s]);
                     }
                 }
                 __syncwarp();
@@ -167,9 +178,12 @@ gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap,
         const uint32_t idesc = idesc_f16_f32(kBM, BN) | (p.b_kmajor ? 0u : (1u << 16)) | (p.a_mnmajor ? (1u << 15) : 0u) |
                                (p.bf16 ? ((1u << 7) | (1u << 10)) : 0u);
         // descriptor strides, and how far a K step of 16 moves along (in the descriptor's 16-byte units)
-        const uint64_t a_form = p.a_mnmajor ? smem_desc(0, 8192u, 1024u, kSwizzle128) : smem_desc(0, 16u, 1024u, kSwizzle128);
-        const uint64_t b_form = p.b_kmajor ? smem_desc(0, 16u, 1024u, kSwizzle128) : smem_desc(0, 8192u, 1024u, kSwizzle128);
+        const uint64_t a_form = p.a_mnmajor ? smem_desc(0, 8192u * KS, 1024u, kSwizzle128) : smem_desc(0, 16u, 1024u, kSwizzle128);
+        const uint64_t b_form = p.b_kmajor ? smem_desc(0, 16u, 1024u, kSwizzle128) : smem_desc(0, 8192u * KS, 1024u, kSwizzle128);
         const uint32_t a_step = p.a_mnmajor ? 128u : 2u, b_step = p.b_kmajor ? 2u : 128u;
+        // ... and a slice of 64; the second 128 rows lie 128 rows of a slice, or two boxes, further on
+        const uint32_t a_next = p.a_mnmajor ? 512u : a_slice >> 4, b_next = p.b_kmajor ? static_cast<uint32_t>(kBSlice) >> 4 : 512u;
+        const uint32_t a_half = p.a_mnmajor ? 1024u * KS : 1024u;
         int s = 0;
         uint32_t par = 0;
         uint32_t acc_par = 0;
@@ -185,12 +199,15 @@ gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap,
                 const uint64_t bdesc = b_form | ((s_u32(b_ring + s * kBStage) >> 4) & 0x3FFFu);
                 if (elect_one()) {
 #pragma unroll
-                    for (int j = 0; j < kBK / 16; ++j) {
-                        const uint64_t bd = bdesc + static_cast<uint64_t>(j * b_step);
-                        const uint32_t add = (ks > 0 || j > 0) ? 1u : 0u;
-                        mma_f16_ss(d_tmem, adesc + static_cast<uint64_t>(j * a_step), bd, idesc, add);
-                        // the second 128 rows: 16 KB further on in either layout
-                        if (MT == 2) mma_f16_ss(d_tmem + BN, adesc + static_cast<uint64_t>(1024u + j * a_step), bd, idesc, add);
+                    for (int sl = 0; sl < KS; ++sl) {
+#pragma unroll
+                        for (int j = 0; j < kBK / 16; ++j) {
+                            const uint64_t ad = adesc + static_cast<uint64_t>(sl * a_next + j * a_step);
+                            const uint64_t bd = bdesc + static_cast<uint64_t>(sl * b_next + j * b_step);
+                            const uint32_t add = (ks > 0 || sl > 0 || j > 0) ? 1u : 0u;
+                            mma_f16_ss(d_tmem, ad, bd, idesc, add);
+                            if (MT == 2) mma_f16_ss(d_tmem + BN, ad + a_half, bd, idesc, add);
+                        }
                     }
                     mma_commit(&bars->empty[s]);
                     if (ks + 1 == ksteps) mma_commit(&bars->acc_full[acc]);
@@ -323,31 +340,48 @@ cudaError_t launch_tile(const GemmParams& p, const void* A, const void* B, int l
     const int a_rows = (!transpose_a && p.M < tile_rows) ? ((p.M + 7) & ~7) : tile_rows;
     GemmParams q = p;
     q.a_tx = static_cast<uint32_t>(a_rows) * kBK * 2u;
+    // Several 64-wide slices per stage while four stages still fit: a stage's barriers and waits cost more than the
+    // MMAs of a slice when the tile is small (16 x 4096 x 4096: 590 clocks a slice with one per stage, 420
+    // with four; the kernel 27.7 -> 21.1 us).
+    // K-major operands are loaded by slice and need whole slices.
+    int ks = 1;
+    const int slice_bytes = static_cast<int>(q.a_tx) + BN * kBK * 2;
+    while (ks < 4 && p.K >= 2 * ks * kBK && ((transpose_a && !transpose_b) || p.K % kBK == 0) && (transpose_a || lda == p.K) &&
+           (!transpose_b || ldb == p.K) && 4 * 2 * ks * slice_bytes <= env.smem_optin - kGemmBarBytes)
+        ks *= 2;
+    q.a_tx *= static_cast<uint32_t>(ks);
     q.a_stage = q.a_tx;     // a multiple of 1024: a_rows is a multiple of 8 rows of 128 bytes
-    const int stage_bytes = static_cast<int>(q.a_stage) + BN * kBK * 2;
+    const int stage_bytes = ks * slice_bytes;
     q.stages = (env.smem_optin - kGemmBarBytes) / stage_bytes;
     if (q.stages > kMaxStages) q.stages = kMaxStages;
     if (q.stages < 2) return cudaErrorNotSupported;
     const int smem = kGemmBarBytes + q.stages * stage_bytes;
     const bool oka = transpose_a
-        ? encode_rows_sw128(&amap, A, static_cast<uint64_t>(p.K), static_cast<uint64_t>(p.M), static_cast<uint64_t>(lda), kBK)
-        : encode_rows_sw128(&amap, A, static_cast<uint64_t>(p.M), static_cast<uint64_t>(p.K), static_cast<uint64_t>(lda), a_rows);
+        ? encode_rows_sw128(&amap, A, static_cast<uint64_t>(p.K), static_cast<uint64_t>(p.M), static_cast<uint64_t>(lda), kBK * ks)
+        : ks > 1 ? encode_f16_slices_sw128(&amap, A, p.M, p.K, a_rows, ks)
+                   : encode_rows_sw128(&amap, A, static_cast<uint64_t>(p.M), static_cast<uint64_t>(p.K), static_cast<uint64_t>(lda), a_rows);
     if (!oka) return cudaErrorNotSupported;
-    const bool okb = transpose_b
-        ? encode_rows_sw128(&bmap, B, static_cast<uint64_t>(p.N), static_cast<uint64_t>(p.K), static_cast<uint64_t>(ldb), BN)
-        : encode_rows_sw128(&bmap, B, static_cast<uint64_t>(p.K), static_cast<uint64_t>(p.N), static_cast<uint64_t>(ldb), kBK);
+    const bool okb = !transpose_b
+        ? encode_rows_sw128(&bmap, B, static_cast<uint64_t>(p.K), static_cast<uint64_t>(p.N), static_cast<uint64_t>(ldb), kBK * ks)
+        : ks > 1 ? encode_f16_slices_sw128(&bmap, B, p.N, p.K, BN, ks)
+                   : encode_rows_sw128(&bmap, B, static_cast<uint64_t>(p.N), static_cast<uint64_t>(p.K), static_cast<uint64_t>(ldb), BN);
     if (!okb) return cudaErrorNotSupported;
     const long tiles = static_cast<long>((p.N + BN - 1) / BN) * ((p.M + tile_rows - 1) / tile_rows);
     const long sms = env.sm_count > 0 ? env.sm_count : 148;
     const dim3 grid(static_cast<unsigned>(tiles < sms ? tiles : sms));     // one CTA per SM walks the tiles
-    gemm_f16_tc_kernel<<<grid, (2 + 4 * p.mt) * 32, smem, stream>>>(q, amap, bmap);
+    auto* kernel = ks == 4 ? gemm_f16_tc_kernel<4> : ks == 2 ? gemm_f16_tc_kernel<2> : gemm_f16_tc_kernel<1>;
+    kernel<<<grid, (2 + 4 * p.mt) * 32, smem, stream>>>(q, amap, bmap);
     return cudaGetLastError();
 }
 
 }  // namespace
 
 cudaError_t init_gemm_tc_kernel(int smem_optin) {
-    return cudaFuncSetAttribute(gemm_f16_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin);
+    for (auto* k : {gemm_f16_tc_kernel<1>, gemm_f16_tc_kernel<2>, gemm_f16_tc_kernel<4>}) {
+        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 // cudaErrorNotSupported when the operands are outside what the tiled copies can describe: the leading

@@ -170,13 +170,6 @@ __device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, volatil
     }
 }
 
-__device__ __forceinline__ void tensor_load_3d(void* dst, const void* tmap, int x, int y, int z, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-        "[%0], [%1, {%2, %3, %4}], [%5];"
-        ::"r"(s_u32(dst)), "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(s_u32(bar)) : "memory");
-}
-
 struct Pos {                                // position in a ring
     int i = 0;
     uint32_t ph = 0;

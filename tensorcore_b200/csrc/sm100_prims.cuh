@@ -86,6 +86,13 @@ __device__ __forceinline__ void tensor_load_2d(void* dst, const void* tmap, int 
         ::"r"(s_u32(dst)), "l"(tmap), "r"(x), "r"(y), "r"(s_u32(bar)) : "memory");
 }
 
+__device__ __forceinline__ void tensor_load_3d(void* dst, const void* tmap, int x, int y, int z, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+        "[%0], [%1, {%2, %3, %4}], [%5];"
+        ::"r"(s_u32(dst)), "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(s_u32(bar)) : "memory");
+}
+
 // Starts the fetch of a tensor map (a kernel parameter) so the first tiled load does not wait for it.
 __device__ __forceinline__ void prefetch_tensormap(const void* tmap) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");
