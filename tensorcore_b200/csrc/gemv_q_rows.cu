@@ -68,17 +68,14 @@ struct RowBlock {
         return d;
     }
 };
-// Quants of elements 4 i .. 4 i + 3 as floats.
+// Quants of elements 4 i .. 4 i + 3 as floats: the unsigned byte becomes the low mantissa of 2^23 and the offset
+// is subtracted, both exactly; a conversion instruction a weight has a quarter of the rate (14.1 -> 13.3 us).
 template <int FMT>
 __device__ __forceinline__ void four_quants(const uint32_t* q, int i, float (&f)[4]) {
-    if (FMT == FMT_Q4_0) {
-        const uint32_t v = (i < 4 ? q[i & 3] : q[i & 3] >> 4) & 0x0F0F0F0Fu;
+    const uint32_t v = FMT == FMT_Q4_0 ? (i < 4 ? q[i & 3] : q[i & 3] >> 4) & 0x0F0F0F0Fu : q[i & 7] ^ 0x80808080u;
+    const float zero = FMT == FMT_Q4_0 ? 8388608.0f + 8.0f : 8388608.0f + 128.0f;
 #pragma unroll
-        for (int t = 0; t < 4; ++t) f[t] = static_cast<float>((v >> (8 * t)) & 0xFFu) - 8.0f;
-    } else {
-#pragma unroll
-        for (int t = 0; t < 4; ++t) f[t] = static_cast<float>(static_cast<int8_t>(q[i] >> (8 * t)));
-    }
+    for (int t = 0; t < 4; ++t) f[t] = __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7440 + t)) - zero;
 }
 
 template <int FMT, int MB>
