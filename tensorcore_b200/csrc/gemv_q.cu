@@ -32,7 +32,7 @@
 
 namespace tcb {
 cudaError_t init_gemm_q_tc_kernels(int smem_optin);
-cudaError_t launch_gemm_q_tc(const GemvQArgs* ops, int n_ops, const LaunchEnv& env, cudaStream_t stream);
+cudaError_t launch_gemm_q_tc(const GemvQArgs* ops, int n_ops, const LaunchEnv& env, cudaStream_t stream, int* launches);
 cudaError_t init_gemv_q_rows_kernels(int smem_optin);
 cudaError_t launch_gemv_q_rows(const GemvQArgs& a, const LaunchEnv& env, cudaStream_t stream);
 cudaError_t init_decode_kernel(int smem_optin);
@@ -656,9 +656,8 @@ cudaError_t launch_gemv_q_group(const GemvQArgs* ops, int n, const LaunchEnv& en
             s[i].X = fuse || copy ? a.norm_scratch : x;
             s[i].Y = static_cast<uint8_t*>(ops[i].Y) + static_cast<size_t>(m0) * ops[i].N * (a.y_f32 ? 4 : 2);
         }
-        e = launch_gemm_q_tc(s, n, env, stream);
+        e = launch_gemm_q_tc(s, n, env, stream, &count);
         if (e != cudaSuccess) return e;      // cudaErrorNotSupported only on the first slab: the others differ in rows alone
-        ++count;
     }
     if (launches) *launches += count;
     if (name) *name = a.M >= gemm_min_rows(a.fmt) && !a.y_f32
