@@ -188,7 +188,9 @@ bool managed(const tc_buffer* b) { return b->kind == BUF_MANAGED || b->kind == B
 // strip), one per CUDA stream: calls on a stream are ordered, calls on different streams must not
 // share it.  Grown on demand, freed when the context goes.
 struct DenseScratch { float* f = nullptr; size_t nf = 0; int* c = nullptr; size_t nc = 0; void* norm = nullptr; size_t norm_bytes = 0;
-                      void* dq = nullptr; size_t dq_bytes = 0; };
+                      void* dq = nullptr; size_t dq_bytes = 0;
+                      std::vector<void*> outgrown; };   // smaller rooms for normalised rows: a graph that a caller has
+                                                        // captured may still use them
 std::mutex g_dense_mutex;
 std::unordered_map<cudaStream_t, DenseScratch> g_dense;
 
@@ -203,6 +205,7 @@ void dense_scratch_for(tc_context* ctx, cudaStream_t st, tcb::DenseNormGemvArgs*
             if (kv.second.f) cudaFree(kv.second.f);
             if (kv.second.c) cudaFree(kv.second.c);
             if (kv.second.norm) cudaFree(kv.second.norm);
+            for (void* p : kv.second.outgrown) cudaFree(p);
             if (kv.second.dq) cudaFree(kv.second.dq);
         }
         g_dense.clear();
@@ -248,17 +251,22 @@ void norm_scratch_for(cudaStream_t st, size_t need, tcb::GemvQArgs* a) {
     std::lock_guard<std::mutex> lock(g_dense_mutex);
     DenseScratch& d = g_dense[st];
     if (d.norm_bytes < need) {
-        cudaStreamSynchronize(st);        // an earlier call on this stream may still use the old one
-        if (d.norm) cudaFree(d.norm);
-        d.norm = nullptr;
-        d.norm_bytes = 0;
-        const size_t want = need > (1u << 20) ? need + need / 2 : (1u << 20);
-        if (cudaMalloc(&d.norm, want) != cudaSuccess) {
-            (void)cudaGetLastError();
-            d.norm = nullptr;
-            return;                        // the launcher then uses the kernels that need no scratch
+        // Nothing can be allocated while the caller captures this stream: the call then goes through the room
+        // there is in slabs.  Rooms at least double, so that the outgrown ones add up to less than the last.
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) { (void)cudaGetLastError(); cs = cudaStreamCaptureStatusNone; }
+        if (cs == cudaStreamCaptureStatusNone) {
+            size_t want = need > (1u << 20) ? need + need / 2 : (1u << 20);
+            if (want < 2 * d.norm_bytes) want = 2 * d.norm_bytes;
+            void* room = nullptr;
+            if (cudaMalloc(&room, want) == cudaSuccess) {
+                if (d.norm) d.outgrown.push_back(d.norm);
+                d.norm = room;
+                d.norm_bytes = want;
+            } else {
+                (void)cudaGetLastError();      // the launcher uses the smaller room, or the kernels that need none
+            }
         }
-        d.norm_bytes = want;
     }
     a->norm_scratch = d.norm;
     a->norm_scratch_bytes = d.norm_bytes;
@@ -301,6 +309,7 @@ void free_dense_scratch() {
         if (kv.second.f) cudaFree(kv.second.f);
         if (kv.second.c) cudaFree(kv.second.c);
         if (kv.second.norm) cudaFree(kv.second.norm);
+        for (void* p : kv.second.outgrown) cudaFree(p);
         if (kv.second.dq) cudaFree(kv.second.dq);
     }
     g_dense.clear();

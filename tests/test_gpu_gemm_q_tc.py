@@ -134,3 +134,35 @@ def test_dependent_products_do_not_share_a_launch(tc, ctx, oracle):
     s.close()
     for b in (bx, b1, b2, by):
         b.close()
+
+
+def test_captured_call_outlives_a_larger_one(tc, ctx, oracle):
+    """A fused call captured in a CUDA graph with more rows than the stream's room for normalised rows holds goes
+    through it in slabs, and the graph stays valid when a later, larger call makes a bigger room."""
+    import torch
+    N, K, M, big = 256, 4096, 300, 700
+    X, Wq = data(oracle, 0, big, N, K)
+    g = (1 + 0.1 * np.random.default_rng(5).standard_normal(K)).astype(np.float16)
+    want = oracle.fused_rmsnorm_gemv_quantized_f32(X[:M].astype(np.float32), g.astype(np.float32), Wq, 0, N)
+    x, w, gam = (torch.from_numpy(t.view(np.uint8) if t.dtype == np.uint8 else t).cuda() for t in (X, Wq, g))
+    y, y2 = torch.zeros(M, N, dtype=torch.float16, device="cuda"), torch.zeros(big, N, dtype=torch.float16, device="cuda")
+    st = torch.cuda.Stream()
+
+    def call(m, out):
+        tc.raw_fused_rmsnorm_gemv_quantized(ctx, x.data_ptr(), gam.data_ptr(), w.data_ptr(), out.data_ptr(), "q4_0", m, N, K,
+                                            1e-5, "f16", "f16", st.cuda_stream)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(st):
+        call(8, y2)                                   # the first room: 1 MB, 127 rows
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=st):
+            call(M, y)
+        call(big, y2)                                 # a larger room
+        torch.cuda.synchronize()
+        y.zero_()
+        graph.replay()
+    torch.cuda.synchronize()
+    assert oracle.scaled_rms(y.cpu().numpy(), want) <= 1.1 * np.sqrt(3.0) * ROUND
+    assert tc.take_device_error(ctx) == 0
+    del graph
