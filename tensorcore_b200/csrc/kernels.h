@@ -49,13 +49,13 @@ struct GemvQArgs {
 // From how many activation rows a call with fp16 activations and results counts as prefill-sized: Q8_0 calls
 // then take the tcgen05 kernel (fp16-rounded weights) instead of the integer kernels (four rows a pass),
 // and calls whose K is no multiple of 256 are dequantised once and multiplied as a GEMM.  Q8_0 14336 x 4096 on the integer
-// kernels: 8 / 12 / 16 / 32 rows 53 / 80 / 105 / 210 us; the tcgen05 kernel takes 20 us for any of them,
+// kernels: 8 / 12 / 16 / 32 rows 53 / 80 / 105 / 210 us; the tcgen05 kernel takes 17 us for 13 to 32 rows,
 // but its results carry the rounding of the weights, which these row counts did not have.
 inline int gemm_min_rows(int fmt) { return fmt == 0 ? 96 : 13; }
 // Whether a Q4_0 call with fp16 activations of M rows goes to the tcgen05 kernel by default.  Five rows or
 // more always; four rows where the matrix is large enough that the integer dot products cost more than
-// the tensor-core kernel's fixed part (M = 4 back to back: 14336 x 4096 21.3 us on the integer kernel;
-// 4096 x 4096 9.6).  Fewer rows stay on the integer kernels, which do not round the weights.
+// the tensor-core kernel's fixed part (M = 4 back to back: 14336 x 4096 21.3 us on the integer kernel, 11.0
+// on this one; 4096 x 4096 9.6 and 8.0, where the exact weights were kept).  Fewer rows stay on the integer kernels, which do not round the weights.
 inline bool batched_tc_rows(int M, int N, int K) { return M >= 5 || (M == 4 && (K >= 8192 || N > 4096)); }
 // Whether a call with fp16 activations and K % 256 == 0 goes to the tcgen05 kernel by default.
 inline bool tc_rows(const GemvQArgs& a) {
