@@ -426,9 +426,14 @@ gemm_q_tc_kernel(const QtcParams p, const __grid_constant__ QtcMaps maps) {
                 const int m = e / rows_c, r = r_lo + e % rows_c;
                 const int row = row0 + r;
                 if (row >= N) continue;
-                float acc = 0.f;
-                for (int c = 0; c < split; ++c)
-                    acc += ld_cluster_f32(red_addr + static_cast<uint32_t>(m * kRows + r) * 4u, c);
+                // every peer's part is asked for before the first is added: one trip across the cluster, not `split`
+                float part[8];
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                    part[c] = c < split ? ld_cluster_f32(red_addr + static_cast<uint32_t>(m * kRows + r) * 4u, c) : 0.f;
+                float acc = part[0];
+#pragma unroll
+                for (int c = 1; c < 8; ++c) acc += part[c];
                 const size_t o = static_cast<size_t>(m0 + m) * N + row;
                 if (p.y_f32) static_cast<float*>(Y)[o] = acc;
                 else static_cast<__half*>(Y)[o] = __float2half_rn(acc);
