@@ -337,9 +337,9 @@ tc_status_t tc_gemm_async(tc_context* ctx, const tc_gemm_desc* desc, const tc_bu
 /* include/tensorcore/attention.h:24-69 (arithmetic: lib/ops/attention_cpu.cpp:131-277).  fp16 Q
  * [batch, heads, seq_q, head_dim], K and V [batch, kv_heads, seq_kv, head_dim], O like Q, optional
  * fp32 LSE [batch, heads, seq_q]; softmax in fp32.  Causal mask (key index > query index), sliding
- * window, ALiBi and grouped-query heads as in the reference.  Here: the forward pass as a
- * streaming kernel per query row - the attention of a decode step (seq_q of one or a few rows over
- * a long K/V cache); head_dim <= 128 (TC_ERR_INVALID_SHAPE above).  The recorded form runs at once,
+ * window, ALiBi and grouped-query heads as in the reference.  Here: the forward pass, on
+ * the tensor cores for head_dim 64 and 128 at 16-byte aligned addresses (decode steps and prefill
+ * blocks), else a streaming kernel per query row; head_dim <= 128 (TC_ERR_INVALID_SHAPE above).  The recorded form runs at once,
  * as the reference's CPU backend does.  tc_attention_backward stays a placeholder. */
 typedef struct {
     int32_t batch, heads, seq_q, seq_kv, head_dim;

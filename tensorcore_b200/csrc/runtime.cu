@@ -1563,9 +1563,8 @@ extern "C" tc_status_t tc_rope_forward(tc_context* ctx, tc_buffer* X, const tc_b
     });
 }
 
-// Attention forward for decode (include/tensorcore/attention.h:54-69; checks in the order of
-// lib/ops/attention_cpu.cpp:138-151).  Any seq_q is accepted, but the kernel is a streaming pass
-// per query row: it is meant for the one to few rows of a decode step.
+// Attention forward (include/tensorcore/attention.h:54-69; checks in the order of
+// lib/ops/attention_cpu.cpp:138-151).
 extern "C" tc_status_t tc_attention_forward(tc_context* ctx, const tc_attention_desc* d, const tc_buffer* Q,
                                             const tc_buffer* K, const tc_buffer* V, tc_buffer* O, tc_buffer* LSE) {
     if (!ctx) return TC_ERR_NOT_INITIALIZED;
