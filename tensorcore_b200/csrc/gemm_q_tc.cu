@@ -542,11 +542,13 @@ cudaError_t launch_gemm_q_tc(const GemvQArgs* ops, int n_ops, const LaunchEnv& e
     const int red_bytes = p.nb * kRows * 4;
 
     // K is split over a cluster when there are fewer tiles than SMs: the largest cluster size whose
-    // clusters can all be resident at once, so that the split shortens the K loop instead of queueing.
+    // clusters can all be resident at once, so that the split shortens the K loop instead of queueing, and
+    // whose CTAs keep a unit for each of four warpgroups (8 rows, split 1 / 2 / 4 / 8: 4096 x 1024 3.4 / 4.5 /
+    // 6.2 us, 4096 x 2048 5.1 / 5.0 / 6.5, 2048 x 4096 - / 6.5 / 4.7 / 10.5, 1024 x 8192 15.9 / 10.1 / 6.3 / 6.0).
     auto split_for = [&](int n) {
         int split = 1;
         for (int s = 8; s > 1; --s) {
-            if (s > p.groups || static_cast<long long>(n) * s > env.sm_count) continue;
+            if (4 * s > p.groups || static_cast<long long>(n) * s > env.sm_count) continue;
             if (n <= max_active_clusters(s, env.smem_optin)) { split = s; break; }
         }
         if (const char* s = std::getenv("TC_TC_SPLIT")) split = std::atoi(s);
@@ -556,8 +558,8 @@ cudaError_t launch_gemm_q_tc(const GemvQArgs* ops, int n_ops, const LaunchEnv& e
         return split;
     };
     // Tiles left over after whole rounds of one per SM go in a launch of their own when their K can be split
-    // over the SMs that would idle beside them (22016 x 4096, 8 rows: 148 tiles, then 24 in clusters of 6,
-    // 20.5 -> 19.9 us).
+    // over the SMs that would idle beside them (22016 x 4096, 8 rows: 148 tiles, then 24 in clusters of 4,
+    // 20.5 -> 18.8 us).
     int first = tiles;
     const int left = env.sm_count > 0 ? tiles % env.sm_count : 0;
     if (tiles > env.sm_count && left > 0 && !std::getenv("TC_TC_SPLIT") && split_for(left) > 1) first = tiles - left;
