@@ -6,8 +6,8 @@
 //
 //   * A CTA owns 128 of those pairs (head fastest, so a tile's rows see about the same keys) and walks the
 //     keys 128 at a time; a long cache is cut into chunks like in the other kernels.
-//   * Three loader warps bring K and V through a three-stage ring (cp.async, written with the 128-byte
-//     swizzle the MMA descriptors read; keys past the end are zeros).
+//   * A loader warp brings K and V through a three-stage ring (TMA boxes of 128 keys x 64 elements, 128-byte
+//     swizzle; keys past the cache's end are zeros).
 //   * One issuing warp: S = Q K^T (M128 x N128, operands in shared memory) into one of two score buffers
 //     in tensor memory, the next step's while this step's softmax runs; then O += P V with P in tensor
 //     memory (the A operand) and V as it lies (MN-major).
@@ -16,13 +16,15 @@
 //     each goes to the tensor core as an fp16 value and the fp16 remainder (22 bits of it), two MMAs.
 //
 // What bounds it: latency.  Causal 512 x 512, 32 heads on 8 K/V heads, head_dim 128 is 128 CTAs of up to four
-// steps; clock stamps of the longest: 8000 clocks until the first scores (loads and cold code), then about
-// 4900 a step - exponentials and masks 2500 to 4000, rescaling 700, storing P 900 - in which 1060 clocks of
-// P V and 530 of Q K^T hide, and 2500 to store O.  31 us through the synchronous call (10 us of it
-// launch and wait), 38 us on the mma.sync kernel, whose tensor instructions run at an eighth of the rate,
-// 388 us as a streaming pass per query row.
+// steps; clock stamps of the longest: about 8000 clocks until the first scores (barriers, tensor memory, Q, cold
+// code), then 3500 a step - exponentials and masks 2100 to 2500, rescaling 600, storing P 500 - in which 1060
+// clocks of P V and 530 of Q K^T hide, and 1900 to store O.  28.7 us through the synchronous call (10 us of it
+// launch and wait; 31 with three warps of cp.async as loaders, which a step then waited 1700 clocks for),
+// 38 us on the mma.sync kernel, whose tensor instructions run at an eighth of the rate, 388 us as a
+// streaming pass per query row.
 #include "kernels.h"
 #include "sm100_prims.cuh"
+#include "tensor_map.h"
 
 #include <cuda_fp16.h>
 
@@ -32,7 +34,7 @@ namespace {
 using namespace sm100;
 
 constexpr int kRows = 128, kKeys = 128, kStages = 3;
-constexpr int kSoftWarps = 8, kLoadWarps = 3, kIssueWarp = kSoftWarps + kLoadWarps;
+constexpr int kSoftWarps = 8, kLoadWarp = kSoftWarps, kIssueWarp = kSoftWarps + 1;
 constexpr int kThreads = (kIssueWarp + 1) * 32;
 constexpr int kBarBytes = 3072;
 constexpr uint32_t kSwizzle128 = 2;
@@ -56,9 +58,6 @@ __device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, volatil
         if (__any_sync(0xffffffffu, stop)) return false;
     }
 }
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
-}
 // exp(x), results below the normal range as zero.
 __device__ __forceinline__ float exp_of(float x) {
     float y;
@@ -74,7 +73,7 @@ __device__ __forceinline__ uint64_t desc128(uint32_t addr, uint32_t lbo) {
 }
 
 template <int D>
-__global__ void __launch_bounds__(kThreads, 1) attention_prefill_kernel(const AttnParams p) {
+__global__ void __launch_bounds__(kThreads, 1) attention_prefill_kernel(const AttnParams p, const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap) {
     constexpr int kSlabs = D / 64;                         // 64-element (128-byte) pieces of a row
     constexpr uint32_t kSlab = kKeys * 128;                // bytes of one piece of 128 rows
     constexpr uint32_t kTile = kSlabs * kSlab;             // Q, or one stage's K or V
@@ -97,30 +96,11 @@ __global__ void __launch_bounds__(kThreads, 1) attention_prefill_kernel(const At
     if (p.window > 0 && i_min - p.window > k0) k0 += (i_min - p.window - k0) / kKeys * kKeys;
     const int steps = k1 > k0 ? (k1 - k0 + kKeys - 1) / kKeys : 0;
 
-    // The first step's K and V are on their way before the barriers exist: nothing has to be waited for.
-    const int lt = tid - kSoftWarps * 32;
-    auto fetch = [&](const __half* src, uint32_t dst, int base) {
-#pragma unroll 4
-        for (int e = lt; e < kKeys * (D / 8); e += kLoadWarps * 32) {
-            const int key = e / (D / 8), c = e % (D / 8);
-            const bool in = base + key < k1;
-            cp_async16(dst + (c / 8) * kSlab + key * 128 + (((c & 7) ^ (key & 7)) * 16),
-                       src + static_cast<size_t>(in ? base + key : k0) * D + c * 8, in);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    const __half* Kh = p.K + static_cast<size_t>(bk) * p.Sk * D;
-    const __half* Vh = p.V + static_cast<size_t>(bk) * p.Sk * D;
-    if (warp >= kSoftWarps && warp < kIssueWarp && steps > 0) {
-        fetch(Kh, ring, k0);
-        fetch(Vh, ring + kTile, k0);
-    }
-
     if (tid == 0) {
         bar_init(&bars->q_full, kSoftWarps);
         for (int i = 0; i < kStages; ++i) {
-            bar_init(&bars->k_full[i], kLoadWarps);
-            bar_init(&bars->v_full[i], kLoadWarps);
+            bar_init(&bars->k_full[i], 1);
+            bar_init(&bars->v_full[i], 1);
             bar_init(&bars->kv_empty[i], 1);
         }
         for (int i = 0; i < 2; ++i) {
@@ -133,6 +113,22 @@ __global__ void __launch_bounds__(kThreads, 1) attention_prefill_kernel(const At
         for (int i = 0; i < 4; ++i) bar_init(&bars->both[i], 2);
         bars->abort_flag = 0;
         fence_barrier_init();
+    }
+    if (tid == kLoadWarp * 32) { prefetch_tensormap(&kmap); prefetch_tensormap(&vmap); }
+    __syncthreads();
+    // The first K and V are on their way while tensor memory is allocated.
+    auto fetch = [&](const CUtensorMap* map, uint64_t* bar, uint32_t offset, int key) {
+        bar_expect_tx(bar, kTile);
+#pragma unroll
+        for (int sl = 0; sl < kSlabs; ++sl)
+            tensor_load_3d(smem + kBarBytes + kTile + offset + sl * kSlab, map, 64 * sl, key, bk, bar);
+    };
+    if (warp == kLoadWarp && steps > 0) {
+        if (elect_one()) {
+            fetch(&kmap, &bars->k_full[0], 0, k0);
+            fetch(&vmap, &bars->v_full[0], kTile, k0);
+        }
+        __syncwarp();
     }
     if (warp == kIssueWarp) tmem_alloc(&bars->tmem_base, kTmemCols);
     tc_fence_before_sync();
@@ -310,33 +306,23 @@ __global__ void __launch_bounds__(kThreads, 1) attention_prefill_kernel(const At
             }
         }
         tc_fence_before_sync();
-    } else if (warp < kIssueWarp) {
-        // ---------------- loaders --------------------------------------------------------------------------
-        auto landed = [&](uint64_t* bar) {                 // this warp's pieces are in shared memory
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) bar_arrive(bar);
-        };
-        for (int t = 0; t < steps; ++t) {
-            const int st = t % kStages, before = (t + kStages - 1) % kStages;
-            if (t == 0) {
-                asm volatile("cp.async.wait_group 1;" ::: "memory");
-                landed(&bars->k_full[0]);
-                continue;
-            }
+    } else if (warp == kLoadWarp) {
+        // ---------------- loader ------------------------------------------------------------------------------
+        int sent = steps > 0 ? 1 : 0;
+        for (int t = 1; t < steps; ++t, ++sent) {
+            const int st = t % kStages;
             if (!wait_all(&bars->kv_empty[st], (static_cast<uint32_t>(t / kStages) & 1u) ^ 1u, abort_flag)) { failed = true; break; }
-            const uint32_t dst = ring + static_cast<uint32_t>(st) * 2u * kTile;
-            fetch(Kh, dst, k0 + t * kKeys);
-            fetch(Vh, dst + kTile, k0 + t * kKeys);
-            asm volatile("cp.async.wait_group 2;" ::: "memory");
-            if (t > 1) landed(&bars->k_full[before]);
-            landed(&bars->v_full[before]);
+            if (elect_one()) {
+                fetch(&kmap, &bars->k_full[st], static_cast<uint32_t>(st) * 2u * kTile, k0 + t * kKeys);
+                fetch(&vmap, &bars->v_full[st], static_cast<uint32_t>(st) * 2u * kTile + kTile, k0 + t * kKeys);
+            }
+            __syncwarp();
         }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        if (steps > 0 && !failed) {
-            const int last = (steps - 1) % kStages;
-            if (steps > 1) landed(&bars->k_full[last]);
-            landed(&bars->v_full[last]);
+        if (failed || *abort_flag) {                       // copies in flight land before the shared memory is released
+            for (int t = sent > kStages ? sent - kStages : 0; t < sent; ++t) {
+                bar_wait(&bars->k_full[t % kStages], static_cast<uint32_t>(t / kStages) & 1u, nullptr, 100000000LL);
+                bar_wait(&bars->v_full[t % kStages], static_cast<uint32_t>(t / kStages) & 1u, nullptr, 100000000LL);
+            }
         }
     } else {
         // ---------------- MMA issue -----------------------------------------------------------------------------
@@ -417,8 +403,12 @@ cudaError_t launch_attention_prefill(const AttnParams& p, cudaStream_t stream) {
     const long long x = static_cast<long long>(p.B) * p.Hkv * ((R + kRows - 1) / kRows);
     if (R > 0x7fffff00LL || x > 0x7fffffffLL) return cudaErrorNotSupported;
     const dim3 grid(static_cast<unsigned>(x), static_cast<unsigned>(p.chunks));
-    if (p.D == 128) attention_prefill_kernel<128><<<grid, kThreads, kSmem<128>, stream>>>(p);
-    else attention_prefill_kernel<64><<<grid, kThreads, kSmem<64>, stream>>>(p);
+    CUtensorMap kmap, vmap;
+    const uint64_t heads = static_cast<uint64_t>(p.B) * p.Hkv;
+    if (!encode_heads_sw128(&kmap, p.K, heads, p.Sk, p.D, kKeys) || !encode_heads_sw128(&vmap, p.V, heads, p.Sk, p.D, kKeys))
+        return cudaErrorNotSupported;
+    if (p.D == 128) attention_prefill_kernel<128><<<grid, kThreads, kSmem<128>, stream>>>(p, kmap, vmap);
+    else attention_prefill_kernel<64><<<grid, kThreads, kSmem<64>, stream>>>(p, kmap, vmap);
     return cudaGetLastError();
 }
 
