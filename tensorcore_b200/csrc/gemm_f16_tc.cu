@@ -29,7 +29,6 @@
 // bounded: it sets the error word and lets the kernel end.
 #include "kernels.h"
 #include "sm100_prims.cuh"
-#include "tensor_map.h"
 
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -143,23 +142,23 @@ gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap,
                 if (!wait_all(&bars->empty[s], par ^ 1u, abort_flag)) { failed = true; break; }
                 if (elect_one()) {
                     bar_expect_tx(&bars->full[s], p.a_tx + kBStage);
-                    // K-major operands: a box is KS slices of 64 k of all rows; MN-major ones ([K][M], B as given): boxes
-                    // of 64 m (n) x KS * 64 k
+                    // K-major operands: a box per slice of 64 k; MN-major ones ([K][M], B as given): boxes of 64 m (n) x
+                    // KS * 64 k.  What lies past K reads as zeros.
                     if (p.a_mnmajor) {
                         for (int c = 0; c < 2 * MT; ++c)
                             tensor_load_2d(a_ring + s * a_stage + c * KS * 8192, &amap, m0 + 64 * c, ks * KS * kBK, &bars->full[s]);
-                    } else if (KS > 1) {
-                        tensor_load_3d(a_ring + s * a_stage, &amap, 0, m0, ks * KS, &bars->full[s]);
                     } else {
-                        tensor_load_2d(a_ring + s * a_stage, &amap, ks * kBK, m0, &bars->full[s]);
+#pragma unroll
+                        for (int sl = 0; sl < KS; ++sl)
+                            tensor_load_2d(a_ring + s * a_stage + sl * a_slice, &amap, (ks * KS + sl) * kBK, m0, &bars->full[s]);
                     }
                     if (!p.b_kmajor) {
                         for (int c = 0; c < BN / 64; ++c)
                             tensor_load_2d(b_ring + s * kBStage + c * KS * 8192, &bmap, n0 + 64 * c, ks * KS * kBK, &bars->full[s]);
-                    } else if (KS > 1) {
-                        tensor_load_3d(b_ring + s * kBStage, &bmap, 0, n0, ks * KS, &bars->full[s]);
                     } else {
-                        tensor_load_2d(b_ring + s * kBStage, &bmap, ks * kBK, n0, &bars->full[s]);
+#pragma unroll
+                        for (int sl = 0; sl < KS; ++sl)
+                            tensor_load_2d(b_ring + s * kBStage + sl * kBSlice, &bmap, (ks * KS + sl) * kBK, n0, &bars->full[s]);
                     }
                 }
                 __syncwarp();
@@ -342,12 +341,11 @@ cudaError_t launch_tile(const GemmParams& p, const void* A, const void* B, int l
     q.a_tx = static_cast<uint32_t>(a_rows) * kBK * 2u;
     // Several 64-wide slices per stage while four stages still fit: a stage's barriers and waits cost more than the
     // MMAs of a slice when the tile is small (16 x 4096 x 4096: 590 clocks a slice with one per stage, 420
-    // with four; the kernel 27.7 -> 21.1 us).
-    // K-major operands are loaded by slice and need whole slices.
+    // with four; the kernel 27.7 -> 21.1 us).  Any K and leading dimension: what a last stage holds past K is zeros
+    // (16 x 9672 x 5136, K not of whole slices: a call 43.7 us with one slice per stage, 39.2 with four).
     int ks = 1;
     const int slice_bytes = static_cast<int>(q.a_tx) + BN * kBK * 2;
-    while (ks < 4 && p.K >= 2 * ks * kBK && ((transpose_a && !transpose_b) || p.K % kBK == 0) && (transpose_a || lda == p.K) &&
-           (!transpose_b || ldb == p.K) && 4 * 2 * ks * slice_bytes <= env.smem_optin - kGemmBarBytes)
+    while (ks < 4 && p.K >= 2 * ks * kBK && 4 * 2 * ks * slice_bytes <= env.smem_optin - kGemmBarBytes)
         ks *= 2;
     q.a_tx *= static_cast<uint32_t>(ks);
     q.a_stage = q.a_tx;     // a multiple of 1024: a_rows is a multiple of 8 rows of 128 bytes
@@ -358,13 +356,11 @@ cudaError_t launch_tile(const GemmParams& p, const void* A, const void* B, int l
     const int smem = kGemmBarBytes + q.stages * stage_bytes;
     const bool oka = transpose_a
         ? encode_rows_sw128(&amap, A, static_cast<uint64_t>(p.K), static_cast<uint64_t>(p.M), static_cast<uint64_t>(lda), kBK * ks)
-        : ks > 1 ? encode_f16_slices_sw128(&amap, A, p.M, p.K, a_rows, ks)
-                   : encode_rows_sw128(&amap, A, static_cast<uint64_t>(p.M), static_cast<uint64_t>(p.K), static_cast<uint64_t>(lda), a_rows);
+        : encode_rows_sw128(&amap, A, static_cast<uint64_t>(p.M), static_cast<uint64_t>(p.K), static_cast<uint64_t>(lda), a_rows);
     if (!oka) return cudaErrorNotSupported;
     const bool okb = !transpose_b
         ? encode_rows_sw128(&bmap, B, static_cast<uint64_t>(p.K), static_cast<uint64_t>(p.N), static_cast<uint64_t>(ldb), kBK * ks)
-        : ks > 1 ? encode_f16_slices_sw128(&bmap, B, p.N, p.K, BN, ks)
-                   : encode_rows_sw128(&bmap, B, static_cast<uint64_t>(p.N), static_cast<uint64_t>(p.K), static_cast<uint64_t>(ldb), BN);
+        : encode_rows_sw128(&bmap, B, static_cast<uint64_t>(p.N), static_cast<uint64_t>(p.K), static_cast<uint64_t>(ldb), BN);
     if (!okb) return cudaErrorNotSupported;
     const long tiles = static_cast<long>((p.N + BN - 1) / BN) * ((p.M + tile_rows - 1) / tile_rows);
     const long sms = env.sm_count > 0 ? env.sm_count : 148;
