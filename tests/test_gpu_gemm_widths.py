@@ -31,3 +31,24 @@ def test_widths_against_64_bit(tc, ctx, M, N, K, ta, tb, dtype):
         b.close()
     assert err <= 1.05 * (2.0 ** -11 if dtype == "f16" else 2.0 ** -8) / np.sqrt(3.0)
     assert tc.take_device_error(ctx) == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(16, 4096, 328), (40, 2000, 1032), (300, 1000, 520)])
+def test_padded_rows_against_64_bit(tc, ctx, M, N, K):
+    # leading dimensions larger than K, K no multiple of 64: what lies behind a row's K elements does not count
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M + N + K)
+    A = torch.randn((M, K + 72), generator=g, device="cuda").half()
+    B = torch.randn((N, K + 200), generator=g, device="cuda").half()
+    C = torch.full((M, N), float("nan"), device="cuda", dtype=torch.float16)
+    bufs = [ctx.buffer_from_ptr(t.data_ptr(), t.numel() * 2) for t in (A, B, C)]
+    torch.cuda.synchronize()
+    tc.gemm(ctx, *bufs, M, N, K, transpose_b=True, lda=K + 72, ldb=K + 200)
+    assert tc.cuda_last_kernel_name() == "gemm_f16_tcgen05_sm100"
+    want = A[:, :K].double() @ B[:, :K].double().t()
+    err = ((C.double() - want).square().mean() / want.square().mean()).sqrt().item()
+    for b in bufs:
+        b.close()
+    assert err <= 1.05 * 2.0 ** -11 / np.sqrt(3.0)
+    assert tc.take_device_error(ctx) == 0
