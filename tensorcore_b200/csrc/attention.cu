@@ -622,7 +622,8 @@ cudaError_t launch_attention_forward(const void* Q, const void* K, const void* V
     p.group = attention_group(Hq, Hkv);
     attention_chunks(B, Hq, Hkv, Sq, Sk, D, sm_count, &p.chunks, &p.keys_per_chunk);
     if (p.chunks > 1 && !scratch) { p.chunks = 1; p.keys_per_chunk = Sk; }
-    p.scale = scale; p.causal = causal ? 1 : 0; p.window = window;
+    // A window that no query can look back beyond hides nothing; so the kernels' `i - window` stays within int.
+    p.scale = scale; p.causal = causal ? 1 : 0; p.window = window < Sq - 1 ? window : 0;
     const uintptr_t at = reinterpret_cast<uintptr_t>(Q) | reinterpret_cast<uintptr_t>(K) | reinterpret_cast<uintptr_t>(V);
     p.vec = (at & 15u) == 0;
     p.err = err_word;

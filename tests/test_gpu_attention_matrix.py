@@ -82,3 +82,22 @@ def test_unaligned_cache_takes_the_vector_kernel(tc, ctx, D):
     for b in [bq, bo] + views + hold:
         b.close()
     assert np.abs(got - want).max() <= 2.0 ** -11 * np.abs(want).max() + 1e-5
+
+
+@pytest.mark.parametrize("D", [64, 96, 128])
+@pytest.mark.parametrize("Sq,Sk", [(1, 300), (1, 3000), (100, 300), (40, 700)])
+@pytest.mark.parametrize("window", [2 ** 31 - 1, 2 ** 31 - 200, 5000])
+def test_a_window_wider_than_the_queries_hides_nothing(tc, ctx, D, Sq, Sk, window):
+    """INT_MAX as "no limit", without the causal mask: keys far ahead of the query stay visible."""
+    B, H, Hkv = 1, 4, 2
+    rng = np.random.default_rng(Sq + Sk + D)
+    Q = rng.standard_normal((B, H, Sq, D)).astype(np.float16)
+    K = rng.standard_normal((B, Hkv, Sk, D)).astype(np.float16)
+    V = rng.standard_normal((B, Hkv, Sk, D)).astype(np.float16)
+    want, _ = exact(Q, K, V, False, 0, None)
+    bufs = [ctx.buffer_from_array(t) for t in (Q, K, V)] + [ctx.buffer(Q.nbytes)]
+    tc.attention_forward(ctx, *bufs, B, H, Sq, Sk, D, causal=False, kv_heads=Hkv, window_size=window)
+    got = bufs[3].to_numpy(Q.shape, np.float16).astype(np.float64)
+    for b in bufs:
+        b.close()
+    assert np.abs(got - want).max() <= 2.0 ** -11 * np.abs(want).max() + 1e-5
