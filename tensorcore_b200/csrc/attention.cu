@@ -15,6 +15,7 @@
 //     online-softmax state (running maximum m, denominator l, unnormalised output o[D]) for its chunk;
 //     with one chunk it writes O (and LSE) itself, else it leaves (m, l, o) in scratch and a second
 //     small kernel merges the chunks.
+#include "attention_math.cuh"
 #include "kernels.h"
 
 #include <cuda_fp16.h>
@@ -22,6 +23,8 @@
 
 namespace tcb {
 namespace {
+
+using namespace attn;
 
 constexpr int kAttnWarps = 4;
 constexpr int kAttnMaxD = 128;
@@ -202,8 +205,8 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_decode_kernel(const
 //   SPLIT_KEYS (16 rows or fewer): all four warps hold the same rows and take 16 keys of a step each,
 //     with softmax states of their own that are merged at the end.
 //   else: a warp owns 16 of the 64 rows and takes all 64 keys.
-// The scores' products are exact and summed in fp32.  The probabilities stay fp32: for the product with V
-// each is split into an fp16 value and the fp16 remainder (22 bits of it), which costs a third
+// The scores' products are exact and summed in fp32.  The probabilities are fp32 numbers; for the product with V
+// each is split into two fp16 numbers (attention_math.cuh says to how many bits), which costs a third
 // more MMAs and keeps the result as close to a 64-bit one as fp32 multiply-adds had it.
 // A decode step is bound by the cache stream; two CTAs per SM overlap the chains of their steps (scores,
 // maximum, exponentials, outputs).  Eight sequences, 32 heads on 8 K/V heads x 4096 keys: 31 us (4.3 TB/s),
@@ -228,22 +231,6 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4],
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// exp(x), results below the normal range as zero.
-__device__ __forceinline__ float exp_of(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f));
-    return y;
-}
-__device__ __forceinline__ uint32_t pack_h2(float a, float b) {
-    const __half2 h = __floats2half2_rn(a, b);
-    return *reinterpret_cast<const uint32_t*>(&h);
-}
-// What the fp16 pair `h` leaves of (a, b), as fp16.
-__device__ __forceinline__ uint32_t rest_h2(uint32_t h, float a, float b) {
-    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
-    return pack_h2(a - f.x, b - f.y);
-}
-
 template <int D> struct MmaShape {
     static constexpr int kStages = D == 128 ? 3 : 4;
     static constexpr int kStageBytes = 2 * kStepKeys * D * 2;
@@ -394,7 +381,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const
         for (int n = 0; n < kNT; ++n)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                s[n][e] = exp_of(s[n][e] - ref[e >> 1]);       // now the probability
+                s[n][e] = scaled_exp(s[n][e] - ref[e >> 1]);   // now the probability, 2^15 times
                 l[e >> 1] += s[n][e];
             }
 #pragma unroll
@@ -403,8 +390,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const
 #pragma unroll
             for (int q = 0; q < 4; ++q) {                  // (rows lo, hi) x (keys 0-7, 8-15)
                 const float a = s[2 * k + (q >> 1)][2 * (q & 1)], c = s[2 * k + (q >> 1)][2 * (q & 1) + 1];
-                hi[q] = pack_h2(a, c);
-                lo[q] = rest_h2(hi[q], a, c);
+                split_h2(a, c, hi[q], lo[q]);
             }
 #pragma unroll
             for (int n = 0; n < D / 8; n += 2) {
@@ -423,6 +409,9 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const
     for (int e = 0; e < 2; ++e) {
         l[e] += __shfl_xor_sync(0xffffffffu, l[e], 1);
         l[e] += __shfl_xor_sync(0xffffffffu, l[e], 2);
+        l[e] *= kProbUnscale;
+#pragma unroll
+        for (int n = 0; n < D / 8; ++n) { o[n][2 * e] *= kProbUnscale; o[n][2 * e + 1] *= kProbUnscale; }
     }
 
     if constexpr (!SPLIT_KEYS) {

@@ -1,0 +1,41 @@
+// Arithmetic shared by the matrix attention kernels (attention.cu, attention_tc.cu).
+#pragma once
+
+#include <cuda_fp16.h>
+#include <stdint.h>
+
+namespace tcb {
+namespace attn {
+
+// The product with V takes a probability p in (0, 1] as two fp16 numbers.  As it stands fp16 ends at 2^-24, and
+// probabilities below that would be lost to the output while the row sum still counts them; so exponentials
+// are carried 2^15 times as large, the largest fp16 power of two, and the factor is taken out of the row's sum and
+// output at the end (exactly: a power of two).  The two numbers then hold p to 22 bits down to 2^-17 and
+// to 2^-40 below: 8192 keys of any size leave out less than 2^-27 of the largest.
+constexpr float kProbScale = 32768.0f, kProbUnscale = 1.0f / 32768.0f;
+
+// exp(x) * kProbScale; exponentials below the normal range are zero.
+__device__ __forceinline__ float scaled_exp(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f));
+    return y * kProbScale;
+}
+// exp(x), the same way.
+__device__ __forceinline__ float exp_of(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f));
+    return y;
+}
+__device__ __forceinline__ uint32_t pack_h2(float a, float b) {
+    const __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+// Two scaled probabilities as fp16 pairs hi + lo.
+__device__ __forceinline__ void split_h2(float a, float b, uint32_t& hi, uint32_t& lo) {
+    hi = pack_h2(a, b);
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+    lo = pack_h2(a - f.x, b - f.y);
+}
+
+}  // namespace attn
+}  // namespace tcb

@@ -12,8 +12,8 @@
 //     in tensor memory, the next step's while this step's softmax runs; then O += P V with P in tensor
 //     memory (the A operand) and V as it lies (MN-major).
 //   * Eight softmax warps, two threads per row with 64 scores each in registers: running maximum (exchanged
-//     between the two), exponentials; O is rescaled in tensor memory only when a row's maximum has grown.  The probabilities stay fp32:
-//     each goes to the tensor core as an fp16 value and the fp16 remainder (22 bits of it), two MMAs.
+//     between the two), exponentials; O is rescaled in tensor memory only when a row's maximum has grown.  The probabilities are fp32
+//     numbers; each goes to the tensor core as two fp16 numbers (attention_math.cuh says to how many bits), two MMAs.
 //
 // What bounds it: latency.  Causal 512 x 512, 32 heads on 8 K/V heads, head_dim 128 is 128 CTAs of up to four
 // steps; clock stamps of the longest: about 8000 clocks until the first scores (barriers, tensor memory, Q, cold
@@ -22,6 +22,7 @@
 // launch and wait; 31 with three warps of cp.async as loaders, which a step then waited 1700 clocks for),
 // 38 us on the mma.sync kernel, whose tensor instructions run at an eighth of the rate, 388 us as a
 // streaming pass per query row.
+#include "attention_math.cuh"
 #include "kernels.h"
 #include "sm100_prims.cuh"
 #include "tensor_map.h"
@@ -32,6 +33,7 @@ namespace tcb {
 namespace {
 
 using namespace sm100;
+using namespace attn;
 
 constexpr int kRows = 128, kKeys = 128, kStages = 3;
 constexpr int kSoftWarps = 8, kLoadWarp = kSoftWarps, kIssueWarp = kSoftWarps + 1;
@@ -57,16 +59,6 @@ __device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, volatil
         const bool stop = *abort_flag || clock64() - t0 > 2000000000LL;
         if (__any_sync(0xffffffffu, stop)) return false;
     }
-}
-// exp(x), results below the normal range as zero.
-__device__ __forceinline__ float exp_of(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f));
-    return y;
-}
-__device__ __forceinline__ uint32_t pack_h2(float a, float b) {
-    const __half2 h = __floats2half2_rn(a, b);
-    return *reinterpret_cast<const uint32_t*>(&h);
 }
 __device__ __forceinline__ uint64_t desc128(uint32_t addr, uint32_t lbo) {
     return smem_desc_kmajor(addr, lbo, 1024u) | (static_cast<uint64_t>(kSwizzle128) << 61);
@@ -216,7 +208,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_prefill_kernel(const At
             float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int e = 0; e < kHalf; ++e) {
-                s[e] = exp_of(s[e] - ref);                               // now the probability
+                s[e] = scaled_exp(s[e] - ref);                           // now the probability, 2^15 times
                 sum[e & 3] += s[e];
             }
             l = l * keep + ((sum[0] + sum[1]) + (sum[2] + sum[3]));      // over this thread's keys
@@ -247,12 +239,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_prefill_kernel(const At
             for (int c = 0; c < kHalf / 32; ++c) {
                 uint32_t hi[16], lo[16];
 #pragma unroll
-                for (int e = 0; e < 16; ++e) {
-                    const float a = s[32 * c + 2 * e], z = s[32 * c + 2 * e + 1];
-                    hi[e] = pack_h2(a, z);
-                    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi[e]));
-                    lo[e] = pack_h2(a - f.x, z - f.y);
-                }
+                for (int e = 0; e < 16; ++e) split_h2(s[32 * c + 2 * e], s[32 * c + 2 * e + 1], hi[e], lo[e]);
                 tmem_st16(lanes + kColPHi + static_cast<uint32_t>(hf * (kHalf / 2) + 16 * c), hi);
                 tmem_st16(lanes + kColPLo + static_cast<uint32_t>(hf * (kHalf / 2) + 16 * c), lo);
             }
@@ -267,7 +254,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_prefill_kernel(const At
         }
         if (!failed) l += exchange(l);
         if (!failed) {
-            const float inv = l != 0.f ? 1.0f / l : 0.f;
+            const float inv = l != 0.f ? 1.0f / l : 0.f;                 // l and O are both 2^15 times as large here
             float* part = p.part + (row_at * p.chunks + chunk) * (D + 2);
             {
                 constexpr int kQ = D / 32;                 // pieces of 16 columns of this thread's half
@@ -296,13 +283,13 @@ __global__ void __launch_bounds__(kThreads, 1) attention_prefill_kernel(const At
                     } else {
 #pragma unroll
                         for (int e = 0; e < 16; e += 2)
-                            *reinterpret_cast<float2*>(part + 2 + c + e) = make_float2(__uint_as_float(v[q][e]), __uint_as_float(v[q][e + 1]));
+                            *reinterpret_cast<float2*>(part + 2 + c + e) = make_float2(__uint_as_float(v[q][e]) * kProbUnscale, __uint_as_float(v[q][e + 1]) * kProbUnscale);
                     }
                 }
             }
             if (live && hf == 0) {
-                if (p.chunks > 1) { part[0] = m; part[1] = l; }
-                else if (p.LSE) p.LSE[row_at] = m + logf(fmaxf(l, 1e-30f));
+                if (p.chunks > 1) { part[0] = m; part[1] = l * kProbUnscale; }
+                else if (p.LSE) p.LSE[row_at] = m + logf(fmaxf(l * kProbUnscale, 1e-30f));
             }
         }
         tc_fence_before_sync();

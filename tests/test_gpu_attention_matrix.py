@@ -101,3 +101,26 @@ def test_a_window_wider_than_the_queries_hides_nothing(tc, ctx, D, Sq, Sk, windo
     for b in bufs:
         b.close()
     assert np.abs(got - want).max() <= 2.0 ** -11 * np.abs(want).max() + 1e-5
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Sq,Sk,gap", [(1, 8192, 18.0), (1, 4096, 22.0), (20, 1024, 18.0), (100, 8192, 18.0), (130, 2048, 22.0)])
+def test_many_small_probabilities_beside_a_large_one(tc, ctx, D, Sq, Sk, gap):
+    """Key 0 scores `gap` above all others (probabilities of e^-gap, down to 2^-32) and has values of zero: the
+    result is made of the small probabilities alone.  Bar: the result's rounding, 2^-11 relative, the exponential's
+    and the sum's, less than 1e-5, and what the two fp16 numbers of a probability leave out, 2^-40 of the largest
+    probability for each key."""
+    B, H, Hkv = 1, 4, 2
+    Q, K, V = (np.zeros((B, h, s, D), np.float16) for h, s in ((H, Sq), (Hkv, Sk), (Hkv, Sk)))
+    Q[..., 0] = 1.0
+    K[:, :, 0, 0] = gap
+    V[:, :, 1:, :] = 1000.0 * (1.0 + np.arange(D) / D)
+    bufs = [ctx.buffer_from_array(t) for t in (Q, K, V)] + [ctx.buffer(Q.nbytes)]
+    tc.attention_forward(ctx, *bufs, B, H, Sq, Sk, D, causal=False, kv_heads=Hkv, softmax_scale=1.0)
+    got = bufs[3].to_numpy(Q.shape, np.float16).astype(np.float64)
+    for b in bufs:
+        b.close()
+    p = np.exp(-gap)
+    want = (Sk - 1) * p / (1.0 + (Sk - 1) * p) * V[0, 0, 1].astype(np.float64)
+    assert want.min() > 2.0 ** -14
+    assert (np.abs(got - want) <= (2.0 ** -11 + 1e-5) * want + Sk * 2.0 ** -40 * V.max()).all()
