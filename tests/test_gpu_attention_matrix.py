@@ -124,3 +124,29 @@ def test_many_small_probabilities_beside_a_large_one(tc, ctx, D, Sq, Sk, gap):
     want = (Sk - 1) * p / (1.0 + (Sk - 1) * p) * V[0, 0, 1].astype(np.float64)
     assert want.min() > 2.0 ** -14
     assert (np.abs(got - want) <= (2.0 ** -11 + 1e-5) * want + Sk * 2.0 ** -40 * V.max()).all()
+
+
+@pytest.mark.parametrize("D", [64, 96, 128])
+@pytest.mark.parametrize("Sq,Sk,causal,window", [(1, 200, False, 0), (1, 3000, False, 0), (20, 70, True, 0), (150, 300, True, 0)])
+def test_an_infinite_value_makes_its_element_infinite(tc, ctx, D, Sq, Sk, causal, window):
+    """V[key, d] = inf: element d of every row that sees the key is inf, as p * inf is, and not NaN; nothing
+    else changes.  The key's score is the row's average, far from underflow."""
+    B, H, Hkv, key, d = 1, 4, 2, 0, 37
+    rng = np.random.default_rng(Sq + Sk + D)
+    Q = rng.standard_normal((B, H, Sq, D)).astype(np.float16)
+    K = rng.standard_normal((B, Hkv, Sk, D)).astype(np.float16)
+    V = rng.standard_normal((B, Hkv, Sk, D)).astype(np.float16)
+    K[:, :, key] = 0
+    bufs = [ctx.buffer_from_array(t) for t in (Q, K, V)] + [ctx.buffer(Q.nbytes)]
+    outs = []
+    for value in (V[0, 0, key, d], np.inf, -np.inf):
+        V[:, :, key, d] = value
+        bufs[2].upload(V)
+        tc.attention_forward(ctx, *bufs, B, H, Sq, Sk, D, causal=causal, kv_heads=Hkv, window_size=window)
+        outs.append(bufs[3].to_numpy(Q.shape, np.float16))
+    for b in bufs:
+        b.close()
+    rest = np.arange(D) != d
+    for got, value in zip(outs[1:], (np.inf, -np.inf)):
+        assert (got[..., d] == value).all()
+        assert np.array_equal(got[..., rest], outs[0][..., rest])
