@@ -5,7 +5,7 @@
 // fp32 LSE [B,H,Sq]; softmax in fp32; causal mask (key index > query index), sliding window
 // (query - key > window), ALiBi (score -= slope * (query - key)), grouped-query heads.
 //
-//   * head_dim 64 and 128 at 16-byte aligned addresses: tensor cores, attention_mma_kernel below for a decode
+//   * head_dim 64 and 128, Q, K and V 16-byte aligned: tensor cores, attention_mma_kernel below for a decode
 //     step (up to 64 query rows per K/V head) and attention_tc.cu for a prefill block.
 //   * Other head_dims and addresses: attention_decode_kernel, a streaming pass per query row on the CUDA
 //     cores.  A lane takes a key for the scores (the query rows in shared memory), then the lanes
@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_decode_kernel(const
 
     // this lane's slice of the output: `per` consecutive elements when D is a multiple of 32 (one
     // vector load per value row), else elements lane, lane + 32, ...
-    const int per = (D & 31) == 0 && p.vec ? D >> 5 : 0;
+    const int per = (D & 31) == 0 && p.v_vec ? D >> 5 : 0;
     auto elem = [&](int t) { return per ? lane * per + t : lane + 32 * t; };
     float o[G][kPer];
     float m[G], l[G];
@@ -420,9 +420,13 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const
             if (!live[e]) continue;
             if (p.chunks == 1) {
                 const float inv = l[e] != 0.f ? 1.0f / l[e] : 0.f;
-                uint32_t* dst = reinterpret_cast<uint32_t*>(p.O + row_at[e] * D) + tq;
+                __half* dst = p.O + row_at[e] * D + 2 * tq;
 #pragma unroll
-                for (int n = 0; n < D / 8; ++n) dst[4 * n] = pack_h2(o[n][2 * e] * inv, o[n][2 * e + 1] * inv);
+                for (int n = 0; n < D / 8; ++n) {
+                    const __half2 v = __floats2half2_rn(o[n][2 * e] * inv, o[n][2 * e + 1] * inv);
+                    if (p.o_vec) *reinterpret_cast<__half2*>(dst + 8 * n) = v;
+                    else { dst[8 * n] = __low2half(v); dst[8 * n + 1] = __high2half(v); }
+                }
                 if (tq == 0 && p.LSE) p.LSE[row_at[e]] = m[e] + logf(fmaxf(l[e], 1e-30f));
             } else {
                 float* dst = p.part + (row_at[e] * p.chunks + chunk) * (D + 2);
@@ -520,12 +524,10 @@ int attention_group(int Hq, int Hkv) {
     return per % 2 == 0 ? 2 : 1;
 }
 
-bool matrix_head_dim(int D) { return D == 64 || D == 128; }
-
 // How a row's keys are cut: chunks of keys_per_chunk keys.
-void attention_chunks(int B, int Hq, int Hkv, int Sq, int Sk, int D, int sm_count, int* chunks, int* keys_per_chunk) {
+void attention_chunks(int B, int Hq, int Hkv, int Sq, int Sk, bool matrix, int sm_count, int* chunks, int* keys_per_chunk) {
     const int sms = sm_count > 0 ? sm_count : 148;
-    if (!matrix_head_dim(D)) {
+    if (!matrix) {
         // Enough CTAs for eight per SM, chunks of at least 128 keys (one step of 32 keys per warp): a
         // step is a few dependent round trips to memory, so the bandwidth comes from many warps in
         // flight, not from long chunks.
@@ -588,9 +590,14 @@ cudaError_t init_attention_kernels() {
     return e == cudaSuccess ? init_attention_prefill_kernels() : e;
 }
 
-size_t attention_scratch_floats(int B, int Hq, int Hkv, int Sq, int Sk, int D, int sm_count, int* chunks_out) {
+bool attention_on_matrix_kernels(int D, const void* Q, const void* K, const void* V) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(Q) | reinterpret_cast<uintptr_t>(K) | reinterpret_cast<uintptr_t>(V);
+    return (D == 64 || D == 128) && (at & 15u) == 0;
+}
+
+size_t attention_scratch_floats(int B, int Hq, int Hkv, int Sq, int Sk, int D, bool matrix, int sm_count, int* chunks_out) {
     int chunks = 1, per = Sk;
-    attention_chunks(B, Hq, Hkv, Sq, Sk, D, sm_count, &chunks, &per);
+    attention_chunks(B, Hq, Hkv, Sq, Sk, matrix, sm_count, &chunks, &per);
     if (chunks_out) *chunks_out = chunks;
     const size_t rows = static_cast<size_t>(B) * Hq * Sq;
     return chunks > 1 ? rows * chunks * (D + 2) : 0;
@@ -599,7 +606,7 @@ size_t attention_scratch_floats(int B, int Hq, int Hkv, int Sq, int Sk, int D, i
 cudaError_t launch_attention_forward(const void* Q, const void* K, const void* V, void* O, float* LSE,
                                      float* scratch, const float* slopes_dev, int B, int Hq, int Hkv, int Sq,
                                      int Sk, int D, float scale, bool causal, int window, int sm_count,
-                                     cudaStream_t stream, int* launches, uint32_t* err_word) {
+                                     cudaStream_t stream, int* launches, uint32_t* err_word, const char** name) {
     if (D <= 0 || D > kAttnMaxD) return cudaErrorNotSupported;
     const long long rows_ll = static_cast<long long>(B) * Hq * Sq;
     if (rows_ll <= 0 || rows_ll > 0x7fffffffLL) return cudaErrorNotSupported;
@@ -609,18 +616,24 @@ cudaError_t launch_attention_forward(const void* Q, const void* K, const void* V
     p.O = static_cast<__half*>(O); p.LSE = LSE; p.part = scratch; p.slopes = slopes_dev;
     p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.Sq = Sq; p.Sk = Sk; p.D = D;
     p.group = attention_group(Hq, Hkv);
-    attention_chunks(B, Hq, Hkv, Sq, Sk, D, sm_count, &p.chunks, &p.keys_per_chunk);
+    const bool matrix = attention_on_matrix_kernels(D, Q, K, V);
+    attention_chunks(B, Hq, Hkv, Sq, Sk, matrix, sm_count, &p.chunks, &p.keys_per_chunk);
     if (p.chunks > 1 && !scratch) { p.chunks = 1; p.keys_per_chunk = Sk; }
     // A window that no query can look back beyond hides nothing; so the kernels' `i - window` stays within int.
     p.scale = scale; p.causal = causal ? 1 : 0; p.window = window < Sq - 1 ? window : 0;
-    const uintptr_t at = reinterpret_cast<uintptr_t>(Q) | reinterpret_cast<uintptr_t>(K) | reinterpret_cast<uintptr_t>(V);
-    p.vec = (at & 15u) == 0;
+    p.o_vec = (reinterpret_cast<uintptr_t>(O) & 15u) == 0;
+    // the vector kernel's lanes load D / 32 elements of a value row at a time
+    p.v_vec = (reinterpret_cast<uintptr_t>(V) & (D == 128 ? 7u : 3u)) == 0;
     p.err = err_word;
     cudaError_t e = cudaErrorNotSupported;
-    if (matrix_head_dim(D) && p.vec && (reinterpret_cast<uintptr_t>(O) & 15u) == 0)
+    if (matrix) {
         e = D == 128 ? launch_matrix<128>(p, stream) : launch_matrix<64>(p, stream);
-    if (e == cudaErrorNotSupported)
+        if (name) *name = static_cast<long long>(Sq) * (Hq / Hkv) > kMmaRows ? "attention_prefill_tcgen05_sm100" : "attention_mma_sm100";
+    }
+    if (e == cudaErrorNotSupported) {
         e = launch_vector(dim3(static_cast<unsigned>(rows / p.group), static_cast<unsigned>(p.chunks)), stream, p);
+        if (name) *name = "attention_decode_sm100";
+    }
     if (e != cudaSuccess) return e;
     if (launches) *launches += 1;
     if (p.chunks > 1) {

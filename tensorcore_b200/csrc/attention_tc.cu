@@ -277,9 +277,15 @@ __global__ void __launch_bounds__(kThreads, 1) attention_prefill_kernel(const At
 #pragma unroll
                         for (int e = 0; e < 8; ++e)
                             o[e] = pack_h2(__uint_as_float(v[q][2 * e]) * inv, __uint_as_float(v[q][2 * e + 1]) * inv);
-                        uint4* dst = reinterpret_cast<uint4*>(p.O + row_at * D + c);
-                        dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-                        dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+                        if (p.o_vec) {
+                            uint4* dst = reinterpret_cast<uint4*>(p.O + row_at * D + c);
+                            dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
+                            dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+                        } else {
+                            uint16_t* dst = reinterpret_cast<uint16_t*>(p.O + row_at * D + c);
+#pragma unroll
+                            for (int e = 0; e < 16; ++e) dst[e] = static_cast<uint16_t>(o[e / 2] >> (16 * (e & 1)));
+                        }
                     } else {
 #pragma unroll
                         for (int e = 0; e < 16; e += 2)

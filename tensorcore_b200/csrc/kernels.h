@@ -271,19 +271,22 @@ struct AttnParams {
     int chunks, keys_per_chunk;
     float scale;
     int causal, window;
-    int vec;              // Q, K and V are 16-byte aligned
+    int o_vec;            // O is 16-byte aligned
+    int v_vec;            // V is aligned to the vector kernel's loads
     uint32_t* err;        // device-visible word for an error bit, or null
 };
-// The tcgen05 kernel for prefill blocks (attention_tc.cu): head_dim 64 or 128, all addresses 16-byte aligned.
+// The tcgen05 kernel for prefill blocks (attention_tc.cu): head_dim 64 or 128; Q, K and V 16-byte aligned.
 cudaError_t init_attention_prefill_kernels();
 cudaError_t launch_attention_prefill(const AttnParams& p, cudaStream_t stream);
 // Floats of scratch the launch needs, and into how many key chunks it will cut a row (1 = no scratch).
-size_t attention_scratch_floats(int B, int Hq, int Hkv, int Sq, int Sk, int D, int sm_count, int* chunks_out);
+size_t attention_scratch_floats(int B, int Hq, int Hkv, int Sq, int Sk, int D, bool matrix, int sm_count, int* chunks_out);
+// Whether a call takes the matrix kernels (O may lie at any even address).
+bool attention_on_matrix_kernels(int D, const void* Q, const void* K, const void* V);
 // cudaErrorNotSupported: head_dim above 128.  slopes_dev: ALiBi slopes on the device, or null.
 cudaError_t launch_attention_forward(const void* Q, const void* K, const void* V, void* O, float* LSE,
                                      float* scratch, const float* slopes_dev, int B, int Hq, int Hkv, int Sq,
                                      int Sk, int D, float scale, bool causal, int window, int sm_count,
-                                     cudaStream_t stream, int* launches, uint32_t* err_word);
+                                     cudaStream_t stream, int* launches, uint32_t* err_word, const char** name);
 
 // --- collectives over NCCL (dist_nccl.cpp); return 0, or -1 bad arguments, -2 NCCL not found,
 // -3 rendezvous failed, -4 NCCL / CUDA error ----------------------------------------------------

@@ -1586,7 +1586,8 @@ extern "C" tc_status_t tc_attention_forward(tc_context* ctx, const tc_attention_
     int chunks = 1;
     const long long rows = static_cast<long long>(B) * Hq * Sq;
     if (rows > 0x7fffffffLL) return TC_ERR_INVALID_SHAPE;
-    size_t want = tcb::attention_scratch_floats(B, Hq, Hkv, Sq, Sk, D, ctx->sm_count, &chunks);
+    size_t want = tcb::attention_scratch_floats(B, Hq, Hkv, Sq, Sk, D, tcb::attention_on_matrix_kernels(D, Q->dptr, K->dptr, V->dptr),
+                                                ctx->sm_count, &chunks);
     const size_t slope_at = want;
     if (d->alibi_slopes) want += static_cast<size_t>(Hq);
     if (want > ctx->attn_scratch_floats) {
@@ -1610,13 +1611,15 @@ extern "C" tc_status_t tc_attention_forward(tc_context* ctx, const tc_attention_
             return record("tc_attention_forward", TC_ERR_DISPATCH);
     }
     int launched = 0;
+    const char* used = "attention_decode_sm100";
     const tc_status_t st = run_step_op(ctx, "tc_attention_forward", "attention_decode_sm100", io, n_io, [&](cudaStream_t s0) {
         return tcb::launch_attention_forward(Q->dptr, K->dptr, V->dptr, O->dptr,
                                              LSE ? static_cast<float*>(LSE->dptr) : nullptr,
                                              chunks > 1 ? ctx->attn_scratch : nullptr, slopes_dev, B, Hq, Hkv, Sq, Sk,
-                                             D, scale, d->causal, d->window_size, ctx->sm_count, s0, &launched, ctx->err_dev);
+                                             D, scale, d->causal, d->window_size, ctx->sm_count, s0, &launched, ctx->err_dev, &used);
     });
     if (launched > 1) g_launches.fetch_add(static_cast<uint64_t>(launched - 1));
+    if (launched > 0) t_last_kernel = used;
     return st;
 }
 
@@ -1640,6 +1643,7 @@ extern "C" tc_status_t tcx_raw_attention_forward(tc_context* ctx, const tc_atten
     cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
     int chunks = 1;
     const size_t want = tcb::attention_scratch_floats(d->batch, d->heads, Hkv, d->seq_q, d->seq_kv, d->head_dim,
+                                                       tcb::attention_on_matrix_kernels(d->head_dim, Q, K, V),
                                                        ctx->sm_count, &chunks);
     if (want > ctx->attn_scratch_floats) {
         cudaDeviceSynchronize();
@@ -1654,12 +1658,13 @@ extern "C" tc_status_t tcx_raw_attention_forward(tc_context* ctx, const tc_atten
     }
     const float scale = d->softmax_scale > 0 ? d->softmax_scale : 1.0f / std::sqrt(static_cast<float>(d->head_dim));
     int launched = 0;
+    const char* used = t_last_kernel;
     const cudaError_t e = tcb::launch_attention_forward(Q, K, V, O, static_cast<float*>(LSE),
                                                         chunks > 1 ? ctx->attn_scratch : nullptr, nullptr, d->batch,
                                                         d->heads, Hkv, d->seq_q, d->seq_kv, d->head_dim, scale, d->causal,
-                                                        d->window_size, ctx->sm_count, st, &launched, ctx->err_dev);
+                                                        d->window_size, ctx->sm_count, st, &launched, ctx->err_dev, &used);
     g_launches.fetch_add(static_cast<uint64_t>(launched));
-    t_last_kernel = "attention_decode_sm100";
+    t_last_kernel = used;
     return record("tcx_raw_attention_forward", from_cuda(e, TC_ERR_DISPATCH));
 }
 

@@ -50,6 +50,7 @@ def test_against_64_bit(tc, ctx, B, H, Hkv, Sq, Sk, D, causal, window, alibi):
     bufs = [ctx.buffer_from_array(t) for t in (Q, K, V)] + [ctx.buffer(Q.nbytes), ctx.buffer(B * H * Sq * 4)]
     tc.attention_forward(ctx, *bufs[:4], B, H, Sq, Sk, D, LSE=bufs[4], causal=causal, kv_heads=Hkv, window_size=window,
                          alibi_slopes=slopes)
+    assert tc.cuda_last_kernel_name() == ("attention_prefill_tcgen05_sm100" if Sq * (H // Hkv) > 64 else "attention_mma_sm100")
     got = bufs[3].to_numpy(Q.shape, np.float16).astype(np.float64)
     got_lse = bufs[4].to_numpy((B, H, Sq), np.float32).astype(np.float64)
     for b in bufs:
@@ -63,9 +64,10 @@ def test_against_64_bit(tc, ctx, B, H, Hkv, Sq, Sk, D, causal, window, alibi):
 
 
 @pytest.mark.parametrize("D", [64, 128])
-def test_unaligned_cache_takes_the_vector_kernel(tc, ctx, D):
-    """A cache 2 bytes past a 16-byte boundary gives the same results."""
-    B, H, Hkv, Sq, Sk = 1, 4, 2, 3, 150
+@pytest.mark.parametrize("off,Sq", [(2, 3), (4, 3), (8, 3), (8, 50)])
+def test_unaligned_cache_takes_the_vector_kernel(tc, ctx, D, off, Sq):
+    """A cache 2, 4 or 8 bytes past a 16-byte boundary gives the same results."""
+    B, H, Hkv, Sk = 1, 4, 2, 150
     rng = np.random.default_rng(D)
     Q = rng.standard_normal((B, H, Sq, D)).astype(np.float16)
     K = rng.standard_normal((B, Hkv, Sk, D)).astype(np.float16)
@@ -75,9 +77,10 @@ def test_unaligned_cache_takes_the_vector_kernel(tc, ctx, D):
     hold = [ctx.buffer(K.nbytes + 16) for _ in range(2)]
     views = []
     for h, t in zip(hold, (K, V)):
-        h.upload(t, 2)
-        views.append(ctx.buffer_from_ptr(h.device_ptr() + 2, t.nbytes))
+        h.upload(t, off)
+        views.append(ctx.buffer_from_ptr(h.device_ptr() + off, t.nbytes))
     tc.attention_forward(ctx, bq, views[0], views[1], bo, B, H, Sq, Sk, D, causal=True, kv_heads=Hkv)
+    assert tc.cuda_last_kernel_name() == "attention_decode_sm100"
     got = bo.to_numpy(Q.shape, np.float16).astype(np.float64)
     for b in [bq, bo] + views + hold:
         b.close()
@@ -150,3 +153,28 @@ def test_an_infinite_value_makes_its_element_infinite(tc, ctx, D, Sq, Sk, causal
     for got, value in zip(outs[1:], (np.inf, -np.inf)):
         assert (got[..., d] == value).all()
         assert np.array_equal(got[..., rest], outs[0][..., rest])
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Sq,Sk", [(1, 3000), (5, 40), (20, 70), (150, 200), (70, 3000)])
+@pytest.mark.parametrize("off", [2, 8])
+def test_results_at_any_even_address(tc, ctx, D, Sq, Sk, off):
+    """O past a 16-byte boundary: the same kernel and the same bits, nothing written beside them."""
+    B, H, Hkv = 1, 4, 2
+    rng = np.random.default_rng(Sq + Sk + D)
+    Q = rng.standard_normal((B, H, Sq, D)).astype(np.float16)
+    K = rng.standard_normal((B, Hkv, Sk, D)).astype(np.float16)
+    V = rng.standard_normal((B, Hkv, Sk, D)).astype(np.float16)
+    bufs = [ctx.buffer_from_array(t) for t in (Q, K, V)] + [ctx.buffer(Q.nbytes)]
+    hold = ctx.buffer(Q.nbytes + 32)
+    hold.upload(np.full(Q.nbytes + 32, 0x5A, np.uint8))
+    view = ctx.buffer_from_ptr(hold.device_ptr() + off, Q.nbytes)
+    tc.attention_forward(ctx, *bufs, B, H, Sq, Sk, D, causal=False, kv_heads=Hkv)
+    name = tc.cuda_last_kernel_name()
+    tc.attention_forward(ctx, *bufs[:3], view, B, H, Sq, Sk, D, causal=False, kv_heads=Hkv)
+    assert tc.cuda_last_kernel_name() == name and name != "attention_decode_sm100"
+    got = hold.to_numpy((Q.nbytes + 32,), np.uint8)
+    assert np.array_equal(got[off:off + Q.nbytes].view(np.uint16).reshape(Q.shape), bufs[3].to_numpy(Q.shape, np.uint16))
+    assert (got[:off] == 0x5A).all() and (got[off + Q.nbytes:] == 0x5A).all()
+    for b in [view, hold] + bufs:
+        b.close()
