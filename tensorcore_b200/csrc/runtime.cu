@@ -28,6 +28,13 @@ cudaError_t init_gemv_kernels(int smem_optin);
 // ---------------------------------------------------------------------------------------
 // Handle definitions
 // ---------------------------------------------------------------------------------------
+// A piece of device memory that calls use as scratch, grown on demand.
+struct Room {
+    void* p = nullptr;
+    size_t bytes = 0;
+    bool captured = false;   // handed out while a stream was being captured: a graph may use it at any time
+};
+
 enum BufKind : int {
     BUF_DEVICE = 0,        // cudaMalloc, owned; never seen by the host
     BUF_MANAGED = 1,       // cudaMallocManaged, owned; host-visible after tc_buffer_map
@@ -51,8 +58,7 @@ struct tc_context {
     uint32_t* err_host;   // pinned, mapped
     uint32_t* err_dev;
     bool mega_on;         // route qualifying recorded lists to the persistent decode kernel
-    float* attn_scratch;  // partial softmax states of tc_attention_forward, grown on demand
-    size_t attn_scratch_floats;
+    Room attn;            // partial softmax states and ALiBi slopes of tc_attention_forward
 };
 
 struct tc_buffer {
@@ -184,60 +190,105 @@ tc_status_t validate(tc_context* ctx, const tc_buffer* b, size_t min_bytes) {
 bool staged(const tc_buffer* b) { return b->kind == BUF_WRAP_HOST || b->kind == BUF_HOST_SHADOW; }
 bool managed(const tc_buffer* b) { return b->kind == BUF_MANAGED || b->kind == BUF_WRAP_MANAGED; }
 
-// Scratch of the dense fused GEMV (partial sums of the K ranges, one ticket counter per column
-// strip), one per CUDA stream: calls on a stream are ordered, calls on different streams must not
-// share it.  Grown on demand, freed when the context goes.
-struct DenseScratch { float* f = nullptr; size_t nf = 0; int* c = nullptr; size_t nc = 0; void* norm = nullptr; size_t norm_bytes = 0;
-                      void* dq = nullptr; size_t dq_bytes = 0;
-                      std::vector<void*> outgrown; };   // smaller rooms for normalised rows: a graph that a caller has
-                                                        // captured may still use them
-std::mutex g_dense_mutex;
-std::unordered_map<cudaStream_t, DenseScratch> g_dense;
+// Scratch that belongs to a CUDA stream: calls on a stream are ordered, calls on different streams must not
+// share it.  A room is made when a call first needs it and grows when one needs more; the one outgrown is
+// freed once the stream is done with it - except where the caller captured the stream while it was handed
+// out: a graph may then be replayed at any time, and the room stays until the context goes.
+// The mutex is held from handing rooms out until the launches that use them are in the stream, so that calls
+// from several threads do not get between another call's launches, nor free its rooms.
+struct StreamRooms {
+    Room partial, counters;   // dense fused GEMV: partial sums of the K ranges, a ticket counter per column strip
+    Room norm;                // normalised rows
+    Room weights;             // weights as fp16
+};
+std::mutex g_rooms_mutex;
+std::unordered_map<cudaStream_t, StreamRooms> g_rooms;
+std::vector<void*> g_kept;    // outgrown rooms of captured graphs
+using RoomsLock = std::unique_lock<std::mutex>;
+constexpr size_t kMaxWeightsRoom = static_cast<size_t>(3) << 29;      // 1.5 GB
 
+bool being_captured(cudaStream_t st) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) { (void)cudaGetLastError(); return false; }
+    return cs != cudaStreamCaptureStatusNone;
+}
+
+// No launch that uses the room is under way.
+void give_back(Room& r) {
+    if (r.p && r.captured) g_kept.push_back(r.p);
+    else if (r.p) cudaFree(r.p);
+    r = Room();
+}
+
+// Makes `r` hold `need` bytes, unless the stream is being captured (nothing can be allocated then) or there
+// is no memory: the caller sees what there is.  `wait` returns when no launch uses the room any more.
+template <typename Wait>
+void grow_room(Room& r, size_t need, size_t most, cudaStream_t st, bool zero, Wait wait) {
+    const bool capture = being_captured(st);
+    if (r.bytes < need && !capture) {
+        // Half as much again as before, so that slowly growing calls do not allocate every time; rooms that have to
+        // stay at least double, so that together they are smaller than the last.
+        size_t want = r.captured ? 2 * r.bytes : r.bytes + r.bytes / 2;
+        if (want > most) want = most;
+        if (want < need) want = need;
+        void* p = nullptr;
+        if (cudaMalloc(&p, want) != cudaSuccess) {
+            (void)cudaGetLastError();
+            p = nullptr;
+            wait();
+            give_back(r);
+            want = need;
+            if (cudaMalloc(&p, want) != cudaSuccess) { (void)cudaGetLastError(); p = nullptr; }
+        }
+        if (p && zero && cudaMemsetAsync(p, 0, want, st) != cudaSuccess) { (void)cudaGetLastError(); cudaFree(p); p = nullptr; }
+        if (p) {
+            if (r.p) { wait(); give_back(r); }
+            r.p = p;
+            r.bytes = want;
+        }
+    }
+    if (capture && r.p) r.captured = true;
+}
+void grow_stream_room(Room& r, size_t need, cudaStream_t st, bool zero = false, size_t most = ~static_cast<size_t>(0)) {
+    grow_room(r, need, most, st, zero, [&] { cudaStreamSynchronize(st); });
+}
+
+StreamRooms& rooms_of(cudaStream_t st) {
+    if (g_rooms.size() > 32 && g_rooms.find(st) == g_rooms.end() && !being_captured(st)) {
+        // many short-lived streams: start over rather than keep scratch for streams that are gone
+        cudaDeviceSynchronize();
+        for (auto& kv : g_rooms)
+            for (Room* r : {&kv.second.partial, &kv.second.counters, &kv.second.norm, &kv.second.weights}) give_back(*r);
+        g_rooms.clear();
+    }
+    return g_rooms[st];
+}
+void free_rooms() {
+    RoomsLock lock(g_rooms_mutex);
+    for (auto& kv : g_rooms)
+        for (Room* r : {&kv.second.partial, &kv.second.counters, &kv.second.norm, &kv.second.weights}) give_back(*r);
+    g_rooms.clear();
+    for (void* p : g_kept) cudaFree(p);
+    g_kept.clear();
+}
+
+// The functions that hand rooms out; the caller holds g_rooms_mutex and goes on holding it until it has launched.
 void dense_scratch_for(tc_context* ctx, cudaStream_t st, tcb::DenseNormGemvArgs* a) {
     size_t nf = 0, nc = 0;
     tcb::dense_norm_gemv_scratch(a->M, a->N, a->K, ctx->sm_count, &nf, &nc);
-    std::lock_guard<std::mutex> lock(g_dense_mutex);
-    if (g_dense.size() > 32 && g_dense.find(st) == g_dense.end()) {
-        // many short-lived streams: start over rather than keep scratch for streams that are gone
-        cudaDeviceSynchronize();
-        for (auto& kv : g_dense) {
-            if (kv.second.f) cudaFree(kv.second.f);
-            if (kv.second.c) cudaFree(kv.second.c);
-            if (kv.second.norm) cudaFree(kv.second.norm);
-            for (void* p : kv.second.outgrown) cudaFree(p);
-            if (kv.second.dq) cudaFree(kv.second.dq);
-        }
-        g_dense.clear();
-    }
-    DenseScratch& d = g_dense[st];
-    if (d.nf < nf || d.nc < nc) {
-        cudaStreamSynchronize(st);        // an earlier call on this stream may still use the old one
-        if (d.f) cudaFree(d.f);
-        if (d.c) cudaFree(d.c);
-        d.f = nullptr; d.c = nullptr; d.nf = 0; d.nc = 0;
-        const size_t wf = nf + nf / 2, wc = nc * 2;
-        if (cudaMalloc(reinterpret_cast<void**>(&d.f), wf * sizeof(float)) != cudaSuccess ||
-            cudaMalloc(reinterpret_cast<void**>(&d.c), wc * sizeof(int)) != cudaSuccess ||
-            cudaMemset(d.c, 0, wc * sizeof(int)) != cudaSuccess) {
-            (void)cudaGetLastError();
-            if (d.f) cudaFree(d.f);
-            if (d.c) cudaFree(d.c);
-            d.f = nullptr; d.c = nullptr; d.nf = 0; d.nc = 0;
-            return;                        // the launcher falls back to the kernel that needs none
-        }
-        d.nf = wf;
-        d.nc = wc;
-    }
-    a->scratch = d.f; a->scratch_floats = d.nf; a->counters = d.c; a->counters_n = d.nc;
+    StreamRooms& d = rooms_of(st);
+    grow_stream_room(d.partial, nf * sizeof(float), st);
+    grow_stream_room(d.counters, nc * sizeof(int), st, true);
+    a->scratch = static_cast<float*>(d.partial.p); a->scratch_floats = d.partial.bytes / sizeof(float);
+    a->counters = static_cast<int*>(d.counters.p); a->counters_n = d.counters.bytes / sizeof(int);
 }
-// Room for the normalised rows of the batched fused RMSNorm GEMV (the tensor-core kernel reads them as
-// plain fp16 activations).
 // Whether the call is prefill-sized: its weights are dequantised once and multiplied as a GEMM.
 bool dequant_gemm_wanted(const tcb::GemvQArgs& a) {
     return a.M >= tcb::gemm_min_rows(a.fmt) && !a.x_f32 && !a.y_f32 && a.K % 256 != 0 && a.K % 32 == 0 &&
-           static_cast<size_t>(a.N) * a.K * 2 <= (static_cast<size_t>(3) << 29);      // at most 1.5 GB of scratch
+           static_cast<size_t>(a.N) * a.K * 2 <= kMaxWeightsRoom;
 }
+// Room for the normalised rows of the batched fused RMSNorm GEMV (the tensor-core kernel reads them as
+// plain fp16 activations).
 size_t norm_scratch_need(const tcb::GemvQArgs& a) {
     if (a.x_f32) return 0;
     if (dequant_gemm_wanted(a)) return a.gamma ? static_cast<size_t>(a.M) * a.K * 2 + static_cast<size_t>(a.M) * 4 : 0;
@@ -246,30 +297,24 @@ size_t norm_scratch_need(const tcb::GemvQArgs& a) {
     const size_t rows = a.M < 2048 ? a.M : 2048;      // larger calls go through the scratch in slabs
     return rows * (static_cast<size_t>(a.K) * 2 + 4);
 }
+// Room for the weights as fp16 of a prefill-sized quantized GEMV (a call that finds none keeps the kernels that
+// stream the blocks).
+size_t dequant_scratch_need(const tcb::GemvQArgs& a) {
+    return dequant_gemm_wanted(a) ? static_cast<size_t>(a.N) * a.K * 2 : 0;
+}
 void norm_scratch_for(cudaStream_t st, size_t need, tcb::GemvQArgs* a) {
     if (need == 0) return;
-    std::lock_guard<std::mutex> lock(g_dense_mutex);
-    DenseScratch& d = g_dense[st];
-    if (d.norm_bytes < need) {
-        // Nothing can be allocated while the caller captures this stream: the call then goes through the room
-        // there is in slabs.  Rooms at least double, so that the outgrown ones add up to less than the last.
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) { (void)cudaGetLastError(); cs = cudaStreamCaptureStatusNone; }
-        if (cs == cudaStreamCaptureStatusNone) {
-            size_t want = need > (1u << 20) ? need + need / 2 : (1u << 20);
-            if (want < 2 * d.norm_bytes) want = 2 * d.norm_bytes;
-            void* room = nullptr;
-            if (cudaMalloc(&room, want) == cudaSuccess) {
-                if (d.norm) d.outgrown.push_back(d.norm);
-                d.norm = room;
-                d.norm_bytes = want;
-            } else {
-                (void)cudaGetLastError();      // the launcher uses the smaller room, or the kernels that need none
-            }
-        }
-    }
-    a->norm_scratch = d.norm;
-    a->norm_scratch_bytes = d.norm_bytes;
+    StreamRooms& d = rooms_of(st);
+    grow_stream_room(d.norm, need > (1u << 20) ? need : (1u << 20), st);
+    a->norm_scratch = d.norm.p;
+    a->norm_scratch_bytes = d.norm.bytes;
+}
+void dequant_scratch_for(cudaStream_t st, size_t need, tcb::GemvQArgs* a) {
+    if (need == 0) return;
+    StreamRooms& d = rooms_of(st);
+    grow_stream_room(d.weights, need, st, false, kMaxWeightsRoom);
+    a->dequant_scratch = d.weights.p;
+    a->dequant_scratch_bytes = d.weights.bytes;
 }
 // Room for the normalised rows of a dense fused norm + GEMV call with five rows or more.
 void dense_norm_rows_for(cudaStream_t st, tcb::DenseNormGemvArgs* a) {
@@ -278,41 +323,6 @@ void dense_norm_rows_for(cudaStream_t st, tcb::DenseNormGemvArgs* a) {
     norm_scratch_for(st, static_cast<size_t>(a->M) * a->K * 2 + static_cast<size_t>(a->M) * 8, &tmp);
     a->norm_scratch = tmp.norm_scratch;
     a->norm_scratch_bytes = tmp.norm_scratch_bytes;
-}
-// Room for the weights as fp16 of a prefill-sized quantized GEMV on this stream (grown on demand; a
-// call that finds none keeps the kernels that stream the blocks).
-void dequant_scratch_for(cudaStream_t st, size_t need, tcb::GemvQArgs* a) {
-    if (need == 0) return;
-    std::lock_guard<std::mutex> lock(g_dense_mutex);
-    DenseScratch& d = g_dense[st];
-    if (d.dq_bytes < need) {
-        cudaStreamSynchronize(st);        // an earlier call on this stream may still use the old one
-        if (d.dq) cudaFree(d.dq);
-        d.dq = nullptr;
-        d.dq_bytes = 0;
-        if (cudaMalloc(&d.dq, need) != cudaSuccess) {
-            (void)cudaGetLastError();
-            d.dq = nullptr;
-            return;
-        }
-        d.dq_bytes = need;
-    }
-    a->dequant_scratch = d.dq;
-    a->dequant_scratch_bytes = d.dq_bytes;
-}
-size_t dequant_scratch_need(const tcb::GemvQArgs& a) {
-    return dequant_gemm_wanted(a) ? static_cast<size_t>(a.N) * a.K * 2 : 0;
-}
-void free_dense_scratch() {
-    std::lock_guard<std::mutex> lock(g_dense_mutex);
-    for (auto& kv : g_dense) {
-        if (kv.second.f) cudaFree(kv.second.f);
-        if (kv.second.c) cudaFree(kv.second.c);
-        if (kv.second.norm) cudaFree(kv.second.norm);
-        for (void* p : kv.second.outgrown) cudaFree(p);
-        if (kv.second.dq) cudaFree(kv.second.dq);
-    }
-    g_dense.clear();
 }
 
 LaunchEnv make_env(tc_context* ctx, bool allow_pdl) {
@@ -399,10 +409,11 @@ tc_status_t setup_device(tc_context* ctx, int device) {
 void teardown_device(tc_context* ctx) {
     if (ctx->stream0) cudaStreamDestroy(ctx->stream0);
     if (ctx->err_host) cudaFreeHost(ctx->err_host);
-    if (ctx->attn_scratch) cudaFree(ctx->attn_scratch);
-    free_dense_scratch();
-    ctx->attn_scratch = nullptr;
-    ctx->attn_scratch_floats = 0;
+    {
+        RoomsLock lock(g_rooms_mutex);
+        give_back(ctx->attn);
+    }
+    free_rooms();
     ctx->stream0 = nullptr;
     ctx->err_host = nullptr;
     ctx->err_dev = nullptr;
@@ -505,8 +516,6 @@ extern "C" tc_status_t tc_init(tc_context** out_ctx) {
     ctx->stream0 = nullptr;
     ctx->err_host = nullptr;
     ctx->err_dev = nullptr;
-    ctx->attn_scratch = nullptr;
-    ctx->attn_scratch_floats = 0;
     if (const char* v = std::getenv("TC_GEMV_VARIANT")) (void)tcx_set_gemv_variant(v);
     ctx->mega_on = env_flag("TC_MEGA", true);
     ctx->pdl = env_flag("TC_PDL", true);
@@ -989,6 +998,7 @@ tc_status_t submit_pending(tc_stream* s) {
     if (s->pending.empty()) return TC_OK;
     bind_device(ctx);
     bool any_staged = false;
+    RoomsLock rooms(g_rooms_mutex, std::defer_lock);
     tcb::GemvQArgs scratch_of;          // the stream's scratch for normalised rows, sized for the widest operation
     {
         size_t need = 0, dq = 0;
@@ -998,6 +1008,7 @@ tc_status_t submit_pending(tc_stream* s) {
             const size_t q = dequant_scratch_need(op.a);
             dq = q > dq ? q : dq;
         }
+        if (need > 0 || dq > 0) rooms.lock();
         norm_scratch_for(s->s, need, &scratch_of);
         dequant_scratch_for(s->s, dq, &scratch_of);
     }
@@ -1353,9 +1364,14 @@ tc_status_t gemv_common(const GemvCall& c, tc_stream* stream, const char* opname
     if (e == cudaSuccess) e = prepare_output(ctx, op.Y, s0);
     int launches = 0;
     const char* name = "none";
-    if (e == cudaSuccess) norm_scratch_for(s0, norm_scratch_need(op.a), &op.a);
-    if (e == cudaSuccess) dequant_scratch_for(s0, dequant_scratch_need(op.a), &op.a);
-    if (e == cudaSuccess) e = launch_recorded(ctx, op, s0, false, &launches, &name);
+    if (e == cudaSuccess) {
+        const size_t need = norm_scratch_need(op.a), dq = dequant_scratch_need(op.a);
+        RoomsLock rooms(g_rooms_mutex, std::defer_lock);
+        if (need > 0 || dq > 0) rooms.lock();
+        norm_scratch_for(s0, need, &op.a);
+        dequant_scratch_for(s0, dq, &op.a);
+        e = launch_recorded(ctx, op, s0, false, &launches, &name);
+    }
     if (e == cudaSuccess) e = finish_output(op.Y, yb, s0);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s0);
     g_launches.fetch_add(static_cast<uint64_t>(launches));
@@ -1452,6 +1468,7 @@ static tc_status_t dense_common(tc_context* ctx, const tc_buffer* X, const tc_bu
     int launches = 0;
     const char* name = "none";
     if (e == cudaSuccess) {
+        RoomsLock rooms(g_rooms_mutex);
         dense_scratch_for(ctx, s0, &a);
         dense_norm_rows_for(s0, &a);
         e = tcb::launch_dense_norm_gemv(a, make_env(ctx, false), s0, &launches, &name);
@@ -1590,21 +1607,13 @@ extern "C" tc_status_t tc_attention_forward(tc_context* ctx, const tc_attention_
                                                 ctx->sm_count, &chunks);
     const size_t slope_at = want;
     if (d->alibi_slopes) want += static_cast<size_t>(Hq);
-    if (want > ctx->attn_scratch_floats) {
-        cudaStreamSynchronize(ctx->stream0);
-        if (ctx->attn_scratch) cudaFree(ctx->attn_scratch);
-    free_dense_scratch();
-        ctx->attn_scratch = nullptr;
-        ctx->attn_scratch_floats = 0;
-        if (cudaMalloc(reinterpret_cast<void**>(&ctx->attn_scratch), want * sizeof(float)) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return record("tc_attention_forward", TC_ERR_ALLOC);
-        }
-        ctx->attn_scratch_floats = want;
-    }
+    RoomsLock rooms(g_rooms_mutex);
+    if (want > 0) grow_room(ctx->attn, want * sizeof(float), ~static_cast<size_t>(0), ctx->stream0, false, [] { cudaDeviceSynchronize(); });
+    if (want * sizeof(float) > ctx->attn.bytes) return record("tc_attention_forward", TC_ERR_ALLOC);
+    float* const scratch = static_cast<float*>(ctx->attn.p);
     float* slopes_dev = nullptr;
     if (d->alibi_slopes) {
-        slopes_dev = ctx->attn_scratch + slope_at;
+        slopes_dev = scratch + slope_at;
         // a small copy from caller memory: staged by the runtime before the call returns
         if (cudaMemcpyAsync(slopes_dev, d->alibi_slopes, static_cast<size_t>(Hq) * sizeof(float),
                             cudaMemcpyHostToDevice, ctx->stream0) != cudaSuccess)
@@ -1613,10 +1622,12 @@ extern "C" tc_status_t tc_attention_forward(tc_context* ctx, const tc_attention_
     int launched = 0;
     const char* used = "attention_decode_sm100";
     const tc_status_t st = run_step_op(ctx, "tc_attention_forward", "attention_decode_sm100", io, n_io, [&](cudaStream_t s0) {
-        return tcb::launch_attention_forward(Q->dptr, K->dptr, V->dptr, O->dptr,
+        const cudaError_t le = tcb::launch_attention_forward(Q->dptr, K->dptr, V->dptr, O->dptr,
                                              LSE ? static_cast<float*>(LSE->dptr) : nullptr,
-                                             chunks > 1 ? ctx->attn_scratch : nullptr, slopes_dev, B, Hq, Hkv, Sq, Sk,
+                                             chunks > 1 ? scratch : nullptr, slopes_dev, B, Hq, Hkv, Sq, Sk,
                                              D, scale, d->causal, d->window_size, ctx->sm_count, s0, &launched, ctx->err_dev, &used);
+        rooms.unlock();
+        return le;
     });
     if (launched > 1) g_launches.fetch_add(static_cast<uint64_t>(launched - 1));
     if (launched > 0) t_last_kernel = used;
@@ -1645,22 +1656,20 @@ extern "C" tc_status_t tcx_raw_attention_forward(tc_context* ctx, const tc_atten
     const size_t want = tcb::attention_scratch_floats(d->batch, d->heads, Hkv, d->seq_q, d->seq_kv, d->head_dim,
                                                        tcb::attention_on_matrix_kernels(d->head_dim, Q, K, V),
                                                        ctx->sm_count, &chunks);
-    if (want > ctx->attn_scratch_floats) {
-        cudaDeviceSynchronize();
-        if (ctx->attn_scratch) cudaFree(ctx->attn_scratch);
-        ctx->attn_scratch = nullptr;
-        ctx->attn_scratch_floats = 0;
-        if (cudaMalloc(reinterpret_cast<void**>(&ctx->attn_scratch), want * sizeof(float)) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return record("tcx_raw_attention_forward", TC_ERR_ALLOC);
-        }
-        ctx->attn_scratch_floats = want;
+    // Under capture nothing can be allocated: a call that finds too little room takes each row's keys in one piece.
+    RoomsLock rooms(g_rooms_mutex, std::defer_lock);
+    float* scratch = nullptr;
+    if (want > 0) {
+        rooms.lock();
+        grow_room(ctx->attn, want * sizeof(float), ~static_cast<size_t>(0), st, false, [] { cudaDeviceSynchronize(); });
+        if (want * sizeof(float) <= ctx->attn.bytes) scratch = static_cast<float*>(ctx->attn.p);
+        else if (!being_captured(st)) return record("tcx_raw_attention_forward", TC_ERR_ALLOC);
     }
     const float scale = d->softmax_scale > 0 ? d->softmax_scale : 1.0f / std::sqrt(static_cast<float>(d->head_dim));
     int launched = 0;
     const char* used = t_last_kernel;
     const cudaError_t e = tcb::launch_attention_forward(Q, K, V, O, static_cast<float*>(LSE),
-                                                        chunks > 1 ? ctx->attn_scratch : nullptr, nullptr, d->batch,
+                                                        scratch, nullptr, d->batch,
                                                         d->heads, Hkv, d->seq_q, d->seq_kv, d->head_dim, scale, d->causal,
                                                         d->window_size, ctx->sm_count, st, &launched, ctx->err_dev, &used);
     g_launches.fetch_add(static_cast<uint64_t>(launched));
@@ -1895,8 +1904,11 @@ static tc_status_t raw_gemv(tc_context* ctx, const void* X, const void* gamma, b
     a.X = X; a.Y = Y; a.gamma = fused ? gamma : nullptr;
     a.fmt = static_cast<int>(fmt); a.M = M; a.N = N; a.K = K;
     a.x_f32 = xd == TC_DTYPE_F32; a.y_f32 = yd == TC_DTYPE_F32; a.eps = eps;
-    norm_scratch_for(static_cast<cudaStream_t>(cuda_stream), norm_scratch_need(a), &a);
-    dequant_scratch_for(static_cast<cudaStream_t>(cuda_stream), dequant_scratch_need(a), &a);
+    const size_t need = norm_scratch_need(a), dq = dequant_scratch_need(a);
+    RoomsLock rooms(g_rooms_mutex, std::defer_lock);
+    if (need > 0 || dq > 0) rooms.lock();
+    norm_scratch_for(static_cast<cudaStream_t>(cuda_stream), need, &a);
+    dequant_scratch_for(static_cast<cudaStream_t>(cuda_stream), dq, &a);
     int launches = 0;
     const char* name = "none";
     const cudaError_t e = tcb::launch_gemv_q(a, make_env(ctx, true),
@@ -1934,6 +1946,7 @@ extern "C" tc_status_t tcx_raw_fused_norm_gemv_f16(tc_context* ctx, const void* 
     a.M = M; a.N = N; a.K = K; a.eps = eps;
     int launches = 0;
     const char* name = "none";
+    RoomsLock rooms(g_rooms_mutex);
     dense_scratch_for(ctx, static_cast<cudaStream_t>(cuda_stream), &a);
     dense_norm_rows_for(static_cast<cudaStream_t>(cuda_stream), &a);
     const cudaError_t e = tcb::launch_dense_norm_gemv(a, make_env(ctx, true),

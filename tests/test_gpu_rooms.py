@@ -1,0 +1,197 @@
+"""GPU: scratch that belongs to a stream, when the caller captures the stream in a CUDA graph: a captured call
+takes the room there is, and the graph stays valid whatever later calls need - more rows on the same stream,
+attention, more streams than the library keeps rooms for.
+
+Bars: fp16 results, 2^-11 / sqrt(3) rms for each rounding (weights, normalised rows, result), a tenth on top."""
+import ctypes
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROUND = 2.0 ** -11 / np.sqrt(3.0)
+
+
+def on_device(*arrays):
+    import torch
+    return [torch.from_numpy(a).cuda() for a in arrays]
+
+
+def capture(stream, call):
+    import torch
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        call()
+    return graph
+
+
+def disturb(tc, ctx, oracle):
+    """Grows every room there is: attention with more and more key chunks, and dense and batched calls on more streams
+    than the library keeps rooms for."""
+    import torch
+    rng = np.random.default_rng(1)
+    for Sk in (4096, 16384):
+        q, k = np.zeros((1, 32, 1, 128), np.float16), np.zeros((1, 8, Sk, 128), np.float16)
+        bufs = [ctx.buffer_from_array(t) for t in (q, k, k, q)]
+        tc.attention_forward(ctx, *bufs, 1, 32, 1, Sk, 128, causal=False, kv_heads=8)
+        for b in bufs:
+            b.close()
+    M, N, K = 3, 264, 512
+    x, g, w = on_device(rng.standard_normal((16, K)).astype(np.float16), np.ones(K, np.float16),
+                        (rng.standard_normal((K, N)) * 0.02).astype(np.float16))
+    y = torch.zeros(16, N, dtype=torch.float16, device="cuda")
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(priority=p) for p in (0, -1) for _ in range(20)]
+    assert len({s.cuda_stream for s in streams}) > 33
+    for s in streams:
+        for m in (M, 16):
+            tc.raw_fused_norm_gemv_f16(ctx, x.data_ptr(), g.data_ptr(), 0, w.data_ptr(), y.data_ptr(), m, N, K, 1e-5, s.cuda_stream)
+        torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("K,M,big", [(4096, 300, 700), (1056, 300, 700)])
+def test_captured_quantized_call(tc, ctx, oracle, K, M, big):
+    """K a multiple of 256: normalised rows in slabs of the room there is.  Else: normalised rows and the weights as
+    fp16, or the kernel that needs neither."""
+    import torch
+    N = 256
+    rng = np.random.default_rng(K)
+    X = rng.standard_normal((big, K)).astype(np.float16)
+    g = (1 + 0.1 * rng.standard_normal(K)).astype(np.float16)
+    Wq = oracle.quantize_weights((rng.standard_normal((N, K)) * 0.02).astype(np.float16), 0)
+    want = oracle.fused_rmsnorm_gemv_quantized_f32(X[:M].astype(np.float32), g.astype(np.float32), Wq, 0, N)
+    x, gam, w = on_device(X, g, Wq)
+    y, y2 = (torch.zeros(m, N, dtype=torch.float16, device="cuda") for m in (M, big))
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+
+    def call(m, out):
+        tc.raw_fused_rmsnorm_gemv_quantized(ctx, x.data_ptr(), gam.data_ptr(), w.data_ptr(), out.data_ptr(), "q4_0", m, N, K,
+                                            1e-5, "f16", "f16", st.cuda_stream)
+    call(100, y2)
+    torch.cuda.synchronize()
+    graph = capture(st, lambda: call(M, y))
+    call(big, y2)
+    torch.cuda.synchronize()
+    disturb(tc, ctx, oracle)
+    call(big, y2)
+    torch.cuda.synchronize()
+    y.zero_()
+    with torch.cuda.stream(st):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert oracle.scaled_rms(y.cpu().numpy(), want) <= 1.1 * np.sqrt(3.0) * ROUND
+    assert tc.take_device_error(ctx) == 0
+
+
+@pytest.mark.parametrize("M,warm", [(2, 0), (2, 2), (4, 1), (16, 0), (16, 5), (40, 16)])
+def test_captured_dense_call(tc, ctx, oracle, M, warm):
+    """The dense fused call: partial sums and tickets up to four rows, normalised rows above; on a stream that has no
+    rooms yet (warm = 0), and on one whose rooms are for fewer rows."""
+    import torch
+    N, K, big = 520, 1536, 64
+    rng = np.random.default_rng(M + warm)
+    X = rng.standard_normal((big, K)).astype(np.float16)
+    g = (1 + 0.1 * rng.standard_normal(K)).astype(np.float16)
+    W = (rng.standard_normal((K, N)) * 0.02).astype(np.float16)
+    x64 = X[:M].astype(np.float64)
+    want = (x64 / np.sqrt((x64 * x64).mean(axis=1, keepdims=True) + 1e-5) * g) @ W.astype(np.float64)
+    x, gam, w = on_device(X, g, W)
+    y, y2 = (torch.zeros(m, N, dtype=torch.float16, device="cuda") for m in (M, big))
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+
+    def call(m, out, n=N):
+        tc.raw_fused_norm_gemv_f16(ctx, x.data_ptr(), gam.data_ptr(), 0, w.data_ptr(), out.data_ptr(), m, n, K, 1e-5, st.cuda_stream)
+    if warm:
+        call(warm, y2)
+        torch.cuda.synchronize()
+    graph = capture(st, lambda: call(M, y))
+    for m in (4, big):
+        call(m, y2)
+    torch.cuda.synchronize()
+    disturb(tc, ctx, oracle)
+    for _ in range(2):                        # the second replay finds the tickets as the first left them
+        y.zero_()
+        with torch.cuda.stream(st):
+            graph.replay()
+        torch.cuda.synchronize()
+        assert oracle.scaled_rms(y.cpu().numpy(), want) <= 1.1 * np.sqrt(2.0) * ROUND
+    assert tc.take_device_error(ctx) == 0
+
+
+def test_captured_attention_without_room_for_its_chunks(tc, ctx):
+    """A raw attention call captured on a context whose scratch is too small takes a row's keys in one piece; one that
+    is captured after an eager call of its size gives the eager call's bits, also after the scratch has grown."""
+    import torch
+    B, H, Sq, Sk, D = 1, 1, 8192, 2048, 128
+    st = torch.cuda.Stream()
+    q, k, v = (torch.randn(B, H, s, D, device="cuda").half() for s in (Sq, Sk, Sk))
+    o, o2, ref = (torch.zeros_like(q) for _ in range(3))
+    torch.cuda.synchronize()
+
+    def call(out, sk=Sk):
+        d = tc.TCAttentionDesc(B, H, Sq, sk, D, tc.TC_DTYPE_F16, tc.TC_DTYPE_F32, 0.0, False, False, H, 0, None)
+        rc = tc.lib().tcx_raw_attention_forward(ctx.handle, ctypes.byref(d), *(ctypes.c_void_p(t.data_ptr()) for t in (q, k, v, out)),
+                                                None, ctypes.c_void_p(st.cuda_stream))
+        assert rc == 0
+    first = capture(st, lambda: call(o))
+    call(ref)
+    torch.cuda.synchronize()
+    second = capture(st, lambda: call(o2))
+    qq, kk = np.zeros((1, 64, 64, 128), np.float16), np.zeros((1, 8, 16384, 128), np.float16)
+    bufs = [ctx.buffer_from_array(t) for t in (qq, kk, kk, qq)]
+    tc.attention_forward(ctx, *bufs, 1, 64, 64, 16384, 128, causal=False, kv_heads=8)
+    for b in bufs:
+        b.close()
+    for graph, out in ((first, o), (second, o2)):
+        out.zero_()
+        with torch.cuda.stream(st):
+            graph.replay()
+        torch.cuda.synchronize()
+    assert torch.equal(o2, ref)
+    assert (o.double() - ref.double()).abs().max() <= 2.0 ** -10 * ref.double().abs().max()
+    assert tc.take_device_error(ctx) == 0
+
+
+def test_threads_on_streams_of_their_own(tc, ctx, oracle):
+    """Fused batched calls of growing size from four threads: no call's rows are normalised into another's room."""
+    import torch
+    N, K = 256, 1024
+    rng = np.random.default_rng(9)
+    X = rng.standard_normal((256, K)).astype(np.float16)
+    g = (1 + 0.1 * rng.standard_normal(K)).astype(np.float16)
+    Wq = oracle.quantize_weights((rng.standard_normal((N, K)) * 0.02).astype(np.float16), 0)
+    x, gam, w = on_device(X, g, Wq)
+    torch.cuda.synchronize()
+    rows = (8, 16, 40, 100, 256)
+
+    def call(m, at, out, st):
+        tc.raw_fused_rmsnorm_gemv_quantized(ctx, x[at:].data_ptr(), gam.data_ptr(), w.data_ptr(), out.data_ptr(), "q4_0", m, N, K,
+                                            1e-5, "f16", "f16", st.cuda_stream)
+    wrong = []
+
+    def work(i):
+        st = torch.cuda.Stream()
+        for m in rows:
+            at = (37 * i) % (257 - m)
+            out, ref = (torch.zeros(m, N, dtype=torch.float16, device="cuda") for _ in range(2))
+            torch.cuda.synchronize()
+            for _ in range(20):
+                call(m, at, out, st)
+            st.synchronize()
+            call(m, at, ref, st)
+            st.synchronize()
+            if not torch.equal(out, ref):
+                wrong.append((i, m))
+            full = oracle.fused_rmsnorm_gemv_quantized_f32(X[at:at + m].astype(np.float32), g.astype(np.float32), Wq, 0, N)
+            if oracle.scaled_rms(out.cpu().numpy(), full) > 1.1 * np.sqrt(3.0) * ROUND:
+                wrong.append((i, m, "values"))
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
