@@ -78,6 +78,7 @@ struct QtcParams {
     int split;         // CTAs per tile = cluster size
     int col_tiles;     // tiles of nb activation rows
     int tile_base;     // first tile of this launch
+    int wait_first;    // the kernel before may write the weights
     int raw_stages;    // per warpgroup (a ring that several groups shared would let one wait on a
                        // barrier phase while an earlier one, which it never observes, is still open)
     int x_stages;      // per issuer
@@ -212,7 +213,7 @@ gemm_q_tc_kernel(const QtcParams p, const __grid_constant__ QtcMaps maps) {
     uint8_t* x_ring = smem + p.off_x;
     const int x_bytes = nb * 128 * XK;
 
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (!p.wait_first) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (tid == kRawWarp * 32) prefetch_tensormap(wmap);
     if (tid == kXWarp * 32) prefetch_tensormap(&maps.x);
     if (tid == 0) {
@@ -278,6 +279,10 @@ gemm_q_tc_kernel(const QtcParams p, const __grid_constant__ QtcMaps maps) {
         }
     } else if (warp == kRawWarp) {
         // ---------------- weight producer: 128 rows x one group per unit; rows past N read as zeros -----
+        if (p.wait_first) {
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        }
         Pos ring;
         for (int r = 0; r < n_units && !failed; r += kActive) {
 #pragma unroll
@@ -301,7 +306,7 @@ gemm_q_tc_kernel(const QtcParams p, const __grid_constant__ QtcMaps maps) {
     } else if (warp == kXWarp) {
         // ---------------- activation producer, in the order the issuers consume ---------------------------
         // Activations belong to the stream's order: wait for the kernel before this one here, with
-        // the weight copies (which no kernel of a decode step writes) already in flight.
+        // the weight copies already in flight where nothing that may still run writes them.
         asm volatile("griddepcontrol.wait;" ::: "memory");
         Pos ring;
         for (int r = 0; r < n_units && !failed; r += I)
@@ -575,6 +580,7 @@ cudaError_t launch_gemm_q_tc(const GemvQArgs* ops, int n_ops, const LaunchEnv& e
     auto launch = [&](int tile, int n) {
         p.tile_base = tile;
         p.split = split_for(n);
+        p.wait_first = tile == 0 && env.wait_first() ? 1 : 0;      // the second launch follows this call's first
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(static_cast<unsigned>(n) * p.split);
         cfg.blockDim = dim3(kThreads);

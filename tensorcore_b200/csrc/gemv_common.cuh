@@ -43,6 +43,7 @@ struct StreamParams {
     int gpr;       // groups per row
     int ns;        // ring stages per warp
     int y_f32;
+    int wait_first; // the kernel before may write the weights (LaunchEnv::weights_ready)
     int x_src_f16; // activations (and gamma) are fp16 in global memory
     int x_acc = 0; // 0: X has the declared type; 1: X points at fp32 accumulators taken as they are;
                    // 2: fp32 accumulators whose values are rounded to fp16 first (the producer's

@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(kMaxStreamThreads, 1) gemv_q_stream_kernel(con
     const int nchunks = (g_count + 31) >> 5;
     const int my_n = nchunks > warp ? (nchunks - warp + nwarps - 1) / nwarps : 0;
 
-    pdl_launch_dependents();
+    if (!p.wait_first) pdl_launch_dependents();
 
     if (tid == 0) {
         for (int i = 0; i < nwarps * ns; ++i) mbar_init(&bars[i], 1);
@@ -85,7 +85,11 @@ __global__ void __launch_bounds__(kMaxStreamThreads, 1) gemv_q_stream_kernel(con
         bulk_g2s(ring + static_cast<size_t>(warp * ns + s) * kChunkBytes,
                  p.W + (g_base + first) * F::kGroupBytes, bytes, bar);
     };
-    // Weights do not depend on the previous kernel in the stream: start streaming now.
+    if (p.wait_first) {
+        pdl_wait();
+        pdl_launch_dependents();
+    }
+    // Weights do not depend on a kernel that may still run: start streaming now.
     if (lane == 0) {
         const int pre = min(ns, my_n);
         for (int i = 0; i < pre; ++i) issue(i);
@@ -209,7 +213,7 @@ gemv_q_box_kernel(const StreamParams p, const __grid_constant__ CUtensorMap wmap
     const int n_units = (rows_pad >> 5) * gpr;
     const int my_n = n_units > warp ? (n_units - warp + nwarps - 1) / nwarps : 0;
 
-    pdl_launch_dependents();
+    if (!p.wait_first) pdl_launch_dependents();
     if (tid == 0) {
         sm100::prefetch_tensormap(&wmap);
         for (int i = 0; i < nwarps * ns; ++i) mbar_init(&bars[i], 1);
@@ -227,7 +231,11 @@ gemv_q_box_kernel(const StreamParams p, const __grid_constant__ CUtensorMap wmap
         sm100::tensor_load_2d(ring + static_cast<size_t>(warp * ns + s) * kBoxBytes, &wmap,
                               kg * (F::kGroupBytes / kElem), r0 + rb * 32, bar);
     };
-    // Weights do not depend on the previous kernel in the stream: start streaming now.
+    if (p.wait_first) {
+        pdl_wait();
+        pdl_launch_dependents();
+    }
+    // Weights do not depend on a kernel that may still run: start streaming now.
     if (lane == 0) {
         const int pre = min(ns, my_n);
         for (int i = 0; i < pre; ++i) issue(i);
@@ -314,8 +322,8 @@ __global__ void __launch_bounds__(kThreads) gemv_q_generic_kernel(const GenericP
     __shared__ float rstd_s;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int bb = p.fmt == FMT_Q4_0 ? 18 : 34;
-    pdl_launch_dependents();
     pdl_wait();
+    pdl_launch_dependents();
     for (int m = 0; m < p.M; ++m) {
         float rstd = 1.f;
         if (p.gamma != nullptr) {
@@ -461,7 +469,7 @@ StreamPlan plan_stream(const GemvQArgs& a, int mb, const LaunchEnv& env) {
     StreamParams& p = pl.p;
     p.W = a.W; p.X = a.X; p.Y = a.Y; p.gamma = a.gamma; p.err = env.err_word;
     p.M = mb; p.N = a.N; p.K = a.K; p.nb = nb; p.gpr = gpr; p.ns = ns;
-    p.y_f32 = a.y_f32 ? 1 : 0; p.eps = a.eps;
+    p.y_f32 = a.y_f32 ? 1 : 0; p.eps = a.eps; p.wait_first = env.wait_first() ? 1 : 0;
     p.off_rowacc = off_rowacc; p.off_sx = off_sx; p.off_x = off_x; p.off_ring = off_ring;
     p.max_rows = max_rows;
     return pl;
@@ -525,7 +533,7 @@ StreamPlan plan_box(const GemvQArgs& a, int mb, const LaunchEnv& env) {
     StreamParams& p = pl.p;
     p.W = a.W; p.X = a.X; p.Y = a.Y; p.gamma = a.gamma; p.err = env.err_word;
     p.M = mb; p.N = a.N; p.K = a.K; p.nb = nb; p.gpr = gpr; p.ns = ns;
-    p.y_f32 = a.y_f32 ? 1 : 0; p.eps = a.eps;
+    p.y_f32 = a.y_f32 ? 1 : 0; p.eps = a.eps; p.wait_first = env.wait_first() ? 1 : 0;
     p.x_src_f16 = a.x_f32 ? 0 : 1;
     p.off_rowacc = off_rowacc; p.off_sx = off_sx; p.off_x = off_x; p.off_ring = off_ring;
     p.max_rows = max_rows;
@@ -626,9 +634,10 @@ bool gemv_q_groupable(const GemvQArgs* ops, int n, const GemvQArgs& b, const Lau
 // fp16-activation bound allows.  The fused RMSNorm form takes it too, behind a pass that normalises the
 // rows into the stream's scratch as fp16 (one more rounding, inside the same bound) - once for all
 // products of a group; rows that are not 16-byte aligned are copied there.
-cudaError_t launch_gemv_q_group(const GemvQArgs* ops, int n, const LaunchEnv& env, cudaStream_t stream, int* launches,
+cudaError_t launch_gemv_q_group(const GemvQArgs* ops, int n, const LaunchEnv& env_in, cudaStream_t stream, int* launches,
                                 const char** name) {
     const GemvQArgs& a = ops[0];
+    LaunchEnv env = env_in;
     const bool fuse = a.gamma != nullptr, copy = !fuse && (reinterpret_cast<uintptr_t>(a.X) & 15u) != 0;
     const size_t row_bytes = static_cast<size_t>(a.K) * 2 + 4;      // a row and its 1/rms
     size_t slab = static_cast<size_t>(a.M);
@@ -643,12 +652,13 @@ cudaError_t launch_gemv_q_group(const GemvQArgs* ops, int n, const LaunchEnv& en
         cudaError_t e = cudaSuccess;
         if (fuse) {
             float* rstd = reinterpret_cast<float*>(static_cast<uint8_t*>(a.norm_scratch) + slab * static_cast<size_t>(a.K) * 2);
-            e = launch_norm_forward(x, a.gamma, nullptr, a.norm_scratch, nullptr, rstd, rows, a.K, a.eps, stream, env.pdl);
+            e = launch_norm_forward(x, a.gamma, nullptr, a.norm_scratch, nullptr, rstd, rows, a.K, a.eps, stream, env.pdl, env.wait_first());
             ++count;
         } else if (copy) {
             e = cudaMemcpyAsync(a.norm_scratch, x, static_cast<size_t>(rows) * a.K * 2, cudaMemcpyDeviceToDevice, stream);
         }
         if (e != cudaSuccess) return e;
+        if (fuse || copy) env.weights_ready = true;        // that waits for what came before this call
         for (int i = 0; i < n; ++i) {
             s[i] = ops[i];
             s[i].M = rows;
@@ -657,6 +667,7 @@ cudaError_t launch_gemv_q_group(const GemvQArgs* ops, int n, const LaunchEnv& en
             s[i].Y = static_cast<uint8_t*>(ops[i].Y) + static_cast<size_t>(m0) * ops[i].N * (a.y_f32 ? 4 : 2);
         }
         e = launch_gemm_q_tc(s, n, env, stream, &count);
+        env.weights_ready = true;
         if (e != cudaSuccess) return e;      // cudaErrorNotSupported only on the first slab: the others differ in rows alone
     }
     if (launches) *launches += count;
@@ -666,8 +677,9 @@ cudaError_t launch_gemv_q_group(const GemvQArgs* ops, int n, const LaunchEnv& en
     return cudaSuccess;
 }
 
-cudaError_t launch_gemv_q(const GemvQArgs& a, const LaunchEnv& env, cudaStream_t stream,
+cudaError_t launch_gemv_q(const GemvQArgs& a, const LaunchEnv& env_in, cudaStream_t stream,
                           int* launches, const char** name) {
+    LaunchEnv env = env_in;
     int count = 0;
     cudaError_t err = cudaSuccess;
     const char* used = "none";
@@ -709,7 +721,7 @@ cudaError_t launch_gemv_q(const GemvQArgs& a, const LaunchEnv& env, cudaStream_t
 
     // Up to kMaxMB activation rows per pass on the integer dot-product kernels.
     int mb = 0;
-    for (int m0 = 0; m0 < a.M && err == cudaSuccess; m0 += mb) {
+    for (int m0 = 0; m0 < a.M && err == cudaSuccess; m0 += mb, env.weights_ready = true) {
         mb = (a.M - m0) < kMaxMB ? (a.M - m0) : kMaxMB;
         GemvQArgs s = a;
         s.X = static_cast<const uint8_t*>(a.X) + static_cast<size_t>(m0) * a.K * xsz;

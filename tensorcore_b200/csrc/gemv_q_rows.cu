@@ -36,6 +36,7 @@ struct RowsParams {
     int cb, chunks;   // blocks per chunk (at most 32), chunks per row
     int max_rows;     // rows of a CTA, rounded up to whole groups
     int x_f32, y_f32;
+    int wait_first;   // the kernel before may write the weights
     int x_vec;        // X and gamma allow 8-byte (fp16) / 16-byte (fp32) loads
     float eps;
     int off_part;
@@ -86,6 +87,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_q_rows_kernel(const Rows
     float4* xs = reinterpret_cast<float4*>(smem);               // [MB][8][nbp]
     float* part = reinterpret_cast<float*>(smem + p.off_part);  // [chunks][max_rows][MB]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (p.wait_first) pdl_wait();
     pdl_launch_dependents();
     const int r0 = static_cast<int>(static_cast<long long>(p.N) * blockIdx.x / gridDim.x);
     const int r1 = static_cast<int>(static_cast<long long>(p.N) * (blockIdx.x + 1) / gridDim.x);
@@ -229,7 +231,7 @@ cudaError_t launch_gemv_q_rows(const GemvQArgs& a, const LaunchEnv& env, cudaStr
     p.nbp = p.nb | 1;
     p.chunks = (p.nb + 31) / 32;
     p.cb = (p.nb + p.chunks - 1) / p.chunks;
-    p.x_f32 = a.x_f32; p.y_f32 = a.y_f32; p.eps = a.eps;
+    p.x_f32 = a.x_f32; p.y_f32 = a.y_f32; p.eps = a.eps; p.wait_first = env.wait_first() ? 1 : 0;
     const uintptr_t mask = a.x_f32 ? 15u : 7u;
     p.x_vec = ((reinterpret_cast<uintptr_t>(a.X) | reinterpret_cast<uintptr_t>(a.gamma)) & mask) == 0;
     const int sms = env.sm_count > 0 ? env.sm_count : 148;

@@ -23,6 +23,10 @@ struct LaunchEnv {
     int sm_count = 0;
     int smem_optin = 0;        // max dynamic shared memory per block (opt-in), bytes
     bool pdl = false;          // launch with programmatic stream serialization
+    // With pdl, whether nothing that may still run on the stream writes the weights: they are then read while the
+    // kernel before runs.  Else a kernel waits for it first, and lets the next one start only after that.
+    bool weights_ready = false;
+    bool wait_first() const { return pdl && !weights_ready; }
     int variant = VARIANT_AUTO;
     uint32_t* err_word = nullptr;  // device-visible word a kernel ORs an error bit into
 };
@@ -240,7 +244,8 @@ cudaError_t launch_gemv_q4_decode_static(const GemvQArgs* ops, int n_ops, const 
 cudaError_t launch_norm_forward(const void* X, const void* gamma, const void* beta /* null = RMSNorm */,
                                 void* Y, float* mean_out /* may be null */, float* rstd_out, int N, int D,
                                 float eps, cudaStream_t stream,
-                                bool pdl = false /* may start while the kernel before it runs */);
+                                bool pdl = false /* may start while the kernel before it runs */,
+                                bool wait_first = false /* the next one only when that has ended */);
 cudaError_t launch_swiglu(const void* gate, const void* up, void* out, int n, cudaStream_t stream);
 cudaError_t launch_rope(void* X, const float* cos_t, const float* sin_t, int batch, int heads, int seq,
                         int head_dim, cudaStream_t stream);

@@ -826,18 +826,31 @@ extern "C" tc_status_t tc_stream_destroy(tc_context* ctx, tc_stream* s) {
 
 namespace {
 
-cudaError_t launch_recorded(tc_context* ctx, const RecordedOp& op, cudaStream_t st, bool pdl,
-                            int* launches, const char** name) {
-    LaunchEnv env = make_env(ctx, pdl);
-    return tcb::launch_gemv_q(op.a, env, st, launches, name);
-}
+// What the operations of a list have written so far.
+struct Written {
+    struct Span { uintptr_t lo, hi; };
+    std::vector<Span> spans;
+    bool overlaps(const void* p, size_t n) const {
+        const uintptr_t lo = reinterpret_cast<uintptr_t>(p);
+        for (const Span& s : spans)
+            if (lo < s.hi && s.lo < lo + n) return true;
+        return false;
+    }
+    void add(const void* p, size_t n) {
+        const uintptr_t lo = reinterpret_cast<uintptr_t>(p);
+        for (const Span& s : spans)
+            if (s.lo <= lo && lo + n <= s.hi) return;      // a list writes the same few buffers over and over
+        spans.push_back({lo, lo + n});
+    }
+};
 
 // The operations of a list in order; neighbours that share their activations (q, k and v; gate and up) run as
 // one launch where their kernel can take several matrices.
 cudaError_t launch_list(tc_context* ctx, const std::vector<RecordedOp>& list, cudaStream_t st, int* launches, const char** name) {
     cudaError_t e = cudaSuccess;
+    Written written;
     for (size_t i = 0; i < list.size() && e == cudaSuccess;) {
-        const LaunchEnv env = make_env(ctx, i > 0);
+        LaunchEnv env = make_env(ctx, i > 0);
         tcb::GemvQArgs group[4];
         int n = 0;
         group[n++] = list[i].a;
@@ -845,14 +858,23 @@ cudaError_t launch_list(tc_context* ctx, const std::vector<RecordedOp>& list, cu
             group[n] = list[i + n].a;
             ++n;
         }
+        // Nothing outside the list runs beside its second operation and those after it.
+        env.weights_ready = true;
+        for (int k = 0; k < n; ++k)
+            if (written.overlaps(list[i + k].a.W, list[i + k].w_bytes)) env.weights_ready = false;
+        for (int k = 0; k < n; ++k) written.add(list[i + k].a.Y, list[i + k].y_bytes);
         if (n > 1) {
             e = tcb::launch_gemv_q_group(group, n, env, st, launches, name);
             if (e == cudaSuccess) { i += n; continue; }
             if (e != cudaErrorNotSupported) break;
             (void)cudaGetLastError();
         }
-        e = launch_recorded(ctx, list[i], st, i > 0, launches, name);
-        ++i;
+        e = cudaSuccess;
+        for (int k = 0; k < n && e == cudaSuccess; ++k) {
+            if (k > 0) env.pdl = ctx->pdl;
+            e = tcb::launch_gemv_q(group[k], env, st, launches, name);
+        }
+        i += n;
     }
     return e;
 }
@@ -1370,7 +1392,7 @@ tc_status_t gemv_common(const GemvCall& c, tc_stream* stream, const char* opname
         if (need > 0 || dq > 0) rooms.lock();
         norm_scratch_for(s0, need, &op.a);
         dequant_scratch_for(s0, dq, &op.a);
-        e = launch_recorded(ctx, op, s0, false, &launches, &name);
+        e = tcb::launch_gemv_q(op.a, make_env(ctx, false), s0, &launches, &name);
     }
     if (e == cudaSuccess) e = finish_output(op.Y, yb, s0);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s0);

@@ -66,13 +66,15 @@ __global__ void __launch_bounds__(256) norm_forward_kernel(const __half* X, cons
 // quantized GEMV (512 rows of 4096) the pass and its launch took 10.8 us as the scalar kernel above.
 template <int V>
 __global__ void __launch_bounds__(256) norm_forward_vec_kernel(const uint4* X, const uint4* gamma, const uint4* beta, uint4* Y,
-                                                               float* mean_out, float* rstd_out, int D, float eps) {
+                                                               float* mean_out, float* rstd_out, int D, float eps, int wait_first) {
     __shared__ double scratch[8];
     // The next kernel's prologue may start; then wait for the one before (launched with programmatic
-    // serialization when it is part of a chain, else this returns at once).
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // serialization when it is part of a chain, else this returns at once).  The other way round where the
+    // next kernel reads ahead what the one before may write.
+    if (!wait_first) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int tid = threadIdx.x, vecs = D >> 3;
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (wait_first) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint4* xr = X + static_cast<size_t>(blockIdx.x) * vecs;
     uint4* yr = Y + static_cast<size_t>(blockIdx.x) * vecs;
     uint4 x[V], g[V];
@@ -184,7 +186,7 @@ __global__ void __launch_bounds__(128) gemm_f16_rows_kernel(const __half* A, con
 }  // namespace
 
 cudaError_t launch_norm_forward(const void* X, const void* gamma, const void* beta, void* Y, float* mean_out,
-                                float* rstd_out, int N, int D, float eps, cudaStream_t stream, bool pdl) {
+                                float* rstd_out, int N, int D, float eps, cudaStream_t stream, bool pdl, bool wait_first) {
     const uintptr_t all = reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(gamma) |
                           reinterpret_cast<uintptr_t>(beta) | reinterpret_cast<uintptr_t>(Y);
     if (D % 8 != 0 || (all & 15u) != 0 || D > 8 * 256 * 8) {
@@ -206,7 +208,7 @@ cudaError_t launch_norm_forward(const void* X, const void* gamma, const void* be
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<const uint4*>(X), static_cast<const uint4*>(gamma),
-                              static_cast<const uint4*>(beta), static_cast<uint4*>(Y), mean_out, rstd_out, D, eps);
+                              static_cast<const uint4*>(beta), static_cast<uint4*>(Y), mean_out, rstd_out, D, eps, wait_first ? 1 : 0);
 }
 
 cudaError_t launch_swiglu(const void* gate, const void* up, void* out, int n, cudaStream_t stream) {
