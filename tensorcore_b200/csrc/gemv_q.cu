@@ -606,7 +606,9 @@ cudaError_t init_gemv_kernels(int smem_optin) {
 }
 
 static bool wants_tc(const GemvQArgs& a, const LaunchEnv& env) {
-    return !a.x_f32 && a.K % 256 == 0 && (env.variant == VARIANT_TC ? a.fmt == FMT_Q4_0 : env.variant == VARIANT_AUTO && tc_rows(a));
+    if (env.variant == VARIANT_TC)
+        return a.fmt == FMT_Q4_0 && !a.x_f32 && a.K % 256 == 0 && (reinterpret_cast<uintptr_t>(a.W) & 15u) == 0;
+    return env.variant == VARIANT_AUTO && tc_rows(a);
 }
 
 bool gemv_q_groupable(const GemvQArgs* ops, int n, const GemvQArgs& b, const LaunchEnv& env) {
@@ -691,11 +693,10 @@ cudaError_t launch_gemv_q(const GemvQArgs& a, const LaunchEnv& env_in, cudaStrea
         if (te != cudaErrorNotSupported) return te;
         (void)cudaGetLastError();
     }
-    // Prefill-sized calls whose K is no multiple of 256: the weights are dequantised once into the
-    // stream's scratch (fp16, the same rounding as above) and multiplied on the tensor cores as a GEMM
-    // with B transposed.
-    if (env.variant == VARIANT_AUTO && a.M >= gemm_min_rows(a.fmt) && !a.x_f32 && !a.y_f32 && a.dequant_scratch &&
-        a.dequant_scratch_bytes >= static_cast<size_t>(a.N) * a.K * 2 && a.K % 32 == 0 &&
+    // Prefill-sized calls that it cannot take: the weights are dequantised once into the stream's scratch
+    // (fp16, the same rounding as above) and multiplied on the tensor cores as a GEMM with B transposed.
+    if (env.variant == VARIANT_AUTO && dequant_once(a) && a.dequant_scratch &&
+        a.dequant_scratch_bytes >= static_cast<size_t>(a.N) * a.K * 2 &&
         (!fuse || (a.norm_scratch && a.norm_scratch_bytes >= static_cast<size_t>(a.M) * a.K * 2 + static_cast<size_t>(a.M) * 4))) {
         cudaError_t e = launch_dequantize(a.W, a.dequant_scratch, a.fmt, a.N, a.K, stream);
         const void* x = a.X;

@@ -44,9 +44,7 @@ struct GemvQArgs {
     // fits); without it that form takes the integer dot-product kernels, four rows per pass
     void* norm_scratch = nullptr;
     size_t norm_scratch_bytes = 0;
-    // scratch of the stream for prefill-sized calls whose K is no multiple of 256 (gemm_min_rows activation
-    // rows or more, fp16 in and out): room for the weights as fp16, N * K halves; with it they are
-    // dequantised once and multiplied on the tensor cores instead of streamed once per four rows
+    // scratch of the stream for the calls of dequant_once: room for the weights as fp16, N * K halves
     void* dequant_scratch = nullptr;
     size_t dequant_scratch_bytes = 0;
 };
@@ -61,9 +59,20 @@ inline int gemm_min_rows(int fmt) { return fmt == 0 ? 96 : 13; }
 // the tensor-core kernel's fixed part (M = 4 back to back: 14336 x 4096 21.3 us on the integer kernel, 11.0
 // on this one; 4096 x 4096 9.6 and 8.0, where the exact weights were kept).  Fewer rows stay on the integer kernels, which do not round the weights.
 inline bool batched_tc_rows(int M, int N, int K) { return M >= 5 || (M == 4 && (K >= 8192 || N > 4096)); }
-// Whether a call with fp16 activations and K % 256 == 0 goes to the tcgen05 kernel by default.
+// Whether a call goes to the tcgen05 kernel by default: its rows are copied 16 bytes at a time, a group of
+// 256 weights whole.
 inline bool tc_rows(const GemvQArgs& a) {
+    if (a.x_f32 || a.K % 256 != 0 || (reinterpret_cast<uintptr_t>(a.W) & 15u) != 0) return false;
     return a.fmt == 0 ? batched_tc_rows(a.M, a.N, a.K) : a.M >= gemm_min_rows(1) && !a.y_f32;
+}
+// Whether the weights of a prefill-sized call are dequantised once, into scratch, and multiplied as a dense GEMM:
+// where the tcgen05 kernel cannot take them (the kernels left would stream them once per four rows).
+constexpr size_t kMaxDequantBytes = static_cast<size_t>(3) << 29;      // 1.5 GB
+inline bool dequant_once(const GemvQArgs& a) {
+    if (a.M < gemm_min_rows(a.fmt) || a.x_f32 || a.y_f32 || a.K % 32 != 0) return false;
+    if (static_cast<size_t>(a.N) * a.K * 2 > kMaxDequantBytes) return false;
+    if ((reinterpret_cast<uintptr_t>(a.W) & 1u) || (!a.gamma && (reinterpret_cast<uintptr_t>(a.X) & 15u))) return false;
+    return !tc_rows(a);
 }
 
 struct DenseNormGemvArgs {

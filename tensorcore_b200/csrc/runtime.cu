@@ -205,7 +205,6 @@ std::mutex g_rooms_mutex;
 std::unordered_map<cudaStream_t, StreamRooms> g_rooms;
 std::vector<void*> g_kept;    // outgrown rooms of captured graphs
 using RoomsLock = std::unique_lock<std::mutex>;
-constexpr size_t kMaxWeightsRoom = static_cast<size_t>(3) << 29;      // 1.5 GB
 
 bool being_captured(cudaStream_t st) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -282,17 +281,11 @@ void dense_scratch_for(tc_context* ctx, cudaStream_t st, tcb::DenseNormGemvArgs*
     a->scratch = static_cast<float*>(d.partial.p); a->scratch_floats = d.partial.bytes / sizeof(float);
     a->counters = static_cast<int*>(d.counters.p); a->counters_n = d.counters.bytes / sizeof(int);
 }
-// Whether the call is prefill-sized: its weights are dequantised once and multiplied as a GEMM.
-bool dequant_gemm_wanted(const tcb::GemvQArgs& a) {
-    return a.M >= tcb::gemm_min_rows(a.fmt) && !a.x_f32 && !a.y_f32 && a.K % 256 != 0 && a.K % 32 == 0 &&
-           static_cast<size_t>(a.N) * a.K * 2 <= kMaxWeightsRoom;
-}
 // Room for the normalised rows of the batched fused RMSNorm GEMV (the tensor-core kernel reads them as
 // plain fp16 activations).
 size_t norm_scratch_need(const tcb::GemvQArgs& a) {
-    if (a.x_f32) return 0;
-    if (dequant_gemm_wanted(a)) return a.gamma ? static_cast<size_t>(a.M) * a.K * 2 + static_cast<size_t>(a.M) * 4 : 0;
-    if (a.K % 256 != 0 || !tcb::tc_rows(a)) return 0;
+    if (tcb::dequant_once(a)) return a.gamma ? static_cast<size_t>(a.M) * a.K * 2 + static_cast<size_t>(a.M) * 4 : 0;
+    if (!tcb::tc_rows(a)) return 0;
     if (!a.gamma && (reinterpret_cast<uintptr_t>(a.X) & 15u) == 0) return 0;
     const size_t rows = a.M < 2048 ? a.M : 2048;      // larger calls go through the scratch in slabs
     return rows * (static_cast<size_t>(a.K) * 2 + 4);
@@ -300,7 +293,7 @@ size_t norm_scratch_need(const tcb::GemvQArgs& a) {
 // Room for the weights as fp16 of a prefill-sized quantized GEMV (a call that finds none keeps the kernels that
 // stream the blocks).
 size_t dequant_scratch_need(const tcb::GemvQArgs& a) {
-    return dequant_gemm_wanted(a) ? static_cast<size_t>(a.N) * a.K * 2 : 0;
+    return tcb::dequant_once(a) ? static_cast<size_t>(a.N) * a.K * 2 : 0;
 }
 void norm_scratch_for(cudaStream_t st, size_t need, tcb::GemvQArgs* a) {
     if (need == 0) return;
@@ -312,7 +305,7 @@ void norm_scratch_for(cudaStream_t st, size_t need, tcb::GemvQArgs* a) {
 void dequant_scratch_for(cudaStream_t st, size_t need, tcb::GemvQArgs* a) {
     if (need == 0) return;
     StreamRooms& d = rooms_of(st);
-    grow_stream_room(d.weights, need, st, false, kMaxWeightsRoom);
+    grow_stream_room(d.weights, need, st, false, tcb::kMaxDequantBytes);
     a->dequant_scratch = d.weights.p;
     a->dequant_scratch_bytes = d.weights.bytes;
 }

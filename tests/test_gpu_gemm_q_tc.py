@@ -166,3 +166,33 @@ def test_captured_call_outlives_a_larger_one(tc, ctx, oracle):
     assert oracle.scaled_rms(y.cpu().numpy(), want) <= 1.1 * np.sqrt(3.0) * ROUND
     assert tc.take_device_error(ctx) == 0
     del graph
+
+
+@pytest.mark.parametrize("fmt", [0, 1])
+@pytest.mark.parametrize("w_off,M,K", [(2, 128, 1024), (8, 128, 1024), (2, 16, 1024), (8, 512, 512)])
+def test_prefill_block_with_weights_at_any_even_address(tc, ctx, oracle, fmt, w_off, M, K):
+    """Weights that no tiled copy can describe although K is a multiple of 256: prefill-sized calls dequantise them once
+    and multiply them as a GEMM - two launches, three with the norm -, smaller ones stream them."""
+    import torch
+    N = 130
+    X, Wq = data(oracle, fmt, M, N, K)
+    g = (1 + 0.1 * np.random.default_rng(8).standard_normal(K)).astype(np.float16)
+    want = oracle.dequant_dot_f64(X.astype(np.float64), Wq, fmt, N)
+    x64 = X.astype(np.float64)
+    wantf = oracle.dequant_dot_f64(x64 / np.sqrt((x64 * x64).mean(axis=1, keepdims=True) + 1e-5) * g, Wq, fmt, N)
+    once = M >= (96 if fmt == 0 else 13)
+    with ctx.buffer_from_array(X) as bx, ctx.buffer_from_array(g) as bg, ctx.buffer(Wq.nbytes + 16) as bw, ctx.buffer(M * N * 2) as by:
+        bw.upload(Wq, w_off)
+        for fused in (False, True):
+            before = tc.launch_count()
+            if fused:
+                tc.raw_fused_rmsnorm_gemv_quantized(ctx, bx.device_ptr(), bg.device_ptr(), bw.device_ptr() + w_off, by.device_ptr(),
+                                                    fmt, M, N, K, 1e-5)
+            else:
+                tc.raw_gemv_quantized(ctx, bx.device_ptr(), bw.device_ptr() + w_off, by.device_ptr(), fmt, M, N, K)
+            torch.cuda.synchronize()
+            assert ("dequant_gemm" if once else "generic_rows") in tc.cuda_last_kernel_name()
+            assert tc.launch_count() - before == (2 + fused if once else (M + 3) // 4)
+            got = by.to_numpy((M, N), np.float16).astype(np.float64)
+            assert oracle.scaled_rms(got, wantf if fused else want) <= 1.1 * np.sqrt(3.0 if fused else 2.0) * ROUND
+    assert tc.take_device_error(ctx) == 0
