@@ -457,7 +457,7 @@ cudaError_t launch_dense_split(const SplitParams& sp, int strips, int smem_optin
         cfg.attrs = attr;
         cfg.numAttrs = 1;
     }
-    cfg.dynamicSmemBytes = 128 + kStages * kStageBytes + static_cast<size_t>(MB) * sp.kc * 2;
+    cfg.dynamicSmemBytes = kSplitSmemBase + static_cast<size_t>(MB) * sp.kc * 2;
     if (static_cast<int>(cfg.dynamicSmemBytes) > smem_optin) return cudaErrorInvalidValue;
     cudaError_t e = cudaFuncSetAttribute(dense_norm_gemv_split_kernel<MB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(cfg.dynamicSmemBytes));
@@ -465,33 +465,40 @@ cudaError_t launch_dense_split(const SplitParams& sp, int strips, int smem_optin
     return cudaLaunchKernelEx(&cfg, dense_norm_gemv_split_kernel<MB>, sp);
 }
 
-// Tiles of the split kernel for one launch of up to kDMaxMB rows.
-void dense_split_shape(int N, int K, int sm_count, int* strips, int* chunks, int* kc) {
-    // The number of K ranges whose waves of tiles take least: three CTAs are resident per SM, and a tile costs
-    // its rows and about 96 rows' time for the row statistics and the fence before its ticket.  4096 x 11008:
-    // ten ranges, one wave of 430 tiles (four tiles per SM before: 602 tiles, a third of a wave left over).
+constexpr int kSplitSmemBase = 128 + kStages * kStageBytes;     // and the normalised K range of every row
+
+// Tiles of the split kernel for launches of up to `mb` rows.
+void dense_split_shape(int mb, int N, int K, int sm_count, int smem_optin, int* strips, int* chunks, int* kc) {
+    // The number of K ranges whose waves of tiles take least: a tile costs its rows and about 96 rows' time for the
+    // row statistics and the fence before its ticket, and as many CTAs are resident per SM as their shared
+    // memory allows, three at most (registers).  4096 x 11008: ten ranges, one wave of 430 tiles (four tiles per SM
+    // before: 602 tiles, a third of a wave left over).
     const int st = (N + kSplitCols - 1) / kSplitCols;
     const int most = (K + 2 * kStageRows - 1) / (2 * kStageRows);
-    int ch = 1;
+    const int optin = smem_optin > 0 ? smem_optin : 48 * 1024;
+    auto rows_of = [&](int c) { return ((K + c - 1) / c + kStageRows - 1) / kStageRows * kStageRows; };
+    int ch = most;
     double best = 0.0;
-    for (int c = 1; c <= most && c <= 256; ++c) {
-        const double waves = static_cast<double>((static_cast<long long>(st) * c + 3 * sm_count - 1) / (3 * sm_count));
+    for (int c = 1; c <= most && (c <= 256 || best == 0.0); ++c) {
+        const long long smem = kSplitSmemBase + static_cast<long long>(mb) * rows_of(c) * 2;
+        if (smem > optin) continue;                                   // the K range of that many rows does not fit
+        // an SM has 1 KB more than one block may take, and every block costs 1 KB of it
+        const long long fit = (optin + 1024) / (smem + 1024), per_wave = (fit < 3 ? fit : 3) * sm_count;
+        const double waves = static_cast<double>((static_cast<long long>(st) * c + per_wave - 1) / per_wave);
         const double cost = waves * (static_cast<double>(K) / c + 96.0);
         if (best == 0.0 || cost < best) { best = cost; ch = c; }
     }
-    int rows = (K + ch - 1) / ch;
-    rows = (rows + kStageRows - 1) / kStageRows * kStageRows;
     *strips = st;
-    *kc = rows;
-    *chunks = (K + rows - 1) / rows;
+    *kc = rows_of(ch);
+    *chunks = (K + *kc - 1) / *kc;
 }
 
 }  // namespace
 
-void dense_norm_gemv_scratch(int M, int N, int K, int sm_count, size_t* floats, size_t* ints) {
+void dense_norm_gemv_scratch(int M, int N, int K, int sm_count, int smem_optin, size_t* floats, size_t* ints) {
     int strips, chunks, kc;
-    dense_split_shape(N, K, sm_count, &strips, &chunks, &kc);
     const int mb = M < kDMaxMB ? M : kDMaxMB;
+    dense_split_shape(mb, N, K, sm_count, smem_optin, &strips, &chunks, &kc);
     *floats = static_cast<size_t>(chunks) * mb * N;
     *ints = static_cast<size_t>(strips);
 }
@@ -503,7 +510,8 @@ cudaError_t launch_dense_norm_gemv(const DenseNormGemvArgs& a, const LaunchEnv& 
     cudaError_t err = cudaSuccess;
     int count = 0;
     size_t need_f = 0, need_i = 0;
-    dense_norm_gemv_scratch(a.M, a.N, a.K, env.sm_count > 0 ? env.sm_count : 148, &need_f, &need_i);
+    const int sms = env.sm_count > 0 ? env.sm_count : 148;
+    dense_norm_gemv_scratch(a.M, a.N, a.K, sms, optin, &need_f, &need_i);
     const bool split = vec && a.scratch && a.counters && a.scratch_floats >= need_f && a.counters_n >= need_i;
     // Five rows or more: the kernels below would read W once per four rows.  Instead the rows are
     // normalised once into the stream's scratch (fp16, as the reference rounds them before its GEMM,
@@ -540,7 +548,7 @@ cudaError_t launch_dense_norm_gemv(const DenseNormGemvArgs& a, const LaunchEnv& 
             sp.partial = a.scratch;
             sp.counters = a.counters;
             int strips = 0;
-            dense_split_shape(a.N, a.K, env.sm_count > 0 ? env.sm_count : 148, &strips, &sp.chunks, &sp.kc);
+            dense_split_shape(a.M < kDMaxMB ? a.M : kDMaxMB, a.N, a.K, sms, optin, &strips, &sp.chunks, &sp.kc);
             switch (mb) {
                 case 1: err = launch_dense_split<1>(sp, strips, optin, stream, env.pdl); break;
                 case 2: err = launch_dense_split<2>(sp, strips, optin, stream, env.pdl); break;

@@ -95,7 +95,7 @@ struct DenseNormGemvArgs {
     int* counters = nullptr;
     size_t counters_n = 0;
 };
-void dense_norm_gemv_scratch(int M, int N, int K, int sm_count, size_t* floats, size_t* ints);
+void dense_norm_gemv_scratch(int M, int N, int K, int sm_count, int smem_optin, size_t* floats, size_t* ints);
 
 // ---------------------------------------------------------------------------------------
 // Persistent decode launch (decode_q4.cu): a list of Q4_0, M = 1 GEMVs as one cooperative kernel.
