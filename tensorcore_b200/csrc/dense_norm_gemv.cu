@@ -247,6 +247,7 @@ constexpr int kRowGroups = kDThreads / 32;   // 8: a warp per row
 constexpr int kStageRows = 32;           // rows of W per ring stage: 16 KB
 constexpr int kStages = 4;               // ring depth: three stages (48 KB) in flight per CTA
 constexpr int kStageBytes = kStageRows * kSplitCols * 2;
+constexpr int kSplitSmemBase = 128 + kStages * kStageBytes;     // and the normalised K range of every row
 
 struct SplitParams {
     DenseParams d;
@@ -464,8 +465,6 @@ cudaError_t launch_dense_split(const SplitParams& sp, int strips, int smem_optin
     if (e != cudaSuccess) return e;
     return cudaLaunchKernelEx(&cfg, dense_norm_gemv_split_kernel<MB>, sp);
 }
-
-constexpr int kSplitSmemBase = 128 + kStages * kStageBytes;     // and the normalised K range of every row
 
 // Tiles of the split kernel for launches of up to `mb` rows.
 void dense_split_shape(int mb, int N, int K, int sm_count, int smem_optin, int* strips, int* chunks, int* kc) {
