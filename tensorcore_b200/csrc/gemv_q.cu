@@ -750,14 +750,14 @@ cudaError_t launch_gemv_q(const GemvQArgs& a, const LaunchEnv& env_in, cudaStrea
             used = a.fmt == FMT_Q4_0 ? "q4_0_gemv_stream_sm100" : "q8_0_gemv_stream_sm100";
         } else {
             // Rows no tiled or bulk copy can describe: a lane per block, as many rows as fit shared memory;
-            // weights at an odd address or very long rows take the byte-wise kernel.
+            // weights at an odd address or very long rows take the byte-wise kernel, all of the pass at once.
             cudaError_t re = cudaErrorNotSupported;
-            for (;; mb = (mb + 1) / 2) {
-                s.M = mb;
+            for (int fit = mb; fit >= 1 && re == cudaErrorNotSupported; fit /= 2) {
+                s.M = fit;
                 re = launch_gemv_q_rows(s, env, stream);
-                if (re != cudaErrorNotSupported || mb == 1) break;
             }
             if (re != cudaErrorNotSupported) {
+                mb = s.M;
                 err = re;
                 used = a.fmt == FMT_Q4_0 ? "q4_0_gemv_generic_rows_sm100" : "q8_0_gemv_generic_rows_sm100";
                 ++count;

@@ -46,3 +46,21 @@ def test_any_weight_and_activation_address(tc, ctx, oracle, fmt, w_off, x_off):
         tc.raw_gemv_quantized(ctx, bx.device_ptr() + x_off, bw.device_ptr() + w_off, by.device_ptr(), fmt, M, N, K, "f16", "f32")
         torch.cuda.synchronize()
         assert oracle.scaled_rms(by.to_numpy((M, N), np.float32).astype(np.float64), want) <= 2e-6
+
+
+@pytest.mark.parametrize("M,launches", [(1, 1), (4, 1), (7, 2)])
+def test_weights_at_an_odd_address_take_four_rows_a_launch(tc, ctx, oracle, M, launches):
+    import torch
+    N, K = 70, 1120
+    rng = np.random.default_rng(M)
+    Wq = oracle.quantize_weights((rng.standard_normal((N, K)) * 0.02).astype(np.float16), 0)
+    X = rng.standard_normal((M, K)).astype(np.float16)
+    want = oracle.dequant_dot_f64(X.astype(np.float64), Wq, 0, N)
+    with ctx.buffer_from_array(X) as bx, ctx.buffer(Wq.nbytes + 16) as bw, ctx.buffer(M * N * 4) as by:
+        bw.upload(Wq, 1)
+        before = tc.launch_count()
+        tc.raw_gemv_quantized(ctx, bx.device_ptr(), bw.device_ptr() + 1, by.device_ptr(), 0, M, N, K, "f16", "f32")
+        torch.cuda.synchronize()
+        assert tc.launch_count() - before == launches
+        assert tc.cuda_last_kernel_name() == "q4_0_gemv_generic_sm100"
+        assert oracle.scaled_rms(by.to_numpy((M, N), np.float32).astype(np.float64), want) <= 2e-6
