@@ -752,7 +752,7 @@ cudaError_t launch_gemv_q(const GemvQArgs& a, const LaunchEnv& env_in, cudaStrea
             // Rows no tiled or bulk copy can describe: a lane per block, as many rows as fit shared memory;
             // weights at an odd address or very long rows take the byte-wise kernel, all of the pass at once.
             cudaError_t re = cudaErrorNotSupported;
-            for (int fit = mb; fit >= 1 && re == cudaErrorNotSupported; fit /= 2) {
+            for (int fit = mb; fit >= 1 && re == cudaErrorNotSupported; fit = fit > 1 ? (fit + 1) / 2 : 0) {
                 s.M = fit;
                 re = launch_gemv_q_rows(s, env, stream);
             }
