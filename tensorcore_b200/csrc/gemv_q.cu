@@ -643,8 +643,13 @@ cudaError_t launch_gemv_q_group(const GemvQArgs* ops, int n, const LaunchEnv& en
     const bool fuse = a.gamma != nullptr, copy = !fuse && (reinterpret_cast<uintptr_t>(a.X) & 15u) != 0;
     const size_t row_bytes = static_cast<size_t>(a.K) * 2 + 4;      // a row and its 1/rms
     size_t slab = static_cast<size_t>(a.M);
-    if (fuse || copy) slab = a.norm_scratch ? a.norm_scratch_bytes / row_bytes : 0;
-    if (slab > static_cast<size_t>(a.M)) slab = static_cast<size_t>(a.M);
+    if (fuse || copy) {
+        // As few slabs as the row limit asks for, equal but for whole tiles of 256 rows, however large the room has
+        // become: the arithmetic of a row follows the slab's shape.  A smaller room (a captured stream) means more.
+        slab = a.M <= kNormRoomRows ? a.M : norm_slab_rows(a.M);
+        const size_t room = a.norm_scratch ? a.norm_scratch_bytes / row_bytes : 0;
+        if (slab > room) slab = room;
+    }
     if (slab == 0) return cudaErrorNotSupported;
     int count = 0;
     for (int m0 = 0; m0 < a.M; m0 += static_cast<int>(slab)) {

@@ -65,6 +65,13 @@ inline bool tc_rows(const GemvQArgs& a) {
     if (a.x_f32 || a.K % 256 != 0 || (reinterpret_cast<uintptr_t>(a.W) & 15u) != 0) return false;
     return a.fmt == 0 ? batched_tc_rows(a.M, a.N, a.K) : a.M >= gemm_min_rows(1) && !a.y_f32;
 }
+// Rows that a fused call of it normalises at a time, at most, and the slab of a larger one: equal slabs but for
+// whole tiles of 256 rows (a last slab of a few rows would read all the weights again for them).
+constexpr int kNormRoomRows = 2048;
+inline int norm_slab_rows(int M) {
+    const int n = (M + kNormRoomRows - 1) / kNormRoomRows;
+    return ((M + n - 1) / n + 255) / 256 * 256;
+}
 // Whether the weights of a prefill-sized call are dequantised once, into scratch, and multiplied as a dense GEMM:
 // where the tcgen05 kernel cannot take them (the kernels left would stream them once per four rows).
 constexpr size_t kMaxDequantBytes = static_cast<size_t>(3) << 29;      // 1.5 GB

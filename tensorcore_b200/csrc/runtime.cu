@@ -287,7 +287,7 @@ size_t norm_scratch_need(const tcb::GemvQArgs& a) {
     if (tcb::dequant_once(a)) return a.gamma ? static_cast<size_t>(a.M) * a.K * 2 + static_cast<size_t>(a.M) * 4 : 0;
     if (!tcb::tc_rows(a)) return 0;
     if (!a.gamma && (reinterpret_cast<uintptr_t>(a.X) & 15u) == 0) return 0;
-    const size_t rows = a.M < 2048 ? a.M : 2048;      // larger calls go through the scratch in slabs
+    const size_t rows = a.M <= tcb::kNormRoomRows ? a.M : tcb::norm_slab_rows(a.M);      // larger calls go through the scratch in slabs
     return rows * (static_cast<size_t>(a.K) * 2 + 4);
 }
 // Room for the weights as fp16 of a prefill-sized quantized GEMV (a call that finds none keeps the kernels that

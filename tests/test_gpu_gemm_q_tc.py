@@ -196,3 +196,32 @@ def test_prefill_block_with_weights_at_any_even_address(tc, ctx, oracle, fmt, w_
             got = by.to_numpy((M, N), np.float16).astype(np.float64)
             assert oracle.scaled_rms(got, wantf if fused else want) <= 1.1 * np.sqrt(3.0 if fused else 2.0) * ROUND
     assert tc.take_device_error(ctx) == 0
+
+
+def test_large_fused_call_does_not_depend_on_the_room_of_earlier_ones(tc, ctx, oracle):
+    """3500 rows with fp32 results go through the room for normalised rows in slabs of the call's own, whatever
+    size the room has grown to: the same bits."""
+    import torch
+    M, N, K = 3500, 1280, 2048
+    X, Wq = data(oracle, 0, 64, N, K)
+    x = torch.from_numpy(X).cuda().repeat(128, 1)
+    g, w = torch.ones(4 * K, dtype=torch.float16, device="cuda"), torch.from_numpy(Wq).cuda()
+    big_w = torch.zeros(128 * 4 * K // 32 * 18, dtype=torch.uint8, device="cuda")
+    outs = [torch.zeros(M, N, dtype=torch.float32, device="cuda") for _ in range(2)]
+    y = torch.zeros(2048, 128, dtype=torch.float32, device="cuda")
+    with ctx.stream() as s:
+        st = s.cuda_handle()
+        torch.cuda.synchronize()
+
+        def call(rows, weights, out, n, k):
+            tc.raw_fused_rmsnorm_gemv_quantized(ctx, x.data_ptr(), g.data_ptr(), weights.data_ptr(), out.data_ptr(), 0, rows, n, k,
+                                                1e-5, "f16", "f32", st)
+        call(M, w, outs[0], N, K)
+        call(2048, big_w, y, 128, 4 * K)         # a room four times as large
+        call(M, w, outs[1], N, K)
+        torch.cuda.synchronize()
+    assert torch.equal(outs[0], outs[1])
+    assert torch.equal(outs[0][:64], outs[0][1792:1856])      # the same rows in the other slab
+    want = oracle.fused_rmsnorm_gemv_quantized_f32(X[:8].astype(np.float32), np.ones(K, np.float32), Wq, 0, N)
+    assert oracle.scaled_rms(outs[0][:8].cpu().numpy(), want) <= 1.1 * np.sqrt(2.0) * ROUND
+    assert tc.take_device_error(ctx) == 0
