@@ -126,7 +126,7 @@ def test_many_small_probabilities_beside_a_large_one(tc, ctx, D, Sq, Sk, gap):
     p = np.exp(-gap)
     want = (Sk - 1) * p / (1.0 + (Sk - 1) * p) * V[0, 0, 1].astype(np.float64)
     assert want.min() > 2.0 ** -14
-    assert (np.abs(got - want) <= (2.0 ** -11 + 1e-5) * want + Sk * 2.0 ** -40 * V.max()).all()
+    assert (np.abs(got - want) <= (2.0 ** -11 + 1e-5) * want + Sk * 2.0 ** -40 * float(V.max())).all()
 
 
 @pytest.mark.parametrize("D", [64, 96, 128])
