@@ -614,6 +614,7 @@ static bool wants_tc(const GemvQArgs& a, const LaunchEnv& env) {
 bool gemv_q_groupable(const GemvQArgs* ops, int n, const GemvQArgs& b, const LaunchEnv& env) {
     const GemvQArgs& a = ops[0];
     if (n >= 4 || !wants_tc(a, env) || !wants_tc(b, env)) return false;
+    if (env.variant == VARIANT_AUTO && (dequant_once(a) || dequant_once(b))) return false;
     if (a.fmt != b.fmt || a.M != b.M || a.K != b.K || a.X != b.X || a.gamma != b.gamma || a.eps != b.eps || a.y_f32 != b.y_f32)
         return false;
     const size_t wb = static_cast<size_t>(a.K / 32) * (a.fmt == FMT_Q4_0 ? 18 : 34), ysz = a.y_f32 ? 4 : 2;
@@ -693,13 +694,8 @@ cudaError_t launch_gemv_q(const GemvQArgs& a, const LaunchEnv& env_in, cudaStrea
     const size_t xsz = a.x_f32 ? 4 : 2, ysz = a.y_f32 ? 4 : 2;
     const bool fuse = a.gamma != nullptr;
 
-    if (wants_tc(a, env)) {
-        const cudaError_t te = launch_gemv_q_group(&a, 1, env, stream, launches, name);
-        if (te != cudaErrorNotSupported) return te;
-        (void)cudaGetLastError();
-    }
-    // Prefill-sized calls that it cannot take: the weights are dequantised once into the stream's scratch
-    // (fp16, the same rounding as above) and multiplied on the tensor cores as a GEMM with B transposed.
+    // The weights are dequantised once into the stream's scratch (fp16, the rounding of the tcgen05 kernel) and
+    // multiplied on the tensor cores as a GEMM with B transposed.
     if (env.variant == VARIANT_AUTO && dequant_once(a) && a.dequant_scratch &&
         a.dequant_scratch_bytes >= static_cast<size_t>(a.N) * a.K * 2 &&
         (!fuse || (a.norm_scratch && a.norm_scratch_bytes >= static_cast<size_t>(a.M) * a.K * 2 + static_cast<size_t>(a.M) * 4))) {
@@ -722,6 +718,11 @@ cudaError_t launch_gemv_q(const GemvQArgs& a, const LaunchEnv& env_in, cudaStrea
             return cudaSuccess;
         }
         if (e != cudaErrorNotSupported) return e;
+        (void)cudaGetLastError();
+    }
+    if (wants_tc(a, env)) {
+        const cudaError_t te = launch_gemv_q_group(&a, 1, env, stream, launches, name);
+        if (te != cudaErrorNotSupported) return te;
         (void)cudaGetLastError();
     }
 

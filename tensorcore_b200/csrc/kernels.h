@@ -67,19 +67,32 @@ inline bool tc_rows(const GemvQArgs& a) {
 }
 // Rows that a fused call of it normalises at a time, at most, and the slab of a larger one: equal slabs but for
 // whole tiles of 256 rows (a last slab of a few rows would read all the weights again for them).
-constexpr int kNormRoomRows = 2048;
+constexpr int kNormRoomRows = 4096;
 inline int norm_slab_rows(int M) {
     const int n = (M + kNormRoomRows - 1) / kNormRoomRows;
     return ((M + n - 1) / n + 255) / 256 * 256;
 }
 // Whether the weights of a prefill-sized call are dequantised once, into scratch, and multiplied as a dense GEMM:
-// where the tcgen05 kernel cannot take them (the kernels left would stream them once per four rows).
+// where the tcgen05 kernel cannot take them (the kernels left would stream them once per four rows), and
+// where the rows are so many that one pass over the weights costs less than dequantising them again for each
+// 256 rows, in a kernel that does not overlap a tile's read-out with the next tile.  That overhead weighs less the
+// longer K is.  Back to back, microseconds, tcgen05 kernel / dequantised copy and GEMM:
+//   rows                          2048        3072        4096        8192
+//   Q4_0 14336 x 4096          191 / 208   306 / 275   409 / 375   834 / 707
+//   Q8_0 14336 x 4096          214 / 232   342 / 301   457 / 420   911 / 778
+//   Q4_0 4096 x 4096            65 /  70    96 /  94   125 / 105   231 / 206
+//   Q4_0 4096 x 14336          182 / 183   286 / 303   367 / 338   764 / 678
+//   Q4_0 1024 x 4096            33 /  43    34 /  48    34 /  50    69 /  59
+// (the last row is bound by its launches: hence a least amount of work, too)
+inline bool dequant_pays(const GemvQArgs& a) {
+    return a.M >= (a.K <= 8192 ? 3072 : 4096) && static_cast<double>(a.M) * a.N * a.K >= 34359738368.0;      // 2^35
+}
 constexpr size_t kMaxDequantBytes = static_cast<size_t>(3) << 29;      // 1.5 GB
 inline bool dequant_once(const GemvQArgs& a) {
     if (a.M < gemm_min_rows(a.fmt) || a.x_f32 || a.y_f32 || a.K % 32 != 0) return false;
     if (static_cast<size_t>(a.N) * a.K * 2 > kMaxDequantBytes) return false;
     if ((reinterpret_cast<uintptr_t>(a.W) & 1u) || (!a.gamma && (reinterpret_cast<uintptr_t>(a.X) & 15u))) return false;
-    return !tc_rows(a);
+    return !tc_rows(a) || dequant_pays(a);
 }
 
 struct DenseNormGemvArgs {

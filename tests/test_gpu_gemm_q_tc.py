@@ -199,10 +199,10 @@ def test_prefill_block_with_weights_at_any_even_address(tc, ctx, oracle, fmt, w_
 
 
 def test_large_fused_call_does_not_depend_on_the_room_of_earlier_ones(tc, ctx, oracle):
-    """3500 rows with fp32 results go through the room for normalised rows in slabs of the call's own, whatever
+    """4700 rows with fp32 results go through the room for normalised rows in slabs of the call's own, whatever
     size the room has grown to: the same bits."""
     import torch
-    M, N, K = 3500, 1280, 2048
+    M, N, K = 4700, 1280, 2048
     X, Wq = data(oracle, 0, 64, N, K)
     x = torch.from_numpy(X).cuda().repeat(128, 1)
     g, w = torch.ones(4 * K, dtype=torch.float16, device="cuda"), torch.from_numpy(Wq).cuda()
@@ -217,11 +217,62 @@ def test_large_fused_call_does_not_depend_on_the_room_of_earlier_ones(tc, ctx, o
             tc.raw_fused_rmsnorm_gemv_quantized(ctx, x.data_ptr(), g.data_ptr(), weights.data_ptr(), out.data_ptr(), 0, rows, n, k,
                                                 1e-5, "f16", "f32", st)
         call(M, w, outs[0], N, K)
-        call(2048, big_w, y, 128, 4 * K)         # a room four times as large
+        call(2048, big_w, y, 128, 4 * K)         # a room more than three times as large
         call(M, w, outs[1], N, K)
         torch.cuda.synchronize()
     assert torch.equal(outs[0], outs[1])
-    assert torch.equal(outs[0][:64], outs[0][1792:1856])      # the same rows in the other slab
     want = oracle.fused_rmsnorm_gemv_quantized_f32(X[:8].astype(np.float32), np.ones(K, np.float32), Wq, 0, N)
     assert oracle.scaled_rms(outs[0][:8].cpu().numpy(), want) <= 1.1 * np.sqrt(2.0) * ROUND
+    assert tc.take_device_error(ctx) == 0
+
+
+@pytest.mark.parametrize("fmt,M,N,K", [(0, 8, 19200, 2048), (0, 5, 22016, 2304), (1, 16, 19000, 4096), (0, 33, 19073, 3072), (0, 260, 9600, 2048),
+                                       (1, 130, 20000, 2048)])
+def test_tiles_left_over_after_whole_rounds(tc, ctx, oracle, fmt, M, N, K):
+    """More tiles than SMs and a few left over, whose K is split in a launch of their own (two launches): the first
+    rows of W, and the last ones, which are in it."""
+    X, Wq = data(oracle, fmt, M, N, K)
+    blocks = np.asarray(Wq).reshape(N, -1)
+    some = np.r_[0:64, N - 700:N]
+    want = oracle.dequant_dot_f64(X.astype(np.float64), np.ascontiguousarray(blocks[some]), fmt, len(some))
+    with ctx.buffer_from_array(X) as bx, ctx.buffer_from_array(Wq) as bw, ctx.buffer(M * N * 2) as by:
+        outs = []
+        for _ in range(3):
+            before = tc.launch_count()
+            ctx.gemv_quantized(bx, bw, by, fmt, M, N, K)
+            assert "tcgen05" in tc.cuda_last_kernel_name() and tc.launch_count() - before == 2
+            outs.append(by.to_numpy((M, N), np.float16))
+    assert np.array_equal(outs[0], outs[1]) and np.array_equal(outs[0], outs[2])
+    assert oracle.scaled_rms(outs[0][:, some].astype(np.float64), want) <= 1.1 * np.sqrt(2.0) * ROUND
+    assert tc.take_device_error(ctx) == 0
+
+
+@pytest.mark.parametrize("fused", [False, True])
+@pytest.mark.parametrize("fmt,M,N,K,once", [(0, 3072, 2816, 4096, True), (0, 3071, 2816, 4096, False), (1, 3072, 2816, 4096, True),
+                                            (0, 4096, 1024, 8448, True), (0, 4095, 1024, 8448, False), (1, 3072, 256, 512, False)])
+def test_very_many_rows_dequantise_once(tc, ctx, oracle, fused, fmt, M, N, K, once):
+    """From some thousands of rows on the weights are dequantised once and multiplied as a GEMM (two launches, three
+    with the norm); below, the tcgen05 kernel dequantises on the way (one or two, and the norm pass)."""
+    import torch
+    X, Wq = data(oracle, fmt, 64, N, K)
+    g = (1 + 0.1 * np.random.default_rng(8).standard_normal(K)).astype(np.float16)
+    x, w, gam = torch.from_numpy(X).cuda().repeat((M + 63) // 64, 1)[:M].contiguous(), torch.from_numpy(Wq).cuda(), torch.from_numpy(g).cuda()
+    x64 = X.astype(np.float64)
+    if fused:
+        x64 = x64 / np.sqrt((x64 * x64).mean(axis=1, keepdims=True) + 1e-5) * g
+    want = oracle.dequant_dot_f64(x64[:8], Wq, fmt, N)
+    y = torch.zeros(M, N, dtype=torch.float16, device="cuda")
+    torch.cuda.synchronize()
+    before = tc.launch_count()
+    if fused:
+        tc.raw_fused_rmsnorm_gemv_quantized(ctx, x.data_ptr(), gam.data_ptr(), w.data_ptr(), y.data_ptr(), fmt, M, N, K, 1e-5)
+    else:
+        tc.raw_gemv_quantized(ctx, x.data_ptr(), w.data_ptr(), y.data_ptr(), fmt, M, N, K)
+    torch.cuda.synchronize()
+    launches = tc.launch_count() - before
+    assert launches == (3 if fused else 2) if once else launches - fused in (1, 2)
+    got = y.cpu().numpy()
+    bar = 1.1 * np.sqrt(3.0 if fused else 2.0) * ROUND
+    for at in (0, 64 * ((M - 8) // 64)):                      # the first copy of the rows and the last
+        assert oracle.scaled_rms(got[at:at + 8].astype(np.float64), want) <= bar
     assert tc.take_device_error(ctx) == 0
