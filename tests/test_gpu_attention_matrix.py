@@ -178,3 +178,28 @@ def test_results_at_any_even_address(tc, ctx, D, Sq, Sk, off):
     assert (got[:off] == 0x5A).all() and (got[off + Q.nbytes:] == 0x5A).all()
     for b in [view, hold] + bufs:
         b.close()
+
+
+@pytest.mark.parametrize("B,H,Hkv,Sq,Sk,D,causal", [(5, 8, 8, 512, 1000, 64, False), (5, 8, 8, 512, 1300, 128, False), (2, 8, 8, 1300, 1300, 128, True), (40, 8, 8, 1, 3000, 128, False),
+                                                    (40, 8, 8, 20, 1500, 64, False)])
+def test_many_key_steps_in_one_block(tc, ctx, B, H, Hkv, Sq, Sk, D, causal):
+    """So many row tiles that a block takes eight key steps or more: the ring of K and V is used several times over."""
+    import torch
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(Sk)
+    q, k, v = (torch.randn(B, h, s, D, device="cuda", generator=gen).half() for h, s in ((H, Sq), (Hkv, Sk), (Hkv, Sk)))
+    o = torch.zeros_like(q)
+    torch.cuda.synchronize()
+    bufs = [ctx.buffer_from_ptr(t.data_ptr(), t.numel() * 2) for t in (q, k, v, o)]
+    before = tc.launch_count()
+    tc.attention_forward(ctx, *bufs, B, H, Sq, Sk, D, causal=causal, kv_heads=Hkv)
+    assert tc.launch_count() - before <= 2
+    for b in bufs:
+        b.close()
+    s = torch.matmul(q.double(), k.double().transpose(2, 3)) / D ** 0.5
+    if causal:
+        s = s.masked_fill(~torch.ones(Sq, Sk, dtype=torch.bool, device="cuda").tril(), float("-inf"))
+    want = torch.matmul(torch.softmax(s, dim=3), v.double())
+    err = (((o.double() - want) ** 2).mean() / (want ** 2).mean()).sqrt().item()
+    assert err <= 1.05 * 2.0 ** -11 / np.sqrt(3.0)
+    assert tc.take_device_error(ctx) == 0
