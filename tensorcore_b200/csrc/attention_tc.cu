@@ -51,15 +51,6 @@ struct PrefillBars {
 };
 static_assert(sizeof(PrefillBars) <= kBarBytes, "barrier block too large");
 
-__device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-    if (__all_sync(0xffffffffu, bar_try_wait(bar, parity))) return true;
-    const long long t0 = clock64();
-    for (;;) {
-        if (__all_sync(0xffffffffu, bar_try_wait(bar, parity))) return true;
-        const bool stop = *abort_flag || clock64() - t0 > 2000000000LL;
-        if (__any_sync(0xffffffffu, stop)) return false;
-    }
-}
 __device__ __forceinline__ uint64_t desc128(uint32_t addr, uint32_t lbo) {
     return smem_desc_kmajor(addr, lbo, 1024u) | (static_cast<uint64_t>(kSwizzle128) << 61);
 }

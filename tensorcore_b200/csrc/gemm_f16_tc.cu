@@ -29,6 +29,7 @@
 // bounded: it sets the error word and lets the kernel end.
 #include "kernels.h"
 #include "sm100_prims.cuh"
+#include "tensor_map.h"
 
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -80,17 +81,6 @@ static_assert(sizeof(GemmBars) <= kGemmBarBytes, "barrier block too large");
 // Shared-memory operand descriptor with a layout type; strides in bytes.
 __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo, uint32_t layout) {
     return smem_desc_kmajor(saddr, lbo, sbo) | (static_cast<uint64_t>(layout) << 61);
-}
-
-// Whole-warp bounded wait that leaves the warp converged.
-__device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-    if (__all_sync(0xffffffffu, bar_try_wait(bar, parity))) return true;
-    const long long t0 = clock64();
-    for (;;) {
-        if (__all_sync(0xffffffffu, bar_try_wait(bar, parity))) return true;
-        const bool stop = *abort_flag || clock64() - t0 > 2000000000LL;
-        if (__any_sync(0xffffffffu, stop)) return false;
-    }
 }
 
 // KS: 64-wide K slices per stage.
@@ -300,31 +290,6 @@ gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap,
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, kGemmTmemCols);
     }
-}
-
-// Row-major fp16 matrix [rows][cols] (leading dimension ld) with a box of box_rows x 64 elements (128
-// bytes), written to shared memory with the 128-byte swizzle.
-bool encode_rows_sw128(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
-    using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                                  CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                  CUtensorMapFloatOOBfill);
-    static EncodeFn encode = [] {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            fn = nullptr;
-        return reinterpret_cast<EncodeFn>(fn);
-    }();
-    if (!encode || ld % 8) return false;
-    const cuuint64_t dims[2] = {cols, rows};
-    const cuuint64_t strides[1] = {ld * 2};
-    const cuuint32_t box[2] = {64, box_rows};
-    const cuuint32_t estr[2] = {1, 1};
-    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 cudaError_t launch_tile(const GemmParams& p, const void* A, const void* B, int lda, int ldb, bool transpose_b,

@@ -11,18 +11,20 @@
 //     cluster of up to 8 CTAs shares a tile along K when there are fewer tiles than SMs.  The unit of
 //     work is one group of 8 blocks (256 weights) of the 128 rows: a single tiled TMA copy of 128 rows
 //     x 144 (Q4_0) or 272 (Q8_0) raw bytes into a ring.
-//   * Four dequantising warpgroups take the units in turn, one thread per weight row.  A thread turns
-//     64 weights (two blocks) at a time into fp16 q * d - the zero point subtracted exactly, one
-//     rounding, the same value a dequantised copy would hold - in natural K order, and stores them
-//     with tcgen05.st into its own TMEM lane: the MMA's A operand (128 lanes = 128 weight rows) lives
-//     in tensor memory, in two or three slots of 32 columns per warpgroup, so that a warpgroup
-//     fills one slot while the MMAs read the other.
+//   * Four dequantising warpgroups (two with more than 64 columns) take the units in turn, one thread per
+//     weight row.  A thread turns 64 weights (two blocks) at a time into fp16 q * d - the zero point
+//     subtracted exactly, one rounding, the same value a dequantised copy would hold - in natural K order,
+//     and stores them with tcgen05.st into its own TMEM lane: the MMA's A operand (128 lanes = 128
+//     weight rows) lives in tensor memory, in slots of 32 columns (two to four per warpgroup), so that
+//     a warpgroup fills one slot while the MMAs read the other.
 //   * Activations arrive as plain 128-byte-swizzled K-major tiles by TMA (natural K order needs no
 //     shuffling by threads); rows past M read as zeros.
-//   * One issuing thread per accumulator: tcgen05.mma M128 x NB x K16, fp32 accumulate.  A thread can
-//     issue one MMA per about 112 clocks whatever its N, so up to 64 columns four threads issue, each
-//     for one warpgroup into an accumulator of its own, with 128 columns two, with 256 columns (128
-//     clocks of tensor work per MMA) one; the accumulators are added in the epilogue in a fixed order.
+//   * One issuing warp per accumulator: tcgen05.mma M128 x NB x K16, fp32 accumulate.  With up to 64 columns four
+//     warps issue, each for one warpgroup into an accumulator of its own, with 128 columns two, with 256
+//     columns (128 clocks of tensor work per MMA) one; the accumulators are added in the epilogue in a
+//     fixed order.  An MMA takes 39 clocks to issue (N up to 64; 66 and 130 at 128 and 256), so the 16 of a
+//     unit are 624 of the 970 clocks a unit takes at 8 rows: two issuers might do.  Four date from an MMA that
+//     took 112 clocks, and fewer have not been measured.
 //   * Epilogue: tcgen05.ld, then a direct store, or with a K split a fixed-order sum over the cluster
 //     through distributed shared memory.  Results do not depend on timing.
 //
@@ -158,17 +160,6 @@ __device__ __forceinline__ void load_quarter(uint32_t row, uint32_t (&g)[4 * QFm
     for (int v = 0; v < F::kVec; ++v) {
         const uint4 t = lds128(row + at + 16 * v);
         g[4 * v] = t.x; g[4 * v + 1] = t.y; g[4 * v + 2] = t.z; g[4 * v + 3] = t.w;
-    }
-}
-
-// Whole-warp bounded wait that leaves the warp converged.
-__device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-    if (__all_sync(0xffffffffu, bar_try_wait(bar, parity))) return true;
-    const long long t0 = clock64();
-    for (;;) {
-        if (__all_sync(0xffffffffu, bar_try_wait(bar, parity))) return true;
-        const bool stop = *abort_flag || clock64() - t0 > 2000000000LL;
-        if (__any_sync(0xffffffffu, stop)) return false;
     }
 }
 
@@ -550,13 +541,14 @@ cudaError_t launch_gemm_q_tc(const GemvQArgs* ops, int n_ops, const LaunchEnv& e
     // clusters can all be resident at once, so that the split shortens the K loop instead of queueing, and
     // whose CTAs keep a unit for each of four warpgroups (8 rows, split 1 / 2 / 4 / 8: 4096 x 1024 3.4 / 4.5 /
     // 6.2 us, 4096 x 2048 5.1 / 5.0 / 6.5, 2048 x 4096 - / 6.5 / 4.7 / 10.5, 1024 x 8192 15.9 / 10.1 / 6.3 / 6.0).
+    const char* const forced = std::getenv("TC_TC_SPLIT");
     auto split_for = [&](int n) {
         int split = 1;
         for (int s = 8; s > 1; --s) {
             if (4 * s > p.groups || static_cast<long long>(n) * s > env.sm_count) continue;
             if (n <= max_active_clusters(s, env.smem_optin)) { split = s; break; }
         }
-        if (const char* s = std::getenv("TC_TC_SPLIT")) split = std::atoi(s);
+        if (forced) split = std::atoi(forced);
         if (split > 8) split = 8;
         if (split > p.groups) split = p.groups;
         if (split < 1 || p.off_x + red_bytes > env.smem_optin) split = 1;
@@ -567,7 +559,7 @@ cudaError_t launch_gemm_q_tc(const GemvQArgs* ops, int n_ops, const LaunchEnv& e
     // 20.5 -> 18.8 us).
     int first = tiles;
     const int left = env.sm_count > 0 ? tiles % env.sm_count : 0;
-    if (tiles > env.sm_count && left > 0 && !std::getenv("TC_TC_SPLIT") && split_for(left) > 1) first = tiles - left;
+    if (tiles > env.sm_count && left > 0 && !forced && split_for(left) > 1) first = tiles - left;
 
     QtcMaps maps;
     const int gb = a.fmt == FMT_Q4_0 ? 144 : 272;

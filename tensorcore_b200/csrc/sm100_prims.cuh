@@ -58,6 +58,16 @@ __device__ __forceinline__ bool bar_wait_warp(uint64_t* bar, uint32_t parity, vo
     if (ok) ok = bar_try_wait(bar, parity, 0u) ? 1 : 0;
     return __all_sync(0xffffffffu, ok) != 0;
 }
+// The same with every lane polling: for warps that wait often and have nothing to do meanwhile.
+__device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+    if (__all_sync(0xffffffffu, bar_try_wait(bar, parity))) return true;
+    const long long t0 = clock64();
+    for (;;) {
+        if (__all_sync(0xffffffffu, bar_try_wait(bar, parity))) return true;
+        const bool stop = *abort_flag || clock64() - t0 > 2000000000LL;
+        if (__any_sync(0xffffffffu, stop)) return false;
+    }
+}
 __device__ __forceinline__ void fence_barrier_init() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }

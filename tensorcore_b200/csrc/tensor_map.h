@@ -60,6 +60,20 @@ inline bool encode_f16_slices_sw128(CUtensorMap* map, const void* base, uint64_t
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Row-major 16-bit matrix [rows][cols] (leading dimension ld, a multiple of 8) with a box of box_rows x 64
+// elements (128 bytes), written to shared memory with the 128-byte swizzle.  Parts outside read as zeros.
+inline bool encode_rows_sw128(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
+    const TensorMapEncodeFn encode = tensor_map_encoder();
+    if (!encode || ld % 8) return false;
+    const cuuint64_t dims[2] = {cols, rows};
+    const cuuint64_t strides[1] = {ld * 2};
+    const cuuint32_t box[2] = {64, box_rows};
+    const cuuint32_t estr[2] = {1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // fp16 [heads][rows][cols] as boxes of box_rows x 64 elements of one head, written to shared memory with the
 // 128-byte swizzle: a load at (64 * slab, row, head).  Rows past the head's end read as zeros.
 inline bool encode_heads_sw128(CUtensorMap* map, const void* base, uint64_t heads, uint64_t rows, uint64_t cols, uint32_t box_rows) {
