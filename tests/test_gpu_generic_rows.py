@@ -64,3 +64,37 @@ def test_weights_at_an_odd_address_take_four_rows_a_launch(tc, ctx, oracle, M, l
         assert tc.launch_count() - before == launches
         assert tc.cuda_last_kernel_name() == "q4_0_gemv_generic_sm100"
         assert oracle.scaled_rms(by.to_numpy((M, N), np.float32).astype(np.float64), want) <= 2e-6
+
+
+@pytest.mark.parametrize("fmt", [0, 1])
+def test_fp32_sums_are_closer_than_one_chain_per_block(tc, ctx, oracle, fmt):
+    """The order of additions: against 64 bits the kernel is closer than 32 fused multiply-adds in a row per block,
+    then the scale, added over 32 lanes' blocks in a tree (restated here in numpy; a few thousand results, so that
+    the two errors stand apart by many times their scatter)."""
+    M, N, K = 3, 1500, 4128
+    rng = np.random.default_rng(4128 + fmt)
+    Wq = oracle.quantize_weights((rng.standard_normal((N, K)) * 0.02).astype(np.float16), fmt)
+    X = rng.standard_normal((M, K)).astype(np.float32)
+    want = oracle.dequant_dot_f64(X.astype(np.float64), Wq, fmt, N)
+    with ctx.buffer_from_array(X) as bx, ctx.buffer_from_array(Wq) as bw, ctx.buffer(M * N * 4) as by:
+        tc.gemv_quantized_ex(ctx, bx, bw, by, fmt, M, N, K, "f32", "f32", None)
+        assert "generic_rows" in tc.cuda_last_kernel_name()
+        got = by.to_numpy((M, N), np.float32).astype(np.float64)
+    blocks = Wq.reshape(N, K // 32, -1)
+    d = blocks[:, :, :2].copy().view(np.float16)[:, :, 0].astype(np.float32)
+    qs = blocks[:, :, 2:]
+    q = np.concatenate([qs & 15, qs >> 4], axis=2).astype(np.float32) - 8 if fmt == 0 else qs.copy().view(np.int8).astype(np.float32)
+    chain = np.zeros((M, N), np.float32)
+    for m in range(M):
+        x = X[m].reshape(-1, 32).astype(np.float64)
+        acc = np.zeros(d.shape, np.float32)
+        for i in range(32):
+            acc = (x[None, :, i] * q[:, :, i] + acc).astype(np.float32)
+        lanes = np.zeros((N, 160), np.float32)
+        lanes[:, :d.shape[1]] = acc * d
+        for c in range(0, 160, 32):
+            v = lanes[:, c:c + 32]
+            while v.shape[1] > 1:
+                v = v[:, :v.shape[1] // 2] + v[:, v.shape[1] // 2:]
+            chain[m] += v[:, 0]
+    assert oracle.scaled_rms(got, want) <= 0.92 * oracle.scaled_rms(chain.astype(np.float64), want)
