@@ -467,7 +467,7 @@ cudaError_t launch_dense_split(const SplitParams& sp, int strips, int smem_optin
 }
 
 // Tiles of the split kernel for launches of up to `mb` rows.
-void dense_split_shape(int mb, int N, int K, int sm_count, int smem_optin, int* strips, int* chunks, int* kc) {
+DenseSplit dense_split_shape(int mb, int N, int K, int sm_count, int smem_optin) {
     // The number of K ranges whose waves of tiles take least: a tile costs its rows and about 96 rows' time for the
     // row statistics and the fence before its ticket, and as many CTAs are resident per SM as their shared
     // memory allows, three at most (registers).  4096 x 11008: ten ranges, one wave of 430 tiles (four tiles per SM
@@ -482,24 +482,22 @@ void dense_split_shape(int mb, int N, int K, int sm_count, int smem_optin, int* 
         const long long smem = kSplitSmemBase + static_cast<long long>(mb) * rows_of(c) * 2;
         if (smem > optin) continue;                                   // the K range of that many rows does not fit
         // an SM has 1 KB more than one block may take, and every block costs 1 KB of it
-        const long long fit = (optin + 1024) / (smem + 1024), per_wave = (fit < 3 ? fit : 3) * sm_count;
-        const double waves = static_cast<double>((static_cast<long long>(st) * c + per_wave - 1) / per_wave);
+        const unsigned per_wave = (3 * (smem + 1024) <= optin + 1024 ? 3u : 2 * (smem + 1024) <= optin + 1024 ? 2u : 1u) * sm_count;
+        const double waves = static_cast<double>((static_cast<unsigned long long>(st) * c + per_wave - 1) / per_wave);
         const double cost = waves * (static_cast<double>(K) / c + 96.0);
         if (best == 0.0 || cost < best) { best = cost; ch = c; }
     }
-    *strips = st;
-    *kc = rows_of(ch);
-    *chunks = (K + *kc - 1) / *kc;
+    const int kc = rows_of(ch);
+    return {st, (K + kc - 1) / kc, kc};
 }
 
 }  // namespace
 
-void dense_norm_gemv_scratch(int M, int N, int K, int sm_count, int smem_optin, size_t* floats, size_t* ints) {
-    int strips, chunks, kc;
-    const int mb = M < kDMaxMB ? M : kDMaxMB;
-    dense_split_shape(mb, N, K, sm_count, smem_optin, &strips, &chunks, &kc);
-    *floats = static_cast<size_t>(chunks) * mb * N;
-    *ints = static_cast<size_t>(strips);
+void plan_dense_norm_gemv(DenseNormGemvArgs* a, int sm_count, int smem_optin, size_t* floats, size_t* ints) {
+    const int mb = a->M < kDMaxMB ? a->M : kDMaxMB;
+    a->split = dense_split_shape(mb, a->N, a->K, sm_count > 0 ? sm_count : 148, smem_optin);
+    *floats = static_cast<size_t>(a->split.chunks) * mb * a->N;
+    *ints = static_cast<size_t>(a->split.strips);
 }
 
 cudaError_t launch_dense_norm_gemv(const DenseNormGemvArgs& a, const LaunchEnv& env,
@@ -508,10 +506,9 @@ cudaError_t launch_dense_norm_gemv(const DenseNormGemvArgs& a, const LaunchEnv& 
     const int optin = env.smem_optin > 0 ? env.smem_optin : 48 * 1024;
     cudaError_t err = cudaSuccess;
     int count = 0;
-    size_t need_f = 0, need_i = 0;
-    const int sms = env.sm_count > 0 ? env.sm_count : 148;
-    dense_norm_gemv_scratch(a.M, a.N, a.K, sms, optin, &need_f, &need_i);
-    const bool split = vec && a.scratch && a.counters && a.scratch_floats >= need_f && a.counters_n >= need_i;
+    const size_t need_f = static_cast<size_t>(a.split.chunks) * (a.M < kDMaxMB ? a.M : kDMaxMB) * a.N;
+    const bool split = vec && a.split.chunks > 0 && a.scratch && a.counters && a.scratch_floats >= need_f &&
+                       a.counters_n >= static_cast<size_t>(a.split.strips);
     // Five rows or more: the kernels below would read W once per four rows.  Instead the rows are
     // normalised once into the stream's scratch (fp16, as the reference rounds them before its GEMM,
     // lib/ops/training_cpu.cpp:799-935) and multiplied by W on the tensor cores: W is read once.
@@ -546,8 +543,9 @@ cudaError_t launch_dense_norm_gemv(const DenseNormGemvArgs& a, const LaunchEnv& 
             sp.d = p;
             sp.partial = a.scratch;
             sp.counters = a.counters;
-            int strips = 0;
-            dense_split_shape(a.M < kDMaxMB ? a.M : kDMaxMB, a.N, a.K, sms, optin, &strips, &sp.chunks, &sp.kc);
+            sp.chunks = a.split.chunks;
+            sp.kc = a.split.kc;
+            const int strips = a.split.strips;
             switch (mb) {
                 case 1: err = launch_dense_split<1>(sp, strips, optin, stream, env.pdl); break;
                 case 2: err = launch_dense_split<2>(sp, strips, optin, stream, env.pdl); break;

@@ -95,6 +95,8 @@ inline bool dequant_once(const GemvQArgs& a) {
     return !tc_rows(a) || dequant_pays(a);
 }
 
+// Tiles of the dense split kernel: column strips, K ranges per strip, rows of a K range.
+struct DenseSplit { int strips = 0, chunks = 0, kc = 0; };
 struct DenseNormGemvArgs {
     const void* X = nullptr;      // [M,K] fp16
     const void* gamma = nullptr;  // [K] fp16
@@ -107,15 +109,17 @@ struct DenseNormGemvArgs {
     // the rows are normalised once and multiplied on the tensor cores, W read once
     void* norm_scratch = nullptr;
     size_t norm_scratch_bytes = 0;
-    // scratch of the stream the call runs on (dense_norm_gemv_scratch says how much): partial sums
+    // scratch of the stream the call runs on (plan_dense_norm_gemv says how much): partial sums
     // and one ticket counter per column strip, all zero between launches; without it a slower
     // kernel that needs none is used
+    DenseSplit split;             // set by plan_dense_norm_gemv
     float* scratch = nullptr;
     size_t scratch_floats = 0;
     int* counters = nullptr;
     size_t counters_n = 0;
 };
-void dense_norm_gemv_scratch(int M, int N, int K, int sm_count, int smem_optin, size_t* floats, size_t* ints);
+// Chooses the tiles (a->split) and says how much scratch they need.
+void plan_dense_norm_gemv(DenseNormGemvArgs* a, int sm_count, int smem_optin, size_t* floats, size_t* ints);
 
 // ---------------------------------------------------------------------------------------
 // Persistent decode launch (decode_q4.cu): a list of Q4_0, M = 1 GEMVs as one cooperative kernel.

@@ -274,7 +274,7 @@ void free_rooms() {
 // The functions that hand rooms out; the caller holds g_rooms_mutex and goes on holding it until it has launched.
 void dense_scratch_for(tc_context* ctx, cudaStream_t st, tcb::DenseNormGemvArgs* a) {
     size_t nf = 0, nc = 0;
-    tcb::dense_norm_gemv_scratch(a->M, a->N, a->K, ctx->sm_count, ctx->smem_optin, &nf, &nc);
+    tcb::plan_dense_norm_gemv(a, ctx->sm_count, ctx->smem_optin, &nf, &nc);
     StreamRooms& d = rooms_of(st);
     grow_stream_room(d.partial, nf * sizeof(float), st);
     grow_stream_room(d.counters, nc * sizeof(int), st, true);
