@@ -7,10 +7,11 @@
 //     at a time, through a ring of stages that keeps running across tiles; two sets of accumulators in
 //     tensor memory where they fit, so that one tile is read out and stored while the next one's MMAs
 //     run.  What bounds it is shared-memory bandwidth: a K step of a 256 x 160 tile writes 52 KB and its
-//     MMAs read 72 KB (B once per 128 rows), 970 clocks at 128 bytes each against 640 of tensor work;
-//     1030 measured.  512 x 11008 x 4096: 128-row tiles 47 us, 256-row tiles 41 us; 4096^3 110 and
-//     100 us.  With few rows of A the waits and the issue of a K step are the bound, so a stage then holds
-//     several.
+//     MMAs read 72 KB (B once per 128 rows), 970 clocks at 128 bytes each against 640 of tensor work.  With few
+//     rows of A the waits and the issue of a K step are the bound, so a stage then holds several.
+//   * The issuing lane runs its loop alone, and the rows of a tile are a constant of the instance: a wait of the
+//     whole warp at each stage and a branch between MMAs cost 70 clocks a stage and more (whole calls,
+//     512 x 4096 x 11008 78.4 -> 55.8 us, 1024 x 4096 x 4096 47.9 -> 37.6, 512 x 11008 x 4096 51.5 -> 48.9).
 //   * Operands reach shared memory by tiled TMA copies of 128-byte rows written with the 128-byte
 //     swizzle, the layout the MMA's shared-memory descriptors read directly:
 //       - A ([M][K]) and a transposed B ([N][K]) are K-major: a box of 64 k x 128 (or BN) rows;
@@ -21,10 +22,10 @@
 //     (Which of the descriptor's two strides is which was settled on the device: for the swizzled
 //     MN-major form the first is the stride along N, the second the one along K; for the K-major
 //     form the second is the stride between 8-row groups and the first is not used.)
-//   * One thread issues tcgen05.mma (M128 x N{128,256} x K16, kind::f16, both operands from shared
-//     memory) into BN columns of tensor memory; tcgen05.commit hands the stage back to the producer.
-//   * Four warps read the accumulator (one TMEM lane = one row of the tile per thread), apply
-//     alpha and beta and store fp16.
+//   * That lane issues tcgen05.mma (M128 x N64..256 x K16, kind::f16, both operands from shared
+//     memory) into BN columns of tensor memory per 128 rows; tcgen05.commit hands the stage back to the producer.
+//   * Four warps per 128 rows read the accumulators (one TMEM lane = one row of the tile per thread), apply
+//     alpha and beta and store 16-bit results.
 // Rows and columns past M, N and K are zero-filled by TMA and masked at the store.  Every wait is
 // bounded: it sets the error word and lets the kernel end.
 #include "kernels.h"
@@ -83,11 +84,14 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint
     return smem_desc_kmajor(saddr, lbo, sbo) | (static_cast<uint64_t>(layout) << 61);
 }
 
-// KS: 64-wide K slices per stage.
-template <int KS>
+// KS: 64-wide K slices per stage.  MT: rows of a tile in units of 128; fixed for each instance, because a branch
+// between two MMAs costs the issuing thread more than the MMA (4096^3 in 128 x 256 tiles 134 us with MT a run-time
+// value, 121 with a constant).
+template <int KS, int MT>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap bmap) {
-    const int BN = p.bn, MT = p.mt, tile_rows = kBM * MT;
+    const int BN = p.bn;
+    constexpr int tile_rows = kBM * MT;
     const int kBSlice = BN * kBK * 2, kBStage = KS * kBSlice;
     const uint32_t a_slice = p.a_stage / KS;
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -97,9 +101,9 @@ gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap,
     const int stages = p.stages;
     const uint32_t a_stage = p.a_stage;
     uint8_t* b_ring = a_ring + stages * a_stage;
-    // The warp number by shuffle and one elected lane inside warp-uniform control flow around every copy, MMA
-    // and commit, so that the compiler has their operands as uniform values: under `lane == 0` an MMA took
-    // 70 to 112 clocks to issue, as long as the tensor core works on a 256-wide one.
+    // The warp number by shuffle and an elected lane for copies, MMAs and commits, so that the compiler has their
+    // operands as uniform values: under `lane == 0` an MMA took 70 to 112 clocks to issue, as long as the tensor
+    // core works on a 256-wide one.
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int ksteps = (p.K + kBK * KS - 1) / (kBK * KS);
     // Tiles of C, numbered column-block-major (the CTAs running at the same time share a block of B's
@@ -109,7 +113,7 @@ gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap,
 
     if (tid == 0) {
         for (int i = 0; i < stages; ++i) { bar_init(&bars->full[i], 1); bar_init(&bars->empty[i], 1); }
-        for (int i = 0; i < 2; ++i) { bar_init(&bars->acc_full[i], 1); bar_init(&bars->acc_empty[i], 4 * p.mt); }
+        for (int i = 0; i < 2; ++i) { bar_init(&bars->acc_full[i], 1); bar_init(&bars->acc_empty[i], 4 * MT); }
         bar_init(&bars->drain, 1);
         bars->abort_flag = 0;
         fence_barrier_init();
@@ -173,20 +177,20 @@ gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap,
         // ... and a slice of 64; the second 128 rows lie 128 rows of a slice, or two boxes, further on
         const uint32_t a_next = p.a_mnmajor ? 512u : a_slice >> 4, b_next = p.b_kmajor ? static_cast<uint32_t>(kBSlice) >> 4 : 512u;
         const uint32_t a_half = p.a_mnmajor ? 1024u * KS : 1024u;
-        int s = 0;
-        uint32_t par = 0;
-        uint32_t acc_par = 0;
-        for (int t = blockIdx.x, acc = 0; t < n_tiles && !failed; t += gridDim.x) {
-            // the accumulator's previous tile has been read out
-            if (!wait_all(&bars->acc_empty[acc], acc_par ^ 1u, abort_flag)) { failed = true; break; }
-            tc_fence_after_sync();
-            const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * MT * BN);
-            for (int ks = 0; ks < ksteps; ++ks) {
-                if (!wait_all(&bars->full[s], par, abort_flag)) { failed = true; break; }
+        if (elect_one()) {
+            int s = 0;
+            uint32_t par = 0;
+            uint32_t acc_par = 0;
+            for (int t = blockIdx.x, acc = 0; t < n_tiles && !failed; t += gridDim.x) {
+                // the accumulator's previous tile has been read out
+                if (!bar_wait(&bars->acc_empty[acc], acc_par ^ 1u, abort_flag)) { failed = true; break; }
                 tc_fence_after_sync();
-                const uint64_t adesc = a_form | ((s_u32(a_ring + s * a_stage) >> 4) & 0x3FFFu);
-                const uint64_t bdesc = b_form | ((s_u32(b_ring + s * kBStage) >> 4) & 0x3FFFu);
-                if (elect_one()) {
+                const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * MT * BN);
+                for (int ks = 0; ks < ksteps; ++ks) {
+                    if (!bar_wait(&bars->full[s], par, abort_flag)) { failed = true; break; }
+                    tc_fence_after_sync();
+                    const uint64_t adesc = a_form | ((s_u32(a_ring + s * a_stage) >> 4) & 0x3FFFu);
+                    const uint64_t bdesc = b_form | ((s_u32(b_ring + s * kBStage) >> 4) & 0x3FFFu);
 #pragma unroll
                     for (int sl = 0; sl < KS; ++sl) {
 #pragma unroll
@@ -200,17 +204,15 @@ gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap,
                     }
                     mma_commit(&bars->empty[s]);
                     if (ks + 1 == ksteps) mma_commit(&bars->acc_full[acc]);
+                    if (++s == stages) { s = 0; par ^= 1u; }
                 }
-                __syncwarp();
-                if (++s == stages) { s = 0; par ^= 1u; }
+                if (++acc == p.accs) { acc = 0; acc_par ^= 1u; }
             }
-            if (++acc == p.accs) { acc = 0; acc_par ^= 1u; }
-        }
-        if (failed || *abort_flag) {
-            // every MMA issued so far has completed before the tensor memory is released
-            if (elect_one()) mma_commit(&bars->drain);
-            __syncwarp();
-            bar_wait(&bars->drain, 0, nullptr, 100000000LL);
+            if (failed || *abort_flag) {
+                // every MMA issued so far has completed before the tensor memory is released
+                mma_commit(&bars->drain);
+                bar_wait(&bars->drain, 0, nullptr, 100000000LL);
+            }
         }
     }
     if (failed) {
@@ -330,7 +332,8 @@ cudaError_t launch_tile(const GemmParams& p, const void* A, const void* B, int l
     const long tiles = static_cast<long>((p.N + BN - 1) / BN) * ((p.M + tile_rows - 1) / tile_rows);
     const long sms = env.sm_count > 0 ? env.sm_count : 148;
     const dim3 grid(static_cast<unsigned>(tiles < sms ? tiles : sms));     // one CTA per SM walks the tiles
-    auto* kernel = ks == 4 ? gemm_f16_tc_kernel<4> : ks == 2 ? gemm_f16_tc_kernel<2> : gemm_f16_tc_kernel<1>;
+    auto* kernel = p.mt == 1 ? (ks == 4 ? gemm_f16_tc_kernel<4, 1> : ks == 2 ? gemm_f16_tc_kernel<2, 1> : gemm_f16_tc_kernel<1, 1>)
+                             : (ks == 4 ? gemm_f16_tc_kernel<4, 2> : ks == 2 ? gemm_f16_tc_kernel<2, 2> : gemm_f16_tc_kernel<1, 2>);
     kernel<<<grid, (2 + 4 * p.mt) * 32, smem, stream>>>(q, amap, bmap);
     return cudaGetLastError();
 }
@@ -338,7 +341,8 @@ cudaError_t launch_tile(const GemmParams& p, const void* A, const void* B, int l
 }  // namespace
 
 cudaError_t init_gemm_tc_kernel(int smem_optin) {
-    for (auto* k : {gemm_f16_tc_kernel<1>, gemm_f16_tc_kernel<2>, gemm_f16_tc_kernel<4>}) {
+    for (auto* k : {gemm_f16_tc_kernel<1, 1>, gemm_f16_tc_kernel<2, 1>, gemm_f16_tc_kernel<4, 1>, gemm_f16_tc_kernel<1, 2>, gemm_f16_tc_kernel<2, 2>,
+                    gemm_f16_tc_kernel<4, 2>}) {
         const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin);
         if (e != cudaSuccess) return e;
     }
@@ -360,12 +364,15 @@ cudaError_t launch_gemm_f16_tc(const void* A, const void* B, void* C, int M, int
     p.b_kmajor = transpose_b ? 1 : 0;
     p.bf16 = bf16 ? 1 : 0;
     p.a_mnmajor = transpose_a ? 1 : 0;
-    // Tile: the one whose rounds over the SMs take least, by a model of a 64-wide K step: four MMAs of N / 2 clocks
-    // per 128 rows, each at least 54 (the measured floor with both operands in shared memory), or the
-    // shared-memory traffic - the stage's bytes written once, A read once and B once per 128 rows - at 110
-    // bytes per clock (measured between 105 and 123 over widths of 64 to 256).  256 rows need less
-    // traffic per flop; their two accumulators leave room for a second set only up to 128 columns, so a
-    // tile's read-out is not hidden beyond that.  B as given is laid out in pieces of 64 columns.
+    // Tile: the one whose rounds over the SMs take least, by a model of a 64-wide K step and of what a tile costs
+    // beside its steps.  A step is four MMAs of N / 2 clocks per 128 rows, each at least 54 (the measured floor with
+    // both operands in shared memory), or the shared-memory traffic - the stage's bytes written once, A read
+    // once and B once per 128 rows - at 120 bytes per clock.  256 rows need less traffic per flop; their two
+    // accumulators leave room for a second set only up to 128 columns, so a wider tile's read-out is not hidden:
+    // 10000 clocks a round, against 1500 per 128 rows where it is.  Fitted to whole calls of 144 shapes (M 64 to
+    // 8192, K 1024 to 11008) in eight tiles each: a step of 128 rows x 64 / 128 / 192 / 256 columns takes 180 / 270 /
+    // 300 / 373 ns, of 256 rows x 128 / 192 / 256 365 / 460 / 635 ns; the tile chosen is 0.3 % slower than the
+    // best of the eight on average, 9 % at most.  B as given is laid out in pieces of 64 columns.
     const long sms = env.sm_count > 0 ? env.sm_count : 148;
     const long ksteps = (K + kBK - 1) / kBK;
     double best = 0.0;
@@ -375,10 +382,8 @@ cudaError_t launch_gemm_f16_tc(const void* A, const void* B, void* C, int M, int
         for (int bn = 256; bn >= 64; bn -= transpose_b ? 16 : 64) {
             const long tiles = tiles_m * ((N + bn - 1) / bn), rounds = (tiles + sms - 1) / sms;
             const int accs = 2 * mt * bn <= static_cast<int>(kGemmTmemCols) ? 2 : 1;
-            const double mma = 4.0 * mt * (bn > 108 ? bn / 2.0 : 54.0), traffic = (a_bytes + bn * kBK * 2L + mt * (kBM + bn) * kBK * 2L) / 110.0;
-            const double read_out = 1000.0 + 8.0 * bn;
-            const double cost = static_cast<double>(rounds) * (ksteps * (mma > traffic ? mma : traffic) + (accs == 1 ? read_out : 0.0)) +
-                                (accs == 1 ? 0.0 : read_out);
+            const double mma = 4.0 * mt * (bn > 108 ? bn / 2.0 : 54.0), traffic = (a_bytes + bn * kBK * 2L + mt * (kBM + bn) * kBK * 2L) / 120.0;
+            const double cost = static_cast<double>(rounds) * (ksteps * (mma > traffic ? mma : traffic) + (accs == 1 ? 10000.0 : 1500.0 * mt));
             if (best == 0.0 || cost < best) { best = cost; p.bn = bn; p.mt = mt; p.accs = accs; }
         }
     }
