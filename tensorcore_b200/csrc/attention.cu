@@ -6,7 +6,7 @@
 // (query - key > window), ALiBi (score -= slope * (query - key)), grouped-query heads.
 //
 //   * head_dim 64 and 128, Q, K and V 16-byte aligned: tensor cores, attention_mma_kernel below for a decode
-//     step (up to 64 query rows per K/V head) and attention_tc.cu for a prefill block.
+//     step or a small block and attention_tc.cu for a prefill block (prefill_block below).
 //   * Other head_dims and addresses: attention_decode_kernel, a streaming pass per query row on the CUDA
 //     cores.  A lane takes a key for the scores (the query rows in shared memory), then the lanes
 //     switch to a slice of D each and walk the step's 32 value rows, eight row loads in flight at a
@@ -198,12 +198,12 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_decode_kernel(const
 // ---------------------------------------------------------------------------------------
 // Matrix kernel, head_dim 64 and 128: scores and outputs on the tensor cores (mma.sync m16n8k16).
 //
-// For decode steps and a few query rows: up to 64 (query, head) pairs that share a K/V head, head fastest,
-// are one tile, so the heads of a grouped-query decode step read the cache once (more rows take
-// attention_tc.cu).  K and V arrive in steps of 64 keys through a ring in shared memory
+// For decode steps and small blocks: up to 64 (query, head) pairs that share a K/V head, head fastest, are one
+// tile, so the heads of a grouped-query decode step read the cache once.  K and V arrive in steps of 64 keys through a ring in shared memory
 // (cp.async, 16-byte pieces, piece index XORed with the row so that ldmatrix is conflict-free).
 //   SPLIT_KEYS (16 rows or fewer): all four warps hold the same rows and take 16 keys of a step each,
-//     with softmax states of their own that are merged at the end.
+//     with softmax states of their own that are merged at the end (a thread per row for the weights, then four
+//     elements a thread at a time: 16 x 16, 8 heads 19.1 us a call with a division and a branch per element).
 //   else: a warp owns 16 of the 64 rows and takes all 64 keys.
 // The scores' products are exact and summed in fp32.  The probabilities are fp32 numbers; for the product with V
 // each is split into two fp16 numbers (attention_math.cuh says to how many bits), which costs a third
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_decode_kernel(const
 // 85 us as a streaming pass of CUDA-core dot products per two heads.
 // ---------------------------------------------------------------------------------------
 constexpr int kStepKeys = 64;
-constexpr int kMmaRows = 64;           // rows (query, head) of a K/V head up to which this kernel is used
+constexpr int kMmaRows = 64;           // rows (query, head) of a tile
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
@@ -241,7 +241,6 @@ template <int D, bool SPLIT_KEYS>
 __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const AttnParams p) {
     asm volatile("griddepcontrol.launch_dependents;");
     using S = MmaShape<D>;
-    constexpr int kTileRows = SPLIT_KEYS ? 16 : 64;
     constexpr int kKeys = SPLIT_KEYS ? 16 : 64;           // keys of a step this warp takes
     constexpr int kNT = kKeys / 8, kPieces = D / 8;
     extern __shared__ __align__(128) uint8_t smem[];
@@ -249,7 +248,8 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, tq = lane & 3;
     const int G = p.Hq / p.Hkv, R = p.Sq * G;
     const int heads = p.B * p.Hkv, bk = blockIdx.x % heads;
-    constexpr int tile0 = 0;
+    const int row_tiles = SPLIT_KEYS ? 1 : (R + kMmaRows - 1) / kMmaRows;
+    const int tile0 = SPLIT_KEYS ? 0 : (row_tiles - 1 - static_cast<int>(blockIdx.x / heads)) * kMmaRows;    // long causal tiles first
     const int b = bk / p.Hkv, hkv = bk % p.Hkv;
     const int chunk = blockIdx.y;
     const __half* Kh = p.K + static_cast<size_t>(bk) * p.Sk * D;
@@ -279,8 +279,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const
         }
     }
     // keys any row of the tile can see, in whole steps from the chunk's start
-    const int r_last = min(R, tile0 + kTileRows) - 1;
-    const int i_min = tile0 / G, i_max = r_last / G;
+    const int i_min = tile0 / G, i_max = (min(R, tile0 + kMmaRows) - 1) / G;
     int k0 = chunk * p.keys_per_chunk, k1 = min(p.Sk, k0 + p.keys_per_chunk);
     if (p.causal) k1 = min(k1, i_max + 1);
     if (p.window > 0 && i_min - p.window > k0) k0 += (i_min - p.window - k0) / kStepKeys * kStepKeys;
@@ -334,13 +333,11 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const
                 mma_16816(s[n], qf[k], bf[0], bf[1]);
                 mma_16816(s[n + 1], qf[k], bf[2], bf[3]);
             }
-        const bool masked = jb + kKeys > k1 || (p.causal && jb + kKeys - 1 > i_min) || p.window > 0 || p.slopes != nullptr;
+        const bool masked = jb + kKeys > k1 || (p.causal && jb + kKeys - 1 > i_min) || p.window > 0;
         // straight-line selects: a branch per element costs more than the arithmetic; a NaN score counts as masked
         float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
-        for (int n = 0; n < kNT; ++n)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) s[n][e] *= p.scale;
+        for (int n = 0; n < kNT; ++n) { scale2(s[n][0], s[n][1], p.scale); scale2(s[n][2], s[n][3], p.scale); }
         if (p.slopes) {
 #pragma unroll
             for (int n = 0; n < kNT; ++n)
@@ -380,9 +377,12 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const
 #pragma unroll
         for (int n = 0; n < kNT; ++n)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                s[n][e] = scaled_exp(s[n][e] - ref[e >> 1]);   // now the probability, 2^15 times
+            for (int e = 0; e < 4; e += 2) {
+                s[n][e] = exp_of(s[n][e] - ref[e >> 1]);       // now the probability ...
+                s[n][e + 1] = exp_of(s[n][e + 1] - ref[e >> 1]);
+                scale2(s[n][e], s[n][e + 1], kProbScale);      // ... 2^15 times
                 l[e >> 1] += s[n][e];
+                l[e >> 1] += s[n][e + 1];
             }
 #pragma unroll
         for (int k = 0; k < kKeys / 16; ++k) {
@@ -437,9 +437,11 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const
             }
         }
     } else {
-        // merge the warps' states through the ring, which everybody has finished reading
+        // Merge the warps' states through the ring, which everybody has finished reading: a thread per row works out
+        // the warps' weights, then all threads go over the elements four at a time.
         float* o_s = reinterpret_cast<float*>(smem);                     // [warp][16][D]
         float* ml_s = o_s + kAttnWarps * 16 * D;                         // [warp][16][2]
+        float* w_s = ml_s + kAttnWarps * 16 * 2;                         // [16][warp]
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
@@ -450,31 +452,53 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const
             if (tq == 0) { ml_s[(warp * 16 + r) * 2] = m[e]; ml_s[(warp * 16 + r) * 2 + 1] = l[e]; }
         }
         __syncthreads();
-        const int rows = min(16, R - tile0);
-        for (int t = tid; t < rows * D; t += kAttnWarps * 32) {
-            const int r = t / D, d = t - r * D;
-            float mm = -INFINITY;
+        auto row_of = [&](int r) { return (static_cast<size_t>(b) * p.Hq + hkv * G + r % G) * p.Sq + r / G; };
+        if (tid < R) {                                                   // at most 16 rows
+            float mm = -INFINITY, ll = 0.f, f[kAttnWarps];
 #pragma unroll
-            for (int w = 0; w < kAttnWarps; ++w) mm = fmaxf(mm, ml_s[(w * 16 + r) * 2]);
-            float ll = 0.f, acc = 0.f;
+            for (int w = 0; w < kAttnWarps; ++w) mm = fmaxf(mm, ml_s[(w * 16 + tid) * 2]);
 #pragma unroll
             for (int w = 0; w < kAttnWarps; ++w) {
-                const float mw = ml_s[(w * 16 + r) * 2];
-                if (mw > -INFINITY) {
-                    const float f = __expf(mw - mm);
-                    ll += ml_s[(w * 16 + r) * 2 + 1] * f;
-                    acc += o_s[(w * 16 + r) * D + d] * f;
-                }
+                const float mw = ml_s[(w * 16 + tid) * 2];
+                f[w] = mw > -INFINITY ? __expf(mw - mm) : 0.f;
+                ll += ml_s[(w * 16 + tid) * 2 + 1] * f[w];
             }
-            const int i = (tile0 + r) / G, h = hkv * G + (tile0 + r) % G;
-            const size_t row = (static_cast<size_t>(b) * p.Hq + h) * p.Sq + i;
-            if (p.chunks == 1) {
-                p.O[row * D + d] = __float2half_rn(ll != 0.f ? acc / ll : 0.f);
-                if (d == 0 && p.LSE) p.LSE[row] = mm + logf(fmaxf(ll, 1e-30f));
+            const float inv = p.chunks > 1 ? 1.f : ll != 0.f ? 1.0f / ll : 0.f;
+#pragma unroll
+            for (int w = 0; w < kAttnWarps; ++w) w_s[tid * kAttnWarps + w] = f[w] * inv;
+            if (p.chunks > 1) {
+                float* dst = p.part + (row_of(tid) * p.chunks + chunk) * (D + 2);
+                dst[0] = mm;
+                dst[1] = ll;
+            } else if (p.LSE) {
+                p.LSE[row_of(tid)] = mm + logf(fmaxf(ll, 1e-30f));
+            }
+        }
+        __syncthreads();
+        for (int t = tid; t < R * (D / 4); t += kAttnWarps * 32) {
+            const int r = t / (D / 4), c = 4 * (t % (D / 4));
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int w = 0; w < kAttnWarps; ++w) {
+                const float4 v = *reinterpret_cast<const float4*>(o_s + (w * 16 + r) * D + c);
+                const float f = w_s[r * kAttnWarps + w];
+                acc.x = fmaf(f, v.x, acc.x); acc.y = fmaf(f, v.y, acc.y);
+                acc.z = fmaf(f, v.z, acc.z); acc.w = fmaf(f, v.w, acc.w);
+            }
+            if (p.chunks > 1) {
+                float2* dst = reinterpret_cast<float2*>(p.part + (row_of(r) * p.chunks + chunk) * (D + 2) + 2 + c);
+                dst[0] = make_float2(acc.x, acc.y);
+                dst[1] = make_float2(acc.z, acc.w);
             } else {
-                float* dst = p.part + (row * p.chunks + chunk) * (D + 2);
-                dst[2 + d] = acc;
-                if (d == 0) { dst[0] = mm; dst[1] = ll; }
+                __half* dst = p.O + row_of(r) * D + c;
+                const uint2 v = make_uint2(pack_h2(acc.x, acc.y), pack_h2(acc.z, acc.w));
+                if (p.o_vec) {
+                    *reinterpret_cast<uint2*>(dst) = v;
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        reinterpret_cast<uint16_t*>(dst)[e] = static_cast<uint16_t>((e < 2 ? v.x : v.y) >> (16 * (e & 1)));
+                }
             }
         }
     }
@@ -524,6 +548,21 @@ int attention_group(int Hq, int Hkv) {
     return per % 2 == 0 ? 2 : 1;
 }
 
+// Whether the tcgen05 kernel takes a call of `heads` K/V heads with R (query, head) pairs each.  It needs about
+// 4 us before its first scores and then takes a step of 128 keys for 128 rows in the time of one step of 64 keys for
+// 64 rows here, so it wins where a block has several steps and there are tiles for more than one wave of this
+// kernel (two CTAs per SM), or so much work that few tiles have to share it.  Whole calls, head_dim 128, tcgen05 /
+// mma.sync kernel, microseconds (8 or 32 heads on 8 K/V heads unless given):
+//   100 x 100, 8 heads 20.3 / 17.9     256 x 256, 32 heads 22.8 / 20.8       512 x 512, 32 heads 27.8 / 37.4
+//   1000 x 128, 32 heads 30.2 / 28.3   4 x 256 x 256, 32 heads 34.2 / 38.8   20 x 1000, 8 heads on 1 27.9 / 19.8
+//   100 x 512, 8 heads 25.6 / 19.2     100 x 512, 32 heads 21.6 / 25.2 (causal)
+bool prefill_block(long long heads, long long R, int Sk, int sms) {
+    if (R <= kMmaRows || Sk <= 128) return false;
+    const long long tiles = heads * ((R + kMmaRows - 1) / kMmaRows);
+    if (Sk <= 256) return tiles > 2LL * sms;
+    return 4 * tiles > sms || tiles * ((Sk + kStepKeys - 1) / kStepKeys) > 640;
+}
+
 // How a row's keys are cut: chunks of keys_per_chunk keys.
 void attention_chunks(int B, int Hq, int Hkv, int Sq, int Sk, bool matrix, int sm_count, int* chunks, int* keys_per_chunk) {
     const int sms = sm_count > 0 ? sm_count : 148;
@@ -544,8 +583,8 @@ void attention_chunks(int B, int Hq, int Hkv, int Sq, int Sk, bool matrix, int s
     // Matrix kernels: the number of chunks whose waves of CTAs (two per SM; one of the prefill kernel) take the
     // fewest key steps, a CTA's start and end counted as two steps and the merge launch as three.
     const long long R = static_cast<long long>(Sq) * (Hq / Hkv);
-    const bool prefill = R > kMmaRows;            // 128-row tiles, one CTA per SM, steps of 128 keys
-    const long long tiles = R <= 16 ? 1 : (prefill ? (R + 127) / 128 : 1);
+    const bool prefill = prefill_block(static_cast<long long>(B) * Hkv, R, Sk, sms);    // 128-row tiles, one CTA per SM, steps of 128 keys
+    const long long tiles = prefill ? (R + 127) / 128 : (R + kMmaRows - 1) / kMmaRows;
     const long long ctas = static_cast<long long>(B) * Hkv * tiles, slots = prefill ? sms : 2LL * sms;
     const int step_keys = prefill ? 128 : kStepKeys, steps = (Sk + step_keys - 1) / step_keys;
     int best = 1;
@@ -561,11 +600,11 @@ void attention_chunks(int B, int Hq, int Hkv, int Sq, int Sk, bool matrix, int s
 }
 
 template <int D>
-cudaError_t launch_matrix(const AttnParams& p, cudaStream_t stream) {
+cudaError_t launch_matrix(const AttnParams& p, bool prefill, cudaStream_t stream) {
     const long long R = static_cast<long long>(p.Sq) * (p.Hq / p.Hkv);
-    if (R > kMmaRows) return launch_attention_prefill(p, stream);
+    if (prefill) return launch_attention_prefill(p, stream);
     const bool split = R <= 16;
-    const long long x = static_cast<long long>(p.B) * p.Hkv;
+    const long long x = static_cast<long long>(p.B) * p.Hkv * ((R + kMmaRows - 1) / kMmaRows);
     if (x > 0x7fffffffLL) return cudaErrorNotSupported;
     const dim3 grid(static_cast<unsigned>(x), static_cast<unsigned>(p.chunks));
     auto* kernel = split ? attention_mma_kernel<D, true> : attention_mma_kernel<D, false>;
@@ -627,8 +666,10 @@ cudaError_t launch_attention_forward(const void* Q, const void* K, const void* V
     p.err = err_word;
     cudaError_t e = cudaErrorNotSupported;
     if (matrix) {
-        e = D == 128 ? launch_matrix<128>(p, stream) : launch_matrix<64>(p, stream);
-        if (name) *name = static_cast<long long>(Sq) * (Hq / Hkv) > kMmaRows ? "attention_prefill_tcgen05_sm100" : "attention_mma_sm100";
+        const bool prefill = prefill_block(static_cast<long long>(B) * Hkv, static_cast<long long>(Sq) * (Hq / Hkv), Sk,
+                                           sm_count > 0 ? sm_count : 148);
+        e = D == 128 ? launch_matrix<128>(p, prefill, stream) : launch_matrix<64>(p, prefill, stream);
+        if (name) *name = prefill ? "attention_prefill_tcgen05_sm100" : "attention_mma_sm100";
     }
     if (e == cudaErrorNotSupported) {
         e = launch_vector(dim3(static_cast<unsigned>(rows / p.group), static_cast<unsigned>(p.chunks)), stream, p);

@@ -14,13 +14,12 @@ namespace attn {
 // to 2^-40 below: 8192 keys of any size leave out less than 2^-27 of the largest.
 constexpr float kProbScale = 32768.0f, kProbUnscale = 1.0f / 32768.0f;
 
-// exp(x) * kProbScale; exponentials below the normal range are zero.
-__device__ __forceinline__ float scaled_exp(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f));
-    return y * kProbScale;
+// a *= k and b *= k, one instruction.
+__device__ __forceinline__ void scale2(float& a, float& b, float k) {
+    asm("{\n\t.reg .b64 v, w;\n\tmov.b64 v, {%0, %1};\n\tmov.b64 w, {%2, %2};\n\tmul.rn.f32x2 v, v, w;\n\tmov.b64 {%0, %1}, v;\n\t}"
+        : "+f"(a), "+f"(b) : "f"(k));
 }
-// exp(x), the same way.
+// exp(x); exponentials below the normal range are zero.
 __device__ __forceinline__ float exp_of(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f));

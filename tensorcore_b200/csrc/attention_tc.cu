@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_prefill_kernel(const At
             // Straight-line selects throughout: a branch per element made this part four times as long.  A NaN
             // score counts as masked, as in the other kernels.
 #pragma unroll
-            for (int e = 0; e < kHalf; ++e) s[e] *= p.scale;
+            for (int e = 0; e < kHalf; e += 2) scale2(s[e], s[e + 1], p.scale);
             if (p.slopes) {
 #pragma unroll
                 for (int e = 0; e < kHalf; ++e) s[e] -= slope * static_cast<float>(i - jb - e);
@@ -198,9 +198,12 @@ __global__ void __launch_bounds__(kThreads, 1) attention_prefill_kernel(const At
             m = m_new;
             float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int e = 0; e < kHalf; ++e) {
-                s[e] = scaled_exp(s[e] - ref);                           // now the probability, 2^15 times
+            for (int e = 0; e < kHalf; e += 2) {
+                s[e] = exp_of(s[e] - ref);                               // now the probability ...
+                s[e + 1] = exp_of(s[e + 1] - ref);
+                scale2(s[e], s[e + 1], kProbScale);                      // ... 2^15 times
                 sum[e & 3] += s[e];
+                sum[(e + 1) & 3] += s[e + 1];
             }
             l = l * keep + ((sum[0] + sum[1]) + (sum[2] + sum[3]));      // over this thread's keys
             if (t > 0) {

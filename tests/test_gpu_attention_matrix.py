@@ -34,12 +34,24 @@ def exact(Q, K, V, causal, window, slopes):
         return o, (m + np.log(l))[..., 0]
 
 
+def tcgen05(B, H, Hkv, Sq, Sk):
+    """Which kernel a call takes on 148 SMs (prefill_block in attention.cu)."""
+    R = Sq * (H // Hkv)
+    tiles = B * Hkv * ((R + 63) // 64)
+    if R <= 64 or Sk <= 128:
+        return False
+    return tiles > 296 if Sk <= 256 else 4 * tiles > 148 or tiles * ((Sk + 63) // 64) > 640
+
+
 @pytest.mark.parametrize("B,H,Hkv,Sq,Sk,D,causal,window,alibi", [
     (1, 1, 1, 1, 1, 128, False, 0, False), (2, 8, 1, 1, 63, 64, False, 0, False), (1, 16, 2, 2, 65, 128, False, 0, False),
     (1, 17, 1, 1, 200, 64, False, 0, True), (3, 4, 4, 16, 16, 64, True, 0, False), (1, 4, 4, 17, 17, 128, True, 0, False),
     (1, 8, 2, 64, 64, 128, True, 0, False), (2, 6, 2, 43, 129, 64, True, 0, True), (1, 8, 4, 200, 200, 128, True, 50, False),
     (1, 2, 2, 130, 70, 128, True, 0, False), (1, 2, 2, 300, 300, 64, False, 20, False), (1, 4, 1, 96, 1000, 128, False, 0, True),
-    (1, 2, 2, 150, 40, 64, False, 30, False)])
+    (1, 2, 2, 150, 40, 64, False, 30, False), (1, 8, 8, 300, 300, 128, True, 50, False), (2, 6, 6, 400, 400, 64, True, 0, True),
+    (1, 8, 8, 310, 257, 128, False, 20, False), (1, 8, 8, 1, 16, 128, False, 0, False), (2, 15, 1, 1, 130, 64, False, 0, True),
+    (1, 8, 8, 130, 300, 128, True, 0, False), (1, 5, 1, 13, 700, 128, True, 40, False), (1, 16, 8, 330, 258, 64, True, 33, True),
+    (1, 40, 40, 600, 250, 64, False, 0, False)])
 def test_against_64_bit(tc, ctx, B, H, Hkv, Sq, Sk, D, causal, window, alibi):
     rng = np.random.default_rng(Sq * 31 + Sk + D)
     Q = rng.standard_normal((B, H, Sq, D)).astype(np.float16)
@@ -50,7 +62,7 @@ def test_against_64_bit(tc, ctx, B, H, Hkv, Sq, Sk, D, causal, window, alibi):
     bufs = [ctx.buffer_from_array(t) for t in (Q, K, V)] + [ctx.buffer(Q.nbytes), ctx.buffer(B * H * Sq * 4)]
     tc.attention_forward(ctx, *bufs[:4], B, H, Sq, Sk, D, LSE=bufs[4], causal=causal, kv_heads=Hkv, window_size=window,
                          alibi_slopes=slopes)
-    assert tc.cuda_last_kernel_name() == ("attention_prefill_tcgen05_sm100" if Sq * (H // Hkv) > 64 else "attention_mma_sm100")
+    assert tc.cuda_last_kernel_name() == ("attention_prefill_tcgen05_sm100" if tcgen05(B, H, Hkv, Sq, Sk) else "attention_mma_sm100")
     got = bufs[3].to_numpy(Q.shape, np.float16).astype(np.float64)
     got_lse = bufs[4].to_numpy((B, H, Sq), np.float32).astype(np.float64)
     for b in bufs:
