@@ -75,17 +75,18 @@ inline int norm_slab_rows(int M) {
 // Whether the weights of a prefill-sized call are dequantised once, into scratch, and multiplied as a dense GEMM:
 // where the tcgen05 kernel cannot take them (the kernels left would stream them once per four rows), and
 // where the rows are so many that one pass over the weights costs less than dequantising them again for each
-// 256 rows, in a kernel that does not overlap a tile's read-out with the next tile.  That overhead weighs less the
-// longer K is.  Back to back, microseconds, tcgen05 kernel / dequantised copy and GEMM:
+// 256 rows, in a kernel that does not overlap a tile's read-out with the next tile.  Back to back, microseconds,
+// tcgen05 kernel / dequantised copy and GEMM:
 //   rows                          2048        3072        4096        8192
-//   Q4_0 14336 x 4096          191 / 208   306 / 275   409 / 375   834 / 707
-//   Q8_0 14336 x 4096          214 / 232   342 / 301   457 / 420   911 / 778
-//   Q4_0 4096 x 4096            65 /  70    96 /  94   125 / 105   231 / 206
-//   Q4_0 4096 x 14336          182 / 183   286 / 303   367 / 338   764 / 678
-//   Q4_0 1024 x 4096            33 /  43    34 /  48    34 /  50    69 /  59
+//   Q4_0 14336 x 4096          204 / 199   316 / 309   409 / 384   850 / 771
+//   Q4_0 11008 x 4096          154 / 171   235 / 254   322 / 299   650 / 561
+//   Q8_0 11008 x 4096          165 / 179   242 / 259   348 / 320   683 / 584
+//   Q4_0 4096 x 4096            56 /  58    89 /  87   120 / 109   230 / 213
+//   Q4_0 4096 x 14336          179 / 189   291 / 275   357 / 366   773 / 771
+//   Q4_0 1024 x 4096            28 /  28    29 /  27    28 /  31    62 /  56
 // (the last row is bound by its launches: hence a least amount of work, too)
 inline bool dequant_pays(const GemvQArgs& a) {
-    return a.M >= (a.K <= 8192 ? 3072 : 4096) && static_cast<double>(a.M) * a.N * a.K >= 34359738368.0;      // 2^35
+    return a.M >= 4096 && static_cast<double>(a.M) * a.N * a.K >= 34359738368.0;      // 2^35
 }
 constexpr size_t kMaxDequantBytes = static_cast<size_t>(3) << 29;      // 1.5 GB
 inline bool dequant_once(const GemvQArgs& a) {

@@ -248,8 +248,8 @@ def test_tiles_left_over_after_whole_rounds(tc, ctx, oracle, fmt, M, N, K):
 
 
 @pytest.mark.parametrize("fused", [False, True])
-@pytest.mark.parametrize("fmt,M,N,K,once", [(0, 3072, 2816, 4096, True), (0, 3071, 2816, 4096, False), (1, 3072, 2816, 4096, True),
-                                            (0, 4096, 1024, 8448, True), (0, 4095, 1024, 8448, False), (1, 3072, 256, 512, False)])
+@pytest.mark.parametrize("fmt,M,N,K,once", [(0, 4096, 2048, 4096, True), (0, 4095, 2048, 4096, False), (1, 4096, 2048, 4096, True),
+                                            (0, 4100, 1024, 8448, True), (1, 4095, 1024, 8448, False), (1, 4096, 1024, 4096, False)])
 def test_very_many_rows_dequantise_once(tc, ctx, oracle, fused, fmt, M, N, K, once):
     """From some thousands of rows on the weights are dequantised once and multiplied as a GEMM (two launches, three
     with the norm); below, the tcgen05 kernel dequantises on the way (one or two, and the norm pass)."""
