@@ -153,10 +153,12 @@ tc_status_t tc_quantize_weights(tc_context* ctx, const tc_buffer* W_fp16, tc_buf
  * By the number of rows M: one to four rows stream the blocks with integer dot products (a
  * recorded list of one-row Q4_0 calls becomes one persistent launch); five rows or more of Q4_0
  * (four, when K >= 8192 or N > 4096) and 13 rows or more of Q8_0 take the tcgen05 kernel that
- * dequantises into tensor memory; K that is no multiple of 256 takes an fp32 kernel, or from 96 rows
- * (Q4_0) or 13 rows (Q8_0) the weights are dequantised once into scratch owned by the stream (N * K
- * halves, at most 1.5 GB) and multiplied as a dense GEMM.  The two tensor-core kinds round the
- * dequantised weights to binary16 (inside the 2e-3 bound of binary16 activations). */
+ * dequantises into tensor memory; K that is no multiple of 256, and weights that are not 16-byte
+ * aligned, take an fp32 kernel, or from 96 rows (Q4_0) or 13 rows (Q8_0) the weights are dequantised
+ * once into scratch owned by the stream (N * K halves, at most 1.5 GB) and multiplied as a dense GEMM,
+ * as are calls of 4096 rows or more.  The two tensor-core kinds round the dequantised weights to
+ * binary16 (inside the 2e-3 bound of binary16 activations).  tc_cuda_last_kernel_name reports both as
+ * ..._dequant_gemm_tcgen05_... from 96 (Q4_0) or 13 (Q8_0) rows on. */
 tc_status_t tc_gemv_quantized(tc_context* ctx, const tc_buffer* X, const tc_buffer* W_quant,
                               tc_buffer* Y, tc_quant_t fmt, int M, int N, int K);
 
@@ -415,8 +417,11 @@ tc_status_t tcx_stream_set_persistent(tc_stream* s, int enable);
 
 /* Raw launches on caller-owned device memory.  Pointers are device addresses valid on the
  * context's device; `cuda_stream` is a cudaStream_t as void* (NULL = the legacy default
- * stream).  The launch is asynchronous; errors detected at launch are returned.  Shapes and
- * dtypes as for the tc_* operations above. */
+ * stream).  The launch is asynchronous and ordered behind all work before it on the stream, the
+ * weights included; errors detected at launch are returned.  Shapes and dtypes as for the tc_*
+ * operations above.  The stream may be captured in a CUDA graph: nothing is allocated then, the call
+ * uses the scratch the stream has (run it once before the capture to have all of it), and that scratch
+ * stays until the context is shut down. */
 tc_status_t tcx_raw_quantize_weights(tc_context* ctx, const void* W_fp16, void* W_quant,
                                      tc_quant_t fmt, int N, int K, void* cuda_stream);
 tc_status_t tcx_raw_gemv_quantized(tc_context* ctx, const void* X, const void* W_quant, void* Y,

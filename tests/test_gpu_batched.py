@@ -163,9 +163,11 @@ def test_fused_rmsnorm_batched_matches_oracle(tc, ctx, oracle, M, N, K):
                                        (1, (1024, 512, 128)), (1, (520, 1056, 200)), (1, (4096, 4096, 512)),
                                        (1, (1024, 2048, 13)), (1, (4096, 4096, 32))])
 def test_prefill_sized_calls_dequantise_once_and_use_the_gemm(tc, ctx, oracle, fmt, shape):
-    """96 activation rows or more (Q4_0; Q8_0, which has no batched kernel, from 13) with fp16 results: the weights are dequantised once to fp16 in the
-    stream's scratch and multiplied on the tensor cores (Q4_0 and Q8_0, plain and fused RMSNorm);
-    same bar as the batched kernel, against the fp64 dequantise-and-dot."""
+    """96 activation rows or more (Q4_0; Q8_0 from 13) with fp16 results: fp16-rounded weights on the tensor cores,
+    Q4_0 and Q8_0, plain and fused RMSNorm; same bar as the batched kernel, against the fp64
+    dequantise-and-dot.  K a multiple of 256: dequantised on the way to the tensor cores, one launch (two where tiles
+    are left over) and the norm pass; else dequantised once in the stream's scratch and multiplied as a GEMM, two
+    launches and the norm pass.  Both report the same kernel name."""
     N, K, M = shape
     rng = np.random.default_rng(N + K * 3 + M * 7 + fmt)
     W = (rng.standard_normal((N, K)) * 0.02).astype(np.float32).astype(np.float16)
@@ -175,8 +177,10 @@ def test_prefill_sized_calls_dequantise_once_and_use_the_gemm(tc, ctx, oracle, f
     want = oracle.dequant_dot_f64(X.astype(np.float64), Wq, fmt, N)
     with ctx.buffer_from_array(X) as bx, ctx.buffer_from_array(Wq) as bw, ctx.buffer_from_array(gam) as bg, \
             ctx.buffer(M * N * 2) as by:
+        before = tc.launch_count()
         ctx.gemv_quantized(bx, bw, by, fmt, M, N, K)
         name = tc.cuda_last_kernel_name()
+        assert tc.launch_count() - before == (1 if K % 256 == 0 else 2)
         got = by.to_numpy((M, N), np.float16).astype(np.float64)
         assert name == ("q4_0" if fmt == 0 else "q8_0") + "_dequant_gemm_tcgen05_sm100"
         assert oracle.scaled_rms(got, want) <= TOL
