@@ -35,7 +35,9 @@ __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
 __device__ __forceinline__ void split_h2(float a, float b, uint32_t& hi, uint32_t& lo) {
     asm("cvt.rz.f16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(b), "f"(a));
     const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi));
-    lo = __vmaxu2(pack_h2(a - f.x, b - f.y), __vminu2(hi, 0x00010001u));
+    uint32_t least;                          // 1, the smallest fp16 number, where hi is not zero
+    asm("min.u16x2 %0, %1, %2;" : "=r"(least) : "r"(hi), "r"(0x00010001u));
+    asm("max.u16x2 %0, %1, %2;" : "=r"(lo) : "r"(pack_h2(a - f.x, b - f.y)), "r"(least));
 }
 
 }  // namespace attn
