@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const
         l[e] += __shfl_xor_sync(0xffffffffu, l[e], 2);
         l[e] *= kProbUnscale;
 #pragma unroll
-        for (int n = 0; n < D / 8; ++n) { o[n][2 * e] *= kProbUnscale; o[n][2 * e + 1] *= kProbUnscale; }
+        for (int n = 0; n < D / 8; ++n) { o[n][2 * e] *= kProbUnscale * kUngrow; o[n][2 * e + 1] *= kProbUnscale * kUngrow; }
     }
 
     if constexpr (!SPLIT_KEYS) {

@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_prefill_kernel(const At
         }
         if (!failed) l += exchange(l);
         if (!failed) {
-            const float inv = l != 0.f ? 1.0f / l : 0.f;                 // l and O are both 2^15 times as large here
+            const float inv = l != 0.f ? kUngrow / l : 0.f;              // l and O are both 2^15 times as large here
             float* part = p.part + (row_at * p.chunks + chunk) * (D + 2);
             {
                 constexpr int kQ = D / 32;                 // pieces of 16 columns of this thread's half
@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_prefill_kernel(const At
                     } else {
 #pragma unroll
                         for (int e = 0; e < 16; e += 2)
-                            *reinterpret_cast<float2*>(part + 2 + c + e) = make_float2(__uint_as_float(v[q][e]) * kProbUnscale, __uint_as_float(v[q][e + 1]) * kProbUnscale);
+                            *reinterpret_cast<float2*>(part + 2 + c + e) = make_float2(__uint_as_float(v[q][e]) * (kProbUnscale * kUngrow), __uint_as_float(v[q][e + 1]) * (kProbUnscale * kUngrow));
                     }
                 }
             }
