@@ -658,8 +658,13 @@ cudaError_t launch_attention_forward(const void* Q, const void* K, const void* V
     const bool matrix = attention_on_matrix_kernels(D, Q, K, V);
     attention_chunks(B, Hq, Hkv, Sq, Sk, matrix, sm_count, &p.chunks, &p.keys_per_chunk);
     if (p.chunks > 1 && !scratch) { p.chunks = 1; p.keys_per_chunk = Sk; }
+    // The tensor core truncates its running sums: a score of D / 16 steps comes out smaller by 2.2e-8 of itself per step
+    // on average (mean over 150,000 scores of normal data, mma.sync and tcgen05 alike: 1.8e-7 at head_dim 128, 0.9e-7
+    // at 64, always towards zero), where fp32 multiply-adds round without a bias.  The scale makes up for it, as far as an
+    // fp32 number can.  LSE of 512 x 512, head_dim 128: 2.8e-7 rms from 64 bits without, 2.0e-7 with multiply-adds.
+    const float matrix_scale = static_cast<float>(static_cast<double>(scale) * (1.0 + 2.2e-8 * (D / 16)));
     // A window that no query can look back beyond hides nothing; so the kernels' `i - window` stays within int.
-    p.scale = scale; p.causal = causal ? 1 : 0; p.window = window < Sq - 1 ? window : 0;
+    p.scale = matrix ? matrix_scale : scale; p.causal = causal ? 1 : 0; p.window = window < Sq - 1 ? window : 0;
     p.o_vec = (reinterpret_cast<uintptr_t>(O) & 15u) == 0;
     // the vector kernel's lanes load D / 32 elements of a value row at a time
     p.v_vec = (reinterpret_cast<uintptr_t>(V) & (D == 128 ? 7u : 3u)) == 0;
