@@ -18,7 +18,7 @@
 // What bounds it: latency.  Causal 512 x 512, 32 heads on 8 K/V heads, head_dim 128 is 128 CTAs of up to four
 // steps; clock stamps of the longest: about 8000 clocks until the first scores (barriers, tensor memory, Q, cold
 // code), then 3500 a step - exponentials and masks 2100 to 2500, rescaling 600, storing P 500 - in which 1060
-// clocks of P V and 530 of Q K^T hide, and 1900 to store O.  28.7 us through the synchronous call (10 us of it
+// clocks of P V and 530 of Q K^T hide, and 1900 to store O.  28.3 us through the synchronous call (10 us of it
 // launch and wait; 31 with three warps of cp.async as loaders, which a step then waited 1700 clocks for),
 // 38 us on the mma.sync kernel, whose tensor instructions run at an eighth of the rate, 388 us as a
 // streaming pass per query row.
