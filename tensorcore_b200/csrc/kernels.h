@@ -26,6 +26,7 @@ struct LaunchEnv {
     // With pdl, whether nothing that may still run on the stream writes the weights: they are then read while the
     // kernel before runs.  Else a kernel waits for it first, and lets the next one start only after that.
     bool weights_ready = false;
+    bool alone = false;        // a synchronous call: nothing follows it before it is through
     bool wait_first() const { return pdl && !weights_ready; }
     int variant = VARIANT_AUTO;
     uint32_t* err_word = nullptr;  // device-visible word a kernel ORs an error bit into
@@ -47,6 +48,10 @@ struct GemvQArgs {
     // scratch of the stream for the calls of dequant_once: room for the weights as fp16, N * K halves
     void* dequant_scratch = nullptr;
     size_t dequant_scratch_bytes = 0;
+    // scratch of the stream for the tcgen05 kernel (tc_rows): sums of tiles that two CTAs work on, all bits set
+    // between launches (gemm_q_tc_share_bytes); without it tiles are whole or split over a cluster
+    void* share_scratch = nullptr;
+    size_t share_scratch_bytes = 0;
 };
 // From how many activation rows a call with fp16 activations and results counts as prefill-sized: Q8_0 calls
 // then take the tcgen05 kernel (fp16-rounded weights) instead of the integer kernels (four rows a pass),
@@ -95,6 +100,9 @@ inline bool dequant_once(const GemvQArgs& a) {
     if ((reinterpret_cast<uintptr_t>(a.W) & 1u) || (!a.gamma && (reinterpret_cast<uintptr_t>(a.X) & 15u))) return false;
     return !tc_rows(a) || dequant_pays(a);
 }
+
+// Bytes of GemvQArgs::share_scratch for M activation rows.
+size_t gemm_q_tc_share_bytes(int M, int sm_count);
 
 // Tiles of the dense split kernel: column strips, K ranges per strip, rows of a K range.
 struct DenseSplit { int strips = 0, chunks = 0, kc = 0; };

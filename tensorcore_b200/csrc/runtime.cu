@@ -196,14 +196,23 @@ bool managed(const tc_buffer* b) { return b->kind == BUF_MANAGED || b->kind == B
 // out: a graph may then be replayed at any time, and the room stays until the context goes.
 // The mutex is held from handing rooms out until the launches that use them are in the stream, so that calls
 // from several threads do not get between another call's launches, nor free its rooms.
-struct StreamRooms {
-    Room partial, counters;   // dense fused GEMV: partial sums of the K ranges, a ticket counter per column strip
-    Room norm;                // normalised rows
-    Room weights;             // weights as fp16
+enum RoomKind : int {
+    ROOM_PARTIAL,    // dense fused GEMV: partial sums of the K ranges
+    ROOM_COUNTERS,   // ... a ticket counter per column strip, zero between launches
+    ROOM_NORM,       // normalised rows
+    ROOM_WEIGHTS,    // weights as fp16
+    ROOM_SHARES,     // batched quantized products: sums of tiles that several CTAs work on, all bits set between launches
+    kRoomKinds
 };
+constexpr int kRoomFill[kRoomKinds] = {-1, 0, -1, -1, 0xFF};      // the byte a new room is filled with
+struct StreamRooms { Room room[kRoomKinds]; };
 std::mutex g_rooms_mutex;
 std::unordered_map<cudaStream_t, StreamRooms> g_rooms;
 std::vector<void*> g_kept;    // outgrown rooms of captured graphs
+// Rooms of streams that have been destroyed, for those that are created later (a cudaMalloc in the first pass over a
+// new session took 0.25 ms): at most kSpareRooms of a kind, none above kSpareBytes.
+std::vector<Room> g_spare[kRoomKinds];
+constexpr size_t kSpareRooms = 4, kSpareBytes = static_cast<size_t>(32) << 20;
 using RoomsLock = std::unique_lock<std::mutex>;
 
 bool being_captured(cudaStream_t st) {
@@ -222,7 +231,7 @@ void give_back(Room& r) {
 // Makes `r` hold `need` bytes, unless the stream is being captured (nothing can be allocated then) or there
 // is no memory: the caller sees what there is.  `wait` returns when no launch uses the room any more.
 template <typename Wait>
-void grow_room(Room& r, size_t need, size_t most, cudaStream_t st, bool zero, Wait wait) {
+void grow_room(Room& r, size_t need, size_t most, cudaStream_t st, int fill, Wait wait) {
     const bool capture = being_captured(st);
     if (r.bytes < need && !capture) {
         // Half as much again as before, so that slowly growing calls do not allocate every time; rooms that have to
@@ -239,7 +248,7 @@ void grow_room(Room& r, size_t need, size_t most, cudaStream_t st, bool zero, Wa
             want = need;
             if (cudaMalloc(&p, want) != cudaSuccess) { (void)cudaGetLastError(); p = nullptr; }
         }
-        if (p && zero && cudaMemsetAsync(p, 0, want, st) != cudaSuccess) { (void)cudaGetLastError(); cudaFree(p); p = nullptr; }
+        if (p && fill >= 0 && cudaMemsetAsync(p, fill, want, st) != cudaSuccess) { (void)cudaGetLastError(); cudaFree(p); p = nullptr; }
         if (p) {
             if (r.p) { wait(); give_back(r); }
             r.p = p;
@@ -248,8 +257,17 @@ void grow_room(Room& r, size_t need, size_t most, cudaStream_t st, bool zero, Wa
     }
     if (capture && r.p) r.captured = true;
 }
-void grow_stream_room(Room& r, size_t need, cudaStream_t st, bool zero = false, size_t most = ~static_cast<size_t>(0)) {
-    grow_room(r, need, most, st, zero, [&] { cudaStreamSynchronize(st); });
+// No work is left on the stream, which goes.
+void retire_rooms(cudaStream_t st) {
+    RoomsLock lock(g_rooms_mutex);
+    auto it = g_rooms.find(st);
+    if (it == g_rooms.end()) return;
+    for (int k = 0; k < kRoomKinds; ++k) {
+        Room& r = it->second.room[k];
+        if (r.p && !r.captured && r.bytes <= kSpareBytes && g_spare[k].size() < kSpareRooms) g_spare[k].push_back(r);
+        else give_back(r);
+    }
+    g_rooms.erase(it);
 }
 
 StreamRooms& rooms_of(cudaStream_t st) {
@@ -257,16 +275,31 @@ StreamRooms& rooms_of(cudaStream_t st) {
         // many short-lived streams: start over rather than keep scratch for streams that are gone
         cudaDeviceSynchronize();
         for (auto& kv : g_rooms)
-            for (Room* r : {&kv.second.partial, &kv.second.counters, &kv.second.norm, &kv.second.weights}) give_back(*r);
+            for (Room& r : kv.second.room) give_back(r);
         g_rooms.clear();
     }
     return g_rooms[st];
 }
+// The stream's room of a kind, grown to `need` bytes where that can be done.
+Room& stream_room(cudaStream_t st, RoomKind k, size_t need, size_t most = ~static_cast<size_t>(0)) {
+    Room& r = rooms_of(st).room[k];
+    if (!r.p && need > 0 && !being_captured(st)) {
+        std::vector<Room>& spare = g_spare[k];
+        for (size_t i = 0; i < spare.size(); ++i)
+            if (spare[i].bytes >= need) { r = spare[i]; spare.erase(spare.begin() + i); break; }
+    }
+    grow_room(r, need, most, st, kRoomFill[k], [&] { cudaStreamSynchronize(st); });
+    return r;
+}
 void free_rooms() {
     RoomsLock lock(g_rooms_mutex);
     for (auto& kv : g_rooms)
-        for (Room* r : {&kv.second.partial, &kv.second.counters, &kv.second.norm, &kv.second.weights}) give_back(*r);
+        for (Room& r : kv.second.room) give_back(r);
     g_rooms.clear();
+    for (std::vector<Room>& spare : g_spare) {
+        for (Room& r : spare) give_back(r);
+        spare.clear();
+    }
     for (void* p : g_kept) cudaFree(p);
     g_kept.clear();
 }
@@ -275,11 +308,10 @@ void free_rooms() {
 void dense_scratch_for(tc_context* ctx, cudaStream_t st, tcb::DenseNormGemvArgs* a) {
     size_t nf = 0, nc = 0;
     tcb::plan_dense_norm_gemv(a, ctx->sm_count, ctx->smem_optin, &nf, &nc);
-    StreamRooms& d = rooms_of(st);
-    grow_stream_room(d.partial, nf * sizeof(float), st);
-    grow_stream_room(d.counters, nc * sizeof(int), st, true);
-    a->scratch = static_cast<float*>(d.partial.p); a->scratch_floats = d.partial.bytes / sizeof(float);
-    a->counters = static_cast<int*>(d.counters.p); a->counters_n = d.counters.bytes / sizeof(int);
+    const Room& partial = stream_room(st, ROOM_PARTIAL, nf * sizeof(float));
+    const Room& counters = stream_room(st, ROOM_COUNTERS, nc * sizeof(int));
+    a->scratch = static_cast<float*>(partial.p); a->scratch_floats = partial.bytes / sizeof(float);
+    a->counters = static_cast<int*>(counters.p); a->counters_n = counters.bytes / sizeof(int);
 }
 // Room for the normalised rows of the batched fused RMSNorm GEMV (the tensor-core kernel reads them as
 // plain fp16 activations).
@@ -295,19 +327,31 @@ size_t norm_scratch_need(const tcb::GemvQArgs& a) {
 size_t dequant_scratch_need(const tcb::GemvQArgs& a) {
     return tcb::dequant_once(a) ? static_cast<size_t>(a.N) * a.K * 2 : 0;
 }
+// Room for the tiles that several CTAs of the tcgen05 kernel work on.
+size_t share_scratch_need(tc_context* ctx, const tcb::GemvQArgs& a) {
+    if (!tcb::tc_rows(a)) return 0;
+    return tcb::gemm_q_tc_share_bytes(a.M <= tcb::kNormRoomRows ? a.M : tcb::norm_slab_rows(a.M), ctx->sm_count);
+}
+void share_scratch_for(cudaStream_t st, size_t need, tcb::GemvQArgs* a) {
+    // A captured call does without: a graph may be replayed beside later calls on the stream, and two launches under
+    // way must not share this.
+    // (nor does the per-thread stream, one handle for many streams)
+    if (need == 0 || st == cudaStreamPerThread || being_captured(st)) return;
+    const Room& r = stream_room(st, ROOM_SHARES, need);
+    a->share_scratch = r.p;
+    a->share_scratch_bytes = r.bytes;
+}
 void norm_scratch_for(cudaStream_t st, size_t need, tcb::GemvQArgs* a) {
     if (need == 0) return;
-    StreamRooms& d = rooms_of(st);
-    grow_stream_room(d.norm, need > (1u << 20) ? need : (1u << 20), st);
-    a->norm_scratch = d.norm.p;
-    a->norm_scratch_bytes = d.norm.bytes;
+    const Room& r = stream_room(st, ROOM_NORM, need > (1u << 20) ? need : (1u << 20));
+    a->norm_scratch = r.p;
+    a->norm_scratch_bytes = r.bytes;
 }
 void dequant_scratch_for(cudaStream_t st, size_t need, tcb::GemvQArgs* a) {
     if (need == 0) return;
-    StreamRooms& d = rooms_of(st);
-    grow_stream_room(d.weights, need, st, false, tcb::kMaxDequantBytes);
-    a->dequant_scratch = d.weights.p;
-    a->dequant_scratch_bytes = d.weights.bytes;
+    const Room& r = stream_room(st, ROOM_WEIGHTS, need, tcb::kMaxDequantBytes);
+    a->dequant_scratch = r.p;
+    a->dequant_scratch_bytes = r.bytes;
 }
 // Room for the normalised rows of a dense fused norm + GEMV call with five rows or more.
 void dense_norm_rows_for(cudaStream_t st, tcb::DenseNormGemvArgs* a) {
@@ -812,6 +856,7 @@ extern "C" tc_status_t tc_stream_destroy(tc_context* ctx, tc_stream* s) {
     cudaStreamSynchronize(s->s);
     drop_graphs(s);
     free_decode_site(s->site);
+    retire_rooms(s->s);
     cudaStreamDestroy(s->s);
     delete s;
     return TC_OK;
@@ -1016,14 +1061,17 @@ tc_status_t submit_pending(tc_stream* s) {
     RoomsLock rooms(g_rooms_mutex, std::defer_lock);
     tcb::GemvQArgs scratch_of;          // the stream's scratch for normalised rows, sized for the widest operation
     {
-        size_t need = 0, dq = 0;
+        size_t need = 0, dq = 0, sh = 0;
         for (const RecordedOp& op : s->pending) {
             const size_t n = norm_scratch_need(op.a);
             need = n > need ? n : need;
             const size_t q = dequant_scratch_need(op.a);
             dq = q > dq ? q : dq;
+            const size_t h = share_scratch_need(ctx, op.a);
+            sh = h > sh ? h : sh;
         }
-        if (need > 0 || dq > 0) rooms.lock();
+        if (need > 0 || dq > 0 || sh > 0) rooms.lock();
+        share_scratch_for(s->s, sh, &scratch_of);
         norm_scratch_for(s->s, need, &scratch_of);
         dequant_scratch_for(s->s, dq, &scratch_of);
     }
@@ -1032,6 +1080,8 @@ tc_status_t submit_pending(tc_stream* s) {
         op.a.norm_scratch_bytes = scratch_of.norm_scratch_bytes;
         op.a.dequant_scratch = scratch_of.dequant_scratch;
         op.a.dequant_scratch_bytes = scratch_of.dequant_scratch_bytes;
+        op.a.share_scratch = scratch_of.share_scratch;
+        op.a.share_scratch_bytes = scratch_of.share_scratch_bytes;
         // Device addresses are resolved now, not when the operation was recorded: a first
         // tc_buffer_map between the two moves a buffer to managed storage.
         op.a.X = op.X->dptr;
@@ -1380,12 +1430,15 @@ tc_status_t gemv_common(const GemvCall& c, tc_stream* stream, const char* opname
     int launches = 0;
     const char* name = "none";
     if (e == cudaSuccess) {
-        const size_t need = norm_scratch_need(op.a), dq = dequant_scratch_need(op.a);
+        const size_t need = norm_scratch_need(op.a), dq = dequant_scratch_need(op.a), sh = share_scratch_need(ctx, op.a);
         RoomsLock rooms(g_rooms_mutex, std::defer_lock);
-        if (need > 0 || dq > 0) rooms.lock();
+        if (need > 0 || dq > 0 || sh > 0) rooms.lock();
+        share_scratch_for(s0, sh, &op.a);
         norm_scratch_for(s0, need, &op.a);
         dequant_scratch_for(s0, dq, &op.a);
-        e = tcb::launch_gemv_q(op.a, make_env(ctx, false), s0, &launches, &name);
+        LaunchEnv env = make_env(ctx, false);
+        env.alone = true;
+        e = tcb::launch_gemv_q(op.a, env, s0, &launches, &name);
     }
     if (e == cudaSuccess) e = finish_output(op.Y, yb, s0);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s0);
@@ -1623,7 +1676,7 @@ extern "C" tc_status_t tc_attention_forward(tc_context* ctx, const tc_attention_
     const size_t slope_at = want;
     if (d->alibi_slopes) want += static_cast<size_t>(Hq);
     RoomsLock rooms(g_rooms_mutex);
-    if (want > 0) grow_room(ctx->attn, want * sizeof(float), ~static_cast<size_t>(0), ctx->stream0, false, [] { cudaDeviceSynchronize(); });
+    if (want > 0) grow_room(ctx->attn, want * sizeof(float), ~static_cast<size_t>(0), ctx->stream0, -1, [] { cudaDeviceSynchronize(); });
     if (want * sizeof(float) > ctx->attn.bytes) return record("tc_attention_forward", TC_ERR_ALLOC);
     float* const scratch = static_cast<float*>(ctx->attn.p);
     float* slopes_dev = nullptr;
@@ -1676,7 +1729,7 @@ extern "C" tc_status_t tcx_raw_attention_forward(tc_context* ctx, const tc_atten
     float* scratch = nullptr;
     if (want > 0) {
         rooms.lock();
-        grow_room(ctx->attn, want * sizeof(float), ~static_cast<size_t>(0), st, false, [] { cudaDeviceSynchronize(); });
+        grow_room(ctx->attn, want * sizeof(float), ~static_cast<size_t>(0), st, -1, [] { cudaDeviceSynchronize(); });
         if (want * sizeof(float) <= ctx->attn.bytes) scratch = static_cast<float*>(ctx->attn.p);
         else if (!being_captured(st)) return record("tcx_raw_attention_forward", TC_ERR_ALLOC);
     }
@@ -1919,9 +1972,10 @@ static tc_status_t raw_gemv(tc_context* ctx, const void* X, const void* gamma, b
     a.X = X; a.Y = Y; a.gamma = fused ? gamma : nullptr;
     a.fmt = static_cast<int>(fmt); a.M = M; a.N = N; a.K = K;
     a.x_f32 = xd == TC_DTYPE_F32; a.y_f32 = yd == TC_DTYPE_F32; a.eps = eps;
-    const size_t need = norm_scratch_need(a), dq = dequant_scratch_need(a);
+    const size_t need = norm_scratch_need(a), dq = dequant_scratch_need(a), sh = share_scratch_need(ctx, a);
     RoomsLock rooms(g_rooms_mutex, std::defer_lock);
-    if (need > 0 || dq > 0) rooms.lock();
+    if (need > 0 || dq > 0 || sh > 0) rooms.lock();
+    share_scratch_for(static_cast<cudaStream_t>(cuda_stream), sh, &a);
     norm_scratch_for(static_cast<cudaStream_t>(cuda_stream), need, &a);
     dequant_scratch_for(static_cast<cudaStream_t>(cuda_stream), dq, &a);
     int launches = 0;
@@ -2033,6 +2087,18 @@ extern "C" uint32_t tcx_take_device_error(tc_context* ctx) {
     if (!ctx || !ctx->err_host) return 0;
     const uint32_t v = *reinterpret_cast<volatile uint32_t*>(ctx->err_host);
     *reinterpret_cast<volatile uint32_t*>(ctx->err_host) = 0;
+    if (v != 0) {
+        // A kernel that gave up may have left sums in the rooms that are empty between launches.
+        RoomsLock lock(g_rooms_mutex);
+        bind_device(ctx);
+        cudaDeviceSynchronize();
+        for (auto& kv : g_rooms) {
+            const Room& r = kv.second.room[ROOM_SHARES];
+            if (r.p) cudaMemset(r.p, kRoomFill[ROOM_SHARES], r.bytes);
+        }
+        for (const Room& r : g_spare[ROOM_SHARES]) cudaMemset(r.p, kRoomFill[ROOM_SHARES], r.bytes);
+        (void)cudaGetLastError();
+    }
     return v;
 }
 
