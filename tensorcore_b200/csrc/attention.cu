@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_decode_kernel(const
 // For decode steps and small blocks: up to 64 (query, head) pairs that share a K/V head, head fastest, are one
 // tile, so the heads of a grouped-query decode step read the cache once.  K and V arrive in steps of 64 keys through a ring in shared memory
 // (cp.async, 16-byte pieces, piece index XORed with the row so that ldmatrix is conflict-free).
-//   SPLIT_KEYS (16 rows or fewer): all four warps hold the same rows and take 16 keys of a step each,
+//   SPLIT_KEYS (9 to 16 rows; attention_mma8_kernel below for up to 8): all four warps hold the same rows and take 16 keys of a step each,
 //     with softmax states of their own that are merged at the end (a thread per row for the weights, then four
 //     elements a thread at a time: 16 x 16, 8 heads 19.1 us a call with a division and a branch per element).
 //   else: a warp owns 16 of the 64 rows and takes all 64 keys.
@@ -209,10 +209,11 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_decode_kernel(const
 // each is split into two fp16 numbers (attention_math.cuh says to how many bits), which costs a third
 // more MMAs and keeps the result as close to a 64-bit one as fp32 multiply-adds had it.
 // A decode step is bound by the cache stream; two CTAs per SM overlap the chains of their steps (scores,
-// maximum, exponentials, outputs).  Eight sequences, 32 heads on 8 K/V heads x 4096 keys: 28 us (4.8 TB/s),
-// 85 us as a streaming pass of CUDA-core dot products per two heads.
+// maximum, exponentials, outputs).
 // ---------------------------------------------------------------------------------------
 constexpr int kStepKeys = 64;
+constexpr int kMergeMaxChunks = 128;
+constexpr int kMergeHere = 8;          // chunks that the attention kernel can merge itself
 constexpr int kMmaRows = 64;           // rows (query, head) of a tile
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
@@ -231,11 +232,165 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4],
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// Partial softmax states that a CTA leaves for the one that merges its row: words that are kNoState until they have
+// been written, so that a reader knows them by their being there (no flag, no fence on either side) and leaves
+// kNoState behind.  A NaN that has these bits is stored as another one.
+constexpr uint32_t kNoState = 0xFFFFFFFFu;
+__device__ __forceinline__ uint32_t state_word(float v) {
+    const uint32_t w = __float_as_uint(v);
+    return w == kNoState ? 0x7FFFFFFFu : w;
+}
+__device__ __forceinline__ void state_store4(uint32_t* dst, float4 v) {
+    asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};"
+                 ::"l"(dst), "r"(state_word(v.x)), "r"(state_word(v.y)), "r"(state_word(v.z)), "r"(state_word(v.w)) : "memory");
+}
+// What n chunks have of four elements, {o, o, o, o} and {m, l, -, -} each: all asked for at a time, until all are
+// there; false after about a second.
+template <int N>
+__device__ __forceinline__ bool state_take(uint32_t* src, size_t stride, int n, uint4 (&o)[N], uint4 (&ml)[N]) {
+    const long long t0 = clock64();
+    auto there = [](const uint4& v) { return v.x != kNoState && v.y != kNoState && v.z != kNoState && v.w != kNoState; };
+    for (;;) {
+        bool all = true;
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            if (i < n) {
+                asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(o[i].x), "=r"(o[i].y), "=r"(o[i].z), "=r"(o[i].w) : "l"(src + i * stride) : "memory");
+                asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(ml[i].x), "=r"(ml[i].y), "=r"(ml[i].z), "=r"(ml[i].w) : "l"(src + i * stride + 4) : "memory");
+            }
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            if (i < n) all = all && there(o[i]) && there(ml[i]);
+        if (all) break;
+        if (clock64() - t0 > 2000000000LL) return false;
+    }
+#pragma unroll
+    for (int i = 0; i < 2 * N; ++i)
+        if (i < 2 * n)
+            asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %1, %1, %1};" ::"l"(src + i / 2 * stride + 4 * (i & 1)), "r"(kNoState) : "memory");
+    return true;
+}
+// An 8 x 8 matrix of 16-bit elements, a thread's two those of row lane / 4, transposed.
+__device__ __forceinline__ uint32_t transpose_8x8(uint32_t v) {
+    uint32_t r;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+    return r;
+}
 template <int D> struct MmaShape {
     static constexpr int kStages = D == 128 ? 3 : 4;
     static constexpr int kStageBytes = 2 * kStepKeys * D * 2;
     static constexpr int kSmem = kStages * kStageBytes;
 };
+
+// The end of the kernels whose warps split the keys of a step (ROWS rows): o_s has each warp's outputs, rows STRIDE
+// elements apart, ml_s its maximum and sum per row, both in the ring, which everybody has finished reading.
+template <int D, int ROWS, int STRIDE>
+__device__ __forceinline__ void merge_warps(const AttnParams& p, float* o_s, float* ml_s, int R, int G, int b, int hkv, int bk, int chunk) {
+    const int tid = threadIdx.x;
+    float* w_s = ml_s + kAttnWarps * ROWS * 2;                       // [ROWS][warp]
+    __syncthreads();
+    auto row_of = [&](int r) { return (static_cast<size_t>(b) * p.Hq + hkv * G + r % G) * p.Sq + r / G; };
+    // With room for them the chunks' states go to the CTA of the last chunk, which started last, and it merges them: a
+    // thread has the same four elements of every chunk, with the row's maximum and sum beside each, so one trip
+    // brings all it needs.
+    const bool here = p.states != nullptr && p.chunks > 1, merges = here && chunk + 1 == p.chunks;
+    const size_t state_words = static_cast<size_t>(R) * D * 2;       // of a chunk
+    uint32_t* const states = here ? p.states + static_cast<size_t>(bk) * (p.chunks - 1) * state_words : nullptr;
+    float* m_s = w_s + ROWS * kAttnWarps;                              // [ROWS]: the CTA's maxima and sums
+    float* l_s = m_s + ROWS;
+    if (tid < R) {                                                   // at most 16 rows
+        float mm = -INFINITY, ll = 0.f, f[kAttnWarps];
+#pragma unroll
+        for (int w = 0; w < kAttnWarps; ++w) mm = fmaxf(mm, ml_s[(w * ROWS + tid) * 2]);
+#pragma unroll
+        for (int w = 0; w < kAttnWarps; ++w) {
+            const float mw = ml_s[(w * ROWS + tid) * 2];
+            f[w] = mw > -INFINITY ? __expf(mw - mm) : 0.f;
+            ll += ml_s[(w * ROWS + tid) * 2 + 1] * f[w];
+        }
+        const float inv = p.chunks > 1 ? 1.f : ll != 0.f ? 1.0f / ll : 0.f;
+#pragma unroll
+        for (int w = 0; w < kAttnWarps; ++w) w_s[tid * kAttnWarps + w] = f[w] * inv;
+        if (here) {
+            m_s[tid] = mm;
+            l_s[tid] = ll;
+        } else if (p.chunks > 1) {
+            float* dst = p.part + (row_of(tid) * p.chunks + chunk) * (D + 2);
+            dst[0] = mm;
+            dst[1] = ll;
+        } else if (p.LSE) {
+            p.LSE[row_of(tid)] = mm + logf(fmaxf(ll, 1e-30f));
+        }
+    }
+    __syncthreads();
+    bool ok = true;
+    for (int t = tid; t < R * (D / 4); t += kAttnWarps * 32) {
+        const int r = t / (D / 4), c = 4 * (t % (D / 4));
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int w = 0; w < kAttnWarps; ++w) {
+            const float4 v = *reinterpret_cast<const float4*>(o_s + (w * ROWS + r) * STRIDE + c);
+            const float f = w_s[r * kAttnWarps + w];
+            acc.x = fmaf(f, v.x, acc.x); acc.y = fmaf(f, v.y, acc.y);
+            acc.z = fmaf(f, v.z, acc.z); acc.w = fmaf(f, v.w, acc.w);
+        }
+        if (here && !merges) {
+            uint32_t* dst = states + chunk * state_words + static_cast<size_t>(t) * 8;
+            state_store4(dst, acc);
+            state_store4(dst + 4, make_float4(m_s[r], l_s[r], 0.f, 0.f));
+            continue;
+        }
+        if (p.chunks > 1 && !here) {
+            float2* dst = reinterpret_cast<float2*>(p.part + (row_of(r) * p.chunks + chunk) * (D + 2) + 2 + c);
+            dst[0] = make_float2(acc.x, acc.y);
+            dst[1] = make_float2(acc.z, acc.w);
+            continue;
+        }
+        if (merges) {
+            constexpr int kOthers = kMergeHere - 1;
+            uint4 o4[kOthers], ml[kOthers];
+            const int n = p.chunks - 1;
+            ok = state_take(states + static_cast<size_t>(t) * 8, state_words, n, o4, ml) && ok;
+            float mm = m_s[r];
+#pragma unroll
+            for (int i = 0; i < kOthers; ++i)
+                if (i < n) mm = fmaxf(mm, __uint_as_float(ml[i].x));
+            // the sums of the merge kernel below in its order, to the bit: a tree of eight, elements by chunk
+            float le[kMergeHere];
+            float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+            auto add = [&](float m_c, float l_c, float4 v) {
+                const float e = m_c > -INFINITY ? __expf(m_c - mm) : 0.f;
+                sum.x = fmaf(v.x, e, sum.x); sum.y = fmaf(v.y, e, sum.y);
+                sum.z = fmaf(v.z, e, sum.z); sum.w = fmaf(v.w, e, sum.w);
+                return l_c * e;
+            };
+#pragma unroll
+            for (int i = 0; i < kMergeHere; ++i) {
+                le[i] = 0.f;
+                if (i < kOthers && i < n)
+                    le[i] = add(__uint_as_float(ml[i].x), __uint_as_float(ml[i].y),
+                                make_float4(__uint_as_float(o4[i].x), __uint_as_float(o4[i].y), __uint_as_float(o4[i].z), __uint_as_float(o4[i].w)));
+                else if (i == n)
+                    le[i] = add(m_s[r], l_s[r], acc);
+            }
+            const float ll = ((le[0] + le[4]) + (le[2] + le[6])) + ((le[1] + le[5]) + (le[3] + le[7]));
+            acc = ll != 0.f ? make_float4(sum.x / ll, sum.y / ll, sum.z / ll, sum.w / ll) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (c == 0 && p.LSE) p.LSE[row_of(r)] = mm + logf(fmaxf(ll, 1e-30f));
+        }
+        __half* dst = p.O + row_of(r) * D + c;
+        const uint2 v = make_uint2(pack_h2(acc.x, acc.y), pack_h2(acc.z, acc.w));
+        if (p.o_vec) {
+            *reinterpret_cast<uint2*>(dst) = v;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                reinterpret_cast<uint16_t*>(dst)[e] = static_cast<uint16_t>((e < 2 ? v.x : v.y) >> (16 * (e & 1)));
+        }
+    }
+    if (!ok && p.err) atomicOr(p.err, ERR_WAIT_TIMEOUT);
+}
 
 template <int D, bool SPLIT_KEYS>
 __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const AttnParams p) {
@@ -437,11 +592,9 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const
             }
         }
     } else {
-        // Merge the warps' states through the ring, which everybody has finished reading: a thread per row works out
-        // the warps' weights, then all threads go over the elements four at a time.
+        // Merge the warps' states through the ring, which everybody has finished reading.
         float* o_s = reinterpret_cast<float*>(smem);                     // [warp][16][D]
         float* ml_s = o_s + kAttnWarps * 16 * D;                         // [warp][16][2]
-        float* w_s = ml_s + kAttnWarps * 16 * 2;                         // [16][warp]
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
@@ -451,62 +604,180 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const
                 *reinterpret_cast<float2*>(o_s + (warp * 16 + r) * D + 8 * n + 2 * tq) = make_float2(o[n][2 * e], o[n][2 * e + 1]);
             if (tq == 0) { ml_s[(warp * 16 + r) * 2] = m[e]; ml_s[(warp * 16 + r) * 2 + 1] = l[e]; }
         }
-        __syncthreads();
-        auto row_of = [&](int r) { return (static_cast<size_t>(b) * p.Hq + hkv * G + r % G) * p.Sq + r / G; };
-        if (tid < R) {                                                   // at most 16 rows
-            float mm = -INFINITY, ll = 0.f, f[kAttnWarps];
-#pragma unroll
-            for (int w = 0; w < kAttnWarps; ++w) mm = fmaxf(mm, ml_s[(w * 16 + tid) * 2]);
-#pragma unroll
-            for (int w = 0; w < kAttnWarps; ++w) {
-                const float mw = ml_s[(w * 16 + tid) * 2];
-                f[w] = mw > -INFINITY ? __expf(mw - mm) : 0.f;
-                ll += ml_s[(w * 16 + tid) * 2 + 1] * f[w];
-            }
-            const float inv = p.chunks > 1 ? 1.f : ll != 0.f ? 1.0f / ll : 0.f;
-#pragma unroll
-            for (int w = 0; w < kAttnWarps; ++w) w_s[tid * kAttnWarps + w] = f[w] * inv;
-            if (p.chunks > 1) {
-                float* dst = p.part + (row_of(tid) * p.chunks + chunk) * (D + 2);
-                dst[0] = mm;
-                dst[1] = ll;
-            } else if (p.LSE) {
-                p.LSE[row_of(tid)] = mm + logf(fmaxf(ll, 1e-30f));
-            }
-        }
-        __syncthreads();
-        for (int t = tid; t < R * (D / 4); t += kAttnWarps * 32) {
-            const int r = t / (D / 4), c = 4 * (t % (D / 4));
-            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int w = 0; w < kAttnWarps; ++w) {
-                const float4 v = *reinterpret_cast<const float4*>(o_s + (w * 16 + r) * D + c);
-                const float f = w_s[r * kAttnWarps + w];
-                acc.x = fmaf(f, v.x, acc.x); acc.y = fmaf(f, v.y, acc.y);
-                acc.z = fmaf(f, v.z, acc.z); acc.w = fmaf(f, v.w, acc.w);
-            }
-            if (p.chunks > 1) {
-                float2* dst = reinterpret_cast<float2*>(p.part + (row_of(r) * p.chunks + chunk) * (D + 2) + 2 + c);
-                dst[0] = make_float2(acc.x, acc.y);
-                dst[1] = make_float2(acc.z, acc.w);
-            } else {
-                __half* dst = p.O + row_of(r) * D + c;
-                const uint2 v = make_uint2(pack_h2(acc.x, acc.y), pack_h2(acc.z, acc.w));
-                if (p.o_vec) {
-                    *reinterpret_cast<uint2*>(dst) = v;
-                } else {
-#pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        reinterpret_cast<uint16_t*>(dst)[e] = static_cast<uint16_t>((e < 2 ? v.x : v.y) >> (16 * (e & 1)));
-                }
-            }
-        }
+        merge_warps<D, 16, D>(p, o_s, ml_s, R, G, b, hkv, bk, chunk);
     }
 }
 
+// The same for up to eight rows per K/V head (a decode step): keys are the rows of the matrices, queries their columns
+// (m16n8k16: S^T = K Q^T, O^T = V^T P^T), so that no half of them is padding.  Half as many MMAs, exponentials
+// and rescalings; P goes from the result's layout to the operand's by movmatrix.  Eight sequences, 32 heads on 8 K/V
+// heads x 4096 keys, whole calls: 40.6 us as rows of 16 with a merge launch, 39.5 merged in the kernel, 38.0 so (of
+// which 12 are launch and wait); 16 sequences, 64 heads x 8192 keys 96.6 -> 93.4 (6.7 TB/s); 8 heads on 2 x 4096 keys
+// 20.1 -> 19.2.
+template <int D>
+__global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma8_kernel(const AttnParams p) {
+    asm volatile("griddepcontrol.launch_dependents;");
+    using S = MmaShape<D>;
+    constexpr int kPieces = D / 8, kStride = D + 4;       // kStride: four rows' stores of a warp on banks of their own
+    extern __shared__ __align__(128) uint8_t smem[];
+    const uint32_t ring = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, tq = lane & 3;
+    const int G = p.Hq / p.Hkv, R = p.Sq * G;             // at most 8
+    const int bk = blockIdx.x, b = bk / p.Hkv, hkv = bk % p.Hkv, chunk = blockIdx.y;
+    const __half* Kh = p.K + static_cast<size_t>(bk) * p.Sk * D;
+    const __half* Vh = p.V + static_cast<size_t>(bk) * p.Sk * D;
+    auto row_at = [&](int r) { return (static_cast<size_t>(b) * p.Hq + hkv * G + r % G) * p.Sq + r / G; };
+
+    const int k0 = chunk * p.keys_per_chunk;
+    int k1 = min(p.Sk, k0 + p.keys_per_chunk);
+    if (p.causal) k1 = min(k1, p.Sq);
+    const int steps = k1 > k0 ? (k1 - k0 + kStepKeys - 1) / kStepKeys : 0;
+
+    // this thread's pieces of a step: piece tid % kPieces of keys tid / kPieces + u * kKeysAtOnce
+    constexpr int kKeysAtOnce = kAttnWarps * 32 / kPieces, kCopies = kStepKeys / kKeysAtOnce;
+    const int my_key = tid / kPieces, my_piece = tid % kPieces;
+    const size_t my_at = static_cast<size_t>(my_key) * D + my_piece * 8;
+    static_assert(kKeysAtOnce % 8 == 0, "the swizzle of a thread's pieces is the same for all of them");
+    const uint32_t my_off = static_cast<uint32_t>(my_key * D * 2 + ((my_piece ^ (my_key & 7)) * 16));
+    auto fetch = [&](int st) {
+        if (st < steps) {
+            const int base = k0 + st * kStepKeys;
+            const uint32_t dst = ring + (st % S::kStages) * S::kStageBytes + my_off;
+            const __half* ks = Kh + static_cast<size_t>(base) * D + my_at;
+            const __half* vs = Vh + static_cast<size_t>(base) * D + my_at;
+            if (base + kStepKeys <= k1) {
+#pragma unroll
+                for (int u = 0; u < kCopies; ++u) {
+                    cp_async16(dst + u * kKeysAtOnce * D * 2, ks + u * kKeysAtOnce * D, true);
+                    cp_async16(dst + kStepKeys * D * 2 + u * kKeysAtOnce * D * 2, vs + u * kKeysAtOnce * D, true);
+                }
+            } else {
+#pragma unroll
+                for (int u = 0; u < kCopies; ++u) {
+                    const bool in = base + my_key + u * kKeysAtOnce < k1;
+                    const size_t at = in ? static_cast<size_t>(u) * kKeysAtOnce * D : 0;
+                    cp_async16(dst + u * kKeysAtOnce * D * 2, in ? ks + at : Kh, in);
+                    cp_async16(dst + kStepKeys * D * 2 + u * kKeysAtOnce * D * 2, in ? vs + at : Vh, in);
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int st = 0; st < S::kStages - 1; ++st) fetch(st);
+
+    // the queries as the second operand, and this thread's two rows of the scores
+    uint32_t qf[D / 16][2];
+    {
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(p.Q + row_at(min(gq, R - 1)) * D) + tq;
+#pragma unroll
+        for (int k = 0; k < D / 16; ++k) { qf[k][0] = src[8 * k]; qf[k][1] = src[8 * k + 4]; }
+    }
+    int qi[2];
+    float slope[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const int r = min(2 * tq + e, R - 1);
+        qi[e] = r / G;
+        slope[e] = p.slopes ? p.slopes[hkv * G + r % G] : 0.f;
+    }
+
+    float o[D / 16][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+#pragma unroll
+    for (int n = 0; n < D / 16; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[n][e] = 0.f;
+    const int mi = lane >> 3, ml = lane & 7;               // ldmatrix: which 8x8 matrix, which of its rows
+
+    for (int st = 0; st < steps; ++st) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(S::kStages - 2) : "memory");
+        __syncthreads();                                   // the step has landed; everyone is done with the one before
+        fetch(st + S::kStages - 1);
+        const uint32_t ks = ring + (st % S::kStages) * S::kStageBytes, vs = ks + kStepKeys * D * 2;
+        const int kw = warp * 16, jb = k0 + st * kStepKeys + kw;   // this warp's 16 keys
+
+        // element e: key gq + 8 (e / 2), row 2 tq + e % 2
+        float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int k = 0; k < D / 16; ++k) {
+            const int key = kw + (mi & 1) * 8 + ml, piece = 2 * k + (mi >> 1);
+            uint32_t af[4];
+            ldmatrix4(af, ks + static_cast<uint32_t>(key * D * 2 + ((piece ^ ml) * 16)));
+            mma_16816(s, af, qf[k][0], qf[k][1]);
+        }
+        scale2(s[0], s[1], p.scale);
+        scale2(s[2], s[3], p.scale);
+        if (p.slopes) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[e] -= slope[e & 1] * static_cast<float>(qi[e & 1] - (jb + gq + 8 * (e >> 1)));
+        }
+        if (jb + 16 > k1 || (p.causal && jb + 15 > 0) || p.window > 0) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int i = qi[e & 1], j = gq + 8 * (e >> 1);
+                const int hi = (p.causal ? min(k1, i + 1) : k1) - jb, lo = p.window > 0 ? i - p.window - jb : 0;
+                s[e] = j < hi && j >= lo ? s[e] : -INFINITY;
+            }
+        }
+        float ref[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            s[e] = fmaxf(s[e], -INFINITY);                 // a NaN score counts as masked
+            s[2 + e] = fmaxf(s[2 + e], -INFINITY);
+            float mx = fmaxf(s[e], s[2 + e]);
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+            const float m_new = fmaxf(m[e], mx);
+            ref[e] = m_new > -INFINITY ? m_new : 0.f;      // a row that sees no key so far keeps zero sums
+            const float keep = exp_of(m[e] - ref[e]);
+            m[e] = m_new;
+            l[e] *= keep;
+#pragma unroll
+            for (int n = 0; n < D / 16; ++n) { o[n][e] *= keep; o[n][2 + e] *= keep; }
+        }
+        uint32_t hi[2], lo[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            float a = exp_of(s[2 * h] - ref[0]), c = exp_of(s[2 * h + 1] - ref[1]);      // the probability ...
+            scale2(a, c, kProbScale);                                                   // ... 2^15 times
+            l[0] += a;
+            l[1] += c;
+            split_h2(a, c, hi[h], lo[h]);
+            hi[h] = transpose_8x8(hi[h]);
+            lo[h] = transpose_8x8(lo[h]);
+        }
+#pragma unroll
+        for (int n = 0; n < D / 16; ++n) {
+            const int key = kw + (mi >> 1) * 8 + ml, piece = 2 * n + (mi & 1);
+            uint32_t af[4];
+            ldmatrix4_trans(af, vs + static_cast<uint32_t>(key * D * 2 + ((piece ^ ml) * 16)));
+            mma_16816(o[n], af, hi[0], hi[1]);
+            mma_16816(o[n], af, lo[0], lo[1]);
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    float* o_s = reinterpret_cast<float*>(smem);                     // [warp][8][kStride]
+    float* ml_s = o_s + kAttnWarps * 8 * kStride;                    // [warp][8][2]
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        l[e] += __shfl_xor_sync(0xffffffffu, l[e], 4);
+        l[e] += __shfl_xor_sync(0xffffffffu, l[e], 8);
+        l[e] += __shfl_xor_sync(0xffffffffu, l[e], 16);
+        l[e] *= kProbUnscale;
+        float* dst = o_s + (warp * 8 + 2 * tq + e) * kStride + gq;
+#pragma unroll
+        for (int n = 0; n < D / 16; ++n) {
+            dst[16 * n] = o[n][e] * (kProbUnscale * kUngrow);
+            dst[16 * n + 8] = o[n][2 + e] * (kProbUnscale * kUngrow);
+        }
+        if (gq == 0) { ml_s[(warp * 8 + 2 * tq + e) * 2] = m[e]; ml_s[(warp * 8 + 2 * tq + e) * 2 + 1] = l[e]; }
+    }
+    merge_warps<D, 8, kStride>(p, o_s, ml_s, R, G, b, hkv, bk, chunk);
+}
 // Merges the chunks of a row: one CTA per row, a thread per chunk for the weights exp(m_c - m), then
 // a thread per output element with the chunks' partial outputs as independent loads.
-constexpr int kMergeMaxChunks = 128;
 __global__ void __launch_bounds__(128) attention_merge_kernel(const AttnParams p) {
     __shared__ float e_s[kMergeMaxChunks];
     __shared__ float red_s[4];
@@ -540,6 +811,9 @@ __global__ void __launch_bounds__(128) attention_merge_kernel(const AttnParams p
     }
     if (tid == 0 && p.LSE) p.LSE[row] = mm + logf(fmaxf(ll, 1e-30f));
 }
+
+// Up to 16 rows per K/V head: the warps of a CTA split the keys of a step.
+bool attention_split_keys(int Hq, int Hkv, int Sq) { return static_cast<long long>(Sq) * (Hq / Hkv) <= 16; }
 
 // Query heads one CTA of the vector kernel takes together: two of those that share a K/V head (the
 // other pairs of the same K/V head run in other CTAs and find the cache in L2).
@@ -603,11 +877,11 @@ template <int D>
 cudaError_t launch_matrix(const AttnParams& p, bool prefill, cudaStream_t stream) {
     const long long R = static_cast<long long>(p.Sq) * (p.Hq / p.Hkv);
     if (prefill) return launch_attention_prefill(p, stream);
-    const bool split = R <= 16;
+    const bool split = attention_split_keys(p.Hq, p.Hkv, p.Sq);
     const long long x = static_cast<long long>(p.B) * p.Hkv * ((R + kMmaRows - 1) / kMmaRows);
     if (x > 0x7fffffffLL) return cudaErrorNotSupported;
     const dim3 grid(static_cast<unsigned>(x), static_cast<unsigned>(p.chunks));
-    auto* kernel = split ? attention_mma_kernel<D, true> : attention_mma_kernel<D, false>;
+    auto* kernel = R <= 8 ? attention_mma8_kernel<D> : split ? attention_mma_kernel<D, true> : attention_mma_kernel<D, false>;
     kernel<<<grid, kAttnWarps * 32, MmaShape<D>::kSmem, stream>>>(p);
     return cudaGetLastError();
 }
@@ -626,6 +900,8 @@ cudaError_t init_attention_kernels() {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_mma_kernel<128, false>, a, MmaShape<128>::kSmem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_mma_kernel<64, true>, a, MmaShape<64>::kSmem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_mma_kernel<64, false>, a, MmaShape<64>::kSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_mma8_kernel<128>, a, MmaShape<128>::kSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_mma8_kernel<64>, a, MmaShape<64>::kSmem);
     return e == cudaSuccess ? init_attention_prefill_kernels() : e;
 }
 
@@ -642,8 +918,13 @@ size_t attention_scratch_floats(int B, int Hq, int Hkv, int Sq, int Sk, int D, b
     return chunks > 1 ? rows * chunks * (D + 2) : 0;
 }
 
+size_t attention_state_bytes(int B, int Hq, int Hkv, int Sq, int D, bool matrix, int chunks) {
+    if (!matrix || chunks < 2 || chunks > kMergeHere || !attention_split_keys(Hq, Hkv, Sq)) return 0;
+    return static_cast<size_t>(B) * Hq * Sq * (chunks - 1) * D * 2 * sizeof(uint32_t);
+}
+
 cudaError_t launch_attention_forward(const void* Q, const void* K, const void* V, void* O, float* LSE,
-                                     float* scratch, const float* slopes_dev, int B, int Hq, int Hkv, int Sq,
+                                     float* scratch, uint32_t* states, const float* slopes_dev, int B, int Hq, int Hkv, int Sq,
                                      int Sk, int D, float scale, bool causal, int window, int sm_count,
                                      cudaStream_t stream, int* launches, uint32_t* err_word, const char** name) {
     if (D <= 0 || D > kAttnMaxD) return cudaErrorNotSupported;
@@ -657,7 +938,8 @@ cudaError_t launch_attention_forward(const void* Q, const void* K, const void* V
     p.group = attention_group(Hq, Hkv);
     const bool matrix = attention_on_matrix_kernels(D, Q, K, V);
     attention_chunks(B, Hq, Hkv, Sq, Sk, matrix, sm_count, &p.chunks, &p.keys_per_chunk);
-    if (p.chunks > 1 && !scratch) { p.chunks = 1; p.keys_per_chunk = Sk; }
+    p.states = matrix && attention_split_keys(Hq, Hkv, Sq) && p.chunks <= kMergeHere ? states : nullptr;
+    if (p.chunks > 1 && !scratch && !p.states) { p.chunks = 1; p.keys_per_chunk = Sk; }
     // The tensor core truncates its running sums: a score of D / 16 steps comes out smaller by 2.2e-8 of itself per step
     // on average (mean over 150,000 scores of normal data, mma.sync and tcgen05 alike: 1.8e-7 at head_dim 128, 0.9e-7
     // at 64, always towards zero), where fp32 multiply-adds round without a bias.  The scale makes up for it, as far as an
@@ -682,7 +964,7 @@ cudaError_t launch_attention_forward(const void* Q, const void* K, const void* V
     }
     if (e != cudaSuccess) return e;
     if (launches) *launches += 1;
-    if (p.chunks > 1) {
+    if (p.chunks > 1 && !p.states) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(static_cast<unsigned>(rows));
         cfg.blockDim = dim3(128);

@@ -312,6 +312,7 @@ struct AttnParams {
     __half* O;
     float* LSE;           // may be null
     float* part;          // [rows][chunks][D + 2] when chunks > 1
+    uint32_t* states;     // the same for the CTA that merges them (attention_state_bytes), all bits set between launches; or null
     const float* slopes;  // device copy of the ALiBi slopes, or null
     int B, Hq, Hkv, Sq, Sk, D;
     int group;            // query heads a CTA handles together (attention_group)
@@ -329,9 +330,12 @@ cudaError_t launch_attention_prefill(const AttnParams& p, cudaStream_t stream);
 size_t attention_scratch_floats(int B, int Hq, int Hkv, int Sq, int Sk, int D, bool matrix, int sm_count, int* chunks_out);
 // Whether a call takes the matrix kernels (O may lie at any even address).
 bool attention_on_matrix_kernels(int D, const void* Q, const void* K, const void* V);
+// Bytes of `states` of a call that can merge its chunks in the kernel (else 0): room of the stream's own, all bits set
+// between launches; with it no other scratch and no merge launch is needed.
+size_t attention_state_bytes(int B, int Hq, int Hkv, int Sq, int D, bool matrix, int chunks);
 // cudaErrorNotSupported: head_dim above 128.  slopes_dev: ALiBi slopes on the device, or null.
 cudaError_t launch_attention_forward(const void* Q, const void* K, const void* V, void* O, float* LSE,
-                                     float* scratch, const float* slopes_dev, int B, int Hq, int Hkv, int Sq,
+                                     float* scratch, uint32_t* states, const float* slopes_dev, int B, int Hq, int Hkv, int Sq,
                                      int Sk, int D, float scale, bool causal, int window, int sm_count,
                                      cudaStream_t stream, int* launches, uint32_t* err_word, const char** name);
 

@@ -202,9 +202,10 @@ enum RoomKind : int {
     ROOM_NORM,       // normalised rows
     ROOM_WEIGHTS,    // weights as fp16
     ROOM_SHARES,     // batched quantized products: sums of tiles that several CTAs work on, all bits set between launches
+    ROOM_STATES,     // attention: softmax states of a row's key chunks, all bits set between launches
     kRoomKinds
 };
-constexpr int kRoomFill[kRoomKinds] = {-1, 0, -1, -1, 0xFF};      // the byte a new room is filled with
+constexpr int kRoomFill[kRoomKinds] = {-1, 0, -1, -1, 0xFF, 0xFF};      // the byte a new room is filled with
 struct StreamRooms { Room room[kRoomKinds]; };
 std::mutex g_rooms_mutex;
 std::unordered_map<cudaStream_t, StreamRooms> g_rooms;
@@ -340,6 +341,13 @@ void share_scratch_for(cudaStream_t st, size_t need, tcb::GemvQArgs* a) {
     const Room& r = stream_room(st, ROOM_SHARES, need);
     a->share_scratch = r.p;
     a->share_scratch_bytes = r.bytes;
+}
+// Room for the softmax states that attention merges in its kernel; null where a call has to do without (captured, as
+// for the shares; no memory).
+uint32_t* attention_states_for(cudaStream_t st, size_t need) {
+    if (need == 0 || st == cudaStreamPerThread || being_captured(st)) return nullptr;
+    const Room& r = stream_room(st, ROOM_STATES, need);
+    return r.bytes >= need ? static_cast<uint32_t*>(r.p) : nullptr;
 }
 void norm_scratch_for(cudaStream_t st, size_t need, tcb::GemvQArgs* a) {
     if (need == 0) return;
@@ -1671,11 +1679,13 @@ extern "C" tc_status_t tc_attention_forward(tc_context* ctx, const tc_attention_
     int chunks = 1;
     const long long rows = static_cast<long long>(B) * Hq * Sq;
     if (rows > 0x7fffffffLL) return TC_ERR_INVALID_SHAPE;
-    size_t want = tcb::attention_scratch_floats(B, Hq, Hkv, Sq, Sk, D, tcb::attention_on_matrix_kernels(D, Q->dptr, K->dptr, V->dptr),
-                                                ctx->sm_count, &chunks);
+    const bool matrix = tcb::attention_on_matrix_kernels(D, Q->dptr, K->dptr, V->dptr);
+    size_t want = tcb::attention_scratch_floats(B, Hq, Hkv, Sq, Sk, D, matrix, ctx->sm_count, &chunks);
+    RoomsLock rooms(g_rooms_mutex);
+    uint32_t* const states = attention_states_for(ctx->stream0, tcb::attention_state_bytes(B, Hq, Hkv, Sq, D, matrix, chunks));
+    if (states) want = 0;
     const size_t slope_at = want;
     if (d->alibi_slopes) want += static_cast<size_t>(Hq);
-    RoomsLock rooms(g_rooms_mutex);
     if (want > 0) grow_room(ctx->attn, want * sizeof(float), ~static_cast<size_t>(0), ctx->stream0, -1, [] { cudaDeviceSynchronize(); });
     if (want * sizeof(float) > ctx->attn.bytes) return record("tc_attention_forward", TC_ERR_ALLOC);
     float* const scratch = static_cast<float*>(ctx->attn.p);
@@ -1692,7 +1702,7 @@ extern "C" tc_status_t tc_attention_forward(tc_context* ctx, const tc_attention_
     const tc_status_t st = run_step_op(ctx, "tc_attention_forward", "attention_decode_sm100", io, n_io, [&](cudaStream_t s0) {
         const cudaError_t le = tcb::launch_attention_forward(Q->dptr, K->dptr, V->dptr, O->dptr,
                                              LSE ? static_cast<float*>(LSE->dptr) : nullptr,
-                                             chunks > 1 ? scratch : nullptr, slopes_dev, B, Hq, Hkv, Sq, Sk,
+                                             chunks > 1 && !states ? scratch : nullptr, states, slopes_dev, B, Hq, Hkv, Sq, Sk,
                                              D, scale, d->causal, d->window_size, ctx->sm_count, s0, &launched, ctx->err_dev, &used);
         rooms.unlock();
         return le;
@@ -1704,7 +1714,8 @@ extern "C" tc_status_t tc_attention_forward(tc_context* ctx, const tc_attention_
 
 // The same on raw device pointers, asynchronous on the caller's stream (no ALiBi: its slopes would
 // have to be staged from host memory).  The scratch for the key chunks belongs to the context:
-// launches on different streams must not overlap.
+// launches on different streams must not overlap, except
+// those whose chunks are merged in the kernel (up to 16 rows per K/V head).
 extern "C" tc_status_t tcx_raw_attention_forward(tc_context* ctx, const tc_attention_desc* d, const void* Q,
                                                  const void* K, const void* V, void* O, void* LSE,
                                                  void* cuda_stream) {
@@ -1721,14 +1732,17 @@ extern "C" tc_status_t tcx_raw_attention_forward(tc_context* ctx, const tc_atten
     bind_device(ctx);
     cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
     int chunks = 1;
-    const size_t want = tcb::attention_scratch_floats(d->batch, d->heads, Hkv, d->seq_q, d->seq_kv, d->head_dim,
-                                                       tcb::attention_on_matrix_kernels(d->head_dim, Q, K, V),
-                                                       ctx->sm_count, &chunks);
+    const bool matrix = tcb::attention_on_matrix_kernels(d->head_dim, Q, K, V);
+    const size_t want = tcb::attention_scratch_floats(d->batch, d->heads, Hkv, d->seq_q, d->seq_kv, d->head_dim, matrix, ctx->sm_count, &chunks);
     // Under capture nothing can be allocated: a call that finds too little room takes each row's keys in one piece.
     RoomsLock rooms(g_rooms_mutex, std::defer_lock);
     float* scratch = nullptr;
+    uint32_t* states = nullptr;
     if (want > 0) {
         rooms.lock();
+        states = attention_states_for(st, tcb::attention_state_bytes(d->batch, d->heads, Hkv, d->seq_q, d->head_dim, matrix, chunks));
+    }
+    if (want > 0 && !states) {
         grow_room(ctx->attn, want * sizeof(float), ~static_cast<size_t>(0), st, -1, [] { cudaDeviceSynchronize(); });
         if (want * sizeof(float) <= ctx->attn.bytes) scratch = static_cast<float*>(ctx->attn.p);
         else if (!being_captured(st)) return record("tcx_raw_attention_forward", TC_ERR_ALLOC);
@@ -1737,7 +1751,7 @@ extern "C" tc_status_t tcx_raw_attention_forward(tc_context* ctx, const tc_atten
     int launched = 0;
     const char* used = t_last_kernel;
     const cudaError_t e = tcb::launch_attention_forward(Q, K, V, O, static_cast<float*>(LSE),
-                                                        scratch, nullptr, d->batch,
+                                                        scratch, states, nullptr, d->batch,
                                                         d->heads, Hkv, d->seq_q, d->seq_kv, d->head_dim, scale, d->causal,
                                                         d->window_size, ctx->sm_count, st, &launched, ctx->err_dev, &used);
     g_launches.fetch_add(static_cast<uint64_t>(launched));
@@ -2092,11 +2106,13 @@ extern "C" uint32_t tcx_take_device_error(tc_context* ctx) {
         RoomsLock lock(g_rooms_mutex);
         bind_device(ctx);
         cudaDeviceSynchronize();
-        for (auto& kv : g_rooms) {
-            const Room& r = kv.second.room[ROOM_SHARES];
-            if (r.p) cudaMemset(r.p, kRoomFill[ROOM_SHARES], r.bytes);
+        for (RoomKind k : {ROOM_SHARES, ROOM_STATES}) {
+            for (auto& kv : g_rooms) {
+                const Room& r = kv.second.room[k];
+                if (r.p) cudaMemset(r.p, kRoomFill[k], r.bytes);
+            }
+            for (const Room& r : g_spare[k]) cudaMemset(r.p, kRoomFill[k], r.bytes);
         }
-        for (const Room& r : g_spare[ROOM_SHARES]) cudaMemset(r.p, kRoomFill[ROOM_SHARES], r.bytes);
         (void)cudaGetLastError();
     }
     return v;

@@ -5,6 +5,8 @@ Bar against 64-bit softmax attention: the one rounding is the fp16 result, 2^-11
 (2^-11 / sqrt(3) = 2.82e-4 scaled RMS; a twentieth on top for the fp32 sums and small samples); the
 log-sum-exp is an fp32 number: half a unit in the last place of its scores (up to 500 with ALiBi), 2^-23
 relative with the sum's own rounding, and 1e-5."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -237,3 +239,56 @@ def test_scores_have_no_bias(tc, ctx, B, H, Hkv, Sq, Sk, D, bar):
     err = lse.double() - want
     assert abs((err * want.sign()).mean().item()) <= 1.2e-7
     assert (err ** 2).mean().sqrt().item() <= bar
+
+
+@pytest.mark.parametrize("B,H,Hkv,Sq,Sk,D,causal,window", [
+    (64, 8, 8, 1, 640, 128, False, 0), (37, 8, 2, 2, 1023, 128, True, 0), (20, 14, 2, 1, 2100, 64, False, 0), (20, 6, 3, 4, 1300, 128, False, 700),
+    (70, 5, 1, 1, 4096, 64, False, 0), (10, 16, 8, 3, 257, 64, True, 0), (20, 48, 3, 1, 1500, 128, False, 0), (50, 8, 4, 1, 1, 128, False, 0)])
+def test_chunks_merged_in_the_kernel(tc, ctx, B, H, Hkv, Sq, Sk, D, causal, window):
+    """Up to 16 rows per K/V head: the chunks of a row's keys are merged by the kernel that has them, in one launch; a
+    captured call merges them in a launch of its own, to the same bits.  Bars: one rounding of O, 2^-11 / sqrt(3) rms (a
+    twentieth for small samples); the log-sum-exp as in test_scores_have_no_bias."""
+    import torch
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(Sk + H * Sq)
+    q, k, v = (torch.randn(B, h, s, D, device="cuda", generator=gen).half() for h, s in ((H, Sq), (Hkv, Sk), (Hkv, Sk)))
+    # another call's chunks, so that the captured one finds room for its own
+    room = [ctx.buffer(64 * 64 * 64 * 256), ctx.buffer(8 * 16384 * 256)]
+    tc.attention_forward(ctx, room[0], room[1], room[1], room[0], 1, 64, 64, 16384, 128, causal=False, kv_heads=8)
+    for b in room:
+        b.close()
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    outs = []
+    for captured in (False, False, True):
+        o, lse = torch.full_like(q, float("nan")), torch.full((B, H, Sq), float("nan"), device="cuda")
+        torch.cuda.synchronize()
+        d = tc.TCAttentionDesc(B, H, Sq, Sk, D, tc.TC_DTYPE_F16, tc.TC_DTYPE_F32, 0.0, causal, True, Hkv, window, None)
+
+        def call():
+            rc = tc.lib().tcx_raw_attention_forward(ctx.handle, ctypes.byref(d), *(ctypes.c_void_p(t.data_ptr()) for t in (q, k, v, o, lse)),
+                                                    ctypes.c_void_p(st.cuda_stream))
+            assert rc == 0
+        if captured:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=st):
+                call()
+            with torch.cuda.stream(st):
+                graph.replay()
+        else:
+            before = tc.launch_count()
+            call()
+            assert tc.launch_count() - before == 1 and tc.cuda_last_kernel_name() == "attention_mma_sm100"
+        torch.cuda.synchronize()
+        outs.append((o, lse))
+    for o, lse in outs[1:]:
+        assert torch.equal(o, outs[0][0]) and torch.equal(lse, outs[0][1])
+    s = torch.matmul(q.double().view(B, Hkv, H // Hkv, Sq, D), k.double().unsqueeze(2).transpose(3, 4)) / D ** 0.5
+    i, j = torch.arange(Sq, device="cuda")[:, None], torch.arange(Sk, device="cuda")[None, :]
+    hidden = ((j > i) if causal else torch.zeros_like(j > i)) | ((i - j > window) if window else torch.zeros_like(j > i))
+    s = s.masked_fill(hidden, float("-inf"))
+    want = torch.matmul(torch.softmax(s, dim=4), v.double().unsqueeze(2)).reshape(B, H, Sq, D)
+    o, lse = outs[0]
+    assert ((o.double() - want).square().mean() / want.square().mean()).sqrt().item() <= 1.05 * 2.0 ** -11 / np.sqrt(3.0)
+    assert (lse.double() - torch.logsumexp(s, 4).reshape(B, H, Sq)).square().mean().sqrt().item() <= 3.8e-7
+    assert tc.take_device_error(ctx) == 0
