@@ -934,7 +934,8 @@ cudaError_t launch_attention_forward(const void* Q, const void* K, const void* V
     AttnParams p;
     p.Q = static_cast<const __half*>(Q); p.K = static_cast<const __half*>(K); p.V = static_cast<const __half*>(V);
     p.O = static_cast<__half*>(O); p.LSE = LSE; p.part = scratch; p.slopes = slopes_dev;
-    p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.Sq = Sq; p.Sk = Sk; p.D = D;
+    p.B = B; p.per_kv = Hq / Hkv; p.Hq = Hq; p.Hkv = Hkv; p.Sq = Sq; p.Sk = Sk; p.D = D;
+    p.by_per_kv.set(p.per_kv); p.by_Hkv.set(Hkv); p.by_heads.set(B * Hkv);
     p.group = attention_group(Hq, Hkv);
     const bool matrix = attention_on_matrix_kernels(D, Q, K, V);
     attention_chunks(B, Hq, Hkv, Sq, Sk, matrix, sm_count, &p.chunks, &p.keys_per_chunk);

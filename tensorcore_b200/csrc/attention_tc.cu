@@ -11,16 +11,20 @@
 //   * One issuing warp: S = Q K^T (M128 x N128, operands in shared memory) into one of two score buffers
 //     in tensor memory, the next step's while this step's softmax runs; then O += P V with P in tensor
 //     memory (the A operand) and V as it lies (MN-major).
-//   * Eight softmax warps, two threads per row with 64 scores each in registers: running maximum (exchanged
-//     between the two), exponentials; O is rescaled in tensor memory only when a row's maximum has grown.  The probabilities are fp32
+//   * Sixteen softmax warps, four threads per row with 32 scores each in registers (two with 64: 3500 clocks a step
+//     where four take 2900): running maximum (an atomic on the row's word in shared memory), exponentials; O is rescaled
+//     in tensor memory only when a row's maximum has grown.  The probabilities are fp32
 //     numbers; each goes to the tensor core as two fp16 numbers (attention_math.cuh says to how many bits), two MMAs.
+//   * Q and O cross global memory by whole rows, O through shared memory: a thread per row takes a clock for each lane
+//     and 16 bytes, 2600 for O.  Rows' queries and heads by multiplication (FastDiv): the device's divisions were 700
+//     clocks of the way to the first load.
 //
 // What bounds it: latency.  Causal 512 x 512, 32 heads on 8 K/V heads, head_dim 128 is 128 CTAs of up to four
-// steps; clock stamps of the longest: about 8000 clocks until the first scores (barriers, tensor memory, Q, cold
-// code), then 3500 a step - exponentials and masks 2100 to 2500, rescaling 600, storing P 500 - in which 1060
-// clocks of P V and 530 of Q K^T hide, and 1900 to store O.  28.3 us through the synchronous call (10 us of it
-// launch and wait; 31 with three warps of cp.async as loaders, which a step then waited 1700 clocks for),
-// 38 us on the mma.sync kernel, whose tensor instructions run at an eighth of the rate, 388 us as a
+// steps; clock stamps of the longest before the last changes: 5500 clocks until the first scores (Q's load 2000 of
+// them, its MMAs 1300), 2900 a step - scores and maximum 1000 to 1300, exponentials 1000, rescaling 500, storing P 350 -
+// in which 1060 clocks of P V and 530 of Q K^T hide, 1600 for the last P V, 2900 to store O.  Whole calls: 28.0 us with two
+// threads per row, 26.1 now (10 us of it launch and wait), 2048 x 2048 97.5 -> 88.3, 4 x 2048 x 2048 without a mask
+// 500 -> 467; 38 us on the mma.sync kernel, whose tensor instructions run at an eighth of the rate, 388 us as a
 // streaming pass per query row.
 #include "attention_math.cuh"
 #include "kernels.h"
@@ -36,7 +40,8 @@ using namespace sm100;
 using namespace attn;
 
 constexpr int kRows = 128, kKeys = 128, kStages = 3;
-constexpr int kSoftWarps = 8, kLoadWarp = kSoftWarps, kIssueWarp = kSoftWarps + 1;
+constexpr int kParts = 4;                      // softmax threads per row
+constexpr int kSoftWarps = 4 * kParts, kLoadWarp = kSoftWarps, kIssueWarp = kSoftWarps + 1;
 constexpr int kThreads = (kIssueWarp + 1) * 32;
 constexpr int kBarBytes = 3072;
 constexpr uint32_t kSwizzle128 = 2;
@@ -47,13 +52,20 @@ struct PrefillBars {
     uint64_t q_full, k_full[kStages], v_full[kStages], kv_empty[kStages], s_full[2], s_empty[2], p_full, pv_done, drain, both[4];
     uint32_t tmem_base;
     int abort_flag;
-    float pair[2][2][kRows];      // what the two threads of a row tell each other, two buffers
+    int best[3][kRows];           // the threads of a row work out its maximum here (order_of), in turn in three buffers
 };
 static_assert(sizeof(PrefillBars) <= kBarBytes, "barrier block too large");
 
 __device__ __forceinline__ uint64_t desc128(uint32_t addr, uint32_t lbo) {
     return smem_desc_kmajor(addr, lbo, 1024u) | (static_cast<uint64_t>(kSwizzle128) << 61);
 }
+
+// Floats (no NaN) as integers of the same order, and back.
+__device__ __forceinline__ int order_of(float v) {
+    const int b = __float_as_int(v);
+    return b >= 0 ? b : b ^ 0x7fffffff;
+}
+__device__ __forceinline__ float value_of(int b) { return __int_as_float(b >= 0 ? b : b ^ 0x7fffffff); }
 
 template <int D>
 __global__ void __launch_bounds__(kThreads, 1) attention_prefill_kernel(const AttnParams p, const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap) {
@@ -67,53 +79,84 @@ __global__ void __launch_bounds__(kThreads, 1) attention_prefill_kernel(const At
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-    const int G = p.Hq / p.Hkv, R = p.Sq * G;
-    const int heads = p.B * p.Hkv, bk = blockIdx.x % heads;
+    const int G = p.per_kv, R = p.Sq * G;
+    const int heads = p.B * p.Hkv, tile_no = p.by_heads(static_cast<int>(blockIdx.x)), bk = static_cast<int>(blockIdx.x) - tile_no * heads;
     const int row_tiles = (R + kRows - 1) / kRows;
-    const int tile0 = (row_tiles - 1 - static_cast<int>(blockIdx.x / heads)) * kRows;    // long causal tiles first
-    const int b = bk / p.Hkv, hkv = bk % p.Hkv, chunk = blockIdx.y;
+    const int tile0 = (row_tiles - 1 - tile_no) * kRows;    // long causal tiles first
+    const int b = p.by_Hkv(bk), hkv = bk - b * p.Hkv, chunk = blockIdx.y;
     // keys any row of the tile can see, in whole steps from the chunk's start
-    const int i_min = tile0 / G, i_max = (min(R, tile0 + kRows) - 1) / G;
+    const int i_min = p.by_per_kv(tile0);
+    auto query_of = [&](int lrow) { return p.by_per_kv(tile0 + lrow); };
+    const int i_max = query_of(min(R - tile0, kRows) - 1);
     int k0 = chunk * p.keys_per_chunk, k1 = min(p.Sk, k0 + p.keys_per_chunk);
     if (p.causal) k1 = min(k1, i_max + 1);
     if (p.window > 0 && i_min - p.window > k0) k0 += (i_min - p.window - k0) / kKeys * kKeys;
     const int steps = k1 > k0 ? (k1 - k0 + kKeys - 1) / kKeys : 0;
 
-    if (tid == 0) {
-        bar_init(&bars->q_full, kSoftWarps);
-        for (int i = 0; i < kStages; ++i) {
-            bar_init(&bars->k_full[i], 1);
-            bar_init(&bars->v_full[i], 1);
-            bar_init(&bars->kv_empty[i], 1);
+    // Rows of Q and O are read and written whole, D / 8 lanes of a warp to a row (a thread per row took a clock per lane
+    // and 16 bytes: 2600 for O, as much for Q); a softmax warp has the eight rows from my_row0.
+    auto row_of = [&](int lrow, bool* there) {
+        *there = tile0 + lrow < R;
+        if (!*there) lrow = R - 1 - tile0;
+        const int i = query_of(lrow);
+        return (b * p.Hq + hkv * G + (tile0 + lrow - i * G)) * p.Sq + i;      // below 2^31 (launch_attention_forward)
+    };
+    constexpr int kLanes = D / 8, kRowsAtOnce = 32 / kLanes, kTurns = 8 / kRowsAtOnce;      // of 16 bytes; rows a load; loads
+    const int quad = warp & 3, part_no = warp >> 2, piece = lane % kLanes;
+    const int my_row0 = quad * 32 + part_no * 8 + lane / kLanes;
+    int rows_at[kTurns];
+    bool rows_live[kTurns];
+    uint4 q_piece[kTurns];
+    if (warp < kSoftWarps) {                 // on its way while barriers and tensor memory are set up
+#pragma unroll
+        for (int u = 0; u < kTurns; ++u) {
+            rows_at[u] = row_of(my_row0 + u * kRowsAtOnce, &rows_live[u]);
+            asm volatile("" : "+r"(rows_at[u]));          // not to be worked out again for O
+            // (volatile: the compiler would move the load down to its use)
+            asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(q_piece[u].x), "=r"(q_piece[u].y), "=r"(q_piece[u].z), "=r"(q_piece[u].w) : "l"(p.Q + static_cast<size_t>(rows_at[u]) * D + piece * 8));
         }
-        for (int i = 0; i < 2; ++i) {
-            bar_init(&bars->s_full[i], 1);
-            bar_init(&bars->s_empty[i], kSoftWarps);
-        }
-        bar_init(&bars->p_full, kSoftWarps);
-        bar_init(&bars->pv_done, 1);
-        bar_init(&bars->drain, 1);
-        for (int i = 0; i < 4; ++i) bar_init(&bars->both[i], 2);
-        bars->abort_flag = 0;
-        fence_barrier_init();
     }
-    if (tid == kLoadWarp * 32) { prefetch_tensormap(&kmap); prefetch_tensormap(&vmap); }
-    __syncthreads();
-    // The first K and V are on their way while tensor memory is allocated.
+    // The loader's own barriers, and the first K and V on their way; tensor memory and the other barriers beside it.
     auto fetch = [&](const CUtensorMap* map, uint64_t* bar, uint32_t offset, int key) {
         bar_expect_tx(bar, kTile);
 #pragma unroll
         for (int sl = 0; sl < kSlabs; ++sl)
             tensor_load_3d(smem + kBarBytes + kTile + offset + sl * kSlab, map, 64 * sl, key, bk, bar);
     };
-    if (warp == kLoadWarp && steps > 0) {
-        if (elect_one()) {
+    if (warp == kLoadWarp) {
+        if (lane == 0) { prefetch_tensormap(&kmap); prefetch_tensormap(&vmap); }
+        if (lane < kStages) {
+            bar_init(&bars->k_full[lane], 1);
+            bar_init(&bars->v_full[lane], 1);
+            bar_init(&bars->kv_empty[lane], 1);
+        }
+        fence_barrier_init();
+        fence_proxy_async();
+        __syncwarp();
+        if (steps > 0 && elect_one()) {
             fetch(&kmap, &bars->k_full[0], 0, k0);
             fetch(&vmap, &bars->v_full[0], kTile, k0);
         }
         __syncwarp();
+    } else if (warp == kIssueWarp) {
+        if (lane < 4) {
+            bar_init(&bars->both[lane], kParts);
+        } else if (lane < 6) {
+            bar_init(&bars->s_full[lane - 4], 1);
+            bar_init(&bars->s_empty[lane - 4], kSoftWarps);
+        } else if (lane == 6) {
+            bar_init(&bars->q_full, kSoftWarps);
+            bar_init(&bars->p_full, kSoftWarps);
+            bar_init(&bars->pv_done, 1);
+            bar_init(&bars->drain, 1);
+            bars->abort_flag = 0;
+        }
+        fence_barrier_init();
+        __syncwarp();
+        tmem_alloc(&bars->tmem_base, kTmemCols);
     }
-    if (warp == kIssueWarp) tmem_alloc(&bars->tmem_base, kTmemCols);
+    for (int e = tid; e < 3 * kRows; e += kThreads) (&bars->best[0][0])[e] = order_of(-INFINITY);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -121,84 +164,83 @@ __global__ void __launch_bounds__(kThreads, 1) attention_prefill_kernel(const At
     bool failed = false;
 
     if (warp < kSoftWarps) {
-        // ---------------- softmax: two threads per row = TMEM lane, half of the keys (or columns of O) each ------
-        constexpr int kHalf = kKeys / 2;
-        const int quad = warp & 3, hf = warp >> 2, lr = quad * 32 + lane, r = tile0 + lr;
-        const bool live = r < R;
-        const int rr = live ? r : R - 1, i = rr / G, h = hkv * G + (rr - i * G);
-        const size_t row_at = (static_cast<size_t>(b) * p.Hq + h) * p.Sq + i;
-        const float slope = p.slopes ? p.slopes[h] : 0.f;
+        // ---------------- softmax: kParts threads per row = TMEM lane, a part of the keys (or columns of O) each ------
+        constexpr int kMine = kKeys / kParts, kCols = D / kParts;
+        const int lr = quad * 32 + lane, r = tile0 + lr, i = query_of(r < R ? lr : R - 1 - tile0);      // this thread's row
+        const float slope = p.slopes ? p.slopes[hkv * G + ((r < R ? r : R - 1) - i * G)] : 0.f;
         const uint32_t lanes = tmem + (static_cast<uint32_t>(quad * 32) << 16);
         {
-            const uint4* src = reinterpret_cast<const uint4*>(p.Q + row_at * D);
 #pragma unroll
-            for (int u = 0; u < D / 16; ++u) {
-                const int c = hf * (D / 16) + u;
-                sts128(q_s + (c / 8) * kSlab + lr * 128 + (((c & 7) ^ (lr & 7)) * 16), src[c]);
+            for (int u = 0; u < kTurns; ++u) {
+                const int lrow = my_row0 + u * kRowsAtOnce;
+                sts128(q_s + (piece / 8) * kSlab + lrow * 128 + (((piece & 7) ^ (lrow & 7)) * 16), q_piece[u]);
             }
             fence_proxy_async();
             __syncwarp();
             if (lane == 0) bar_arrive(&bars->q_full);
         }
-        // the row's other thread is in warp +-4: a value each through shared memory
-        uint32_t turn = 0;
-        auto exchange = [&](float v) {
-            bars->pair[turn][hf][lr] = v;
+        // The row's other threads are four warps apart.  A buffer is cleared once the barrier after its use has shown
+        // that all of them have read it, and used again behind the next.
+        auto row_wait = [&](uint32_t parity) {
             __syncwarp();
             if (lane == 0) bar_arrive(&bars->both[quad]);
-            if (!wait_all(&bars->both[quad], turn, abort_flag)) failed = true;
-            const float other = bars->pair[turn][hf ^ 1][lr];
-            turn ^= 1u;
-            return other;
+            if (!wait_all(&bars->both[quad], parity, abort_flag)) failed = true;
+        };
+        auto row_max = [&](float v, int t) {
+            atomicMax(&bars->best[t % 3][lr], order_of(v));
+            row_wait(static_cast<uint32_t>(t) & 1u);
+            const float all = value_of(bars->best[t % 3][lr]);
+            if (part_no == 0) bars->best[(t + 2) % 3][lr] = order_of(-INFINITY);
+            return all;
         };
         float m = -INFINITY, l = 0.f;
         for (int t = 0; t < steps; ++t) {
-            const int buf = t & 1, jb = k0 + t * kKeys + hf * kHalf;      // this thread's first key
+            const int buf = t & 1, jb = k0 + t * kKeys + part_no * kMine;      // this thread's first key
             if (!wait_all(&bars->s_full[buf], static_cast<uint32_t>(t >> 1) & 1u, abort_flag)) { failed = true; break; }
             tc_fence_after_sync();
-            uint32_t raw[kHalf / 16][16];
+            uint32_t raw[kMine / 16][16];
 #pragma unroll
-            for (int c = 0; c < kHalf / 16; ++c)
-                tmem_ld16(lanes + kColS + static_cast<uint32_t>(buf * kKeys + hf * kHalf + 16 * c), raw[c]);
+            for (int c = 0; c < kMine / 16; ++c)
+                tmem_ld16(lanes + kColS + static_cast<uint32_t>(buf * kKeys + part_no * kMine + 16 * c), raw[c]);
             tmem_wait_ld();
-            float s[kHalf];
+            float s[kMine];
 #pragma unroll
-            for (int e = 0; e < kHalf; ++e) {
+            for (int e = 0; e < kMine; ++e) {
                 asm volatile("" : "+r"(raw[e / 16][e % 16]));                    // read behind the wait
                 s[e] = __uint_as_float(raw[e / 16][e % 16]);
             }
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) bar_arrive(&bars->s_empty[buf]);
-            const bool masked = jb + kHalf > k1 || (p.causal && jb + kHalf - 1 > i_min) || p.window > 0;
+            const bool masked = jb + kMine > k1 || (p.causal && jb + kMine - 1 > i_min) || p.window > 0;
             // Straight-line selects throughout: a branch per element made this part four times as long.  A NaN
             // score counts as masked, as in the other kernels.
 #pragma unroll
-            for (int e = 0; e < kHalf; e += 2) scale2(s[e], s[e + 1], p.scale);
+            for (int e = 0; e < kMine; e += 2) scale2(s[e], s[e + 1], p.scale);
             if (p.slopes) {
 #pragma unroll
-                for (int e = 0; e < kHalf; ++e) s[e] -= slope * static_cast<float>(i - jb - e);
+                for (int e = 0; e < kMine; ++e) s[e] -= slope * static_cast<float>(i - jb - e);
             }
             if (masked) {
                 const int hi_e = (p.causal ? min(k1, i + 1) : k1) - jb, lo_e = p.window > 0 ? i - p.window - jb : 0;
 #pragma unroll
-                for (int e = 0; e < kHalf; ++e) s[e] = e < hi_e && e >= lo_e ? s[e] : -INFINITY;
+                for (int e = 0; e < kMine; ++e) s[e] = e < hi_e && e >= lo_e ? s[e] : -INFINITY;
             }
             float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-            for (int e = 0; e < kHalf; ++e) {
+            for (int e = 0; e < kMine; ++e) {
                 s[e] = fmaxf(s[e], -INFINITY);
                 mx[e & 3] = fmaxf(mx[e & 3], s[e]);
             }
             const float mine = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-            const float m_new = fmaxf(m, fmaxf(mine, exchange(mine)));
+            const float m_new = fmaxf(m, row_max(mine, t));
             if (failed) break;
             const float ref = m_new > -INFINITY ? m_new : 0.f;          // a row that sees no key so far keeps zero sums
             const float keep = exp_of(m - ref);
             m = m_new;
             float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int e = 0; e < kHalf; e += 2) {
+            for (int e = 0; e < kMine; e += 2) {
                 s[e] = exp_of(s[e] - ref);                               // now the probability ...
                 s[e + 1] = exp_of(s[e + 1] - ref);
                 scale2(s[e], s[e + 1], kProbScale);                      // ... 2^15 times
@@ -211,31 +253,29 @@ __global__ void __launch_bounds__(kThreads, 1) attention_prefill_kernel(const At
                 if (!wait_all(&bars->pv_done, static_cast<uint32_t>(t - 1) & 1u, abort_flag)) { failed = true; break; }
                 tc_fence_after_sync();
                 if (__any_sync(0xffffffffu, keep != 1.f)) {
+                    uint32_t v[kCols / 16][16];
+                    const uint32_t at = lanes + kColO + static_cast<uint32_t>(part_no * kCols);
 #pragma unroll
-                    for (int c = 0; c < D / 2; c += 32) {
-                        const uint32_t at = lanes + kColO + static_cast<uint32_t>(hf * (D / 2) + c);
-                        uint32_t v[16], w[16];
-                        tmem_ld16(at, v);
-                        tmem_ld16(at + 16u, w);
-                        tmem_wait_ld();
+                    for (int c = 0; c < kCols / 16; ++c) tmem_ld16(at + 16u * c, v[c]);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int c = 0; c < kCols / 16; ++c) {
 #pragma unroll
                         for (int e = 0; e < 16; ++e) {
-                            asm volatile("" : "+r"(v[e]), "+r"(w[e]));
-                            v[e] = __float_as_uint(__uint_as_float(v[e]) * keep);
-                            w[e] = __float_as_uint(__uint_as_float(w[e]) * keep);
+                            asm volatile("" : "+r"(v[c][e]));
+                            v[c][e] = __float_as_uint(__uint_as_float(v[c][e]) * keep);
                         }
-                        tmem_st16(at, v);
-                        tmem_st16(at + 16u, w);
+                        tmem_st16(at + 16u * c, v[c]);
                     }
                 }
             }
 #pragma unroll
-            for (int c = 0; c < kHalf / 32; ++c) {
+            for (int c = 0; c < kMine / 32; ++c) {
                 uint32_t hi[16], lo[16];
 #pragma unroll
                 for (int e = 0; e < 16; ++e) split_h2(s[32 * c + 2 * e], s[32 * c + 2 * e + 1], hi[e], lo[e]);
-                tmem_st16(lanes + kColPHi + static_cast<uint32_t>(hf * (kHalf / 2) + 16 * c), hi);
-                tmem_st16(lanes + kColPLo + static_cast<uint32_t>(hf * (kHalf / 2) + 16 * c), lo);
+                tmem_st16(lanes + kColPHi + static_cast<uint32_t>(part_no * (kMine / 2) + 16 * c), hi);
+                tmem_st16(lanes + kColPLo + static_cast<uint32_t>(part_no * (kMine / 2) + 16 * c), lo);
             }
             tmem_wait_st();
             tc_fence_before_sync();
@@ -246,50 +286,86 @@ __global__ void __launch_bounds__(kThreads, 1) attention_prefill_kernel(const At
             if (!wait_all(&bars->pv_done, static_cast<uint32_t>(steps - 1) & 1u, abort_flag)) failed = true;
             tc_fence_after_sync();
         }
-        if (!failed) l += exchange(l);
+        if (!failed) {                                       // the row's sum, through the ring: every copy and MMA is done
+            float* sums = reinterpret_cast<float*>(smem + kBarBytes + kTile);
+            sums[part_no * kRows + lr] = l;
+            row_wait(static_cast<uint32_t>(steps) & 1u);
+            l = sums[lr];
+#pragma unroll
+            for (int k = 1; k < kParts; ++k) l += sums[k * kRows + lr];
+        }
         if (!failed) {
-            const float inv = l != 0.f ? kUngrow / l : 0.f;              // l and O are both 2^15 times as large here
-            float* part = p.part + (row_at * p.chunks + chunk) * (D + 2);
-            {
-                constexpr int kQ = D / 32;                 // pieces of 16 columns of this thread's half
-                uint32_t v[kQ][16];
+            // Through shared memory, so that rows leave whole: results as they go to O, or fp32 as they go to scratch.
+            const float scale = p.chunks > 1 ? kProbUnscale * kUngrow : l != 0.f ? kUngrow / l : 0.f;      // l and O are both 2^15 times as large here
+            constexpr int kStrideH = D * 2 + 16, kStrideF = D * 4 + 16;                  // bytes; odd multiples of 16
+            const uint32_t rows_s = ring + kRows * 4 * kParts;                           // behind the sums
+            uint32_t v[kCols / 16][16];
 #pragma unroll
-                for (int q = 0; q < kQ; ++q) {
+            for (int q = 0; q < kCols / 16; ++q) {
 #pragma unroll
-                    for (int e = 0; e < 16; ++e) v[q][e] = 0u;
-                    if (steps > 0) tmem_ld16(lanes + kColO + static_cast<uint32_t>(hf * (D / 2) + 16 * q), v[q]);
+                for (int e = 0; e < 16; ++e) v[q][e] = 0u;
+                if (steps > 0) tmem_ld16(lanes + kColO + static_cast<uint32_t>(part_no * kCols + 16 * q), v[q]);
+            }
+            tmem_wait_ld();
+#pragma unroll
+            for (int q = 0; q < kCols / 16; ++q) {
+                float f[16];
+#pragma unroll
+                for (int e = 0; e < 16; ++e) {
+                    asm volatile("" : "+r"(v[q][e]));
+                    f[e] = __uint_as_float(v[q][e]) * scale;
                 }
-                tmem_wait_ld();
+                const int c = part_no * kCols + 16 * q;
+                if (p.chunks == 1) {
 #pragma unroll
-                for (int q = 0; q < kQ; ++q) {
+                    for (int e = 0; e < 16; e += 8)
+                        sts128(rows_s + lr * kStrideH + (c + e) * 2,
+                               make_uint4(pack_h2(f[e], f[e + 1]), pack_h2(f[e + 2], f[e + 3]), pack_h2(f[e + 4], f[e + 5]), pack_h2(f[e + 6], f[e + 7])));
+                } else {
 #pragma unroll
-                    for (int e = 0; e < 16; ++e) asm volatile("" : "+r"(v[q][e]));
-                    const int c = hf * (D / 2) + 16 * q;
-                    if (!live) continue;
-                    if (p.chunks == 1) {
-                        uint32_t o[8];
-#pragma unroll
-                        for (int e = 0; e < 8; ++e)
-                            o[e] = pack_h2(__uint_as_float(v[q][2 * e]) * inv, __uint_as_float(v[q][2 * e + 1]) * inv);
-                        if (p.o_vec) {
-                            uint4* dst = reinterpret_cast<uint4*>(p.O + row_at * D + c);
-                            dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-                            dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
-                        } else {
-                            uint16_t* dst = reinterpret_cast<uint16_t*>(p.O + row_at * D + c);
-#pragma unroll
-                            for (int e = 0; e < 16; ++e) dst[e] = static_cast<uint16_t>(o[e / 2] >> (16 * (e & 1)));
-                        }
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 16; e += 2)
-                            *reinterpret_cast<float2*>(part + 2 + c + e) = make_float2(__uint_as_float(v[q][e]) * (kProbUnscale * kUngrow), __uint_as_float(v[q][e + 1]) * (kProbUnscale * kUngrow));
-                    }
+                    for (int e = 0; e < 16; e += 4)
+                        sts128(rows_s + lr * kStrideF + (c + e) * 4,
+                               make_uint4(__float_as_uint(f[e]), __float_as_uint(f[e + 1]), __float_as_uint(f[e + 2]), __float_as_uint(f[e + 3])));
                 }
             }
-            if (live && hf == 0) {
-                if (p.chunks > 1) { part[0] = m; part[1] = l * kProbUnscale; }
-                else if (p.LSE) p.LSE[row_at] = m + logf(fmaxf(l * kProbUnscale, 1e-30f));
+            if (r < R && part_no == 0) {
+                bool there;
+                const size_t at = row_of(lr, &there);
+                if (p.chunks > 1) {
+                    float* part = p.part + (at * p.chunks + chunk) * (D + 2);
+                    part[0] = m;
+                    part[1] = l * kProbUnscale;
+                } else if (p.LSE) {
+                    p.LSE[at] = m + logf(fmaxf(l * kProbUnscale, 1e-30f));
+                }
+            }
+            row_wait(static_cast<uint32_t>(steps + 1) & 1u);
+            if (!failed) {
+#pragma unroll
+                for (int u = 0; u < kTurns; ++u) {
+                    const int lrow = my_row0 + u * kRowsAtOnce;
+                    if (!rows_live[u]) continue;
+                    if (p.chunks > 1) {
+                        float* part = p.part + (static_cast<size_t>(rows_at[u]) * p.chunks + chunk) * (D + 2) + 2;
+#pragma unroll
+                        for (int x = 0; x < 2; ++x) {
+                            const int c = (x * kLanes + piece) * 4;
+                            const uint4 w = lds128(rows_s + lrow * kStrideF + c * 4);
+                            reinterpret_cast<uint2*>(part + c)[0] = make_uint2(w.x, w.y);
+                            reinterpret_cast<uint2*>(part + c)[1] = make_uint2(w.z, w.w);
+                        }
+                        continue;
+                    }
+                    const uint4 w = lds128(rows_s + lrow * kStrideH + piece * 16);
+                    __half* dst = p.O + static_cast<size_t>(rows_at[u]) * D + piece * 8;
+                    if (p.o_vec) {
+                        *reinterpret_cast<uint4*>(dst) = w;
+                    } else {
+                        const uint32_t o[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) reinterpret_cast<uint16_t*>(dst)[e] = static_cast<uint16_t>(o[e / 2] >> (16 * (e & 1)));
+                    }
+                }
             }
         }
         tc_fence_before_sync();

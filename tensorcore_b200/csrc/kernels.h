@@ -305,6 +305,22 @@ cudaError_t launch_gemm_f16_tc(const void* A, const void* B, void* C, int M, int
 
 // --- attention forward (attention.cu); fp16 data, fp32 softmax ----------------------------
 cudaError_t init_attention_kernels();
+// Division of 0 <= n < 2^31 by a number known to the host: mul = 2^(31 + s) / d rounded up, s = ceil(log2 d), is exact
+// there; two instructions where the device's division is a chain of 150 clocks and more.
+struct FastDiv {
+    uint32_t mul = 0;
+    int shift = -1;       // s - 1
+    void set(int d) {
+        shift = -1;
+        while ((1ll << (shift + 1)) < d) ++shift;
+        mul = static_cast<uint32_t>(((1ull << (32 + shift)) / static_cast<uint64_t>(d)) + 1);
+    }
+#ifdef __CUDACC__
+    __device__ __forceinline__ int operator()(int n) const {
+        return shift < 0 ? n : static_cast<int>(__umulhi(static_cast<uint32_t>(n), mul) >> shift);
+    }
+#endif
+};
 struct AttnParams {
     const __half* Q;
     const __half* K;
@@ -315,6 +331,8 @@ struct AttnParams {
     uint32_t* states;     // the same for the CTA that merges them (attention_state_bytes), all bits set between launches; or null
     const float* slopes;  // device copy of the ALiBi slopes, or null
     int B, Hq, Hkv, Sq, Sk, D;
+    int per_kv;           // Hq / Hkv
+    FastDiv by_per_kv, by_Hkv, by_heads;      // by_heads: B * Hkv
     int group;            // query heads a CTA handles together (attention_group)
     int chunks, keys_per_chunk;
     float scale;

@@ -292,3 +292,31 @@ def test_chunks_merged_in_the_kernel(tc, ctx, B, H, Hkv, Sq, Sk, D, causal, wind
     assert ((o.double() - want).square().mean() / want.square().mean()).sqrt().item() <= 1.05 * 2.0 ** -11 / np.sqrt(3.0)
     assert (lse.double() - torch.logsumexp(s, 4).reshape(B, H, Sq)).square().mean().sqrt().item() <= 3.8e-7
     assert tc.take_device_error(ctx) == 0
+
+
+@pytest.mark.parametrize("B,H,Hkv,Sq,Sk,D,causal,off", [
+    (5, 21, 3, 130, 300, 128, True, 0), (9, 15, 5, 77, 700, 64, False, 0), (2, 22, 2, 65, 2000, 128, False, 1), (37, 8, 8, 129, 260, 64, True, 3),
+    (3, 39, 13, 200, 450, 128, True, 0), (40, 8, 8, 65, 300, 128, False, 0)])
+def test_prefill_rows_of_odd_groups(tc, ctx, B, H, Hkv, Sq, Sk, D, causal, off):
+    """The prefill kernel's rows - queries of 3 to 11 heads per K/V head, tiles that are not full, results `off` elements past a
+    16-byte boundary, key chunks - against 64 bits; bars as in test_chunks_merged_in_the_kernel."""
+    import torch
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(Sk)
+    q, k, v = (torch.randn(B, h, s, D, device="cuda", generator=gen).half() for h, s in ((H, Sq), (Hkv, Sk), (Hkv, Sk)))
+    room = torch.full((q.numel() + 16,), float("nan"), device="cuda").half()
+    o, lse = room[off:off + q.numel()].view(q.shape), torch.full((B, H, Sq), float("nan"), device="cuda")
+    torch.cuda.synchronize()
+    bufs = [ctx.buffer_from_ptr(t.data_ptr(), t.numel() * t.element_size()) for t in (q, k, v, o, lse)]
+    tc.attention_forward(ctx, *bufs[:4], B, H, Sq, Sk, D, LSE=bufs[4], causal=causal, kv_heads=Hkv)
+    assert tc.cuda_last_kernel_name() == "attention_prefill_tcgen05_sm100"
+    for b in bufs:
+        b.close()
+    s = torch.matmul(q.double().view(B, Hkv, H // Hkv, Sq, D), k.double().unsqueeze(2).transpose(3, 4)) / D ** 0.5
+    if causal:
+        s = s.masked_fill(~torch.ones(Sq, Sk, dtype=torch.bool, device="cuda").tril(), float("-inf"))
+    want = torch.matmul(torch.softmax(s, dim=4), v.double().unsqueeze(2)).reshape(B, H, Sq, D)
+    assert ((o.double() - want).square().mean() / want.square().mean()).sqrt().item() <= 1.05 * 2.0 ** -11 / np.sqrt(3.0)
+    assert (lse.double() - torch.logsumexp(s, 4).reshape(B, H, Sq)).square().mean().sqrt().item() <= 3.8e-7
+    assert torch.isnan(room[off + q.numel():]).all() and torch.isnan(room[:off]).all()
+    assert tc.take_device_error(ctx) == 0
