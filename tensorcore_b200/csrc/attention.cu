@@ -16,6 +16,7 @@
 //     with one chunk it writes O (and LSE) itself, else it leaves (m, l, o) in scratch and a second
 //     small kernel merges the chunks.
 #include "attention_math.cuh"
+#include "handover.cuh"
 #include "kernels.h"
 
 #include <cuda_fp16.h>
@@ -232,44 +233,34 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4],
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// Partial softmax states that a CTA leaves for the one that merges its row: words that are kNoState until they have
-// been written, so that a reader knows them by their being there (no flag, no fence on either side) and leaves
-// kNoState behind.  A NaN that has these bits is stored as another one.
-constexpr uint32_t kNoState = 0xFFFFFFFFu;
-__device__ __forceinline__ uint32_t state_word(float v) {
-    const uint32_t w = __float_as_uint(v);
-    return w == kNoState ? 0x7FFFFFFFu : w;
-}
+// Partial softmax states that a CTA leaves for the one that merges its row (handover.cuh).
 __device__ __forceinline__ void state_store4(uint32_t* dst, float4 v) {
-    asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};"
-                 ::"l"(dst), "r"(state_word(v.x)), "r"(state_word(v.y)), "r"(state_word(v.z)), "r"(state_word(v.w)) : "memory");
+    using handover::word_of;
+    handover::store4(dst, make_uint4(word_of(v.x), word_of(v.y), word_of(v.z), word_of(v.w)));
 }
 // What n chunks have of four elements, {o, o, o, o} and {m, l, -, -} each: all asked for at a time, until all are
 // there; false after about a second.
 template <int N>
 __device__ __forceinline__ bool state_take(uint32_t* src, size_t stride, int n, uint4 (&o)[N], uint4 (&ml)[N]) {
     const long long t0 = clock64();
-    auto there = [](const uint4& v) { return v.x != kNoState && v.y != kNoState && v.z != kNoState && v.w != kNoState; };
     for (;;) {
         bool all = true;
 #pragma unroll
         for (int i = 0; i < N; ++i)
             if (i < n) {
-                asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-                             : "=r"(o[i].x), "=r"(o[i].y), "=r"(o[i].z), "=r"(o[i].w) : "l"(src + i * stride) : "memory");
-                asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-                             : "=r"(ml[i].x), "=r"(ml[i].y), "=r"(ml[i].z), "=r"(ml[i].w) : "l"(src + i * stride + 4) : "memory");
+                o[i] = handover::load4(src + i * stride);
+                ml[i] = handover::load4(src + i * stride + 4);
             }
 #pragma unroll
         for (int i = 0; i < N; ++i)
-            if (i < n) all = all && there(o[i]) && there(ml[i]);
+            if (i < n) all = all && handover::there(o[i]) && handover::there(ml[i]);
         if (all) break;
         if (clock64() - t0 > 2000000000LL) return false;
     }
+    constexpr uint32_t w = handover::kNothing;
 #pragma unroll
     for (int i = 0; i < 2 * N; ++i)
-        if (i < 2 * n)
-            asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %1, %1, %1};" ::"l"(src + i / 2 * stride + 4 * (i & 1)), "r"(kNoState) : "memory");
+        if (i < 2 * n) handover::store4(src + i / 2 * stride + 4 * (i & 1), make_uint4(w, w, w, w));
     return true;
 }
 // An 8 x 8 matrix of 16-bit elements, a thread's two those of row lane / 4, transposed.

@@ -11,13 +11,13 @@
 // four-stage ring in shared memory; a thread reads back exactly the pieces it copied, so the
 // ring needs no barrier), works out the row statistics meanwhile (K values from L2; cheaper than
 // a separate kernel and an fp16 round trip), normalises its K range into shared memory, streams
-// its tile and leaves its partial sums in scratch;
-// the CTA that finishes a column strip last adds the strip's partial sums in K order - the result
-// does not depend on which CTA that is - and writes fp16 Y.  The scratch (partial sums and one
-// ticket counter per strip, which the last CTA resets) belongs to the stream the call runs on.
+// its tile and leaves its partial sums in scratch (handover.cuh);
+// the CTA of a column strip's last K range, which started last, adds them in K order, its own at the end, and writes
+// fp16 Y.  The scratch belongs to the stream the call runs on.
 //
 // Without scratch, for N not a multiple of 8 or an unaligned W: a CTA owns a strip of 32 columns
 // and all of K (dense_norm_gemv_kernel), or one thread owns a column (scalar kernel).
+#include "handover.cuh"
 #include "kernels.h"
 
 #include <cuda_fp16.h>
@@ -251,8 +251,8 @@ constexpr int kSplitSmemBase = 128 + kStages * kStageBytes;     // and the norma
 
 struct SplitParams {
     DenseParams d;
-    float* partial;      // [chunks][M][N]
-    int* counters;       // [strips], zero between launches
+    uint32_t* partial;   // [chunks - 1][M][N] sums, nothing between launches
+    uint32_t* err;
     int kc;              // K rows per tile (a multiple of kStageRows)
     int chunks;
 };
@@ -269,7 +269,6 @@ template <int MB>
 __global__ void __launch_bounds__(kDThreads) dense_norm_gemv_split_kernel(const SplitParams sp) {
     extern __shared__ __align__(128) uint8_t dsm[];
     double* scratch = reinterpret_cast<double*>(dsm);                 // kDWarps doubles
-    int* ticket_s = reinterpret_cast<int*>(dsm + 64);
     uint8_t* ring = dsm + 128;                                        // kStages x 16 KB; reused for the reduction
     float* red = reinterpret_cast<float*>(ring);                      // [8][MB][256] floats <= 32 KB
     __half* xn = reinterpret_cast<__half*>(ring + kStages * kStageBytes);   // [MB][kc]
@@ -359,31 +358,46 @@ __global__ void __launch_bounds__(kDThreads) dense_norm_gemv_split_kernel(const 
 #pragma unroll
         for (int e = 0; e < 8; ++e) red[(r0 * MB + m) * kSplitCols + hl * 8 + e] = acc[m][e];
     __syncthreads();
-    for (int i = tid; i < MB * kSplitCols; i += kDThreads) {
-        const int m = i / kSplitCols, c = i - m * kSplitCols;
-        float v = 0.f;
-#pragma unroll
-        for (int g = 0; g < kRowGroups; ++g) v += red[(g * MB + m) * kSplitCols + c];
-        const int n = strip * kSplitCols + c;
-        if (n < p.N) sp.partial[(static_cast<size_t>(chunk) * p.M + m) * p.N + n] = v;
-    }
-    // The last CTA of the strip adds the K ranges in order and writes the result.
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) *ticket_s = atomicAdd(&sp.counters[strip], 1);
-    __syncthreads();
-    if (*ticket_s != sp.chunks - 1) return;
-    __threadfence();
+    const int others = sp.chunks - 1;
     for (int i = tid; i < MB * kSplitCols; i += kDThreads) {
         const int m = i / kSplitCols, c = i - m * kSplitCols;
         const int n = strip * kSplitCols + c;
         if (n >= p.N) continue;
+        float mine = 0.f;
+#pragma unroll
+        for (int g = 0; g < kRowGroups; ++g) mine += red[(g * MB + m) * kSplitCols + c];
+        const size_t step = static_cast<size_t>(p.M) * p.N, at = static_cast<size_t>(m) * p.N + n;
+        if (chunk < others) {
+            handover::store(sp.partial + chunk * step + at, handover::word_of(mine));
+            continue;
+        }
         float v = 0.f;
-        for (int ch = 0; ch < sp.chunks; ++ch)
-            v += __ldcg(sp.partial + (static_cast<size_t>(ch) * p.M + m) * p.N + n);
-        p.Y[static_cast<size_t>(m) * p.N + n] = __float2half_rn(v);
+        constexpr int kAtOnce = 8;
+        for (int c0 = 0; c0 < others; c0 += kAtOnce) {
+            uint32_t* src = sp.partial + c0 * step + at;
+            const int some = min(kAtOnce, others - c0);
+            uint32_t w[kAtOnce];
+            const long long t0 = clock64();
+            for (bool all = false; !all;) {
+                all = true;
+#pragma unroll
+                for (int k = 0; k < kAtOnce; ++k) w[k] = k < some ? handover::load(src + k * step) : 0u;
+#pragma unroll
+                for (int k = 0; k < kAtOnce; ++k) all = all && handover::there(w[k]);
+                if (!all && clock64() - t0 > 2000000000LL) {
+                    if (sp.err) atomicOr(sp.err, ERR_WAIT_TIMEOUT);
+                    break;
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < kAtOnce; ++k) {
+                if (k >= some) continue;
+                handover::store(src + k * step, handover::kNothing);
+                v += __uint_as_float(w[k]);
+            }
+        }
+        p.Y[at] = __float2half_rn(v + mine);
     }
-    if (tid == 0) sp.counters[strip] = 0;      // ready for the next launch on this stream
 }
 
 // Fallback for N % 8 != 0 or unaligned W: one thread per column, scalar loads (still
@@ -493,11 +507,10 @@ DenseSplit dense_split_shape(int mb, int N, int K, int sm_count, int smem_optin)
 
 }  // namespace
 
-void plan_dense_norm_gemv(DenseNormGemvArgs* a, int sm_count, int smem_optin, size_t* floats, size_t* ints) {
+void plan_dense_norm_gemv(DenseNormGemvArgs* a, int sm_count, int smem_optin, size_t* floats) {
     const int mb = a->M < kDMaxMB ? a->M : kDMaxMB;
     a->split = dense_split_shape(mb, a->N, a->K, sm_count > 0 ? sm_count : 148, smem_optin);
-    *floats = static_cast<size_t>(a->split.chunks) * mb * a->N;
-    *ints = static_cast<size_t>(a->split.strips);
+    *floats = static_cast<size_t>(a->split.chunks - 1) * mb * a->N;
 }
 
 cudaError_t launch_dense_norm_gemv(const DenseNormGemvArgs& a, const LaunchEnv& env,
@@ -506,9 +519,8 @@ cudaError_t launch_dense_norm_gemv(const DenseNormGemvArgs& a, const LaunchEnv& 
     const int optin = env.smem_optin > 0 ? env.smem_optin : 48 * 1024;
     cudaError_t err = cudaSuccess;
     int count = 0;
-    const size_t need_f = static_cast<size_t>(a.split.chunks) * (a.M < kDMaxMB ? a.M : kDMaxMB) * a.N;
-    const bool split = vec && a.split.chunks > 0 && a.scratch && a.counters && a.scratch_floats >= need_f &&
-                       a.counters_n >= static_cast<size_t>(a.split.strips);
+    const size_t need_f = static_cast<size_t>(a.split.chunks - 1) * (a.M < kDMaxMB ? a.M : kDMaxMB) * a.N;
+    const bool split = vec && a.split.chunks > 0 && a.scratch && a.scratch_floats >= need_f;
     // Five rows or more: the kernels below would read W once per four rows.  Instead the rows are
     // normalised once into the stream's scratch (fp16, as the reference rounds them before its GEMM,
     // lib/ops/training_cpu.cpp:799-935) and multiplied by W on the tensor cores: W is read once.
@@ -542,7 +554,7 @@ cudaError_t launch_dense_norm_gemv(const DenseNormGemvArgs& a, const LaunchEnv& 
             SplitParams sp;
             sp.d = p;
             sp.partial = a.scratch;
-            sp.counters = a.counters;
+            sp.err = env.err_word;
             sp.chunks = a.split.chunks;
             sp.kc = a.split.kc;
             const int strips = a.split.strips;

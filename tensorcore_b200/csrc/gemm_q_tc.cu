@@ -46,6 +46,7 @@
 // 8 rows 20.4 -> 15.2, Q8_0 28672 x 4096, 16 rows 33.2 -> 27.8 (4.5 TB/s).
 // Per 128-row unit of 256 weights in steady state: Q4_0 0.51 us at 8 rows, 1.9 us at 256 rows (1.08 us
 // of tensor work at the clock's peak); Q8_0 0.82 us at 16 rows, which is the weight stream at 6.3 TB/s.
+#include "handover.cuh"
 #include "kernels.h"
 #include "sm100_prims.cuh"
 #include "tensor_map.h"
@@ -94,7 +95,7 @@ struct QtcParams {
     int split;         // > 1: a cluster of that many CTAs per tile
     int chunk;         // split == 1: CTAs take runs of so many units: 1, or all of a tile
     int run, longer;   // ... run of them each, the first `longer` CTAs one more
-    uint32_t* part;    // shares: [grid][nb][128], what a CTA has of a tile that began in the CTA before it (kNothing else)
+    uint32_t* part;    // shares: [grid][nb][128], what a CTA has of a tile that began in the CTA before it (nothing else: handover.cuh)
     int wait_first;    // the kernel before may write the weights
     int raw_stages;    // per warpgroup (a ring that several groups shared would let one wait on a
                        // barrier phase while an earlier one, which it never observes, is still open)
@@ -189,9 +190,7 @@ struct Pos {                                // position in a ring
 __device__ __forceinline__ int first_unit(const QtcParams& p, int c) {
     return (c * p.run + (c < p.longer ? c : p.longer)) * p.chunk;
 }
-// What CB of the partial sums that another CTA of this launch leaves in scratch are: a word is kNothing until it
-// has been written, so that a reader knows a sum by its being there - no flag, and no fence on either side.
-constexpr uint32_t kNothing = 0xFFFFFFFFu;         // a NaN no sum has: such a sum is stored as another NaN
+// CB of the partial sums that another CTA of this launch leaves in scratch (handover.cuh), by a whole warp.
 template <int CB>
 __device__ __forceinline__ bool take_sums(uint32_t* src, uint32_t (&v)[CB], volatile int* abort_flag) {
     const long long t0 = clock64();
@@ -199,14 +198,14 @@ __device__ __forceinline__ bool take_sums(uint32_t* src, uint32_t (&v)[CB], vola
         bool all = true;
 #pragma unroll
         for (int e = 0; e < CB; ++e)
-            asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v[e]) : "l"(src + e * kRows) : "memory");
+            v[e] = handover::load(src + e * kRows);
 #pragma unroll
-        for (int e = 0; e < CB; ++e) all = all && v[e] != kNothing;
+        for (int e = 0; e < CB; ++e) all = all && handover::there(v[e]);
         if (__all_sync(0xffffffffu, all)) break;
         if (__any_sync(0xffffffffu, *abort_flag || clock64() - t0 > 2000000000LL)) return false;
     }
 #pragma unroll
-    for (int e = 0; e < CB; ++e) asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(src + e * kRows), "r"(kNothing) : "memory");
+    for (int e = 0; e < CB; ++e) handover::store(src + e * kRows, handover::kNothing);
     return true;
 }
 template <int CB>
@@ -350,11 +349,7 @@ gemm_q_tc_kernel(const QtcParams p, const __grid_constant__ QtcMaps maps) {
                 for (int e = 0; e < CB; ++e) red[(c0 + e) * kRows + r] = f[e];
             } else if (RUNS && !begins) {
 #pragma unroll
-                for (int e = 0; e < CB; ++e) {
-                    const uint32_t w = __float_as_uint(f[e]);
-                    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;"
-                                 ::"l"(mine + (c0 + e) * kRows), "r"(w == kNothing ? 0x7FFFFFFFu : w) : "memory");
-                }
+                for (int e = 0; e < CB; ++e) handover::store(mine + (c0 + e) * kRows, handover::word_of(f[e]));
             } else if (row < N) {
                 const size_t o = static_cast<size_t>(m0 + c0) * N + row;
                 if (p.y_f32) {

@@ -118,17 +118,14 @@ struct DenseNormGemvArgs {
     // the rows are normalised once and multiplied on the tensor cores, W read once
     void* norm_scratch = nullptr;
     size_t norm_scratch_bytes = 0;
-    // scratch of the stream the call runs on (plan_dense_norm_gemv says how much): partial sums
-    // and one ticket counter per column strip, all zero between launches; without it a slower
-    // kernel that needs none is used
+    // scratch of the stream the call runs on (plan_dense_norm_gemv says how much): partial sums, all bits set
+    // between launches; without it a slower kernel that needs none is used
     DenseSplit split;             // set by plan_dense_norm_gemv
-    float* scratch = nullptr;
+    uint32_t* scratch = nullptr;
     size_t scratch_floats = 0;
-    int* counters = nullptr;
-    size_t counters_n = 0;
 };
 // Chooses the tiles (a->split) and says how much scratch they need.
-void plan_dense_norm_gemv(DenseNormGemvArgs* a, int sm_count, int smem_optin, size_t* floats, size_t* ints);
+void plan_dense_norm_gemv(DenseNormGemvArgs* a, int sm_count, int smem_optin, size_t* floats);
 
 // ---------------------------------------------------------------------------------------
 // Persistent decode launch (decode_q4.cu): a list of Q4_0, M = 1 GEMVs as one cooperative kernel.

@@ -197,15 +197,14 @@ bool managed(const tc_buffer* b) { return b->kind == BUF_MANAGED || b->kind == B
 // The mutex is held from handing rooms out until the launches that use them are in the stream, so that calls
 // from several threads do not get between another call's launches, nor free its rooms.
 enum RoomKind : int {
-    ROOM_PARTIAL,    // dense fused GEMV: partial sums of the K ranges
-    ROOM_COUNTERS,   // ... a ticket counter per column strip, zero between launches
+    ROOM_PARTIAL,    // dense fused GEMV: partial sums of the K ranges, all bits set between launches
     ROOM_NORM,       // normalised rows
     ROOM_WEIGHTS,    // weights as fp16
     ROOM_SHARES,     // batched quantized products: sums of tiles that several CTAs work on, all bits set between launches
     ROOM_STATES,     // attention: softmax states of a row's key chunks, all bits set between launches
     kRoomKinds
 };
-constexpr int kRoomFill[kRoomKinds] = {-1, 0, -1, -1, 0xFF, 0xFF};      // the byte a new room is filled with
+constexpr int kRoomFill[kRoomKinds] = {0xFF, -1, -1, 0xFF, 0xFF};      // the byte a new room is filled with
 struct StreamRooms { Room room[kRoomKinds]; };
 std::mutex g_rooms_mutex;
 std::unordered_map<cudaStream_t, StreamRooms> g_rooms;
@@ -307,12 +306,11 @@ void free_rooms() {
 
 // The functions that hand rooms out; the caller holds g_rooms_mutex and goes on holding it until it has launched.
 void dense_scratch_for(tc_context* ctx, cudaStream_t st, tcb::DenseNormGemvArgs* a) {
-    size_t nf = 0, nc = 0;
-    tcb::plan_dense_norm_gemv(a, ctx->sm_count, ctx->smem_optin, &nf, &nc);
-    const Room& partial = stream_room(st, ROOM_PARTIAL, nf * sizeof(float));
-    const Room& counters = stream_room(st, ROOM_COUNTERS, nc * sizeof(int));
-    a->scratch = static_cast<float*>(partial.p); a->scratch_floats = partial.bytes / sizeof(float);
-    a->counters = static_cast<int*>(counters.p); a->counters_n = counters.bytes / sizeof(int);
+    size_t nf = 0;
+    tcb::plan_dense_norm_gemv(a, ctx->sm_count, ctx->smem_optin, &nf);
+    const Room& partial = stream_room(st, ROOM_PARTIAL, nf > 1024 ? nf * sizeof(float) : 4096);
+    a->scratch = static_cast<uint32_t*>(partial.p);
+    a->scratch_floats = partial.bytes / sizeof(float);
 }
 // Room for the normalised rows of the batched fused RMSNorm GEMV (the tensor-core kernel reads them as
 // plain fp16 activations).
@@ -2106,7 +2104,7 @@ extern "C" uint32_t tcx_take_device_error(tc_context* ctx) {
         RoomsLock lock(g_rooms_mutex);
         bind_device(ctx);
         cudaDeviceSynchronize();
-        for (RoomKind k : {ROOM_SHARES, ROOM_STATES}) {
+        for (RoomKind k : {ROOM_PARTIAL, ROOM_SHARES, ROOM_STATES}) {
             for (auto& kv : g_rooms) {
                 const Room& r = kv.second.room[k];
                 if (r.p) cudaMemset(r.p, kRoomFill[k], r.bytes);
