@@ -483,9 +483,10 @@ cudaError_t launch_dense_split(const SplitParams& sp, int strips, int smem_optin
 // Tiles of the split kernel for launches of up to `mb` rows.
 DenseSplit dense_split_shape(int mb, int N, int K, int sm_count, int smem_optin) {
     // The number of K ranges whose waves of tiles take least: a tile costs its rows and about 96 rows' time for the
-    // row statistics and the fence before its ticket, and as many CTAs are resident per SM as their shared
-    // memory allows, three at most (registers).  4096 x 11008: ten ranges, one wave of 430 tiles (four tiles per SM
-    // before: 602 tiles, a third of a wave left over).
+    // row statistics and its end, the last of a strip ten rows' time for each range it adds (hidden behind other waves), and as many CTAs are
+    // resident per SM as their shared memory allows, three at most (registers).  4096 x 11008: ten ranges, one wave of
+    // 430 tiles (four tiles per SM before: 602 tiles, a third of a wave left over).  8192 x 1024, one row: 16 / 24 / 32 / 111
+    // ranges 21.3 / 20.3 / 20.1 / 23.2 us a call.
     const int st = (N + kSplitCols - 1) / kSplitCols;
     const int most = (K + 2 * kStageRows - 1) / (2 * kStageRows);
     const int optin = smem_optin > 0 ? smem_optin : 48 * 1024;
@@ -498,7 +499,7 @@ DenseSplit dense_split_shape(int mb, int N, int K, int sm_count, int smem_optin)
         // an SM has 1 KB more than one block may take, and every block costs 1 KB of it
         const unsigned per_wave = (3 * (smem + 1024) <= optin + 1024 ? 3u : 2 * (smem + 1024) <= optin + 1024 ? 2u : 1u) * sm_count;
         const double waves = static_cast<double>((static_cast<unsigned long long>(st) * c + per_wave - 1) / per_wave);
-        const double cost = waves * (static_cast<double>(K) / c + 96.0);
+        const double cost = waves * (static_cast<double>(K) / c + 96.0) + 10.0 * c / waves;
         if (best == 0.0 || cost < best) { best = cost; ch = c; }
     }
     const int kc = rows_of(ch);
