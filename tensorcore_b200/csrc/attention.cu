@@ -282,7 +282,10 @@ __device__ __forceinline__ void merge_warps(const AttnParams& p, float* o_s, flo
     const int tid = threadIdx.x;
     float* w_s = ml_s + kAttnWarps * ROWS * 2;                       // [ROWS][warp]
     __syncthreads();
-    auto row_of = [&](int r) { return (static_cast<size_t>(b) * p.Hq + hkv * G + r % G) * p.Sq + r / G; };
+    auto row_of = [&](int r) {
+        const int i = p.by_per_kv(r);
+        return (static_cast<size_t>(b) * p.Hq + hkv * G + (r - i * G)) * p.Sq + i;
+    };
     // With room for them the chunks' states go to the CTA of the last chunk, which started last, and it merges them: a
     // thread has the same four elements of every chunk, with the row's maximum and sum beside each, so one trip
     // brings all it needs.
@@ -613,11 +616,14 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma8_kernel(cons
     extern __shared__ __align__(128) uint8_t smem[];
     const uint32_t ring = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, tq = lane & 3;
-    const int G = p.Hq / p.Hkv, R = p.Sq * G;             // at most 8
-    const int bk = blockIdx.x, b = bk / p.Hkv, hkv = bk % p.Hkv, chunk = blockIdx.y;
+    const int G = p.per_kv, R = p.Sq * G;                 // at most 8
+    const int bk = blockIdx.x, b = p.by_Hkv(bk), hkv = bk - b * p.Hkv, chunk = blockIdx.y;
     const __half* Kh = p.K + static_cast<size_t>(bk) * p.Sk * D;
     const __half* Vh = p.V + static_cast<size_t>(bk) * p.Sk * D;
-    auto row_at = [&](int r) { return (static_cast<size_t>(b) * p.Hq + hkv * G + r % G) * p.Sq + r / G; };
+    auto row_at = [&](int r) {
+        const int i = p.by_per_kv(r);
+        return (static_cast<size_t>(b) * p.Hq + hkv * G + (r - i * G)) * p.Sq + i;
+    };
 
     const int k0 = chunk * p.keys_per_chunk;
     int k1 = min(p.Sk, k0 + p.keys_per_chunk);
@@ -669,8 +675,8 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma8_kernel(cons
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
         const int r = min(2 * tq + e, R - 1);
-        qi[e] = r / G;
-        slope[e] = p.slopes ? p.slopes[hkv * G + r % G] : 0.f;
+        qi[e] = p.by_per_kv(r);
+        slope[e] = p.slopes ? p.slopes[hkv * G + (r - qi[e] * G)] : 0.f;
     }
 
     float o[D / 16][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};

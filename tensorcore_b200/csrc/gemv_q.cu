@@ -57,8 +57,7 @@ __global__ void __launch_bounds__(kMaxStreamThreads, 1) gemv_q_stream_kernel(con
     constexpr int kChunkBytes = 32 * F::kGroupBytes;
 
     // Row range of this CTA and the corresponding run of groups.
-    const int r0 = static_cast<int>(static_cast<long long>(p.N) * blockIdx.x / gridDim.x);
-    const int r1 = static_cast<int>(static_cast<long long>(p.N) * (blockIdx.x + 1) / gridDim.x);
+    const int r0 = p.rows_of.first(blockIdx.x), r1 = p.rows_of.first(blockIdx.x + 1);
     const int rows = r1 - r0;
     const long long g_base = static_cast<long long>(r0) * gpr;
     const int g_count = rows * gpr;
@@ -141,7 +140,7 @@ __global__ void __launch_bounds__(kMaxStreamThreads, 1) gemv_q_stream_kernel(con
         for (int m = 0; m < MB; ++m) out[m] = 0.f;
         int row = -1 - lane;  // distinct negatives for idle lanes
         if (valid) {
-            row = gl / gpr;
+            row = p.by_gpr(gl);
             const int kg = gl - row * gpr;
             group_dot_i16<FMT, MB>(w, xs, reinterpret_cast<const float2*>(sx), kg, gpr, p.K, p.nb, out);
         }
@@ -206,8 +205,7 @@ gemv_q_box_kernel(const StreamParams p, const __grid_constant__ CUtensorMap wmap
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nwarps = blockDim.x >> 5, nthreads = blockDim.x;
     const int ns = p.ns, gpr = p.gpr;
-    const int r0 = static_cast<int>(static_cast<long long>(p.N) * blockIdx.x / gridDim.x);
-    const int r1 = static_cast<int>(static_cast<long long>(p.N) * (blockIdx.x + 1) / gridDim.x);
+    const int r0 = p.rows_of.first(blockIdx.x), r1 = p.rows_of.first(blockIdx.x + 1);
     const int rows = r1 - r0;
     const int rows_pad = (rows + 31) & ~31;
     const int n_units = (rows_pad >> 5) * gpr;
@@ -224,7 +222,7 @@ gemv_q_box_kernel(const StreamParams p, const __grid_constant__ CUtensorMap wmap
 
     auto issue = [&](int i) {  // lane 0 only: start the copy of this warp's i-th box
         const int u = warp + nwarps * i;
-        const int rb = u / gpr, kg = u - rb * gpr;
+        const int rb = p.by_gpr(u), kg = u - rb * gpr;
         const int s = i % ns;
         uint64_t* bar = &bars[warp * ns + s];
         mbar_expect_tx(bar, kBoxBytes);
@@ -254,7 +252,7 @@ gemv_q_box_kernel(const StreamParams p, const __grid_constant__ CUtensorMap wmap
         if (!mbar_wait_bounded(bar, static_cast<uint32_t>((i / ns) & 1))) { failed = true; break; }
         waited = i + 1;
         const int u = warp + nwarps * i;
-        const int rb = u / gpr, kg = u - rb * gpr;
+        const int rb = p.by_gpr(u), kg = u - rb * gpr;
         const int rl = rb * 32 + lane;
         uint32_t w[F::kGroupV4 * 4];
         {
@@ -290,7 +288,7 @@ gemv_q_box_kernel(const StreamParams p, const __grid_constant__ CUtensorMap wmap
     __syncthreads();
     if (failed) return;
     for (int i = tid; i < rows * MB; i += nthreads) {
-        const int m = i / rows, r = i - m * rows;
+        const int m = MB == 1 ? 0 : i / rows, r = i - m * rows;
         const float v = rowacc[m * rows_pad + r];
         const size_t o = static_cast<size_t>(m) * p.N + r0 + r;
         if (p.y_f32) static_cast<float*>(p.Y)[o] = v;
@@ -472,6 +470,8 @@ StreamPlan plan_stream(const GemvQArgs& a, int mb, const LaunchEnv& env) {
     p.y_f32 = a.y_f32 ? 1 : 0; p.eps = a.eps; p.wait_first = env.wait_first() ? 1 : 0;
     p.off_rowacc = off_rowacc; p.off_sx = off_sx; p.off_x = off_x; p.off_ring = off_ring;
     p.max_rows = max_rows;
+    p.rows_of.set(a.N, grid);
+    p.by_gpr.set(gpr);
     return pl;
 }
 
@@ -537,6 +537,8 @@ StreamPlan plan_box(const GemvQArgs& a, int mb, const LaunchEnv& env) {
     p.x_src_f16 = a.x_f32 ? 0 : 1;
     p.off_rowacc = off_rowacc; p.off_sx = off_sx; p.off_x = off_x; p.off_ring = off_ring;
     p.max_rows = max_rows;
+    p.rows_of.set(a.N, grid);
+    p.by_gpr.set(gpr);
     return pl;
 }
 

@@ -36,6 +36,7 @@ struct RowsParams {
     int nbp;          // blocks of a staged row, padded to an odd count (bank conflicts while staging)
     int cb, chunks;   // blocks per chunk (at most 32), chunks per row
     int max_rows;     // rows of a CTA, rounded up to whole groups
+    EvenSplit rows_of;
     int x_f32, y_f32;
     int wait_first;   // the kernel before may write the weights
     int x_vec;        // X and gamma allow 8-byte (fp16) / 16-byte (fp32) loads
@@ -90,15 +91,16 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_q_rows_kernel(const Rows
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (p.wait_first) pdl_wait();
     pdl_launch_dependents();
-    const int r0 = static_cast<int>(static_cast<long long>(p.N) * blockIdx.x / gridDim.x);
-    const int r1 = static_cast<int>(static_cast<long long>(p.N) * (blockIdx.x + 1) / gridDim.x);
+    const int r0 = p.rows_of.first(blockIdx.x), r1 = p.rows_of.first(blockIdx.x + 1);
     const int groups = (r1 - r0 + kGroupRows - 1) / kGroupRows, units = groups * p.chunks;
     const size_t row_bytes = static_cast<size_t>(p.nb) * kBlock;
     // Blocks of this warp's next unit, on their way while the activations are staged or a unit is computed.
     RowBlock<FMT> blk[kGroupRows];
     int off[kGroupRows];
     auto fetch = [&](int u) {
-        const int g = u % groups, c = u / groups, b = c * p.cb + lane;
+        int c = 0, g = u;                                       // few chunks: subtractions beat a division
+        for (; g >= groups && c < p.chunks; g -= groups) ++c;
+        const int b = c * p.cb + lane;
         const bool active = u < units && lane < p.cb && b < p.nb;
 #pragma unroll
         for (int r = 0; r < kGroupRows; ++r) {
@@ -153,7 +155,8 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_q_rows_kernel(const Rows
     __syncthreads();
 
     for (int u = warp; u < units; u += kRowsWarps) {
-        const int g = u % groups, c = u / groups;
+        int c = 0, g = u;
+        for (; g >= groups; g -= groups) ++c;
         const int b = c * p.cb + lane;
         const bool active = lane < p.cb && b < p.nb;
         const int bx = active ? b : 0;
@@ -197,7 +200,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_q_rows_kernel(const Rows
     }
     __syncthreads();
     for (int e = tid; e < (r1 - r0) * MB; e += kRowsThreads) {
-        const int m = e / (r1 - r0), r = e - m * (r1 - r0);
+        const int m = MB == 1 ? 0 : e / (r1 - r0), r = e - m * (r1 - r0);
         float v = 0.f;
         for (int c = 0; c < p.chunks; ++c) v += part[(c * p.max_rows + r) * MB + m];
         const size_t o = static_cast<size_t>(m) * p.N + r0 + r;
@@ -240,6 +243,7 @@ cudaError_t launch_gemv_q_rows(const GemvQArgs& a, const LaunchEnv& env, cudaStr
     const int groups = (a.N + kGroupRows - 1) / kGroupRows;
     const int grid = groups < sms ? groups : sms;
     p.max_rows = ((a.N + grid - 1) / grid + kGroupRows) / kGroupRows * kGroupRows;
+    p.rows_of.set(a.N, grid);
     const long long off = static_cast<long long>(a.M) * 8 * p.nbp * 16;
     const long long bytes = off + static_cast<long long>(p.chunks) * p.max_rows * a.M * 4;
     if (bytes > env.smem_optin - 1024) return cudaErrorNotSupported;

@@ -8,6 +8,32 @@
 
 namespace tcb {
 
+// Division of 0 <= n < 2^31 by a number known to the host: mul = 2^(31 + s) / d rounded up, s = ceil(log2 d), is exact
+// there; two instructions where the device's division is a chain of 150 clocks and more.
+struct FastDiv {
+    uint32_t mul = 0;
+    int shift = -1;       // s - 1
+    void set(int d) {
+        shift = -1;
+        while ((1ll << (shift + 1)) < d) ++shift;
+        mul = static_cast<uint32_t>(((1ull << (32 + shift)) / static_cast<uint64_t>(d)) + 1);
+    }
+#ifdef __CUDACC__
+    __device__ __forceinline__ int operator()(int n) const {
+        return shift < 0 ? n : static_cast<int>(__umulhi(static_cast<uint32_t>(n), mul) >> shift);
+    }
+#endif
+};
+// Items of CTA i when n items go to `parts` CTAs in order, the first ones one more: two instructions, where n * i / parts
+// in 64 bits was 300 clocks and more before a kernel's first copy.
+struct EvenSplit {
+    int run = 0, longer = 0;
+    void set(int n, int parts) { run = n / parts; longer = n % parts; }
+#ifdef __CUDACC__
+    __device__ __forceinline__ int first(int i) const { return i * run + (i < longer ? i : longer); }
+#endif
+};
+
 enum QuantFmt : int { FMT_Q4_0 = 0, FMT_Q8_0 = 1 };
 
 // Kernel families for the quantized GEMV (see gemv_q.cu).
@@ -302,22 +328,6 @@ cudaError_t launch_gemm_f16_tc(const void* A, const void* B, void* C, int M, int
 
 // --- attention forward (attention.cu); fp16 data, fp32 softmax ----------------------------
 cudaError_t init_attention_kernels();
-// Division of 0 <= n < 2^31 by a number known to the host: mul = 2^(31 + s) / d rounded up, s = ceil(log2 d), is exact
-// there; two instructions where the device's division is a chain of 150 clocks and more.
-struct FastDiv {
-    uint32_t mul = 0;
-    int shift = -1;       // s - 1
-    void set(int d) {
-        shift = -1;
-        while ((1ll << (shift + 1)) < d) ++shift;
-        mul = static_cast<uint32_t>(((1ull << (32 + shift)) / static_cast<uint64_t>(d)) + 1);
-    }
-#ifdef __CUDACC__
-    __device__ __forceinline__ int operator()(int n) const {
-        return shift < 0 ? n : static_cast<int>(__umulhi(static_cast<uint32_t>(n), mul) >> shift);
-    }
-#endif
-};
 struct AttnParams {
     const __half* Q;
     const __half* K;
