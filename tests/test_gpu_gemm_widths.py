@@ -52,3 +52,27 @@ def test_padded_rows_against_64_bit(tc, ctx, M, N, K):
         b.close()
     assert err <= 1.05 * 2.0 ** -11 / np.sqrt(3.0)
     assert tc.take_device_error(ctx) == 0
+
+
+@pytest.mark.parametrize("M,N,ldc", [(1021, 160, 160), (130, 96, 104), (131, 40, 48), (257, 248, 248), (66, 32, 40), (5, 304, 304)])
+@pytest.mark.parametrize("dtype", ["f16", "bf16"])
+def test_rows_and_columns_past_the_result_stay(tc, ctx, M, N, ldc, dtype):
+    """Rows and columns that are no multiples of the groups of four rows and 32 columns a store covers, rows of C further
+    apart than its columns: results within one rounding, everything around them untouched."""
+    import torch
+    dt, K = torch.float16 if dtype == "f16" else torch.bfloat16, 192
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M + N)
+    A, B = torch.randn(M, K, generator=g, device="cuda").to(dt), torch.randn(N, K, generator=g, device="cuda").to(dt)
+    C = torch.full((M + 8, ldc), 7.0, device="cuda", dtype=dt)
+    bufs = [ctx.buffer_from_ptr(t.data_ptr(), t.numel() * 2) for t in (A, B, C)]
+    torch.cuda.synchronize()
+    tc.gemm(ctx, *bufs, M, N, K, dtype=dtype, transpose_b=True, ldc=ldc)
+    assert tc.cuda_last_kernel_name() == "gemm_f16_tcgen05_sm100"
+    for b in bufs:
+        b.close()
+    want = A.double() @ B.double().t()
+    err = ((C[:M, :N].double() - want).square().mean() / want.square().mean()).sqrt().item()
+    assert err <= 1.05 * (2.0 ** -11 if dtype == "f16" else 2.0 ** -8) / np.sqrt(3.0)
+    assert (C[M:] == 7.0).all() and (C[:, N:] == 7.0).all()
+    assert tc.take_device_error(ctx) == 0
