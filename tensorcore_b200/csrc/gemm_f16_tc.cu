@@ -26,8 +26,8 @@
 //     memory) into BN columns of tensor memory per 128 rows; tcgen05.commit hands the stage back to the producer.
 //   * Four warps per 128 rows read the accumulators (one TMEM lane = one row of the tile per thread), apply
 //     alpha and beta and store 16-bit results, 64 bytes of eight rows a store: threads exchange pieces by shuffles.
-//     (16 bytes of 32 rows took the load/store unit a clock a row: whole calls, 512 x 11008 x 4096 54.1 -> 49.9 us,
-//     512 x 12288 x 512 23.8 -> 21.0, 4096^3 109.4 -> 105.6, 512 x 11008 x 4096 with B as given 53.0 -> 47.8.)
+//     (16 bytes of 32 rows took the load/store unit a clock a row: whole calls, 512 x 11008 x 4096 54.1 -> 49.8 us,
+//     512 x 12288 x 512 23.8 -> 20.9, 4096^3 109.4 -> 105.8, 512 x 11008 x 4096 with B as given 53.0 -> 47.4.)
 // Rows and columns past M, N and K are zero-filled by TMA and masked at the store.  Every wait is
 // bounded: it sets the error word and lets the kernel end.
 #include "kernels.h"
@@ -418,7 +418,8 @@ cudaError_t launch_gemm_f16_tc(const void* A, const void* B, void* C, int M, int
     // both operands in shared memory), or the shared-memory traffic - the stage's bytes written once, A read
     // once and B once per 128 rows - at 120 bytes per clock.  256 rows need less traffic per flop; their two
     // accumulators leave room for a second set only up to 128 columns, so a wider tile's read-out is not hidden:
-    // 10000 clocks a round, against 1500 per 128 rows where it is.  Fitted to whole calls of 144 shapes (M 64 to
+    // 10000 clocks a round, against 1500 per 128 rows where it is (3000 to 7000 choose worse tiles: 256 x 14336 x 4096
+    // 47 us instead of 44.5, 2048^3 30 instead of 28.7).  Fitted to whole calls of 144 shapes (M 64 to
     // 8192, K 1024 to 11008) in eight tiles each: a step of 128 rows x 64 / 128 / 192 / 256 columns takes 180 / 270 /
     // 300 / 373 ns, of 256 rows x 128 / 192 / 256 365 / 460 / 635 ns; the tile chosen is 0.3 % slower than the
     // best of the eight on average, 9 % at most.  B as given is laid out in pieces of 64 columns.
