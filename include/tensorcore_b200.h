@@ -531,6 +531,8 @@ tc_status_t tcx_stream_decode_tp(tc_stream* s, const tcx_decode_tp_op* ops, int 
 tc_status_t tcx_set_gemv_variant(const char* name);
 /* Device-side error word: non-zero after a kernel gave up on a bounded wait.  Reading clears. */
 uint32_t tcx_take_device_error(tc_context* ctx);
+/* Sets bits of that word as a kernel that gives up would, so that a caller can try out its error handling. */
+tc_status_t tcx_set_device_error(tc_context* ctx, uint32_t bits);
 /* Number of kernel launches this library has issued in the calling process. */
 uint64_t tcx_launch_count(void);
 

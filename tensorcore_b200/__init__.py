@@ -218,6 +218,7 @@ def _declare(L) -> None:
     sig("tcx_raw_decode_q4_static", i, vp, POINTER(TCXDecodeOp), i, vp)
     sig("tcx_set_gemv_variant", i, c_char_p)
     sig("tcx_take_device_error", c_uint32, vp)
+    sig("tcx_set_device_error", i, vp, c_uint32)
     sig("tcx_launch_count", c_uint64)
 
 
@@ -651,6 +652,10 @@ def set_gemv_variant(name: str) -> None:
 
 def take_device_error(ctx) -> int:
     return int(lib().tcx_take_device_error(_h(ctx)))
+
+
+def set_device_error(ctx, bits: int) -> None:
+    _check(lib().tcx_set_device_error(_h(ctx), bits))
 
 
 def launch_count() -> int:

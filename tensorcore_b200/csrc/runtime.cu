@@ -408,6 +408,13 @@ tc_status_t check_device_error(tc_context* ctx) {
     return TC_OK;
 }
 
+// The status of a synchronous operation whose last CUDA call gave e: a kernel that gave up on a wait has left a wrong
+// result, whichever operation it belongs to.
+tc_status_t finished(tc_context* ctx, cudaError_t e) {
+    const tc_status_t st = from_cuda(e, TC_ERR_DISPATCH);
+    return st == TC_OK ? check_device_error(ctx) : st;
+}
+
 cudaError_t bind_device(tc_context* ctx) { return cudaSetDevice(ctx->device); }
 
 tc_status_t setup_device(tc_context* ctx, int device) {
@@ -1357,7 +1364,7 @@ extern "C" tc_status_t tc_quantize_weights(tc_context* ctx, const tc_buffer* W_f
     if (e == cudaSuccess) e = cudaStreamSynchronize(s0);
     g_launches.fetch_add(static_cast<uint64_t>(launches));
     t_last_kernel = name;
-    return record("tc_quantize_weights", from_cuda(e, TC_ERR_DISPATCH));
+    return record("tc_quantize_weights", finished(ctx, e));
 }
 
 namespace {
@@ -1450,9 +1457,7 @@ tc_status_t gemv_common(const GemvCall& c, tc_stream* stream, const char* opname
     if (e == cudaSuccess) e = cudaStreamSynchronize(s0);
     g_launches.fetch_add(static_cast<uint64_t>(launches));
     t_last_kernel = name;
-    tc_status_t out = from_cuda(e, TC_ERR_DISPATCH);
-    if (out == TC_OK) out = check_device_error(ctx);
-    return record(opname, out);
+    return record(opname, finished(ctx, e));
 }
 
 }  // namespace
@@ -1551,7 +1556,7 @@ static tc_status_t dense_common(tc_context* ctx, const tc_buffer* X, const tc_bu
     if (e == cudaSuccess) e = cudaStreamSynchronize(s0);
     g_launches.fetch_add(static_cast<uint64_t>(launches));
     t_last_kernel = name;
-    return record(opname, from_cuda(e, TC_ERR_DISPATCH));
+    return record(opname, finished(ctx, e));
 }
 
 extern "C" tc_status_t tc_fused_rmsnorm_gemv(tc_context* ctx, const tc_buffer* X,
@@ -1593,7 +1598,7 @@ tc_status_t run_step_op(tc_context* ctx, const char* opname, const char* kname, 
     if (e == cudaSuccess) e = cudaStreamSynchronize(s0);
     g_launches.fetch_add(1);
     t_last_kernel = kname;
-    return record(opname, from_cuda(e, TC_ERR_DISPATCH));
+    return record(opname, finished(ctx, e));
 }
 
 tc_buffer* mut(const tc_buffer* b) { return const_cast<tc_buffer*>(b); }
@@ -1879,7 +1884,7 @@ tc_status_t run_collective(tc_dist_ctx* d, const char* opname, StepIo* io, int n
     for (int i = 0; i < n_io && e == cudaSuccess; ++i)
         if (io[i].write) e = finish_output(io[i].b, io[i].bytes, s0);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s0);
-    return record(opname, from_cuda(e, TC_ERR_DISPATCH));
+    return record(opname, finished(ctx, e));
 }
 }  // namespace
 
@@ -2092,6 +2097,12 @@ extern "C" tc_status_t tcx_set_gemv_variant(const char* name) {
     else if (!std::strcmp(name, "generic")) v = tcb::VARIANT_GENERIC;
     if (v < 0) return TC_ERR_INVALID_ARG;
     g_variant.store(v);
+    return TC_OK;
+}
+
+extern "C" tc_status_t tcx_set_device_error(tc_context* ctx, uint32_t bits) {
+    if (!ctx || !ctx->err_host) return TC_ERR_NOT_INITIALIZED;
+    *reinterpret_cast<volatile uint32_t*>(ctx->err_host) |= bits;
     return TC_OK;
 }
 
