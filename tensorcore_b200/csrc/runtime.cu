@@ -14,6 +14,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <limits>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <unordered_map>
@@ -193,7 +194,8 @@ bool managed(const tc_buffer* b) { return b->kind == BUF_MANAGED || b->kind == B
 // Scratch that belongs to a CUDA stream: calls on a stream are ordered, calls on different streams must not
 // share it.  A room is made when a call first needs it and grows when one needs more; the one outgrown is
 // freed once the stream is done with it - except where the caller captured the stream while it was handed
-// out: a graph may then be replayed at any time, and the room stays until the context goes.
+// out: a graph may then be replayed at any time, and the room stays until the context goes (words handed from one CTA to
+// another belong to the graph: graph_room).
 // The mutex is held from handing rooms out until the launches that use them are in the stream, so that calls
 // from several threads do not get between another call's launches, nor free its rooms.
 enum RoomKind : int {
@@ -206,14 +208,23 @@ enum RoomKind : int {
 };
 constexpr int kRoomFill[kRoomKinds] = {0xFF, -1, -1, 0xFF, 0xFF};      // the byte a new room is filled with
 struct StreamRooms { Room room[kRoomKinds]; };
+// A stream's rooms are found by its handle; cudaStreamPerThread is a stream for every thread under one handle, and is
+// found by the stream's number.
+using RoomKey = unsigned long long;
 std::mutex g_rooms_mutex;
-std::unordered_map<cudaStream_t, StreamRooms> g_rooms;
+std::unordered_map<RoomKey, StreamRooms> g_rooms;
 std::vector<void*> g_kept;    // outgrown rooms of captured graphs
 // Rooms of streams that have been destroyed, for those that are created later (a cudaMalloc in the first pass over a
 // new session took 0.25 ms): at most kSpareRooms of a kind, none above kSpareBytes.
 std::vector<Room> g_spare[kRoomKinds];
 constexpr size_t kSpareRooms = 4, kSpareBytes = static_cast<size_t>(32) << 20;
 using RoomsLock = std::unique_lock<std::mutex>;
+
+RoomKey room_key(cudaStream_t st) {
+    unsigned long long id = 0;
+    if (st == cudaStreamPerThread && cudaStreamGetId(st, &id) == cudaSuccess) return id | 1ull << 63;
+    return reinterpret_cast<uintptr_t>(st);
+}
 
 bool being_captured(cudaStream_t st) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -260,7 +271,7 @@ void grow_room(Room& r, size_t need, size_t most, cudaStream_t st, int fill, Wai
 // No work is left on the stream, which goes.
 void retire_rooms(cudaStream_t st) {
     RoomsLock lock(g_rooms_mutex);
-    auto it = g_rooms.find(st);
+    auto it = g_rooms.find(room_key(st));
     if (it == g_rooms.end()) return;
     for (int k = 0; k < kRoomKinds; ++k) {
         Room& r = it->second.room[k];
@@ -271,14 +282,15 @@ void retire_rooms(cudaStream_t st) {
 }
 
 StreamRooms& rooms_of(cudaStream_t st) {
-    if (g_rooms.size() > 32 && g_rooms.find(st) == g_rooms.end() && !being_captured(st)) {
+    const RoomKey key = room_key(st);
+    if (g_rooms.size() > 32 && g_rooms.find(key) == g_rooms.end() && !being_captured(st)) {
         // many short-lived streams: start over rather than keep scratch for streams that are gone
         cudaDeviceSynchronize();
         for (auto& kv : g_rooms)
             for (Room& r : kv.second.room) give_back(r);
         g_rooms.clear();
     }
-    return g_rooms[st];
+    return g_rooms[key];
 }
 // The stream's room of a kind, grown to `need` bytes where that can be done.
 Room& stream_room(cudaStream_t st, RoomKind k, size_t need, size_t most = ~static_cast<size_t>(0)) {
@@ -291,8 +303,99 @@ Room& stream_room(cudaStream_t st, RoomKind k, size_t need, size_t most = ~stati
     grow_room(r, need, most, st, kRoomFill[k], [&] { cudaStreamSynchronize(st); });
     return r;
 }
+
+// A captured call's graph may be replayed on any stream beside later calls, and two launches under way must not share
+// words that say by their bits whether they have been written.  So what a captured call uses of that kind belongs to its
+// graph: the graph holds a reference, and when the last executable graph is gone another may have the room.
+struct GraphRoom {
+    Room room;
+    RoomKind kind;
+    unsigned long long capture;                  // which capture, and which of its streams (whose calls are in order)
+    RoomKey stream;
+    std::shared_ptr<std::atomic<bool>> gone;     // set by the driver, from a thread of its own
+};
+std::vector<GraphRoom> g_graph_rooms;            // those of graphs that are gone: kSpareRooms at most after an eager call
+
+void CUDART_CB graph_gone(void* flag) {
+    auto* gone = static_cast<std::shared_ptr<std::atomic<bool>>*>(flag);
+    (*gone)->store(true);
+    delete gone;
+}
+// Memory that is allocated or freed meanwhile is no part of a capture that is under way, here or in another thread.
+struct OutsideCaptures {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    OutsideCaptures() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~OutsideCaptures() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+// The room of a call that is being captured on `st`; empty where there is no memory.  `aside` is a stream that nobody
+// captures.
+Room graph_room(cudaStream_t st, RoomKind k, size_t need, cudaStream_t aside) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long capture = 0;
+    cudaGraph_t graph = nullptr;
+    if (cudaStreamGetCaptureInfo(st, &status, &capture, &graph) != cudaSuccess || status != cudaStreamCaptureStatusActive) {
+        (void)cudaGetLastError();
+        return Room();
+    }
+    const RoomKey key = room_key(st);
+    GraphRoom* reuse = nullptr;
+    for (GraphRoom& g : g_graph_rooms) {
+        if (g.kind != k || g.room.bytes < need) continue;
+        if (!*g.gone && g.capture == capture && g.stream == key) return g.room;
+        if (*g.gone) reuse = &g;
+    }
+    GraphRoom fresh;
+    fresh.kind = k;
+    if (!reuse) {
+        const OutsideCaptures outside;
+        if (cudaMalloc(&fresh.room.p, need) != cudaSuccess) fresh.room.p = nullptr;
+        if (fresh.room.p && (cudaMemsetAsync(fresh.room.p, kRoomFill[k], need, aside) != cudaSuccess || cudaStreamSynchronize(aside) != cudaSuccess)) {
+            cudaFree(fresh.room.p);
+            fresh.room.p = nullptr;
+        }
+        if (!fresh.room.p) { (void)cudaGetLastError(); return Room(); }
+        fresh.room.bytes = need;
+    }
+    GraphRoom& g = reuse ? *reuse : fresh;
+    auto gone = std::make_shared<std::atomic<bool>>(false);
+    auto* held = new std::shared_ptr<std::atomic<bool>>(gone);
+    cudaUserObject_t object = nullptr;
+    if (cudaUserObjectCreate(&object, held, graph_gone, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+        (void)cudaGetLastError();
+        delete held;
+        if (!reuse) cudaFree(fresh.room.p);
+        return Room();
+    }
+    g.capture = capture;
+    g.stream = key;
+    g.gone = gone;
+    const Room r = g.room;
+    if (!reuse) g_graph_rooms.push_back(fresh);
+    if (cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+        (void)cudaGetLastError();
+        cudaUserObjectRelease(object, 1);        // the room is another graph's from here on
+        return Room();
+    }
+    return r;
+}
+// From a call that is not captured: rooms of graphs that are gone, beyond a few.
+void trim_graph_rooms() {
+    const OutsideCaptures outside;
+    size_t spare = 0;
+    for (size_t i = 0; i < g_graph_rooms.size();) {
+        if (*g_graph_rooms[i].gone && ++spare > kSpareRooms) {
+            cudaFree(g_graph_rooms[i].room.p);
+            g_graph_rooms.erase(g_graph_rooms.begin() + i);
+        } else {
+            ++i;
+        }
+    }
+}
+
 void free_rooms() {
     RoomsLock lock(g_rooms_mutex);
+    for (GraphRoom& g : g_graph_rooms) cudaFree(g.room.p);
+    g_graph_rooms.clear();
     for (auto& kv : g_rooms)
         for (Room& r : kv.second.room) give_back(r);
     g_rooms.clear();
@@ -304,11 +407,19 @@ void free_rooms() {
     g_kept.clear();
 }
 
+// Room for words that one CTA hands to another: the stream's, or that of the graph the call is captured for.
+Room hand_over_room(tc_context* ctx, cudaStream_t st, RoomKind k, size_t need) {
+    if (being_captured(st)) return graph_room(st, k, need, ctx->stream0);
+    if (!g_graph_rooms.empty()) trim_graph_rooms();
+    return stream_room(st, k, need);
+}
+
 // The functions that hand rooms out; the caller holds g_rooms_mutex and goes on holding it until it has launched.
 void dense_scratch_for(tc_context* ctx, cudaStream_t st, tcb::DenseNormGemvArgs* a) {
     size_t nf = 0;
     tcb::plan_dense_norm_gemv(a, ctx->sm_count, ctx->smem_optin, &nf);
-    const Room& partial = stream_room(st, ROOM_PARTIAL, nf > 1024 ? nf * sizeof(float) : 4096);
+    const size_t need = nf > 1024 ? nf * sizeof(float) : 4096;
+    const Room partial = hand_over_room(ctx, st, ROOM_PARTIAL, need);
     a->scratch = static_cast<uint32_t*>(partial.p);
     a->scratch_floats = partial.bytes / sizeof(float);
 }
@@ -332,10 +443,9 @@ size_t share_scratch_need(tc_context* ctx, const tcb::GemvQArgs& a) {
     return tcb::gemm_q_tc_share_bytes(a.M <= tcb::kNormRoomRows ? a.M : tcb::norm_slab_rows(a.M), ctx->sm_count);
 }
 void share_scratch_for(cudaStream_t st, size_t need, tcb::GemvQArgs* a) {
-    // A captured call does without: a graph may be replayed beside later calls on the stream, and two launches under
-    // way must not share this.
-    // (nor does the per-thread stream, one handle for many streams)
-    if (need == 0 || st == cudaStreamPerThread || being_captured(st)) return;
+    // A captured call does without (its graph could have a room of its own, as the dense call's; but whole tiles and
+    // clusters need none).
+    if (need == 0 || being_captured(st)) return;
     const Room& r = stream_room(st, ROOM_SHARES, need);
     a->share_scratch = r.p;
     a->share_scratch_bytes = r.bytes;
@@ -343,7 +453,7 @@ void share_scratch_for(cudaStream_t st, size_t need, tcb::GemvQArgs* a) {
 // Room for the softmax states that attention merges in its kernel; null where a call has to do without (captured, as
 // for the shares; no memory).
 uint32_t* attention_states_for(cudaStream_t st, size_t need) {
-    if (need == 0 || st == cudaStreamPerThread || being_captured(st)) return nullptr;
+    if (need == 0 || being_captured(st)) return nullptr;
     const Room& r = stream_room(st, ROOM_STATES, need);
     return r.bytes >= need ? static_cast<uint32_t*>(r.p) : nullptr;
 }

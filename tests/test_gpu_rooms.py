@@ -156,6 +156,124 @@ def test_captured_attention_without_room_for_its_chunks(tc, ctx):
     assert tc.take_device_error(ctx) == 0
 
 
+def dense_case(seed, M, N=520, K=1536):
+    """Inputs of a dense fused call, and that call on a stream."""
+    rng = np.random.default_rng(seed)
+    x, g, w = on_device(rng.standard_normal((M, K)).astype(np.float16), (1 + 0.1 * rng.standard_normal(K)).astype(np.float16),
+                        (rng.standard_normal((K, N)) * 0.02).astype(np.float16))
+    import torch
+    x64 = x.double()
+    want = (x64 * torch.rsqrt((x64 * x64).mean(dim=1, keepdim=True) + 1e-5) * g.double()) @ w.double()
+
+    def call(tc, ctx, out, handle):
+        tc.raw_fused_norm_gemv_f16(ctx, x.data_ptr(), g.data_ptr(), 0, w.data_ptr(), out.data_ptr(), M, N, K, 1e-5, handle)
+    return call, want.cpu().numpy()
+
+
+def test_captured_dense_calls_beside_others(tc, ctx, oracle):
+    """Graphs captured on one stream, replayed on two others at a time beside eager calls on the first: no launch takes
+    another's sums."""
+    import torch
+    cases = [dense_case(i, 2) for i in range(3)]
+    outs = [torch.zeros(2, 520, dtype=torch.float16, device="cuda") for _ in cases]
+    streams = [torch.cuda.Stream() for _ in cases]
+    torch.cuda.synchronize()
+    first = streams[0]
+    cases[0][0](tc, ctx, outs[0], first.cuda_stream)
+    torch.cuda.synchronize()
+    graphs = [capture(first, lambda i=i: cases[i][0](tc, ctx, outs[i], first.cuda_stream)) for i in (1, 2)]
+    for _ in range(20):
+        for o in outs:
+            o.fill_(float("nan"))
+        torch.cuda.synchronize()
+        for _ in range(10):
+            for graph, st in zip(graphs, streams[1:]):
+                with torch.cuda.stream(st):
+                    graph.replay()
+            cases[0][0](tc, ctx, outs[0], first.cuda_stream)
+        torch.cuda.synchronize()
+        for o, (_, want) in zip(outs, cases):
+            assert oracle.scaled_rms(o.cpu().numpy(), want) <= 1.1 * np.sqrt(2.0) * ROUND
+    assert tc.take_device_error(ctx) == 0
+
+
+def test_rooms_of_graphs_that_are_gone_are_used_again(tc, ctx, oracle):
+    """48 graphs captured and dropped, a room of 1.6 MB each: what is held at the end is a few of them."""
+    import gc
+    import time
+    import torch
+    call, want = dense_case(7, 4, 11008, 4096)
+    out = torch.zeros(4, 11008, dtype=torch.float16, device="cuda")
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    free = None
+    for i in range(48):
+        graph = capture(st, lambda: call(tc, ctx, out, st.cuda_stream))
+        out.zero_()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(st):
+            graph.replay()
+        torch.cuda.synchronize()
+        assert i % 16 or oracle.scaled_rms(out.cpu().numpy(), want) <= 1.1 * np.sqrt(2.0) * ROUND
+        del graph
+        gc.collect()
+        time.sleep(0.01)                      # the driver tells of it from a thread of its own
+        if i == 7:
+            free = torch.cuda.mem_get_info()[0]
+    assert free - torch.cuda.mem_get_info()[0] <= 16 << 20
+    assert tc.take_device_error(ctx) == 0
+
+
+def test_threads_on_the_per_thread_stream(tc, ctx, oracle):
+    """cudaStreamPerThread is one handle and a stream for each thread: dense, batched and attention calls of four threads
+    at a time, none in another's room."""
+    import torch
+    per_thread = 2
+    N, K, M, S, B = 19968, 2048, 8, 1300, 20
+    Wq = oracle.quantize_weights((np.random.default_rng(4).standard_normal((128, K)) * 0.02).astype(np.float16), 0)
+    w = on_device(np.asarray(Wq))[0].reshape(128, -1).repeat(N // 128, 1).contiguous()
+    d = tc.TCAttentionDesc(B, 8, 1, S, 128, tc.TC_DTYPE_F16, tc.TC_DTYPE_F32, 0.0, False, False, 2, 0, None)
+    wrong = []
+
+    def work(i):
+        gen = torch.Generator(device="cuda")
+        gen.manual_seed(i)
+        half = lambda *shape: torch.randn(*shape, device="cuda", generator=gen).half()
+        dense, want = dense_case(20 + i, 3)
+        x, q, k, v = half(M, K), half(B, 8, 1, 128), half(B, 2, S, 128), half(B, 2, S, 128)
+        y, o, z = torch.zeros(M, N, device="cuda").half(), torch.zeros_like(q), torch.zeros(3, 520, device="cuda").half()
+        torch.cuda.synchronize()
+        first = None
+        for _ in range(10):
+            for _ in range(5):
+                dense(tc, ctx, z, per_thread)
+                tc.raw_gemv_quantized(ctx, x.data_ptr(), w.data_ptr(), y.data_ptr(), 0, M, N, K, "f16", "f16", per_thread)
+                rc = tc.lib().tcx_raw_attention_forward(ctx.handle, ctypes.byref(d), *(ctypes.c_void_p(t.data_ptr()) for t in (q, k, v, o)),
+                                                        None, ctypes.c_void_p(per_thread))
+                assert rc == 0
+            torch.cuda.synchronize()
+            got = [t.clone() for t in (z, y, o)]
+            torch.cuda.synchronize()
+            first = first or got
+            if not all(torch.equal(a, b) for a, b in zip(got, first)):
+                wrong.append((i, "bits"))
+        if oracle.scaled_rms(first[0].cpu().numpy(), want) > 1.1 * np.sqrt(2.0) * ROUND:
+            wrong.append((i, "dense"))
+        rows = oracle.dequant_dot_f64(x.cpu().numpy().astype(np.float64), Wq, 0, 128)
+        if oracle.scaled_rms(first[1][:, N - 128:].cpu().numpy(), rows) > 1.1 * np.sqrt(2.0) * ROUND:
+            wrong.append((i, "batched"))
+        s = torch.softmax(q.double().view(B, 2, 4, 128) @ k.double().transpose(2, 3) / 128 ** 0.5, 3) @ v.double()
+        if oracle.scaled_rms(first[2].cpu().numpy().reshape(B, 2, 4, 128), s.cpu().numpy()) > 1.1 * ROUND:
+            wrong.append((i, "attention"))
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+    assert tc.take_device_error(ctx) == 0
+
+
 def test_threads_on_streams_of_their_own(tc, ctx, oracle):
     """Fused batched calls of growing size from four threads: no call's rows are normalised into another's room."""
     import torch
