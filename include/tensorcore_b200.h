@@ -529,7 +529,10 @@ tc_status_t tcx_stream_decode_tp(tc_stream* s, const tcx_decode_tp_op* ops, int 
  * kernel), "tc" (tcgen05 kernel where it applies), "generic".  Returns TC_ERR_INVALID_ARG for an
  * unknown name.  Process-wide. */
 tc_status_t tcx_set_gemv_variant(const char* name);
-/* Device-side error word: non-zero after a kernel gave up on a bounded wait.  Reading clears. */
+/* Device-side error word: non-zero after a kernel gave up on a bounded wait.  Reading clears it.  Where it is set this
+ * waits for the whole device and empties the scratch that kernels hand partial results over in; let no other thread
+ * replay a graph with captured calls meanwhile.  Until then synchronous operations return TC_ERR_INTERNAL, and raw calls
+ * run on kernels that need no such scratch. */
 uint32_t tcx_take_device_error(tc_context* ctx);
 /* Sets bits of that word as a kernel that gives up would, so that a caller can try out its error handling. */
 tc_status_t tcx_set_device_error(tc_context* ctx, uint32_t bits);

@@ -191,6 +191,13 @@ tc_status_t validate(tc_context* ctx, const tc_buffer* b, size_t min_bytes) {
 bool staged(const tc_buffer* b) { return b->kind == BUF_WRAP_HOST || b->kind == BUF_HOST_SHADOW; }
 bool managed(const tc_buffer* b) { return b->kind == BUF_MANAGED || b->kind == BUF_WRAP_MANAGED; }
 
+tc_status_t check_device_error(tc_context* ctx) {
+    if (ctx->err_host && *reinterpret_cast<volatile uint32_t*>(ctx->err_host) != 0) {
+        return TC_ERR_INTERNAL;  // left set; tcx_take_device_error reads and clears it
+    }
+    return TC_OK;
+}
+
 // Scratch that belongs to a CUDA stream: calls on a stream are ordered, calls on different streams must not
 // share it.  A room is made when a call first needs it and grows when one needs more; the one outgrown is
 // freed once the stream is done with it - except where the caller captured the stream while it was handed
@@ -407,8 +414,20 @@ void free_rooms() {
     g_kept.clear();
 }
 
-// Room for words that one CTA hands to another: the stream's, or that of the graph the call is captured for.
+// Every room that is empty between launches.
+template <typename F>
+void for_hand_over_rooms(F f) {
+    for (RoomKind k : {ROOM_PARTIAL, ROOM_SHARES, ROOM_STATES}) {
+        for (auto& kv : g_rooms)
+            if (kv.second.room[k].p) f(kv.second.room[k], k);
+        for (const Room& r : g_spare[k]) f(r, k);
+    }
+    for (const GraphRoom& g : g_graph_rooms) f(g.room, g.kind);
+}
+// Room for words that one CTA hands to another: the stream's, or that of the graph the call is captured for.  None once
+// a kernel has given up: its words may be in any of them until the error is taken, and the kernels that need none do.
 Room hand_over_room(tc_context* ctx, cudaStream_t st, RoomKind k, size_t need) {
+    if (check_device_error(ctx) != TC_OK) return Room();
     if (being_captured(st)) return graph_room(st, k, need, ctx->stream0);
     if (!g_graph_rooms.empty()) trim_graph_rooms();
     return stream_room(st, k, need);
@@ -442,19 +461,19 @@ size_t share_scratch_need(tc_context* ctx, const tcb::GemvQArgs& a) {
     if (!tcb::tc_rows(a)) return 0;
     return tcb::gemm_q_tc_share_bytes(a.M <= tcb::kNormRoomRows ? a.M : tcb::norm_slab_rows(a.M), ctx->sm_count);
 }
-void share_scratch_for(cudaStream_t st, size_t need, tcb::GemvQArgs* a) {
+void share_scratch_for(tc_context* ctx, cudaStream_t st, size_t need, tcb::GemvQArgs* a) {
     // A captured call does without (its graph could have a room of its own, as the dense call's; but whole tiles and
     // clusters need none).
     if (need == 0 || being_captured(st)) return;
-    const Room& r = stream_room(st, ROOM_SHARES, need);
+    const Room r = hand_over_room(ctx, st, ROOM_SHARES, need);
     a->share_scratch = r.p;
     a->share_scratch_bytes = r.bytes;
 }
 // Room for the softmax states that attention merges in its kernel; null where a call has to do without (captured, as
 // for the shares; no memory).
-uint32_t* attention_states_for(cudaStream_t st, size_t need) {
+uint32_t* attention_states_for(tc_context* ctx, cudaStream_t st, size_t need) {
     if (need == 0 || being_captured(st)) return nullptr;
-    const Room& r = stream_room(st, ROOM_STATES, need);
+    const Room r = hand_over_room(ctx, st, ROOM_STATES, need);
     return r.bytes >= need ? static_cast<uint32_t*>(r.p) : nullptr;
 }
 void norm_scratch_for(cudaStream_t st, size_t need, tcb::GemvQArgs* a) {
@@ -509,13 +528,6 @@ cudaError_t prepare_output(tc_context* ctx, tc_buffer* b, cudaStream_t st) {
 cudaError_t finish_output(tc_buffer* b, size_t bytes, cudaStream_t st) {
     if (staged(b)) return cudaMemcpyAsync(b->hptr, b->dptr, bytes, cudaMemcpyDeviceToHost, st);
     return cudaSuccess;
-}
-
-tc_status_t check_device_error(tc_context* ctx) {
-    if (ctx->err_host && *reinterpret_cast<volatile uint32_t*>(ctx->err_host) != 0) {
-        return TC_ERR_INTERNAL;  // left set; tcx_take_device_error reads and clears it
-    }
-    return TC_OK;
 }
 
 // The status of a synchronous operation whose last CUDA call gave e: a kernel that gave up on a wait has left a wrong
@@ -1059,11 +1071,11 @@ void free_decode_site(DecodeSite& d) {
 }
 
 // After a launch that gave up on a bounded wait the counter and the accumulators hold arbitrary
-// values: start over from zero.
-void reset_decode_site(DecodeSite& d) {
+// values: start over from zero, in the stream's order.
+void reset_decode_site(DecodeSite& d, cudaStream_t st) {
     if (d.n_ranks > 1) return;   // tensor parallel: the ranks must agree on a restart (tcx_stream_tp_reset)
-    if (d.counter) cudaMemset(d.counter, 0, kMegaFlagBytes);
-    if (d.pool) cudaMemset(d.pool, 0, d.pool_floats * sizeof(float));
+    if (d.counter) cudaMemsetAsync(d.counter, 0, kMegaFlagBytes, st);
+    if (d.pool) cudaMemsetAsync(d.pool, 0, d.pool_floats * sizeof(float), st);
     d.base = 0;
 }
 
@@ -1194,7 +1206,7 @@ tc_status_t submit_pending(tc_stream* s) {
             sh = h > sh ? h : sh;
         }
         if (need > 0 || dq > 0 || sh > 0) rooms.lock();
-        share_scratch_for(s->s, sh, &scratch_of);
+        share_scratch_for(ctx, s->s, sh, &scratch_of);
         norm_scratch_for(s->s, need, &scratch_of);
         dequant_scratch_for(s->s, dq, &scratch_of);
     }
@@ -1299,7 +1311,7 @@ extern "C" tc_status_t tc_stream_sync(tc_stream* s) {
     const cudaError_t e = cudaStreamSynchronize(s->s);
     if (st == TC_OK) st = from_cuda(e, TC_ERR_DISPATCH);
     if (st == TC_OK) st = check_device_error(s->owner);
-    if (st != TC_OK) reset_decode_site(s->site);
+    if (st != TC_OK) reset_decode_site(s->site, s->s);
     return st;
 }
 
@@ -1556,7 +1568,7 @@ tc_status_t gemv_common(const GemvCall& c, tc_stream* stream, const char* opname
         const size_t need = norm_scratch_need(op.a), dq = dequant_scratch_need(op.a), sh = share_scratch_need(ctx, op.a);
         RoomsLock rooms(g_rooms_mutex, std::defer_lock);
         if (need > 0 || dq > 0 || sh > 0) rooms.lock();
-        share_scratch_for(s0, sh, &op.a);
+        share_scratch_for(ctx, s0, sh, &op.a);
         norm_scratch_for(s0, need, &op.a);
         dequant_scratch_for(s0, dq, &op.a);
         LaunchEnv env = make_env(ctx, false);
@@ -1795,7 +1807,7 @@ extern "C" tc_status_t tc_attention_forward(tc_context* ctx, const tc_attention_
     const bool matrix = tcb::attention_on_matrix_kernels(D, Q->dptr, K->dptr, V->dptr);
     size_t want = tcb::attention_scratch_floats(B, Hq, Hkv, Sq, Sk, D, matrix, ctx->sm_count, &chunks);
     RoomsLock rooms(g_rooms_mutex);
-    uint32_t* const states = attention_states_for(ctx->stream0, tcb::attention_state_bytes(B, Hq, Hkv, Sq, D, matrix, chunks));
+    uint32_t* const states = attention_states_for(ctx, ctx->stream0, tcb::attention_state_bytes(B, Hq, Hkv, Sq, D, matrix, chunks));
     if (states) want = 0;
     const size_t slope_at = want;
     if (d->alibi_slopes) want += static_cast<size_t>(Hq);
@@ -1853,7 +1865,7 @@ extern "C" tc_status_t tcx_raw_attention_forward(tc_context* ctx, const tc_atten
     uint32_t* states = nullptr;
     if (want > 0) {
         rooms.lock();
-        states = attention_states_for(st, tcb::attention_state_bytes(d->batch, d->heads, Hkv, d->seq_q, d->head_dim, matrix, chunks));
+        states = attention_states_for(ctx, st, tcb::attention_state_bytes(d->batch, d->heads, Hkv, d->seq_q, d->head_dim, matrix, chunks));
     }
     if (want > 0 && !states) {
         grow_room(ctx->attn, want * sizeof(float), ~static_cast<size_t>(0), st, -1, [] { cudaDeviceSynchronize(); });
@@ -2102,7 +2114,7 @@ static tc_status_t raw_gemv(tc_context* ctx, const void* X, const void* gamma, b
     const size_t need = norm_scratch_need(a), dq = dequant_scratch_need(a), sh = share_scratch_need(ctx, a);
     RoomsLock rooms(g_rooms_mutex, std::defer_lock);
     if (need > 0 || dq > 0 || sh > 0) rooms.lock();
-    share_scratch_for(static_cast<cudaStream_t>(cuda_stream), sh, &a);
+    share_scratch_for(ctx, static_cast<cudaStream_t>(cuda_stream), sh, &a);
     norm_scratch_for(static_cast<cudaStream_t>(cuda_stream), need, &a);
     dequant_scratch_for(static_cast<cudaStream_t>(cuda_stream), dq, &a);
     int launches = 0;
@@ -2218,23 +2230,20 @@ extern "C" tc_status_t tcx_set_device_error(tc_context* ctx, uint32_t bits) {
 
 extern "C" uint32_t tcx_take_device_error(tc_context* ctx) {
     if (!ctx || !ctx->err_host) return 0;
-    const uint32_t v = *reinterpret_cast<volatile uint32_t*>(ctx->err_host);
-    *reinterpret_cast<volatile uint32_t*>(ctx->err_host) = 0;
-    if (v != 0) {
-        // A kernel that gave up may have left sums in the rooms that are empty between launches.
-        RoomsLock lock(g_rooms_mutex);
-        bind_device(ctx);
-        cudaDeviceSynchronize();
-        for (RoomKind k : {ROOM_PARTIAL, ROOM_SHARES, ROOM_STATES}) {
-            for (auto& kv : g_rooms) {
-                const Room& r = kv.second.room[k];
-                if (r.p) cudaMemset(r.p, kRoomFill[k], r.bytes);
-            }
-            for (const Room& r : g_spare[k]) cudaMemset(r.p, kRoomFill[k], r.bytes);
-        }
-        (void)cudaGetLastError();
-    }
-    return v;
+    volatile uint32_t* const word = ctx->err_host;
+    if (*word == 0) return 0;
+    // A kernel that gave up may have left words in the rooms that are empty between launches, and others that wait for
+    // it may still be about to give up too: nothing runs any more before the word is read, and no call is handed a
+    // room before all of them are empty again.
+    RoomsLock lock(g_rooms_mutex);
+    bind_device(ctx);
+    cudaDeviceSynchronize();
+    const uint32_t bits = *word;
+    for_hand_over_rooms([&](const Room& r, RoomKind k) { cudaMemsetAsync(r.p, kRoomFill[k], r.bytes, ctx->stream0); });
+    cudaStreamSynchronize(ctx->stream0);
+    (void)cudaGetLastError();
+    *word = 0;
+    return bits;
 }
 
 extern "C" uint64_t tcx_launch_count(void) { return g_launches.load(); }

@@ -1,5 +1,7 @@
 """GPU: the device error word.  A kernel that gives up on a bounded wait sets it and leaves a wrong result; every
 synchronous operation reports it until it is taken.  No kernel gives up here: the word is set from the host."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -58,3 +60,50 @@ def test_synchronous_operations_report_a_device_error(tc, ctx):
     assert tc.take_device_error(ctx) == 0
     for b in bufs:
         b.close()
+
+
+def test_raw_calls_do_without_hand_over_scratch_until_the_error_is_taken(tc, ctx):
+    """Once a kernel has given up, words of its launch may lie in the scratch that sums are handed over in.  Raw calls
+    then take kernels that need none (merged chunks: the same bits), and the first ones after the error was taken have
+    empty scratch again."""
+    import torch
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(5)
+    half = lambda *shape: torch.randn(*shape, device="cuda", generator=gen).half()
+    st = torch.cuda.Stream()
+    x, g, w, y = half(2, 1536), half(1536), half(1536, 520) * 0.02, torch.zeros(2, 520, device="cuda").half()
+    q, k, v, o = half(20, 8, 1, 128), half(20, 2, 1300, 128), half(20, 2, 1300, 128), torch.zeros(20, 8, 1, 128, device="cuda").half()
+    N, K = 19200, 2048
+    wf = half(N, K) * 0.02
+    wq, xb, yb = torch.zeros(tc.quantized_size("q4_0", N, K), dtype=torch.uint8, device="cuda"), half(8, K), torch.zeros(8, N, device="cuda").half()
+    torch.cuda.synchronize()
+    tc.raw_quantize_weights(ctx, wf.data_ptr(), wq.data_ptr(), "q4_0", N, K, st.cuda_stream)
+    d = tc.TCAttentionDesc(20, 8, 1, 1300, 128, tc.TC_DTYPE_F16, tc.TC_DTYPE_F32, 0.0, False, False, 2, 0, None)
+
+    def run():
+        """Results, and how many launches each call took."""
+        outs = []
+        for call, out in ((lambda: tc.raw_fused_norm_gemv_f16(ctx, x.data_ptr(), g.data_ptr(), 0, w.data_ptr(), y.data_ptr(), 2, 520, 1536, 1e-5,
+                                                              st.cuda_stream), y),
+                          (lambda: tc.lib().tcx_raw_attention_forward(ctx.handle, ctypes.byref(d), *(ctypes.c_void_p(t.data_ptr()) for t in (q, k, v, o)),
+                                                                      None, ctypes.c_void_p(st.cuda_stream)), o),
+                          (lambda: tc.raw_gemv_quantized(ctx, xb.data_ptr(), wq.data_ptr(), yb.data_ptr(), "q4_0", 8, N, K, "f16", "f16", st.cuda_stream), yb)):
+            before = tc.launch_count()
+            assert not call()
+            outs.append((tc.cuda_last_kernel_name(), tc.launch_count() - before))
+            st.synchronize()
+            outs[-1] += (out.clone(),)
+        torch.cuda.synchronize()
+        return outs
+    usual = run()
+    assert [u[1] for u in usual] == [1, 1, 1] and "split" in usual[0][0]
+    tc.set_device_error(ctx, 1)
+    without = run()
+    assert [u[1] for u in without] == [1, 2, 2] and "split" not in without[0][0]
+    assert torch.equal(without[1][2], usual[1][2])
+    for i, bar in ((0, 2.0 ** -11), (2, 2.0 ** -11)):       # sums in another order: a few roundings of the results differ
+        a, b = usual[i][2].double(), without[i][2].double()
+        assert ((a - b).square().mean() / a.square().mean()).sqrt().item() <= bar
+    assert tc.take_device_error(ctx) == 1 and tc.take_device_error(ctx) == 0
+    for a, b in zip(run(), usual):
+        assert a[:2] == b[:2] and torch.equal(a[2], b[2])
