@@ -434,7 +434,9 @@ tc_status_t tcx_raw_fused_rmsnorm_gemv_quantized(tc_context* ctx, const void* X,
                                                  void* cuda_stream);
 /* tc_attention_forward on raw device pointers, asynchronous on `cuda_stream` (desc->alibi_slopes must
  * be NULL).  The scratch that holds the partial softmax states of a row's key chunks belongs to the
- * context: do not let two of these launches overlap on different streams. */
+ * context: do not let two of these launches overlap on different streams.  (Launches of up to 16 rows - queries
+ * times query heads - per K/V head whose keys are cut into at most eight chunks merge them in the kernel, in scratch
+ * of the stream or of the captured graph, and may overlap; how many chunks there are depends on sizes and GPU.) */
 tc_status_t tcx_raw_attention_forward(tc_context* ctx, const tc_attention_desc* desc, const void* Q,
                                       const void* K, const void* V, void* O, void* LSE /* or NULL */,
                                       void* cuda_stream);

@@ -469,10 +469,9 @@ void share_scratch_for(tc_context* ctx, cudaStream_t st, size_t need, tcb::GemvQ
     a->share_scratch = r.p;
     a->share_scratch_bytes = r.bytes;
 }
-// Room for the softmax states that attention merges in its kernel; null where a call has to do without (captured, as
-// for the shares; no memory).
+// Room for the softmax states that attention merges in its kernel; null where a call has to do without.
 uint32_t* attention_states_for(tc_context* ctx, cudaStream_t st, size_t need) {
-    if (need == 0 || being_captured(st)) return nullptr;
+    if (need == 0) return nullptr;
     const Room r = hand_over_room(ctx, st, ROOM_STATES, need);
     return r.bytes >= need ? static_cast<uint32_t*>(r.p) : nullptr;
 }
@@ -1838,9 +1837,8 @@ extern "C" tc_status_t tc_attention_forward(tc_context* ctx, const tc_attention_
 }
 
 // The same on raw device pointers, asynchronous on the caller's stream (no ALiBi: its slopes would
-// have to be staged from host memory).  The scratch for the key chunks belongs to the context:
-// launches on different streams must not overlap, except
-// those whose chunks are merged in the kernel (up to 16 rows per K/V head).
+// have to be staged from host memory).  The scratch for the key chunks belongs to the context: launches on different
+// streams must not overlap, except those whose chunks are merged in the kernel (attention_state_bytes says which).
 extern "C" tc_status_t tcx_raw_attention_forward(tc_context* ctx, const tc_attention_desc* d, const void* Q,
                                                  const void* K, const void* V, void* O, void* LSE,
                                                  void* cuda_stream) {
@@ -1859,7 +1857,7 @@ extern "C" tc_status_t tcx_raw_attention_forward(tc_context* ctx, const tc_atten
     int chunks = 1;
     const bool matrix = tcb::attention_on_matrix_kernels(d->head_dim, Q, K, V);
     const size_t want = tcb::attention_scratch_floats(d->batch, d->heads, Hkv, d->seq_q, d->seq_kv, d->head_dim, matrix, ctx->sm_count, &chunks);
-    // Under capture nothing can be allocated: a call that finds too little room takes each row's keys in one piece.
+    // The context's scratch does not grow under capture: a call that finds too little takes each row's keys in one piece.
     RoomsLock rooms(g_rooms_mutex, std::defer_lock);
     float* scratch = nullptr;
     uint32_t* states = nullptr;

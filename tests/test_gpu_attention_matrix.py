@@ -245,22 +245,18 @@ def test_scores_have_no_bias(tc, ctx, B, H, Hkv, Sq, Sk, D, bar):
     (64, 8, 8, 1, 640, 128, False, 0), (37, 8, 2, 2, 1023, 128, True, 0), (20, 14, 2, 1, 2100, 64, False, 0), (20, 6, 3, 4, 1300, 128, False, 700),
     (70, 5, 1, 1, 4096, 64, False, 0), (10, 16, 8, 3, 257, 64, True, 0), (20, 48, 3, 1, 1500, 128, False, 0), (50, 8, 4, 1, 1, 128, False, 0)])
 def test_chunks_merged_in_the_kernel(tc, ctx, B, H, Hkv, Sq, Sk, D, causal, window):
-    """Up to 16 rows per K/V head: the chunks of a row's keys are merged by the kernel that has them, in one launch; a
-    captured call merges them in a launch of its own, to the same bits.  Bars: one rounding of O, 2^-11 / sqrt(3) rms (a
+    """Up to 16 rows per K/V head: the chunks of a row's keys are merged by the kernel that has them, in one launch, eager
+    or captured; a call that has no scratch to hand them over in (an error is set) merges them in a launch of its own, to
+    the same bits.  Bars: one rounding of O, 2^-11 / sqrt(3) rms (a
     twentieth for small samples); the log-sum-exp as in test_scores_have_no_bias."""
     import torch
     gen = torch.Generator(device="cuda")
     gen.manual_seed(Sk + H * Sq)
     q, k, v = (torch.randn(B, h, s, D, device="cuda", generator=gen).half() for h, s in ((H, Sq), (Hkv, Sk), (Hkv, Sk)))
-    # another call's chunks, so that the captured one finds room for its own
-    room = [ctx.buffer(64 * 64 * 64 * 256), ctx.buffer(8 * 16384 * 256)]
-    tc.attention_forward(ctx, room[0], room[1], room[1], room[0], 1, 64, 64, 16384, 128, causal=False, kv_heads=8)
-    for b in room:
-        b.close()
     st = torch.cuda.Stream()
     torch.cuda.synchronize()
     outs = []
-    for captured in (False, False, True):
+    for form in ("eager", "eager", "captured", "without"):
         o, lse = torch.full_like(q, float("nan")), torch.full((B, H, Sq), float("nan"), device="cuda")
         torch.cuda.synchronize()
         d = tc.TCAttentionDesc(B, H, Sq, Sk, D, tc.TC_DTYPE_F16, tc.TC_DTYPE_F32, 0.0, causal, True, Hkv, window, None)
@@ -269,16 +265,20 @@ def test_chunks_merged_in_the_kernel(tc, ctx, B, H, Hkv, Sq, Sk, D, causal, wind
             rc = tc.lib().tcx_raw_attention_forward(ctx.handle, ctypes.byref(d), *(ctypes.c_void_p(t.data_ptr()) for t in (q, k, v, o, lse)),
                                                     ctypes.c_void_p(st.cuda_stream))
             assert rc == 0
-        if captured:
+        before = tc.launch_count()
+        if form == "captured":
             graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(graph, stream=st):
                 call()
             with torch.cuda.stream(st):
                 graph.replay()
-        else:
-            before = tc.launch_count()
+        elif form == "without":
+            tc.set_device_error(ctx, 1)
             call()
-            assert tc.launch_count() - before == 1 and tc.cuda_last_kernel_name() == "attention_mma_sm100"
+            assert tc.take_device_error(ctx) == 1
+        else:
+            call()
+        assert tc.launch_count() - before == (2 if form == "without" else 1) and tc.cuda_last_kernel_name() == "attention_mma_sm100"
         torch.cuda.synchronize()
         outs.append((o, lse))
     for o, lse in outs[1:]:

@@ -197,6 +197,48 @@ def test_captured_dense_calls_beside_others(tc, ctx, oracle):
     assert tc.take_device_error(ctx) == 0
 
 
+def test_captured_decode_attention_beside_others(tc, ctx):
+    """Two captures of a decode step's attention have their chunks' states in rooms of their own: one launch each, the
+    eager call's bits, also when they run at a time, beside eager calls on the stream they were captured on."""
+    import torch
+    B, H, Hkv, Sk, D = 8, 32, 8, 2048, 128
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(11)
+    half = lambda *shape: torch.randn(*shape, device="cuda", generator=gen).half()
+    cases = [[half(B, h, s, D) for h, s in ((H, 1), (Hkv, Sk), (Hkv, Sk))] for _ in range(3)]
+    outs = [torch.zeros(B, H, 1, D, device="cuda").half() for _ in cases]
+    streams = [torch.cuda.Stream() for _ in cases]
+    d = tc.TCAttentionDesc(B, H, 1, Sk, D, tc.TC_DTYPE_F16, tc.TC_DTYPE_F32, 0.0, False, False, Hkv, 0, None)
+    torch.cuda.synchronize()
+
+    def call(i):
+        rc = tc.lib().tcx_raw_attention_forward(ctx.handle, ctypes.byref(d), *(ctypes.c_void_p(t.data_ptr()) for t in cases[i] + [outs[i]]),
+                                                None, ctypes.c_void_p(streams[0].cuda_stream))
+        assert rc == 0
+    before = tc.launch_count()
+    graphs = [capture(streams[0], lambda i=i: call(i)) for i in (1, 2)]
+    assert tc.launch_count() - before == 2
+    refs = []
+    for i in range(3):
+        call(i)
+        torch.cuda.synchronize()
+        refs.append(outs[i].clone())
+        s = torch.softmax(cases[i][0].double().view(B, Hkv, 4, D) @ cases[i][1].double().transpose(2, 3) / D ** 0.5, 3) @ cases[i][2].double()
+        assert ((refs[i].double().view(s.shape) - s).square().mean() / s.square().mean()).sqrt().item() <= 1.05 * ROUND
+    for _ in range(20):
+        for o in outs:
+            o.fill_(float("nan"))
+        torch.cuda.synchronize()
+        for _ in range(10):
+            for graph, st in zip(graphs, streams[1:]):
+                with torch.cuda.stream(st):
+                    graph.replay()
+            call(0)
+        torch.cuda.synchronize()
+        assert all(torch.equal(o, r) for o, r in zip(outs, refs))
+    assert tc.take_device_error(ctx) == 0
+
+
 def test_rooms_of_graphs_that_are_gone_are_used_again(tc, ctx, oracle):
     """48 graphs captured and dropped, a room of 1.6 MB each: what is held at the end is a few of them."""
     import gc
