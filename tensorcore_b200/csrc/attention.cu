@@ -319,7 +319,6 @@ __device__ __forceinline__ void merge_warps(const AttnParams& p, float* o_s, flo
         }
     }
     __syncthreads();
-    bool ok = true;
     for (int t = tid; t < R * (D / 4); t += kAttnWarps * 32) {
         const int r = t / (D / 4), c = 4 * (t % (D / 4));
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -346,7 +345,10 @@ __device__ __forceinline__ void merge_warps(const AttnParams& p, float* o_s, flo
             constexpr int kOthers = kMergeHere - 1;
             uint4 o4[kOthers], ml[kOthers];
             const int n = p.chunks - 1;
-            ok = state_take(states + static_cast<size_t>(t) * 8, state_words, n, o4, ml) && ok;
+            if (!state_take(states + static_cast<size_t>(t) * 8, state_words, n, o4, ml)) {
+                if (p.err) atomicOr(p.err, ERR_WAIT_TIMEOUT);      // a thread waits once: the others' chunks are as late
+                return;
+            }
             float mm = m_s[r];
 #pragma unroll
             for (int i = 0; i < kOthers; ++i)
@@ -383,7 +385,6 @@ __device__ __forceinline__ void merge_warps(const AttnParams& p, float* o_s, flo
                 reinterpret_cast<uint16_t*>(dst)[e] = static_cast<uint16_t>((e < 2 ? v.x : v.y) >> (16 * (e & 1)));
         }
     }
-    if (!ok && p.err) atomicOr(p.err, ERR_WAIT_TIMEOUT);
 }
 
 template <int D, bool SPLIT_KEYS>

@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(kDThreads) dense_norm_gemv_split_kernel(const 
                 for (int k = 0; k < kAtOnce; ++k) all = all && handover::there(w[k]);
                 if (!all && clock64() - t0 > 2000000000LL) {
                     if (sp.err) atomicOr(sp.err, ERR_WAIT_TIMEOUT);
-                    break;
+                    return;                                  // a thread waits once: the other sums are as late
                 }
             }
 #pragma unroll

@@ -2,7 +2,10 @@
 // kNothing until its value has been written, so a reader knows the value by its being there, in one trip.  The reader
 // leaves kNothing behind for the next launch.  Store to use takes about 1.2 us; with a fence and a flag or a ticket 3 to 4.
 //
-// Who may wait: a CTA for those that started before it, or for what another's first piece of work is.  Waits are bounded.
+// Who may wait: a CTA for those that started before it, or for what another's first piece of work is.  That CTAs of lower
+// index start first is an assumption: GPUs deal them out so, CUDA does not promise it.  Were it otherwise, CTAs that wait
+// could keep those they wait for from starting.  So waits are bounded, about a second and once a thread; then the error
+// word is set, the kernel ends, and the words stay out of use until the host has emptied them (tcx_take_device_error).
 #pragma once
 
 #include <cuda_runtime.h>
