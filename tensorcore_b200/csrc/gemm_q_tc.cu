@@ -737,8 +737,8 @@ cudaError_t launch_gemm_q_tc(const GemvQArgs* ops, int n_ops, const LaunchEnv& e
         if (split < 1 || p.off_x + red_bytes > env.smem_optin) split = 1;
         return split;
     };
-    // Tiles left over after whole rounds of one per SM can go in a launch of their own when their K can be split
-    // over the SMs that would idle beside them.
+    // Without shares (a call that is captured has no scratch for them), tiles left over after whole rounds of one per SM go
+    // in a launch of their own when their K can be split over the SMs that would idle beside them.
     const bool two_launches = tiles > sms && left > 0 && !forced && split_for(left) > 1;
     // Shares, where they save enough units of the CTA with most of them.  What they cost: a tile more to read out
     // on the way, and, where a share is shorter than a tile, the sums that cross the L2 at the very end (a tile of 8 /
@@ -756,8 +756,6 @@ cudaError_t launch_gemm_q_tc(const GemvQArgs* ops, int n_ops, const LaunchEnv& e
     bool share = tiles > sms ? saved > (p.nb <= 32 ? 4.0 : p.nb <= 128 ? 7.0 : 5.6)
                              : p.nb <= 32 && units >= 3 * sms && saved > (a.fmt == FMT_Q4_0 ? 5.5 : 4.0);
     if (forced || !a.share_scratch || a.share_scratch_bytes < static_cast<size_t>(shares) * p.nb * kRows * 4) share = false;
-    // The launches of a synchronous call can be counted by its caller, and where these are two they stay two.
-    if (env.alone && two_launches) share = false;
     p.part = static_cast<uint32_t*>(a.share_scratch);
     const int first = two_launches && !share ? tiles - left : tiles;
 
