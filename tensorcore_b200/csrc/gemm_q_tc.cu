@@ -658,6 +658,27 @@ int mma_columns(int M, int* col_tiles) {
     return ((M + *col_tiles - 1) / *col_tiles + 15) & ~15;
 }
 
+// Shares, where they save enough units of the CTA with most of them.  What they cost: a tile more to read out
+// on the way, and, where a share is shorter than a tile, the sums that cross the L2 at the very end (a tile of 8 /
+// 32 / 64 / 128 / 256 columns: 2.2 / 2.5 / 6.5 / 6.7 / 10 us).  Whole tiles or clusters / shares, microseconds back to
+// back, units of 256 weights by 128 rows of the longest CTA in brackets:
+//   Q4_0, rows           8            32            64           128           256           512
+//   11008 x 4096 (16 / 9.3)   11.7 / 11.3   12.5 / 12.3   16.1 / 18.4   17.7 / 19.2   29.1 / 29.9   -
+//   14336 x 4096 (16 / 12.1)  12.0 / 12.5   12.8 / 13.7   16.4 / 20.1   17.8 / 21.0   28.9 / 33.2   59.5 / 56.2 (32 / 24.2)
+//   28672 x 4096 (32 / 24.2)  21.5 / 18.2   22.7 / 19.7   30.5 / 31.5   33.4 / 34.0   58.0 / 54.8   112 / 102 (64 / 48.4)
+//   20000 x 2048 (16 / 8.5)   15.7 / 10.2   16.4 / 11.1   19.7 / 16.2   22.5 / 18.5   39.2 / 29.5   62.0 / 46.8 (24 / 17)
+//   4096 x 4096 (4 / 3.5)      8.7 /  8.0    9.2 /  8.8   10.9 / 15.0 (clusters of four)
+// Q8_0's units take longer up to 32 columns (0.82 against 0.5 us), so fewer of them pay.
+struct Shares { int n; bool pay; };
+Shares shares_of(int fmt, int nb, long long tiles, int groups, int sms) {
+    const long long units = tiles * groups;
+    const int n = units < sms ? static_cast<int>(units) : sms;
+    const double saved = static_cast<double>((tiles + sms - 1) / sms) * groups - static_cast<double>(units) / n;
+    return {n, tiles > sms ? saved > (nb <= 32 ? 4.0 : nb <= 128 ? 7.0 : 5.6)
+                           : nb <= 32 && units >= 3 * sms && saved > (fmt == FMT_Q4_0 ? 5.5 : 4.0)};
+}
+size_t share_bytes(const Shares& s, int nb) { return static_cast<size_t>(s.n) * nb * kRows * 4; }
+
 }  // namespace
 
 cudaError_t init_gemm_q_tc_kernels(int smem_optin) {
@@ -670,9 +691,13 @@ cudaError_t init_gemm_q_tc_kernels(int smem_optin) {
     return cudaSuccess;
 }
 
-size_t gemm_q_tc_share_bytes(int M, int sm_count) {
+size_t gemm_q_tc_share_bytes(const GemvQArgs* ops, int n_ops, int M, int sm_count) {
     int col_tiles = 1;
-    return static_cast<size_t>(sm_count) * mma_columns(M, &col_tiles) * kRows * 4;
+    const int nb = mma_columns(M, &col_tiles);
+    long long row_tiles = 0;
+    for (int i = 0; i < n_ops; ++i) row_tiles += (ops[i].N + kRows - 1) / kRows;
+    const Shares s = shares_of(ops[0].fmt, nb, row_tiles * col_tiles, ops[0].K / 256, sm_count > 0 ? sm_count : 148);
+    return s.pay ? share_bytes(s, nb) : 0;
 }
 
 // Up to kMaxMats products of the same activation rows in one launch: ops[1 ..] differ from ops[0] in W, Y and N
@@ -740,22 +765,8 @@ cudaError_t launch_gemm_q_tc(const GemvQArgs* ops, int n_ops, const LaunchEnv& e
     // Without shares (a call that is captured has no scratch for them), tiles left over after whole rounds of one per SM go
     // in a launch of their own when their K can be split over the SMs that would idle beside them.
     const bool two_launches = tiles > sms && left > 0 && !forced && split_for(left) > 1;
-    // Shares, where they save enough units of the CTA with most of them.  What they cost: a tile more to read out
-    // on the way, and, where a share is shorter than a tile, the sums that cross the L2 at the very end (a tile of 8 /
-    // 32 / 64 / 128 / 256 columns: 2.2 / 2.5 / 6.5 / 6.7 / 10 us).  Whole tiles or clusters / shares, microseconds back to
-    // back, units of 256 weights by 128 rows of the longest CTA in brackets:
-    //   Q4_0, rows           8            32            64           128           256           512
-    //   11008 x 4096 (16 / 9.3)   11.7 / 11.3   12.5 / 12.3   16.1 / 18.4   17.7 / 19.2   29.1 / 29.9   -
-    //   14336 x 4096 (16 / 12.1)  12.0 / 12.5   12.8 / 13.7   16.4 / 20.1   17.8 / 21.0   28.9 / 33.2   59.5 / 56.2 (32 / 24.2)
-    //   28672 x 4096 (32 / 24.2)  21.5 / 18.2   22.7 / 19.7   30.5 / 31.5   33.4 / 34.0   58.0 / 54.8   112 / 102 (64 / 48.4)
-    //   20000 x 2048 (16 / 8.5)   15.7 / 10.2   16.4 / 11.1   19.7 / 16.2   22.5 / 18.5   39.2 / 29.5   62.0 / 46.8 (24 / 17)
-    //   4096 x 4096 (4 / 3.5)      8.7 /  8.0    9.2 /  8.8   10.9 / 15.0 (clusters of four)
-    // Q8_0's units take longer up to 32 columns (0.82 against 0.5 us), so fewer of them pay.
-    const int shares = units < sms ? static_cast<int>(units) : sms;
-    const double saved = static_cast<double>((tiles + sms - 1) / sms) * p.groups - static_cast<double>(units) / shares;
-    bool share = tiles > sms ? saved > (p.nb <= 32 ? 4.0 : p.nb <= 128 ? 7.0 : 5.6)
-                             : p.nb <= 32 && units >= 3 * sms && saved > (a.fmt == FMT_Q4_0 ? 5.5 : 4.0);
-    if (forced || !a.share_scratch || a.share_scratch_bytes < static_cast<size_t>(shares) * p.nb * kRows * 4) share = false;
+    const Shares shares = shares_of(a.fmt, p.nb, tiles, p.groups, sms);
+    const bool share = shares.pay && !forced && a.share_scratch && a.share_scratch_bytes >= share_bytes(shares, p.nb);
     p.part = static_cast<uint32_t*>(a.share_scratch);
     const int first = two_launches && !share ? tiles - left : tiles;
 
@@ -773,7 +784,7 @@ cudaError_t launch_gemm_q_tc(const GemvQArgs* ops, int n_ops, const LaunchEnv& e
         p.split = share ? 1 : split_for(n);
         p.wait_first = tile == 0 && env.wait_first() ? 1 : 0;      // the second launch follows this call's first
         cudaLaunchConfig_t cfg = {};
-        const int ctas = p.split > 1 ? n * p.split : share ? shares : n < sms ? n : sms;
+        const int ctas = p.split > 1 ? n * p.split : share ? shares.n : n < sms ? n : sms;
         const int chunks = share ? static_cast<int>(units) : n;
         p.chunk = share ? 1 : p.groups;
         p.run = chunks / ctas;

@@ -456,10 +456,16 @@ size_t norm_scratch_need(const tcb::GemvQArgs& a) {
 size_t dequant_scratch_need(const tcb::GemvQArgs& a) {
     return tcb::dequant_once(a) ? static_cast<size_t>(a.N) * a.K * 2 : 0;
 }
-// Room for the tiles that several CTAs of the tcgen05 kernel work on.
-size_t share_scratch_need(tc_context* ctx, const tcb::GemvQArgs& a) {
-    if (!tcb::tc_rows(a)) return 0;
-    return tcb::gemm_q_tc_share_bytes(a.M <= tcb::kNormRoomRows ? a.M : tcb::norm_slab_rows(a.M), ctx->sm_count);
+// Room for the tiles that several CTAs of the tcgen05 kernel work on, where its rule deals out shares: products that are
+// one launch, or a launch for each slab of their rows.
+size_t share_scratch_need(tc_context* ctx, const tcb::GemvQArgs* ops, int n) {
+    const tcb::GemvQArgs& a = ops[0];
+    if (!tcb::tc_rows(a) || tcb::dequant_once(a)) return 0;
+    const bool through_room = a.gamma || (reinterpret_cast<uintptr_t>(a.X) & 15u);
+    const int rows = through_room && a.M > tcb::kNormRoomRows ? tcb::norm_slab_rows(a.M) : a.M;
+    const size_t need = tcb::gemm_q_tc_share_bytes(ops, n, rows, ctx->sm_count);
+    const size_t last = a.M % rows ? tcb::gemm_q_tc_share_bytes(ops, n, a.M % rows, ctx->sm_count) : 0;
+    return need > last ? need : last;
 }
 void share_scratch_for(tc_context* ctx, cudaStream_t st, size_t need, tcb::GemvQArgs* a) {
     // A captured call does without (its graph could have a room of its own, as the dense call's; but whole tiles and
@@ -1016,20 +1022,26 @@ struct Written {
     }
 };
 
-// The operations of a list in order; neighbours that share their activations (q, k and v; gate and up) run as
-// one launch where their kernel can take several matrices.
+// Neighbours that share their activations (q, k and v; gate and up) run as one launch where their kernel can take several
+// matrices: the operations of a list that do with the i-th, copied to `group`, and how many they are.
+int group_of(const std::vector<RecordedOp>& list, size_t i, const LaunchEnv& env, tcb::GemvQArgs (&group)[4]) {
+    int n = 0;
+    group[n++] = list[i].a;
+    while (i + n < list.size() && tcb::gemv_q_groupable(group, n, list[i + n].a, env)) {
+        group[n] = list[i + n].a;
+        ++n;
+    }
+    return n;
+}
+
+// The operations of a list in order.
 cudaError_t launch_list(tc_context* ctx, const std::vector<RecordedOp>& list, cudaStream_t st, int* launches, const char** name) {
     cudaError_t e = cudaSuccess;
     Written written;
     for (size_t i = 0; i < list.size() && e == cudaSuccess;) {
         LaunchEnv env = make_env(ctx, i > 0);
         tcb::GemvQArgs group[4];
-        int n = 0;
-        group[n++] = list[i].a;
-        while (i + n < list.size() && tcb::gemv_q_groupable(group, n, list[i + n].a, env)) {
-            group[n] = list[i + n].a;
-            ++n;
-        }
+        const int n = group_of(list, i, env, group);
         // Nothing outside the list runs beside its second operation and those after it.
         env.weights_ready = true;
         for (int k = 0; k < n; ++k)
@@ -1192,17 +1204,34 @@ tc_status_t submit_pending(tc_stream* s) {
     if (s->pending.empty()) return TC_OK;
     bind_device(ctx);
     bool any_staged = false;
+    for (RecordedOp& op : s->pending) {
+        // Device addresses are resolved now, not when the operation was recorded: a first
+        // tc_buffer_map between the two moves a buffer to managed storage.
+        op.a.X = op.X->dptr;
+        op.a.W = static_cast<const uint8_t*>(op.W->dptr);
+        op.a.Y = op.Y->dptr;
+        op.a.gamma = op.gamma ? op.gamma->dptr : nullptr;
+        tc_buffer* bufs[4] = {op.X, op.W, op.Y, op.gamma};
+        for (tc_buffer* b : bufs)
+            if (b && staged(b)) any_staged = true;
+    }
     RoomsLock rooms(g_rooms_mutex, std::defer_lock);
     tcb::GemvQArgs scratch_of;          // the stream's scratch for normalised rows, sized for the widest operation
     {
         size_t need = 0, dq = 0, sh = 0;
-        for (const RecordedOp& op : s->pending) {
-            const size_t n = norm_scratch_need(op.a);
-            need = n > need ? n : need;
-            const size_t q = dequant_scratch_need(op.a);
-            dq = q > dq ? q : dq;
-            const size_t h = share_scratch_need(ctx, op.a);
+        const LaunchEnv env = make_env(ctx, false);
+        for (size_t i = 0; i < s->pending.size();) {
+            tcb::GemvQArgs group[4];
+            const int n = group_of(s->pending, i, env, group);
+            for (int k = 0; k < n; ++k) {
+                const size_t r = norm_scratch_need(group[k]);
+                need = r > need ? r : need;
+                const size_t q = dequant_scratch_need(group[k]);
+                dq = q > dq ? q : dq;
+            }
+            const size_t h = share_scratch_need(ctx, group, n);
             sh = h > sh ? h : sh;
+            i += n;
         }
         if (need > 0 || dq > 0 || sh > 0) rooms.lock();
         share_scratch_for(ctx, s->s, sh, &scratch_of);
@@ -1216,15 +1245,6 @@ tc_status_t submit_pending(tc_stream* s) {
         op.a.dequant_scratch_bytes = scratch_of.dequant_scratch_bytes;
         op.a.share_scratch = scratch_of.share_scratch;
         op.a.share_scratch_bytes = scratch_of.share_scratch_bytes;
-        // Device addresses are resolved now, not when the operation was recorded: a first
-        // tc_buffer_map between the two moves a buffer to managed storage.
-        op.a.X = op.X->dptr;
-        op.a.W = static_cast<const uint8_t*>(op.W->dptr);
-        op.a.Y = op.Y->dptr;
-        op.a.gamma = op.gamma ? op.gamma->dptr : nullptr;
-        tc_buffer* bufs[4] = {op.X, op.W, op.Y, op.gamma};
-        for (tc_buffer* b : bufs)
-            if (b && staged(b)) any_staged = true;
     }
     cudaError_t e = cudaSuccess;
     // Host-visible inputs first (staging copies or prefetch hints), outside any graph.
@@ -1564,7 +1584,7 @@ tc_status_t gemv_common(const GemvCall& c, tc_stream* stream, const char* opname
     int launches = 0;
     const char* name = "none";
     if (e == cudaSuccess) {
-        const size_t need = norm_scratch_need(op.a), dq = dequant_scratch_need(op.a), sh = share_scratch_need(ctx, op.a);
+        const size_t need = norm_scratch_need(op.a), dq = dequant_scratch_need(op.a), sh = share_scratch_need(ctx, &op.a, 1);
         RoomsLock rooms(g_rooms_mutex, std::defer_lock);
         if (need > 0 || dq > 0 || sh > 0) rooms.lock();
         share_scratch_for(ctx, s0, sh, &op.a);
@@ -2107,7 +2127,7 @@ static tc_status_t raw_gemv(tc_context* ctx, const void* X, const void* gamma, b
     a.X = X; a.Y = Y; a.gamma = fused ? gamma : nullptr;
     a.fmt = static_cast<int>(fmt); a.M = M; a.N = N; a.K = K;
     a.x_f32 = xd == TC_DTYPE_F32; a.y_f32 = yd == TC_DTYPE_F32; a.eps = eps;
-    const size_t need = norm_scratch_need(a), dq = dequant_scratch_need(a), sh = share_scratch_need(ctx, a);
+    const size_t need = norm_scratch_need(a), dq = dequant_scratch_need(a), sh = share_scratch_need(ctx, &a, 1);
     RoomsLock rooms(g_rooms_mutex, std::defer_lock);
     if (need > 0 || dq > 0 || sh > 0) rooms.lock();
     share_scratch_for(ctx, static_cast<cudaStream_t>(cuda_stream), sh, &a);

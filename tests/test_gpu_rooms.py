@@ -266,6 +266,27 @@ def test_rooms_of_graphs_that_are_gone_are_used_again(tc, ctx, oracle):
     assert tc.take_device_error(ctx) == 0
 
 
+def test_no_room_for_shares_that_are_not_dealt_out(tc, ctx):
+    """Calls whose tiles stay whole leave memory as it is: scratch for the shares of 256 columns is 19 MB a stream."""
+    import torch
+    M, N, K = 256, 4096, 1024
+    x, y = torch.randn(M, K, device="cuda").half(), torch.zeros(M, N, device="cuda").half()
+    w = torch.zeros(tc.quantized_size("q4_0", N, K), dtype=torch.uint8, device="cuda")
+    streams = [torch.cuda.Stream() for _ in range(8)]
+
+    def call(st):
+        tc.raw_gemv_quantized(ctx, x.data_ptr(), w.data_ptr(), y.data_ptr(), "q4_0", M, N, K, "f16", "f16", st.cuda_stream)
+        torch.cuda.synchronize()
+    torch.cuda.synchronize()
+    call(streams[0])
+    free = torch.cuda.mem_get_info()[0]
+    for st in streams:
+        call(st)
+    assert "tcgen05" in tc.cuda_last_kernel_name()
+    assert free - torch.cuda.mem_get_info()[0] <= 16 << 20
+    assert (y == 0).all() and tc.take_device_error(ctx) == 0
+
+
 def test_threads_on_the_per_thread_stream(tc, ctx, oracle):
     """cudaStreamPerThread is one handle and a stream for each thread: dense, batched and attention calls of four threads
     at a time, none in another's room."""
