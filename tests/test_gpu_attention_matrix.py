@@ -241,10 +241,11 @@ def test_scores_have_no_bias(tc, ctx, B, H, Hkv, Sq, Sk, D, bar):
     assert (err ** 2).mean().sqrt().item() <= bar
 
 
-@pytest.mark.parametrize("B,H,Hkv,Sq,Sk,D,causal,window", [
-    (64, 8, 8, 1, 640, 128, False, 0), (37, 8, 2, 2, 1023, 128, True, 0), (20, 14, 2, 1, 2100, 64, False, 0), (20, 6, 3, 4, 1300, 128, False, 700),
-    (70, 5, 1, 1, 4096, 64, False, 0), (10, 16, 8, 3, 257, 64, True, 0), (20, 48, 3, 1, 1500, 128, False, 0), (50, 8, 4, 1, 1, 128, False, 0)])
-def test_chunks_merged_in_the_kernel(tc, ctx, B, H, Hkv, Sq, Sk, D, causal, window):
+@pytest.mark.parametrize("B,H,Hkv,Sq,Sk,D,causal,window,chunked", [
+    (64, 8, 8, 1, 640, 128, False, 0, False), (37, 8, 2, 2, 1023, 128, True, 0, True), (20, 14, 2, 1, 2100, 64, False, 0, True),
+    (20, 6, 3, 4, 1300, 128, False, 700, True), (70, 5, 1, 1, 4096, 64, False, 0, True), (10, 16, 8, 3, 257, 64, True, 0, False),
+    (20, 48, 3, 1, 1500, 128, False, 0, True), (50, 8, 4, 1, 1, 128, False, 0, False)])
+def test_chunks_merged_in_the_kernel(tc, ctx, B, H, Hkv, Sq, Sk, D, causal, window, chunked):
     """Up to 16 rows per K/V head: the chunks of a row's keys are merged by the kernel that has them, in one launch, eager
     or captured; a call that has no scratch to hand them over in (an error is set) merges them in a launch of its own, to
     the same bits.  Bars: one rounding of O, 2^-11 / sqrt(3) rms (a
@@ -278,7 +279,7 @@ def test_chunks_merged_in_the_kernel(tc, ctx, B, H, Hkv, Sq, Sk, D, causal, wind
             assert tc.take_device_error(ctx) == 1
         else:
             call()
-        assert tc.launch_count() - before == (2 if form == "without" else 1) and tc.cuda_last_kernel_name() == "attention_mma_sm100"
+        assert tc.launch_count() - before == (2 if form == "without" and chunked else 1) and tc.cuda_last_kernel_name() == "attention_mma_sm100"
         torch.cuda.synchronize()
         outs.append((o, lse))
     for o, lse in outs[1:]:
