@@ -295,6 +295,30 @@ def test_very_many_rows_dequantise_once(tc, ctx, oracle, fused, fmt, M, N, K, on
     assert tc.take_device_error(ctx) == 0
 
 
+def distinct_tiles(oracle, fmt, M, N, K, seed=0):
+    """Weights whose tiles of 128 rows differ, for the price of one: the same rows, further on in every tile, times a power
+    of two of its own.  Returns activations, weights, the 64-bit results without those factors, and the factors."""
+    import torch
+    X, Wq = data(oracle, fmt, M, 128, K)
+    if seed:
+        _, Wq = data(oracle, fmt, M + seed, 128, K)
+    rows = torch.arange(N, device="cuda")
+    tile = rows // 128
+    at, power = (rows + tile) % 128, tile % 5 - 2
+    w = torch.from_numpy(np.asarray(Wq)).cuda().reshape(128, K // 32, -1)[at].contiguous()
+    d = w[:, :, :2].contiguous().view(torch.float16)
+    w[:, :, :2] = (d * torch.pow(2.0, power.half()).view(-1, 1, 1)).view(torch.uint8)
+    want = torch.from_numpy(oracle.dequant_dot_f64(X.astype(np.float64), Wq, fmt, 128)).cuda()[:, at]
+    return torch.from_numpy(X).cuda(), w, want, torch.pow(2.0, power.double())
+
+
+def check_tiles(got, want, factors, bar):
+    """All results against `bar`, and each column: one wrong tile would vanish in the mean of all."""
+    err = ((got.double() / factors - want) / want.square().mean().sqrt()).square()
+    assert err.mean().sqrt().item() <= bar
+    assert err.mean(0).sqrt().max().item() <= 4 * bar
+
+
 @pytest.mark.parametrize("fmt,M,N,K", [
     (0, 5, 3841, 4096), (0, 16, 3900, 4352), (0, 32, 4096, 14336), (0, 17, 8192, 8192), (1, 16, 3800, 4096), (1, 13, 11008, 4096),
     (0, 8, 19200, 2048), (0, 16, 38000, 768), (0, 32, 57000, 256), (0, 33, 19073, 3072), (0, 64, 38100, 2048), (0, 100, 20000, 2048),
@@ -303,11 +327,7 @@ def test_shares_of_the_unit_list(tc, ctx, oracle, fmt, M, N, K):
     """Every CTA has the same number of units, wherever tiles end: shares shorter than a tile (a tile of two to six
     CTAs), longer, of one unit more or less, in every accumulator layout.  One launch; the same bits each time."""
     import torch
-    X, Wq = data(oracle, fmt, M, 128, K)
-    reps = (N + 127) // 128                                   # every tile the same 128 rows: one oracle call for all of them
-    want = oracle.dequant_dot_f64(X.astype(np.float64), Wq, fmt, 128)
-    x, w = torch.from_numpy(X).cuda(), torch.from_numpy(np.asarray(Wq)).cuda().reshape(128, -1).repeat(reps, 1)[:N].contiguous()
-    want = torch.from_numpy(want).cuda().repeat(1, reps)[:, :N]
+    x, w, want, factors = distinct_tiles(oracle, fmt, M, N, K)
     y = torch.empty(M, N, dtype=torch.float16, device="cuda")
     st = torch.cuda.current_stream().cuda_stream
     outs = []
@@ -318,9 +338,39 @@ def test_shares_of_the_unit_list(tc, ctx, oracle, fmt, M, N, K):
         assert "tcgen05" in tc.cuda_last_kernel_name() and tc.launch_count() - before == 1
         outs.append(y.clone())
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
-    err = ((outs[0].double() - want) / want.square().mean().sqrt()).square()
-    bar = 1.1 * np.sqrt(2.0) * ROUND
-    assert err.mean().sqrt().item() <= bar
-    # a tile's share of the error: one wrong tile would vanish in the mean of all
-    assert err.mean(0).sqrt().max().item() <= 4 * bar
+    check_tiles(outs[0], want, factors, 1.1 * np.sqrt(2.0) * ROUND)
+    assert tc.take_device_error(ctx) == 0
+
+
+@pytest.mark.parametrize("fmt,M,K,Ns", [(0, 8, 2048, (9000, 5000, 5100)), (0, 5, 4096, (130, 11009, 127, 7700)), (1, 16, 2304, (10010, 9001)),
+                                        (0, 40, 3072, (6400, 6500, 6337)), (0, 130, 2048, (10011, 9990)), (0, 300, 2304, (4993, 4700))])
+def test_shares_that_go_on_in_the_next_matrix(tc, ctx, oracle, fmt, M, K, Ns):
+    """Products that share their activations, recorded: one launch whose runs of units cross from one matrix to the next
+    (another tensor map, row count and result), with row counts that are no whole tiles.  Launched directly, captured and
+    replayed, always the same bits."""
+    import torch
+    cases = [distinct_tiles(oracle, fmt, M, n, K, seed=i) for i, n in enumerate(Ns)]
+    x = cases[0][0]                             # the same activations in each
+    ys = [torch.empty(M, n, dtype=torch.float16, device="cuda") for n in Ns]
+    torch.cuda.synchronize()
+    wrap = lambda t: ctx.buffer_from_ptr(t.data_ptr(), t.numel() * t.element_size())
+    bx, bws, bys = wrap(x), [wrap(w) for _, w, _, _ in cases], [wrap(y) for y in ys]
+    first = None
+    with ctx.stream() as s:
+        for _ in range(4):
+            for y in ys:
+                y.fill_(float("nan"))
+            torch.cuda.synchronize()
+            before = tc.launch_count()
+            for bw, by, n in zip(bws, bys, Ns):
+                ctx.gemv_quantized_async(bx, bw, by, fmt, M, n, K, s)
+            s.sync()
+            assert tc.launch_count() - before == 1 and "tcgen05" in tc.cuda_last_kernel_name()
+            got = [y.clone() for y in ys]
+            first = first or got
+            assert all(torch.equal(a, b) for a, b in zip(got, first))
+    for got, (_, _, want, factors) in zip(first, cases):
+        check_tiles(got, want, factors, 1.1 * np.sqrt(2.0) * ROUND)
+    for b in [bx] + bws + bys:
+        b.close()
     assert tc.take_device_error(ctx) == 0

@@ -88,8 +88,8 @@ def test_captured_quantized_call(tc, ctx, oracle, K, M, big):
 
 @pytest.mark.parametrize("M,warm", [(2, 0), (2, 2), (4, 1), (16, 0), (16, 5), (40, 16)])
 def test_captured_dense_call(tc, ctx, oracle, M, warm):
-    """The dense fused call: partial sums and tickets up to four rows, normalised rows above; on a stream that has no
-    rooms yet (warm = 0), and on one whose rooms are for fewer rows."""
+    """The dense fused call: partial sums in a room of the graph's up to four rows, normalised rows in the stream's above; on
+    a stream that has no rooms yet (warm = 0), and on one whose rooms are for fewer rows."""
     import torch
     N, K, big = 520, 1536, 64
     rng = np.random.default_rng(M + warm)
@@ -113,7 +113,7 @@ def test_captured_dense_call(tc, ctx, oracle, M, warm):
         call(m, y2)
     torch.cuda.synchronize()
     disturb(tc, ctx, oracle)
-    for _ in range(2):                        # the second replay finds the tickets as the first left them
+    for _ in range(2):                        # the second replay finds the room as the first left it
         y.zero_()
         with torch.cuda.stream(st):
             graph.replay()
@@ -287,11 +287,11 @@ def test_no_room_for_shares_that_are_not_dealt_out(tc, ctx):
     assert (y == 0).all() and tc.take_device_error(ctx) == 0
 
 
-def test_threads_on_the_per_thread_stream(tc, ctx, oracle):
-    """cudaStreamPerThread is one handle and a stream for each thread: dense, batched and attention calls of four threads
-    at a time, none in another's room."""
+@pytest.mark.parametrize("per_thread", [True, False])
+def test_threads_that_hand_sums_over(tc, ctx, oracle, per_thread):
+    """Dense, batched and attention calls of four threads at a time, none in another's room: on streams of their own, and on
+    cudaStreamPerThread, which is one handle and a stream for each thread."""
     import torch
-    per_thread = 2
     N, K, M, S, B = 19968, 2048, 8, 1300, 20
     Wq = oracle.quantize_weights((np.random.default_rng(4).standard_normal((128, K)) * 0.02).astype(np.float16), 0)
     w = on_device(np.asarray(Wq))[0].reshape(128, -1).repeat(N // 128, 1).contiguous()
@@ -303,16 +303,18 @@ def test_threads_on_the_per_thread_stream(tc, ctx, oracle):
         gen.manual_seed(i)
         half = lambda *shape: torch.randn(*shape, device="cuda", generator=gen).half()
         dense, want = dense_case(20 + i, 3)
+        own = torch.cuda.Stream()
+        st = 2 if per_thread else own.cuda_stream
         x, q, k, v = half(M, K), half(B, 8, 1, 128), half(B, 2, S, 128), half(B, 2, S, 128)
         y, o, z = torch.zeros(M, N, device="cuda").half(), torch.zeros_like(q), torch.zeros(3, 520, device="cuda").half()
         torch.cuda.synchronize()
         first = None
         for _ in range(10):
             for _ in range(5):
-                dense(tc, ctx, z, per_thread)
-                tc.raw_gemv_quantized(ctx, x.data_ptr(), w.data_ptr(), y.data_ptr(), 0, M, N, K, "f16", "f16", per_thread)
+                dense(tc, ctx, z, st)
+                tc.raw_gemv_quantized(ctx, x.data_ptr(), w.data_ptr(), y.data_ptr(), 0, M, N, K, "f16", "f16", st)
                 rc = tc.lib().tcx_raw_attention_forward(ctx.handle, ctypes.byref(d), *(ctypes.c_void_p(t.data_ptr()) for t in (q, k, v, o)),
-                                                        None, ctypes.c_void_p(per_thread))
+                                                        None, ctypes.c_void_p(st))
                 assert rc == 0
             torch.cuda.synchronize()
             got = [t.clone() for t in (z, y, o)]
@@ -334,6 +336,44 @@ def test_threads_on_the_per_thread_stream(tc, ctx, oracle):
     for t in threads:
         t.join()
     assert not wrong
+    assert tc.take_device_error(ctx) == 0
+
+
+def test_streams_in_the_rooms_of_closed_ones(tc, ctx, oracle):
+    """A stream that is opened after another was closed takes its rooms: the sums handed over in them are the new
+    stream's, smaller calls and larger ones."""
+    import torch
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(2)
+    half = lambda *shape: torch.randn(*shape, device="cuda", generator=gen).half()
+    S, B, N, K = 1300, 20, 19200, 2048
+    w = torch.zeros(tc.quantized_size("q4_0", N, K), dtype=torch.uint8, device="cuda")
+    tc.raw_quantize_weights(ctx, (half(N, K) * 0.02).data_ptr(), w.data_ptr(), "q4_0", N, K)
+    q, k, v, x = half(B, 8, 1, 128), half(B, 2, S, 128), half(B, 2, S, 128), half(32, K)
+    dense = [dense_case(30 + m, m) for m in (1, 4)]
+    torch.cuda.synchronize()
+
+    def work(s, m, b):
+        st = s.cuda_handle()
+        z, y, o = torch.zeros(m, 520, device="cuda").half(), torch.zeros(8 * m, N, device="cuda").half(), torch.zeros(b, 8, 1, 128, device="cuda").half()
+        torch.cuda.synchronize()
+        d = tc.TCAttentionDesc(b, 8, 1, S, 128, tc.TC_DTYPE_F16, tc.TC_DTYPE_F32, 0.0, False, False, 2, 0, None)
+        before = tc.launch_count()
+        dense[m > 1][0](tc, ctx, z, st)
+        tc.raw_gemv_quantized(ctx, x.data_ptr(), w.data_ptr(), y.data_ptr(), 0, 8 * m, N, K, "f16", "f16", st)
+        rc = tc.lib().tcx_raw_attention_forward(ctx.handle, ctypes.byref(d), *(ctypes.c_void_p(t.data_ptr()) for t in (q, k, v, o)), None,
+                                                ctypes.c_void_p(st))
+        assert rc == 0 and tc.launch_count() - before == 3
+        torch.cuda.synchronize()
+        assert oracle.scaled_rms(z.cpu().numpy(), dense[m > 1][1]) <= 1.1 * np.sqrt(2.0) * ROUND
+        return z, y, o
+    sizes = [(1, 16), (4, 20), (1, 16), (4, 20), (4, 20), (1, 16)]
+    with ctx.stream() as s:
+        refs = {size: work(s, *size) for size in sizes}
+    for size in sizes:
+        with ctx.stream() as s, ctx.stream() as s2:
+            for st in (s, s2, s):
+                assert all(torch.equal(a, b) for a, b in zip(work(st, *size), refs[size]))
     assert tc.take_device_error(ctx) == 0
 
 
