@@ -1220,18 +1220,19 @@ tc_status_t submit_pending(tc_stream* s) {
     {
         size_t need = 0, dq = 0, sh = 0;
         const LaunchEnv env = make_env(ctx, false);
-        for (size_t i = 0; i < s->pending.size();) {
+        size_t grouped = 0;             // operations before this one are in a group that has been asked about
+        for (size_t i = 0; i < s->pending.size(); ++i) {
+            const tcb::GemvQArgs& a = s->pending[i].a;
+            const size_t n = norm_scratch_need(a);
+            need = n > need ? n : need;
+            const size_t q = dequant_scratch_need(a);
+            dq = q > dq ? q : dq;
+            if (i < grouped || !tcb::tc_rows(a)) continue;      // (most lists are a token of one row)
             tcb::GemvQArgs group[4];
-            const int n = group_of(s->pending, i, env, group);
-            for (int k = 0; k < n; ++k) {
-                const size_t r = norm_scratch_need(group[k]);
-                need = r > need ? r : need;
-                const size_t q = dequant_scratch_need(group[k]);
-                dq = q > dq ? q : dq;
-            }
-            const size_t h = share_scratch_need(ctx, group, n);
+            const int m = group_of(s->pending, i, env, group);
+            const size_t h = share_scratch_need(ctx, group, m);
             sh = h > sh ? h : sh;
-            i += n;
+            grouped = i + static_cast<size_t>(m);
         }
         if (need > 0 || dq > 0 || sh > 0) rooms.lock();
         share_scratch_for(ctx, s->s, sh, &scratch_of);
