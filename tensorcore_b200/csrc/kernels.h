@@ -52,6 +52,7 @@ struct LaunchEnv {
     // With pdl, whether nothing that may still run on the stream writes the weights: they are then read while the
     // kernel before runs.  Else a kernel waits for it first, and lets the next one start only after that.
     bool weights_ready = false;
+    bool alone = false;        // a synchronous call
     bool wait_first() const { return pdl && !weights_ready; }
     int variant = VARIANT_AUTO;
     uint32_t* err_word = nullptr;  // device-visible word a kernel ORs an error bit into

@@ -1591,7 +1591,9 @@ tc_status_t gemv_common(const GemvCall& c, tc_stream* stream, const char* opname
         share_scratch_for(ctx, s0, sh, &op.a);
         norm_scratch_for(s0, need, &op.a);
         dequant_scratch_for(s0, dq, &op.a);
-        e = tcb::launch_gemv_q(op.a, make_env(ctx, false), s0, &launches, &name);
+        LaunchEnv env = make_env(ctx, false);
+        env.alone = true;
+        e = tcb::launch_gemv_q(op.a, env, s0, &launches, &name);
     }
     if (e == cudaSuccess) e = finish_output(op.Y, yb, s0);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s0);
