@@ -241,23 +241,26 @@ def test_scores_have_no_bias(tc, ctx, B, H, Hkv, Sq, Sk, D, bar):
     assert (err ** 2).mean().sqrt().item() <= bar
 
 
-@pytest.mark.parametrize("B,H,Hkv,Sq,Sk,D,causal,window,chunked", [
-    (64, 8, 8, 1, 640, 128, False, 0, False), (37, 8, 2, 2, 1023, 128, True, 0, True), (20, 14, 2, 1, 2100, 64, False, 0, True),
-    (20, 6, 3, 4, 1300, 128, False, 700, True), (70, 5, 1, 1, 4096, 64, False, 0, True), (10, 16, 8, 3, 257, 64, True, 0, False),
-    (20, 48, 3, 1, 1500, 128, False, 0, True), (50, 8, 4, 1, 1, 128, False, 0, False)])
-def test_chunks_merged_in_the_kernel(tc, ctx, B, H, Hkv, Sq, Sk, D, causal, window, chunked):
-    """Up to 16 rows per K/V head: the chunks of a row's keys are merged by the kernel that has them, in one launch, eager
-    or captured; a call that has no scratch to hand them over in (an error is set) merges them in a launch of its own, to
-    the same bits.  Bars: one rounding of O, 2^-11 / sqrt(3) rms (a
+@pytest.mark.parametrize("B,H,Hkv,Sq,Sk,D,causal,window", [
+    (64, 8, 8, 1, 640, 128, False, 0), (37, 8, 2, 2, 1023, 128, True, 0), (20, 14, 2, 1, 2100, 64, False, 0), (20, 6, 3, 4, 1300, 128, False, 700),
+    (70, 5, 1, 1, 4096, 64, False, 0), (10, 16, 8, 3, 257, 64, True, 0), (20, 48, 3, 1, 1500, 128, False, 0), (50, 8, 4, 1, 1, 128, False, 0)])
+def test_chunks_merged_in_the_kernel(tc, ctx, B, H, Hkv, Sq, Sk, D, causal, window):
+    """Up to 16 rows per K/V head: the chunks of a row's keys are merged by the kernel that has them, in one launch,
+    to the same bits when captured.  Bars: one rounding of O, 2^-11 / sqrt(3) rms (a
     twentieth for small samples); the log-sum-exp as in test_scores_have_no_bias."""
     import torch
     gen = torch.Generator(device="cuda")
     gen.manual_seed(Sk + H * Sq)
     q, k, v = (torch.randn(B, h, s, D, device="cuda", generator=gen).half() for h, s in ((H, Sq), (Hkv, Sk), (Hkv, Sk)))
+    # another call's chunks, so that the captured one finds room for its own
+    room = [ctx.buffer(64 * 64 * 64 * 256), ctx.buffer(8 * 16384 * 256)]
+    tc.attention_forward(ctx, room[0], room[1], room[1], room[0], 1, 64, 64, 16384, 128, causal=False, kv_heads=8)
+    for b in room:
+        b.close()
     st = torch.cuda.Stream()
     torch.cuda.synchronize()
     outs = []
-    for form in ("eager", "eager", "captured", "without"):
+    for captured in (False, False, True):
         o, lse = torch.full_like(q, float("nan")), torch.full((B, H, Sq), float("nan"), device="cuda")
         torch.cuda.synchronize()
         d = tc.TCAttentionDesc(B, H, Sq, Sk, D, tc.TC_DTYPE_F16, tc.TC_DTYPE_F32, 0.0, causal, True, Hkv, window, None)
@@ -266,20 +269,16 @@ def test_chunks_merged_in_the_kernel(tc, ctx, B, H, Hkv, Sq, Sk, D, causal, wind
             rc = tc.lib().tcx_raw_attention_forward(ctx.handle, ctypes.byref(d), *(ctypes.c_void_p(t.data_ptr()) for t in (q, k, v, o, lse)),
                                                     ctypes.c_void_p(st.cuda_stream))
             assert rc == 0
-        before = tc.launch_count()
-        if form == "captured":
+        if captured:
             graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(graph, stream=st):
                 call()
             with torch.cuda.stream(st):
                 graph.replay()
-        elif form == "without":
-            tc.set_device_error(ctx, 1)
-            call()
-            assert tc.take_device_error(ctx) == 1
         else:
+            before = tc.launch_count()
             call()
-        assert tc.launch_count() - before == (2 if form == "without" and chunked else 1) and tc.cuda_last_kernel_name() == "attention_mma_sm100"
+            assert tc.launch_count() - before == 1 and tc.cuda_last_kernel_name() == "attention_mma_sm100"
         torch.cuda.synchronize()
         outs.append((o, lse))
     for o, lse in outs[1:]:
@@ -321,3 +320,45 @@ def test_prefill_rows_of_odd_groups(tc, ctx, B, H, Hkv, Sq, Sk, D, causal, off):
     assert (lse.double() - torch.logsumexp(s, 4).reshape(B, H, Sq)).square().mean().sqrt().item() <= 3.8e-7
     assert torch.isnan(room[off + q.numel():]).all() and torch.isnan(room[:off]).all()
     assert tc.take_device_error(ctx) == 0
+
+
+@pytest.mark.parametrize("B,H,Hkv,Sq,Sk,D,causal,window,chunked", [
+    (64, 8, 8, 1, 640, 128, False, 0, False), (37, 8, 2, 2, 1023, 128, True, 0, True), (20, 14, 2, 1, 2100, 64, False, 0, True),
+    (20, 6, 3, 4, 1300, 128, False, 700, True), (70, 5, 1, 1, 4096, 64, False, 0, True), (20, 48, 3, 1, 1500, 128, False, 0, True)])
+def test_chunks_merged_in_the_kernel_in_other_forms(tc, ctx, B, H, Hkv, Sq, Sk, D, causal, window, chunked):
+    """A captured call has room of its graph's and is the same one launch, whatever ran before; a call without scratch to hand
+    chunks over in (an error is set) merges them in a launch of its own.  Both to the eager call's bits."""
+    import torch
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(Sk + H * Sq)
+    q, k, v = (torch.randn(B, h, s, D, device="cuda", generator=gen).half() for h, s in ((H, Sq), (Hkv, Sk), (Hkv, Sk)))
+    st = torch.cuda.Stream()
+    d = tc.TCAttentionDesc(B, H, Sq, Sk, D, tc.TC_DTYPE_F16, tc.TC_DTYPE_F32, 0.0, causal, True, Hkv, window, None)
+    outs = []
+    for form in ("captured", "eager", "without"):
+        o, lse = torch.full_like(q, float("nan")), torch.full((B, H, Sq), float("nan"), device="cuda")
+        torch.cuda.synchronize()
+
+        def call():
+            rc = tc.lib().tcx_raw_attention_forward(ctx.handle, ctypes.byref(d), *(ctypes.c_void_p(t.data_ptr()) for t in (q, k, v, o, lse)),
+                                                    ctypes.c_void_p(st.cuda_stream))
+            assert rc == 0
+        before = tc.launch_count()
+        if form == "captured":
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=st):
+                call()
+            with torch.cuda.stream(st):
+                graph.replay()
+        elif form == "without":
+            tc.set_device_error(ctx, 1)
+            call()
+            assert tc.take_device_error(ctx) == 1
+        else:
+            call()
+        assert tc.launch_count() - before == (2 if form == "without" and chunked else 1) and tc.cuda_last_kernel_name() == "attention_mma_sm100"
+        torch.cuda.synchronize()
+        outs.append((o, lse))
+    for o, lse in outs[1:]:
+        assert torch.equal(o, outs[0][0]) and torch.equal(lse, outs[0][1])
+    assert not torch.isnan(outs[0][0]).any() and tc.take_device_error(ctx) == 0

@@ -278,6 +278,37 @@ def test_very_many_rows_dequantise_once(tc, ctx, oracle, fused, fmt, M, N, K, on
     assert tc.take_device_error(ctx) == 0
 
 
+@pytest.mark.parametrize("fmt,M,N,K", [
+    (0, 5, 3841, 4096), (0, 16, 3900, 4352), (0, 32, 4096, 14336), (0, 17, 8192, 8192), (1, 16, 3800, 4096), (1, 13, 11008, 4096),
+    (0, 8, 19200, 2048), (0, 16, 38000, 768), (0, 32, 57000, 256), (0, 33, 19073, 3072), (0, 64, 38100, 2048), (0, 100, 20000, 2048),
+    (0, 130, 20000, 2048), (0, 300, 9700, 2304), (0, 256, 19100, 2048), (1, 48, 20000, 2048), (1, 128, 28672, 2304), (1, 520, 7000, 4096)])
+def test_shares_of_the_unit_list(tc, ctx, oracle, fmt, M, N, K):
+    """Every CTA has the same number of units, wherever tiles end: shares shorter than a tile (a tile of two to six
+    CTAs), longer, of one unit more or less, in every accumulator layout.  One launch; the same bits each time."""
+    import torch
+    X, Wq = data(oracle, fmt, M, 128, K)
+    reps = (N + 127) // 128                                   # every tile the same 128 rows: one oracle call for all of them
+    want = oracle.dequant_dot_f64(X.astype(np.float64), Wq, fmt, 128)
+    x, w = torch.from_numpy(X).cuda(), torch.from_numpy(np.asarray(Wq)).cuda().reshape(128, -1).repeat(reps, 1)[:N].contiguous()
+    want = torch.from_numpy(want).cuda().repeat(1, reps)[:, :N]
+    y = torch.empty(M, N, dtype=torch.float16, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    outs = []
+    for _ in range(3):
+        y.fill_(float("nan"))
+        before = tc.launch_count()
+        tc.raw_gemv_quantized(ctx, x.data_ptr(), w.data_ptr(), y.data_ptr(), fmt, M, N, K, "f16", "f16", st)
+        assert "tcgen05" in tc.cuda_last_kernel_name() and tc.launch_count() - before == 1
+        outs.append(y.clone())
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    err = ((outs[0].double() - want) / want.square().mean().sqrt()).square()
+    bar = 1.1 * np.sqrt(2.0) * ROUND
+    assert err.mean().sqrt().item() <= bar
+    # a tile's share of the error: one wrong tile would vanish in the mean of all
+    assert err.mean(0).sqrt().max().item() <= 4 * bar
+    assert tc.take_device_error(ctx) == 0
+
+
 def distinct_tiles(oracle, fmt, M, N, K, seed=0):
     """Weights whose tiles of 128 rows differ, for the price of one: the same rows, further on in every tile, times a power
     of two of its own.  Returns activations, weights, the 64-bit results without those factors, and the factors."""
@@ -306,9 +337,9 @@ def check_tiles(got, want, factors, bar):
     (0, 5, 3841, 4096), (0, 16, 3900, 4352), (0, 32, 4096, 14336), (0, 17, 8192, 8192), (1, 16, 3800, 4096), (1, 13, 11008, 4096),
     (0, 8, 19200, 2048), (0, 16, 38000, 768), (0, 32, 57000, 256), (0, 33, 19073, 3072), (0, 64, 38100, 2048), (0, 100, 20000, 2048),
     (0, 130, 20000, 2048), (0, 300, 9700, 2304), (0, 256, 19100, 2048), (1, 48, 20000, 2048), (1, 128, 28672, 2304), (1, 520, 7000, 4096)])
-def test_shares_of_the_unit_list(tc, ctx, oracle, fmt, M, N, K):
-    """Every CTA has the same number of units, wherever tiles end: shares shorter than a tile (a tile of two to six
-    CTAs), longer, of one unit more or less, in every accumulator layout.  One launch; the same bits each time."""
+def test_shares_over_tiles_that_differ(tc, ctx, oracle, fmt, M, N, K):
+    """The shapes of the test above over tiles that can be told apart: a unit of the wrong tile, or a neighbour's sums at
+    the wrong place, shows."""
     import torch
     x, w, want, factors = distinct_tiles(oracle, fmt, M, N, K)
     y = torch.empty(M, N, dtype=torch.float16, device="cuda")
@@ -356,4 +387,32 @@ def test_shares_that_go_on_in_the_next_matrix(tc, ctx, oracle, fmt, M, K, Ns):
         check_tiles(got, want, factors, 1.1 * np.sqrt(2.0) * ROUND)
     for b in [bx] + bws + bys:
         b.close()
+    assert tc.take_device_error(ctx) == 0
+
+
+@pytest.mark.parametrize("fmt,M,N,K", [(0, 8, 19200, 2048), (0, 5, 22016, 2304), (1, 16, 19000, 4096), (0, 33, 19073, 3072), (0, 260, 9600, 2048),
+                                       (1, 130, 20000, 2048)])
+def test_tiles_left_over_in_a_captured_call(tc, ctx, oracle, fmt, M, N, K):
+    """A captured call has no scratch for shares: whole rounds of tiles, and the rest in a launch of its own in which their K
+    is split."""
+    import torch
+    x, w, want, factors = distinct_tiles(oracle, fmt, M, N, K)
+    y = torch.empty(M, N, dtype=torch.float16, device="cuda")
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    before = tc.launch_count()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=st):
+        tc.raw_gemv_quantized(ctx, x.data_ptr(), w.data_ptr(), y.data_ptr(), fmt, M, N, K, "f16", "f16", st.cuda_stream)
+    assert tc.launch_count() - before == 2 and "tcgen05" in tc.cuda_last_kernel_name()
+    outs = []
+    for _ in range(3):
+        y.fill_(float("nan"))
+        torch.cuda.synchronize()
+        with torch.cuda.stream(st):
+            graph.replay()
+        torch.cuda.synchronize()
+        outs.append(y.clone())
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    check_tiles(outs[0], want, factors, 1.1 * np.sqrt(2.0) * ROUND)
     assert tc.take_device_error(ctx) == 0
