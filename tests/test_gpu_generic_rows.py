@@ -98,3 +98,24 @@ def test_fp32_sums_are_closer_than_one_chain_per_block(tc, ctx, oracle, fmt):
                 v = v[:, :v.shape[1] // 2] + v[:, v.shape[1] // 2:]
             chain[m] += v[:, 0]
     assert oracle.scaled_rms(got, want) <= 0.92 * oracle.scaled_rms(chain.astype(np.float64), want)
+
+
+@pytest.mark.parametrize("fmt", [0, 1])
+@pytest.mark.parametrize("M,N,K", [(1, 3, 50016), (1, 200, 40032), (2, 1190, 16416), (1, 9571, 2080), (3, 9472, 1056), (4, 9546, 1056), (1, 2300, 28704)])
+def test_units_of_a_warp_over_groups_and_chunks(tc, ctx, oracle, fmt, M, N, K):
+    """A warp goes from unit to unit by a step of so many chunks and row groups: one group a CTA to more than there are warps,
+    CTAs with a row more that have a group more, rows of up to the length that fits shared memory, each unit once.
+    Bar as above: 32 products in two chains, 32 blocks in a tree and up to 49 chunks in order round less often than
+    a chain of 9000."""
+    rng = np.random.default_rng(N + K + fmt)
+    rows = min(N, 97)                                    # the weights repeat, N / 97 no whole number: the oracle's share of the time
+    Wq = np.asarray(oracle.quantize_weights((rng.standard_normal((rows, K)) * 0.02).astype(np.float16), fmt)).reshape(rows, -1)
+    X = rng.standard_normal((M, K)).astype(np.float32)
+    at = np.arange(N) % rows
+    want = oracle.dequant_dot_f64(X.astype(np.float64), Wq, fmt, rows)[:, at]
+    with ctx.buffer_from_array(X) as bx, ctx.buffer_from_array(np.ascontiguousarray(Wq[at])) as bw, ctx.buffer(M * N * 4) as by:
+        tc.gemv_quantized_ex(ctx, bx, bw, by, fmt, M, N, K, "f32", "f32", None)
+        assert "generic" in tc.cuda_last_kernel_name()
+        got = by.to_numpy((M, N), np.float32).astype(np.float64)
+    assert oracle.scaled_rms(got, want) <= 2e-6
+    assert np.abs(got - want).max() <= 2e-5 * np.sqrt((want * want).mean())      # ten times the bar: a wrong unit would be 1e4 times it
