@@ -217,6 +217,9 @@ constexpr int kMergeMaxChunks = 128;
 constexpr int kMergeHere = 8;          // chunks that the attention kernel can merge itself
 constexpr int kMmaRows = 64;           // rows (query, head) of a tile
 
+// Words of a chunk's states for R rows that another CTA merges: sums, then maximum and sum of each row; in 16 bytes.
+__host__ __device__ constexpr int attention_state_words(int R, int D) { return R * D + ((2 * R + 3) & ~3); }
+
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
@@ -238,31 +241,6 @@ __device__ __forceinline__ void state_store4(uint32_t* dst, float4 v) {
     using handover::word_of;
     handover::store4(dst, make_uint4(word_of(v.x), word_of(v.y), word_of(v.z), word_of(v.w)));
 }
-// What n chunks have of four elements, {o, o, o, o} and {m, l, -, -} each: all asked for at a time, until all are
-// there; false after about a second.
-template <int N>
-__device__ __forceinline__ bool state_take(uint32_t* src, size_t stride, int n, uint4 (&o)[N], uint4 (&ml)[N]) {
-    const long long t0 = clock64();
-    for (;;) {
-        bool all = true;
-#pragma unroll
-        for (int i = 0; i < N; ++i)
-            if (i < n) {
-                o[i] = handover::load4(src + i * stride);
-                ml[i] = handover::load4(src + i * stride + 4);
-            }
-#pragma unroll
-        for (int i = 0; i < N; ++i)
-            if (i < n) all = all && handover::there(o[i]) && handover::there(ml[i]);
-        if (all) break;
-        if (clock64() - t0 > 2000000000LL) return false;
-    }
-    constexpr uint32_t w = handover::kNothing;
-#pragma unroll
-    for (int i = 0; i < 2 * N; ++i)
-        if (i < 2 * n) handover::store4(src + i / 2 * stride + 4 * (i & 1), make_uint4(w, w, w, w));
-    return true;
-}
 // An 8 x 8 matrix of 16-bit elements, a thread's two those of row lane / 4, transposed.
 __device__ __forceinline__ uint32_t transpose_8x8(uint32_t v) {
     uint32_t r;
@@ -277,7 +255,14 @@ template <int D> struct MmaShape {
 
 // The end of the kernels whose warps split the keys of a step (ROWS rows): o_s has each warp's outputs, rows STRIDE
 // elements apart, ml_s its maximum and sum per row, both in the ring, which everybody has finished reading.
-template <int D, int ROWS, int STRIDE>
+// HERE: the chunks' states - sums, then maximum and sum per row - go to the CTA of the last chunk, which started last, and
+// it merges them: all words it needs are asked for at a time, however many elements a thread has, and the weights are
+// worked out once per row.  (With a trip for every four elements of a thread, and maximum and sum beside them, 16 rows
+// of head_dim 128 took up to 4 us longer than with a merge launch.  Raw calls back to back, merge launch / that / this: 18
+// sequences, 64 heads on 4 x 527 keys 14.5 / 16.6 / 14.4 us, 6 sequences, 256 on 16 x 2338 27.9 / 30.0 / 27.2, head_dim 64,
+// 39 sequences, 24 on 8, four queries x 1624 35.0 / 33.0 / 31.1, 160 on 16 x 456, eight chunks of a step, 8.4 / 12.5 / 10.4.)
+// Calls whose chunks are not merged here run an instance without that code, which cost them up to 1 us.
+template <int D, int ROWS, int STRIDE, bool HERE>
 __device__ __forceinline__ void merge_warps(const AttnParams& p, float* o_s, float* ml_s, int R, int G, int b, int hkv, int bk, int chunk) {
     const int tid = threadIdx.x;
     float* w_s = ml_s + kAttnWarps * ROWS * 2;                       // [ROWS][warp]
@@ -286,13 +271,11 @@ __device__ __forceinline__ void merge_warps(const AttnParams& p, float* o_s, flo
         const int i = p.by_per_kv(r);
         return (static_cast<size_t>(b) * p.Hq + hkv * G + (r - i * G)) * p.Sq + i;
     };
-    // With room for them the chunks' states go to the CTA of the last chunk, which started last, and it merges them: a
-    // thread has the same four elements of every chunk, with the row's maximum and sum beside each, so one trip
-    // brings all it needs.
-    const bool here = p.states != nullptr && p.chunks > 1, merges = here && chunk + 1 == p.chunks;
-    const size_t state_words = static_cast<size_t>(R) * D * 2;       // of a chunk
-    uint32_t* const states = here ? p.states + static_cast<size_t>(bk) * (p.chunks - 1) * state_words : nullptr;
-    float* m_s = w_s + ROWS * kAttnWarps;                              // [ROWS]: the CTA's maxima and sums
+    const int n = p.chunks - 1;                                      // HERE: chunks that others have
+    const bool merges = HERE && chunk == n;
+    const int state_words = attention_state_words(R, D);
+    uint32_t* const states = HERE ? p.states + static_cast<size_t>(bk) * n * state_words : nullptr;
+    float* m_s = w_s + ROWS * kAttnWarps;                            // [ROWS]: the CTA's maxima and sums
     float* l_s = m_s + ROWS;
     if (tid < R) {                                                   // at most 16 rows
         float mm = -INFINITY, ll = 0.f, f[kAttnWarps];
@@ -307,9 +290,13 @@ __device__ __forceinline__ void merge_warps(const AttnParams& p, float* o_s, flo
         const float inv = p.chunks > 1 ? 1.f : ll != 0.f ? 1.0f / ll : 0.f;
 #pragma unroll
         for (int w = 0; w < kAttnWarps; ++w) w_s[tid * kAttnWarps + w] = f[w] * inv;
-        if (here) {
+        if (merges) {
             m_s[tid] = mm;
             l_s[tid] = ll;
+        } else if (HERE) {
+            uint32_t* dst = states + static_cast<size_t>(chunk) * state_words + R * D + 2 * tid;
+            handover::store(dst, handover::word_of(mm));
+            handover::store(dst + 1, handover::word_of(ll));
         } else if (p.chunks > 1) {
             float* dst = p.part + (row_of(tid) * p.chunks + chunk) * (D + 2);
             dst[0] = mm;
@@ -319,8 +306,7 @@ __device__ __forceinline__ void merge_warps(const AttnParams& p, float* o_s, flo
         }
     }
     __syncthreads();
-    for (int t = tid; t < R * (D / 4); t += kAttnWarps * 32) {
-        const int r = t / (D / 4), c = 4 * (t % (D / 4));
+    auto sum_of = [&](int r, int c) {                                // four elements of the CTA's own
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int w = 0; w < kAttnWarps; ++w) {
@@ -329,52 +315,9 @@ __device__ __forceinline__ void merge_warps(const AttnParams& p, float* o_s, flo
             acc.x = fmaf(f, v.x, acc.x); acc.y = fmaf(f, v.y, acc.y);
             acc.z = fmaf(f, v.z, acc.z); acc.w = fmaf(f, v.w, acc.w);
         }
-        if (here && !merges) {
-            uint32_t* dst = states + chunk * state_words + static_cast<size_t>(t) * 8;
-            state_store4(dst, acc);
-            state_store4(dst + 4, make_float4(m_s[r], l_s[r], 0.f, 0.f));
-            continue;
-        }
-        if (p.chunks > 1 && !here) {
-            float2* dst = reinterpret_cast<float2*>(p.part + (row_of(r) * p.chunks + chunk) * (D + 2) + 2 + c);
-            dst[0] = make_float2(acc.x, acc.y);
-            dst[1] = make_float2(acc.z, acc.w);
-            continue;
-        }
-        if (merges) {
-            constexpr int kOthers = kMergeHere - 1;
-            uint4 o4[kOthers], ml[kOthers];
-            const int n = p.chunks - 1;
-            if (!state_take(states + static_cast<size_t>(t) * 8, state_words, n, o4, ml)) {
-                if (p.err) atomicOr(p.err, ERR_WAIT_TIMEOUT);      // a thread waits once: the others' chunks are as late
-                return;
-            }
-            float mm = m_s[r];
-#pragma unroll
-            for (int i = 0; i < kOthers; ++i)
-                if (i < n) mm = fmaxf(mm, __uint_as_float(ml[i].x));
-            // the sums of the merge kernel below in its order, to the bit: a tree of eight, elements by chunk
-            float le[kMergeHere];
-            float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-            auto add = [&](float m_c, float l_c, float4 v) {
-                const float e = m_c > -INFINITY ? __expf(m_c - mm) : 0.f;
-                sum.x = fmaf(v.x, e, sum.x); sum.y = fmaf(v.y, e, sum.y);
-                sum.z = fmaf(v.z, e, sum.z); sum.w = fmaf(v.w, e, sum.w);
-                return l_c * e;
-            };
-#pragma unroll
-            for (int i = 0; i < kMergeHere; ++i) {
-                le[i] = 0.f;
-                if (i < kOthers && i < n)
-                    le[i] = add(__uint_as_float(ml[i].x), __uint_as_float(ml[i].y),
-                                make_float4(__uint_as_float(o4[i].x), __uint_as_float(o4[i].y), __uint_as_float(o4[i].z), __uint_as_float(o4[i].w)));
-                else if (i == n)
-                    le[i] = add(m_s[r], l_s[r], acc);
-            }
-            const float ll = ((le[0] + le[4]) + (le[2] + le[6])) + ((le[1] + le[5]) + (le[3] + le[7]));
-            acc = ll != 0.f ? make_float4(sum.x / ll, sum.y / ll, sum.z / ll, sum.w / ll) : make_float4(0.f, 0.f, 0.f, 0.f);
-            if (c == 0 && p.LSE) p.LSE[row_of(r)] = mm + logf(fmaxf(ll, 1e-30f));
-        }
+        return acc;
+    };
+    auto write = [&](int r, int c, float4 acc) {
         __half* dst = p.O + row_of(r) * D + c;
         const uint2 v = make_uint2(pack_h2(acc.x, acc.y), pack_h2(acc.z, acc.w));
         if (p.o_vec) {
@@ -384,10 +327,116 @@ __device__ __forceinline__ void merge_warps(const AttnParams& p, float* o_s, flo
             for (int e = 0; e < 4; ++e)
                 reinterpret_cast<uint16_t*>(dst)[e] = static_cast<uint16_t>((e < 2 ? v.x : v.y) >> (16 * (e & 1)));
         }
+    };
+    constexpr int kThreads = kAttnWarps * 32;
+    if (!merges) {
+        for (int t = tid; t < R * (D / 4); t += kThreads) {
+            const int r = t / (D / 4), c = 4 * (t % (D / 4));
+            const float4 acc = sum_of(r, c);
+            if (HERE) {
+                state_store4(states + static_cast<size_t>(chunk) * state_words + 4 * t, acc);
+            } else if (p.chunks > 1) {
+                float2* dst = reinterpret_cast<float2*>(p.part + (row_of(r) * p.chunks + chunk) * (D + 2) + 2 + c);
+                dst[0] = make_float2(acc.x, acc.y);
+                dst[1] = make_float2(acc.z, acc.w);
+            } else {
+                write(r, c, acc);
+            }
+        }
+        return;
+    }
+    if constexpr (HERE) {
+        constexpr int kOthers = kMergeHere - 1, kTurns = ROWS * (D / 4) / kThreads;
+        static_assert(ROWS * kMergeHere <= kThreads && ROWS * (D / 4) % kThreads == 0, "");
+        constexpr uint32_t kNone = handover::kNothing;
+        const long long t0 = clock64();
+        uint4 o[kTurns][kOthers];
+        auto ask = [&]() {
+#pragma unroll
+            for (int u = 0; u < kTurns; ++u)
+#pragma unroll
+                for (int i = 0; i < kOthers; ++i)
+                    if (i < n && u * kThreads + tid < R * (D / 4)) o[u][i] = handover::load4(states + static_cast<size_t>(i) * state_words + 4 * (u * kThreads + tid));
+        };
+        ask();
+        // Weights: eight threads per row, one per chunk (the last is this CTA's), sums of them as in the merge kernel below.
+        float* e_s = l_s + ROWS;                                     // [ROWS][chunk]
+        float* ll_s = e_s + ROWS * kMergeHere;
+        bool ok = true;
+        if (tid < ROWS * kMergeHere) {
+            const int r = tid / kMergeHere, c = tid % kMergeHere;
+            float m = -INFINITY, l = 0.f;
+            if (r < R && c == n) {
+                m = m_s[r];
+                l = l_s[r];
+            } else if (r < R && c < n) {
+                uint32_t* src = states + static_cast<size_t>(c) * state_words + R * D + 2 * r;
+                uint32_t mw, lw;
+                for (;;) {
+                    mw = handover::load(src);
+                    lw = handover::load(src + 1);
+                    ok = handover::there(mw) && handover::there(lw);
+                    if (ok || clock64() - t0 > 2000000000LL) break;
+                }
+                handover::store(src, kNone);
+                handover::store(src + 1, kNone);
+                m = __uint_as_float(mw);
+                l = __uint_as_float(lw);
+            }
+            __syncwarp();
+            float mm = m;
+#pragma unroll
+            for (int x = 4; x > 0; x >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, x));
+            const float e = m > -INFINITY ? __expf(m - mm) : 0.f;
+            float ll = l * e;
+#pragma unroll
+            for (int x = 4; x > 0; x >>= 1) ll += __shfl_xor_sync(0xffffffffu, ll, x);
+            e_s[tid] = e;
+            if (c == 0 && r < R) {
+                ll_s[r] = ll;
+                if (p.LSE) p.LSE[row_of(r)] = mm + logf(fmaxf(ll, 1e-30f));
+            }
+        }
+        __syncthreads();
+        while (ok) {
+            bool all = true;
+#pragma unroll
+            for (int u = 0; u < kTurns; ++u)
+#pragma unroll
+                for (int i = 0; i < kOthers; ++i)
+                    if (i < n && u * kThreads + tid < R * (D / 4)) all = all && handover::there(o[u][i]);
+            if (all) break;
+            ok = clock64() - t0 <= 2000000000LL;
+            ask();
+        }
+        if (!ok) {                               // a thread waits once; what it has not taken is emptied with the error
+            if (p.err) atomicOr(p.err, ERR_WAIT_TIMEOUT);
+            return;
+        }
+#pragma unroll
+        for (int u = 0; u < kTurns; ++u) {
+            const int t = u * kThreads + tid, r = t / (D / 4), c = 4 * (t % (D / 4));
+            if (t >= R * (D / 4)) break;
+            float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+            auto add = [&](float e, float4 v) {
+                sum.x = fmaf(v.x, e, sum.x); sum.y = fmaf(v.y, e, sum.y);
+                sum.z = fmaf(v.z, e, sum.z); sum.w = fmaf(v.w, e, sum.w);
+            };
+#pragma unroll
+            for (int i = 0; i < kOthers; ++i) {
+                if (i >= n) continue;
+                handover::store4(states + static_cast<size_t>(i) * state_words + 4 * t, make_uint4(kNone, kNone, kNone, kNone));
+                add(e_s[r * kMergeHere + i], make_float4(__uint_as_float(o[u][i].x), __uint_as_float(o[u][i].y),
+                                                         __uint_as_float(o[u][i].z), __uint_as_float(o[u][i].w)));
+            }
+            add(e_s[r * kMergeHere + n], sum_of(r, c));
+            const float ll = ll_s[r];
+            write(r, c, ll != 0.f ? make_float4(sum.x / ll, sum.y / ll, sum.z / ll, sum.w / ll) : make_float4(0.f, 0.f, 0.f, 0.f));
+        }
     }
 }
 
-template <int D, bool SPLIT_KEYS>
+template <int D, bool SPLIT_KEYS, bool HERE>
 __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const AttnParams p) {
     asm volatile("griddepcontrol.launch_dependents;");
     using S = MmaShape<D>;
@@ -599,7 +648,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const
                 *reinterpret_cast<float2*>(o_s + (warp * 16 + r) * D + 8 * n + 2 * tq) = make_float2(o[n][2 * e], o[n][2 * e + 1]);
             if (tq == 0) { ml_s[(warp * 16 + r) * 2] = m[e]; ml_s[(warp * 16 + r) * 2 + 1] = l[e]; }
         }
-        merge_warps<D, 16, D>(p, o_s, ml_s, R, G, b, hkv, bk, chunk);
+        merge_warps<D, 16, D, HERE>(p, o_s, ml_s, R, G, b, hkv, bk, chunk);
     }
 }
 
@@ -609,7 +658,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const
 // heads x 4096 keys, whole calls: 40.6 us as rows of 16 with a merge launch, 39.5 merged in the kernel, 38.0 so (of
 // which 12 are launch and wait); 16 sequences, 64 heads x 8192 keys 96.6 -> 93.4 (6.7 TB/s); 8 heads on 2 x 4096 keys
 // 20.1 -> 19.2.
-template <int D>
+template <int D, bool HERE>
 __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma8_kernel(const AttnParams p) {
     asm volatile("griddepcontrol.launch_dependents;");
     using S = MmaShape<D>;
@@ -772,7 +821,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma8_kernel(cons
         }
         if (gq == 0) { ml_s[(warp * 8 + 2 * tq + e) * 2] = m[e]; ml_s[(warp * 8 + 2 * tq + e) * 2 + 1] = l[e]; }
     }
-    merge_warps<D, 8, kStride>(p, o_s, ml_s, R, G, b, hkv, bk, chunk);
+    merge_warps<D, 8, kStride, HERE>(p, o_s, ml_s, R, G, b, hkv, bk, chunk);
 }
 // Merges the chunks of a row: one CTA per row, a thread per chunk for the weights exp(m_c - m), then
 // a thread per output element with the chunks' partial outputs as independent loads.
@@ -881,7 +930,9 @@ cudaError_t launch_matrix(const AttnParams& p, bool prefill, cudaStream_t stream
     const long long x = static_cast<long long>(p.B) * p.Hkv * ((R + kMmaRows - 1) / kMmaRows);
     if (x > 0x7fffffffLL) return cudaErrorNotSupported;
     const dim3 grid(static_cast<unsigned>(x), static_cast<unsigned>(p.chunks));
-    auto* kernel = R <= 8 ? attention_mma8_kernel<D> : split ? attention_mma_kernel<D, true> : attention_mma_kernel<D, false>;
+    auto* kernel = R <= 8 ? (p.states ? attention_mma8_kernel<D, true> : attention_mma8_kernel<D, false>)
+                 : !split ? attention_mma_kernel<D, false, false>
+                          : p.states ? attention_mma_kernel<D, true, true> : attention_mma_kernel<D, true, false>;
     kernel<<<grid, kAttnWarps * 32, MmaShape<D>::kSmem, stream>>>(p);
     return cudaGetLastError();
 }
@@ -895,13 +946,14 @@ cudaError_t launch_vector(dim3 grid, cudaStream_t stream, const AttnParams& p) {
 }  // namespace
 
 cudaError_t init_attention_kernels() {
-    const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    cudaError_t e = cudaFuncSetAttribute(attention_mma_kernel<128, true>, a, MmaShape<128>::kSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_mma_kernel<128, false>, a, MmaShape<128>::kSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_mma_kernel<64, true>, a, MmaShape<64>::kSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_mma_kernel<64, false>, a, MmaShape<64>::kSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_mma8_kernel<128>, a, MmaShape<128>::kSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_mma8_kernel<64>, a, MmaShape<64>::kSmem);
+    auto allow = [](auto* kernel, int bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); };
+    cudaError_t e = cudaSuccess;
+    for (auto* k : {attention_mma_kernel<128, true, true>, attention_mma_kernel<128, true, false>, attention_mma_kernel<128, false, false>,
+                    attention_mma8_kernel<128, true>, attention_mma8_kernel<128, false>})
+        if (e == cudaSuccess) e = allow(k, MmaShape<128>::kSmem);
+    for (auto* k : {attention_mma_kernel<64, true, true>, attention_mma_kernel<64, true, false>, attention_mma_kernel<64, false, false>,
+                    attention_mma8_kernel<64, true>, attention_mma8_kernel<64, false>})
+        if (e == cudaSuccess) e = allow(k, MmaShape<64>::kSmem);
     return e == cudaSuccess ? init_attention_prefill_kernels() : e;
 }
 
@@ -920,7 +972,7 @@ size_t attention_scratch_floats(int B, int Hq, int Hkv, int Sq, int Sk, int D, b
 
 size_t attention_state_bytes(int B, int Hq, int Hkv, int Sq, int D, bool matrix, int chunks) {
     if (!matrix || chunks < 2 || chunks > kMergeHere || !attention_split_keys(Hq, Hkv, Sq)) return 0;
-    return static_cast<size_t>(B) * Hq * Sq * (chunks - 1) * D * 2 * sizeof(uint32_t);
+    return static_cast<size_t>(B) * Hkv * (chunks - 1) * attention_state_words(Sq * (Hq / Hkv), D) * sizeof(uint32_t);
 }
 
 cudaError_t launch_attention_forward(const void* Q, const void* K, const void* V, void* O, float* LSE,
@@ -939,7 +991,7 @@ cudaError_t launch_attention_forward(const void* Q, const void* K, const void* V
     p.group = attention_group(Hq, Hkv);
     const bool matrix = attention_on_matrix_kernels(D, Q, K, V);
     attention_chunks(B, Hq, Hkv, Sq, Sk, matrix, sm_count, &p.chunks, &p.keys_per_chunk);
-    p.states = matrix && attention_split_keys(Hq, Hkv, Sq) && p.chunks <= kMergeHere ? states : nullptr;
+    p.states = matrix && attention_split_keys(Hq, Hkv, Sq) && p.chunks > 1 && p.chunks <= kMergeHere ? states : nullptr;
     if (p.chunks > 1 && !scratch && !p.states) { p.chunks = 1; p.keys_per_chunk = Sk; }
     // The tensor core truncates its running sums: a score of D / 16 steps comes out smaller by 2.2e-8 of itself per step
     // on average (mean over 150,000 scores of normal data, mma.sync and tcgen05 alike: 1.8e-7 at head_dim 128, 0.9e-7

@@ -324,7 +324,9 @@ def test_prefill_rows_of_odd_groups(tc, ctx, B, H, Hkv, Sq, Sk, D, causal, off):
 
 @pytest.mark.parametrize("B,H,Hkv,Sq,Sk,D,causal,window,chunked", [
     (64, 8, 8, 1, 640, 128, False, 0, False), (37, 8, 2, 2, 1023, 128, True, 0, True), (20, 14, 2, 1, 2100, 64, False, 0, True),
-    (20, 6, 3, 4, 1300, 128, False, 700, True), (70, 5, 1, 1, 4096, 64, False, 0, True), (20, 48, 3, 1, 1500, 128, False, 0, True)])
+    (20, 6, 3, 4, 1300, 128, False, 700, True), (70, 5, 1, 1, 4096, 64, False, 0, True), (20, 48, 3, 1, 1500, 128, False, 0, True),
+    (1, 160, 16, 1, 456, 128, False, 0, True), (4, 72, 8, 1, 274, 128, False, 0, True), (22, 30, 2, 1, 700, 64, False, 0, True),
+    (40, 1, 1, 1, 500, 128, False, 0, True), (13, 39, 3, 1, 1100, 128, False, 0, True), (2, 16, 8, 8, 377, 64, False, 0, True)])
 def test_chunks_merged_in_the_kernel_in_other_forms(tc, ctx, B, H, Hkv, Sq, Sk, D, causal, window, chunked):
     """A captured call has room of its graph's and is the same one launch, whatever ran before; a call without scratch to hand
     chunks over in (an error is set) merges them in a launch of its own.  Both to the eager call's bits."""
