@@ -266,7 +266,7 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 template <int MB>
-__global__ void __launch_bounds__(kDThreads) dense_norm_gemv_split_kernel(const SplitParams sp) {
+__global__ void __launch_bounds__(kDThreads, 3) dense_norm_gemv_split_kernel(const SplitParams sp) {
     extern __shared__ __align__(128) uint8_t dsm[];
     double* scratch = reinterpret_cast<double*>(dsm);                 // kDWarps doubles
     uint8_t* ring = dsm + 128;                                        // kStages x 16 KB; reused for the reduction
@@ -358,46 +358,65 @@ __global__ void __launch_bounds__(kDThreads) dense_norm_gemv_split_kernel(const 
 #pragma unroll
         for (int e = 0; e < 8; ++e) red[(r0 * MB + m) * kSplitCols + hl * 8 + e] = acc[m][e];
     __syncthreads();
-    const int others = sp.chunks - 1;
-    for (int i = tid; i < MB * kSplitCols; i += kDThreads) {
-        const int m = i / kSplitCols, c = i - m * kSplitCols;
-        const int n = strip * kSplitCols + c;
-        if (n >= p.N) continue;
-        float mine = 0.f;
+    // A thread has one column: it adds the warps' sums of every row, and in the last K range the other ranges'.
+    static_assert(kDThreads == kSplitCols, "");
+    const int n = strip * kSplitCols + tid, others = sp.chunks - 1;
+    if (n >= p.N) return;
+    float mine[MB];
 #pragma unroll
-        for (int g = 0; g < kRowGroups; ++g) mine += red[(g * MB + m) * kSplitCols + c];
-        const size_t step = static_cast<size_t>(p.M) * p.N, at = static_cast<size_t>(m) * p.N + n;
-        if (chunk < others) {
-            handover::store(sp.partial + chunk * step + at, handover::word_of(mine));
-            continue;
-        }
-        float v = 0.f;
-        constexpr int kAtOnce = 8;
-        for (int c0 = 0; c0 < others; c0 += kAtOnce) {
-            uint32_t* src = sp.partial + c0 * step + at;
-            const int some = min(kAtOnce, others - c0);
-            uint32_t w[kAtOnce];
-            const long long t0 = clock64();
-            for (bool all = false; !all;) {
-                all = true;
+    for (int m = 0; m < MB; ++m) {
+        mine[m] = 0.f;
 #pragma unroll
-                for (int k = 0; k < kAtOnce; ++k) w[k] = k < some ? handover::load(src + k * step) : 0u;
-#pragma unroll
-                for (int k = 0; k < kAtOnce; ++k) all = all && handover::there(w[k]);
-                if (!all && clock64() - t0 > 2000000000LL) {
-                    if (sp.err) atomicOr(sp.err, ERR_WAIT_TIMEOUT);
-                    return;                                  // a thread waits once: the other sums are as late
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < kAtOnce; ++k) {
-                if (k >= some) continue;
-                handover::store(src + k * step, handover::kNothing);
-                v += __uint_as_float(w[k]);
-            }
-        }
-        p.Y[at] = __float2half_rn(v + mine);
+        for (int g = 0; g < kRowGroups; ++g) mine[m] += red[(g * MB + m) * kSplitCols + tid];
     }
+    const size_t step = static_cast<size_t>(MB) * p.N;
+    uint32_t* const sums = sp.partial + n;
+    if (chunk < others) {
+#pragma unroll
+        for (int m = 0; m < MB; ++m) handover::store(sums + chunk * step + static_cast<size_t>(m) * p.N, handover::word_of(mine[m]));
+        return;
+    }
+    float v[MB];
+#pragma unroll
+    for (int m = 0; m < MB; ++m) v[m] = 0.f;
+    // As many words at a time as registers allow at three CTAs per SM, those of all rows together: with eight of one row
+    // after the other a strip of 86 ranges ended in 44 trips to L2 at four rows.  Raw calls back to back, tickets / eight
+    // of a row / this: 26808 x 1216, four rows 46.3 / 52.6 / 42.7 us, 8082 x 1400 26.3 / 30.0 / 20.5,
+    // 22976 x 1264, two rows 26.2 / 28.8 / 24.8 (the last with the ranges chosen anew, see dense_split_shape).
+    constexpr int kAtOnce = MB == 1 ? 16 : 20 / MB;
+#pragma unroll 1
+    for (int c0 = 0; c0 < others; c0 += kAtOnce) {
+        uint32_t* src = sums + c0 * step;
+        const int some = min(kAtOnce, others - c0);
+        uint32_t w[kAtOnce][MB];
+        const long long t0 = clock64();
+        for (bool all = false; !all;) {
+            all = true;
+#pragma unroll
+            for (int k = 0; k < kAtOnce; ++k)
+#pragma unroll
+                for (int m = 0; m < MB; ++m) w[k][m] = k < some ? handover::load(src + k * step + static_cast<size_t>(m) * p.N) : 0u;
+#pragma unroll
+            for (int k = 0; k < kAtOnce; ++k)
+#pragma unroll
+                for (int m = 0; m < MB; ++m) all = all && handover::there(w[k][m]);
+            if (!all && clock64() - t0 > 2000000000LL) {
+                if (sp.err) atomicOr(sp.err, ERR_WAIT_TIMEOUT);
+                return;                                  // a thread waits once: the other sums are as late
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kAtOnce; ++k) {
+            if (k >= some) continue;
+#pragma unroll
+            for (int m = 0; m < MB; ++m) {
+                handover::store(src + k * step + static_cast<size_t>(m) * p.N, handover::kNothing);
+                v[m] += __uint_as_float(w[k][m]);
+            }
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < MB; ++m) p.Y[static_cast<size_t>(m) * p.N + n] = __float2half_rn(v[m] + mine[m]);
 }
 
 // Fallback for N % 8 != 0 or unaligned W: one thread per column, scalar loads (still
@@ -483,10 +502,11 @@ cudaError_t launch_dense_split(const SplitParams& sp, int strips, int smem_optin
 // Tiles of the split kernel for launches of up to `mb` rows.
 DenseSplit dense_split_shape(int mb, int N, int K, int sm_count, int smem_optin) {
     // The number of K ranges whose waves of tiles take least: a tile costs its rows and about 96 rows' time for the
-    // row statistics and its end, the last of a strip ten rows' time for each range it adds (hidden behind other waves), and as many CTAs are
-    // resident per SM as their shared memory allows, three at most (registers).  4096 x 11008: ten ranges, one wave of
-    // 430 tiles (four tiles per SM before: 602 tiles, a third of a wave left over).  8192 x 1024, one row: 16 / 24 / 32 / 111
-    // ranges 21.3 / 20.3 / 20.1 / 23.2 us a call.
+    // row statistics and its end, the last of a strip so many rows' time for each range it adds (hidden behind other waves),
+    // and as many CTAs are resident per SM as their shared memory allows, three at most (registers).  4096 x 11008: ten ranges,
+    // one wave of 430 tiles (four tiles per SM before: 602 tiles, a third of a wave left over).  The price of a range was
+    // swept over 275 shapes, raw calls back to back against the ticket kernel without it: 4 / 6 / 8 / 10 rows' time 0.872 /
+    // 0.885 / 0.894 / 0.899 of its time on average at one row, 0.821 / 0.817 / 0.823 / 0.823 at two, 0.752 / 0.745 / 0.745 / 0.760 at four.
     const int st = (N + kSplitCols - 1) / kSplitCols;
     const int most = (K + 2 * kStageRows - 1) / (2 * kStageRows);
     const int optin = smem_optin > 0 ? smem_optin : 48 * 1024;
@@ -499,7 +519,7 @@ DenseSplit dense_split_shape(int mb, int N, int K, int sm_count, int smem_optin)
         // an SM has 1 KB more than one block may take, and every block costs 1 KB of it
         const unsigned per_wave = (3 * (smem + 1024) <= optin + 1024 ? 3u : 2 * (smem + 1024) <= optin + 1024 ? 2u : 1u) * sm_count;
         const double waves = static_cast<double>((static_cast<unsigned long long>(st) * c + per_wave - 1) / per_wave);
-        const double cost = waves * (static_cast<double>(K) / c + 96.0) + 10.0 * c / waves;
+        const double cost = waves * (static_cast<double>(K) / c + 96.0) + (mb == 1 ? 4.0 : 6.0) * c / waves;
         if (best == 0.0 || cost < best) { best = cost; ch = c; }
     }
     const int kc = rows_of(ch);
