@@ -687,3 +687,24 @@ def test_raw_attention_entry_matches_oracle(tc, ctx, oracle):
     assert np.abs(O.astype(np.float32) - Oo.astype(np.float32)).max() < 1e-3
     for b in [bq, bo] + bks + bvs:
         b.close()
+
+
+@pytest.mark.parametrize("fmt", [0, 1])
+@pytest.mark.parametrize("M", [1, 2, 3, 4])
+@pytest.mark.parametrize("N,K", [(4700, 256), (8900, 768), (9472, 256), (14000, 2816), (4763, 11008), (300, 14336), (1, 14336)])
+def test_boxes_of_a_warp_over_row_blocks_and_groups(tc, ctx, oracle, fmt, M, N, K):
+    """A warp's boxes go over the K groups of a row block and on to the next: one group a row to more than there are warps,
+    CTAs of one row, with a row more, and with rows in a second or third block of which few are theirs.
+    Bar: that of fp32 activations (16-bit staging)."""
+    rng = np.random.default_rng(N + K + M + fmt)
+    rows = min(N, 131)                                   # the weights repeat: the oracle's share of the time
+    Wq = np.asarray(oracle.quantize_weights((rng.standard_normal((rows, K)) * 0.02).astype(np.float16), fmt)).reshape(rows, -1)
+    X = rng.standard_normal((M, K)).astype(np.float32)
+    at = np.arange(N) % rows
+    want = oracle.dequant_dot_f64(X.astype(np.float64), Wq, fmt, rows)[:, at]
+    with ctx.buffer_from_array(X) as bx, ctx.buffer_from_array(np.ascontiguousarray(Wq[at])) as bw, ctx.buffer(M * N * 4) as by:
+        tc.gemv_quantized_ex(ctx, bx, bw, by, fmt, M, N, K, "f32", "f32", None)
+        assert "box" in tc.cuda_last_kernel_name() or M * K > 40000      # (longer rows leave no room for the rings)
+        got = by.to_numpy((M, N), np.float32).astype(np.float64)
+    assert oracle.scaled_rms(got, want) <= 1e-4
+    assert np.abs(got - want).max() <= 1e-2 * np.sqrt((want * want).mean() + 1e-30)     # a wrong box would be far above
