@@ -668,14 +668,22 @@ int mma_columns(int M, int* col_tiles) {
 //   28672 x 4096 (32 / 24.2)  21.5 / 18.2   22.7 / 19.7   30.5 / 31.5   33.4 / 34.0   58.0 / 54.8   112 / 102 (64 / 48.4)
 //   20000 x 2048 (16 / 8.5)   15.7 / 10.2   16.4 / 11.1   19.7 / 16.2   22.5 / 18.5   39.2 / 29.5   62.0 / 46.8 (24 / 17)
 //   4096 x 4096 (4 / 3.5)      8.7 /  8.0    9.2 /  8.8   10.9 / 15.0 (clusters of four)
-// Q8_0's units take longer up to 32 columns (0.82 against 0.5 us), so fewer of them pay.
+// Q8_0's units take longer up to 32 columns (0.82 against 0.5 us), so fewer of them pay; and the longer the tiles the more
+// they have to be, because the weights then come at HBM's rate either way.  With fewer tiles than SMs (differences of 200
+// calls of 104 to 147 tiles): saved 5 units of 16 / 32 / 50 / 80 Q4_0 +0.1 / +0.1 / +0.2 / +1.5 us, 8 units - / -0.9 / -0.8 / -0.7;
+// Q8_0 5 units -0.5 / -0.2 / +2.3 / +1.0, 8 units - / -1.8 / +0.2 / -0.5.
+// And not where a tile is in the hands of many CTAs, whose sums are taken one after the other: more than seven, or ten where
+// shares are seven units or more.  Clusters / shares: Q4_0, 32 rows, 768 x 28672 12.9 / 18.0 us, 1024 x 20480 11.5 / 14.7;
+// 16 rows 2048 x 28672 15.6 / 14.5, Q8_0 21.7 / 19.2; 2560 x 14336 15.0 / 13.6 but 2560 x 11008 12.6 / 13.3.
 struct Shares { int n; bool pay; };
 Shares shares_of(int fmt, int nb, long long tiles, int groups, int sms) {
     const long long units = tiles * groups;
     const int n = units < sms ? static_cast<int>(units) : sms;
     const double saved = static_cast<double>((tiles + sms - 1) / sms) * groups - static_cast<double>(units) / n;
-    return {n, tiles > sms ? saved > (nb <= 32 ? 4.0 : nb <= 128 ? 7.0 : 5.6)
-                           : nb <= 32 && units >= 3 * sms && saved > (fmt == FMT_Q4_0 ? 5.5 : 4.0)};
+    if (tiles > sms) return {n, saved > (nb <= 32 ? 4.0 : nb <= 128 ? 7.0 : 5.6)};
+    const bool few = 7 * tiles > sms || (10 * tiles > sms && units >= 7 * sms);
+    const double least = fmt == FMT_Q4_0 ? 5.5 : 4.0, by_length = (fmt == FMT_Q4_0 ? 0.1 : 0.15) * groups;
+    return {n, nb <= 32 && few && units >= 3 * sms && saved > (by_length < least ? least : by_length > 8.0 ? 8.0 : by_length)};
 }
 size_t share_bytes(const Shares& s, int nb) { return static_cast<size_t>(s.n) * nb * kRows * 4; }
 

@@ -416,3 +416,22 @@ def test_tiles_left_over_in_a_captured_call(tc, ctx, oracle, fmt, M, N, K):
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
     check_tiles(outs[0], want, factors, 1.1 * np.sqrt(2.0) * ROUND)
     assert tc.take_device_error(ctx) == 0
+
+
+@pytest.mark.parametrize("fmt,M,N,K", [(0, 32, 768, 28672), (0, 16, 1024, 20480), (0, 8, 1400, 10240), (1, 16, 2048, 28672), (0, 16, 2048, 28672),
+                                       (1, 14, 2400, 14336), (0, 32, 2560, 11008), (1, 32, 2560, 14336), (0, 8, 2800, 8192)])
+def test_few_tiles_of_long_rows(tc, ctx, oracle, fmt, M, N, K):
+    """Fewer tiles than SMs by far: split over clusters, or shares with up to ten CTAs a tile; one launch, the same bits."""
+    import torch
+    x, w, want, factors = distinct_tiles(oracle, fmt, M, N, K)
+    st = torch.cuda.current_stream().cuda_stream
+    outs = []
+    for _ in range(3):
+        y = torch.full((M, N), float("nan"), device="cuda").half()
+        before = tc.launch_count()
+        tc.raw_gemv_quantized(ctx, x.data_ptr(), w.data_ptr(), y.data_ptr(), fmt, M, N, K, "f16", "f16", st)
+        assert "tcgen05" in tc.cuda_last_kernel_name() and tc.launch_count() - before == 1
+        outs.append(y)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    check_tiles(outs[0], want, factors, 1.1 * np.sqrt(2.0) * ROUND)
+    assert tc.take_device_error(ctx) == 0
