@@ -445,11 +445,11 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const
     extern __shared__ __align__(128) uint8_t smem[];
     const uint32_t ring = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, tq = lane & 3;
-    const int G = p.Hq / p.Hkv, R = p.Sq * G;
-    const int heads = p.B * p.Hkv, bk = blockIdx.x % heads;
+    const int G = p.per_kv, R = p.Sq * G;
+    const int tile_no = SPLIT_KEYS ? 0 : p.by_heads(static_cast<int>(blockIdx.x)), bk = static_cast<int>(blockIdx.x) - tile_no * p.B * p.Hkv;
     const int row_tiles = SPLIT_KEYS ? 1 : (R + kMmaRows - 1) / kMmaRows;
-    const int tile0 = SPLIT_KEYS ? 0 : (row_tiles - 1 - static_cast<int>(blockIdx.x / heads)) * kMmaRows;    // long causal tiles first
-    const int b = bk / p.Hkv, hkv = bk % p.Hkv;
+    const int tile0 = SPLIT_KEYS ? 0 : (row_tiles - 1 - tile_no) * kMmaRows;    // long causal tiles first
+    const int b = p.by_Hkv(bk), hkv = bk - b * p.Hkv;
     const int chunk = blockIdx.y;
     const __half* Kh = p.K + static_cast<size_t>(bk) * p.Sk * D;
     const __half* Vh = p.V + static_cast<size_t>(bk) * p.Sk * D;
@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const
         const int r = r_lo + 8 * e;
         live[e] = r < R;
         const int rr = live[e] ? r : R - 1;
-        qi[e] = rr / G;
+        qi[e] = p.by_per_kv(rr);
         const int h = hkv * G + (rr - qi[e] * G);
         row_at[e] = (static_cast<size_t>(b) * p.Hq + h) * p.Sq + qi[e];
         slope[e] = p.slopes ? p.slopes[h] : 0.f;
@@ -478,7 +478,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 2) attention_mma_kernel(const
         }
     }
     // keys any row of the tile can see, in whole steps from the chunk's start
-    const int i_min = tile0 / G, i_max = (min(R, tile0 + kMmaRows) - 1) / G;
+    const int i_min = p.by_per_kv(tile0), i_max = p.by_per_kv(min(R, tile0 + kMmaRows) - 1);
     int k0 = chunk * p.keys_per_chunk, k1 = min(p.Sk, k0 + p.keys_per_chunk);
     if (p.causal) k1 = min(k1, i_max + 1);
     if (p.window > 0 && i_min - p.window > k0) k0 += (i_min - p.window - k0) / kStepKeys * kStepKeys;
