@@ -708,6 +708,11 @@ size_t gemm_q_tc_share_bytes(const GemvQArgs* ops, int n_ops, int M, int sm_coun
     return s.pay ? share_bytes(s, nb) : 0;
 }
 
+size_t gemm_q_tc_share_room(int M, int sm_count) {
+    int col_tiles = 1;
+    return share_bytes({sm_count > 0 ? sm_count : 148, true}, mma_columns(M, &col_tiles));
+}
+
 // Up to kMaxMats products of the same activation rows in one launch: ops[1 ..] differ from ops[0] in W, Y and N
 // only.  cudaErrorNotSupported when the operation is outside this kernel's domain.
 cudaError_t launch_gemm_q_tc(const GemvQArgs* ops, int n_ops, const LaunchEnv& env, cudaStream_t stream, int* launches) {

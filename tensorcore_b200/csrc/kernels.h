@@ -129,6 +129,8 @@ inline bool dequant_once(const GemvQArgs& a) {
 
 // Bytes of GemvQArgs::share_scratch for M activation rows of n_ops products in one launch; 0 where tiles stay whole.
 size_t gemm_q_tc_share_bytes(const GemvQArgs* ops, int n_ops, int M, int sm_count);
+// As many as any products of M rows can need.
+size_t gemm_q_tc_share_room(int M, int sm_count);
 
 // Tiles of the dense split kernel: column strips, K ranges per strip, rows of a K range.
 struct DenseSplit { int strips = 0, chunks = 0, kc = 0; };
