@@ -15,17 +15,18 @@
 //     where four take 2900): running maximum (an atomic on the row's word in shared memory), exponentials; O is rescaled
 //     in tensor memory only when a row's maximum has grown.  The probabilities are fp32
 //     numbers; each goes to the tensor core as two fp16 numbers (attention_math.cuh says to how many bits), two MMAs.
-//   * Q and O cross global memory by whole rows, O through shared memory: a thread per row takes a clock for each lane
-//     and 16 bytes, 2600 for O.  Rows' queries and heads by multiplication (FastDiv): the device's divisions were 700
-//     clocks of the way to the first load.
+//   * Q and O cross global memory by whole rows, O through shared memory (a thread per row takes a clock for each lane
+//     and 16 bytes: O 2650 clocks instead of 2400).  Rows' queries and heads by multiplication (FastDiv): the device's
+//     divisions were 700 clocks of the way to the first load.
 //
 // What bounds it: latency.  Causal 512 x 512, 32 heads on 8 K/V heads, head_dim 128 is 128 CTAs of up to four
-// steps; clock stamps of the longest before the last changes: 5500 clocks until the first scores (Q's load 2000 of
-// them, its MMAs 1300), 2900 a step - scores and maximum 1000 to 1300, exponentials 1000, rescaling 500, storing P 350 -
-// in which 1060 clocks of P V and 530 of Q K^T hide, 1600 for the last P V, 2900 to store O.  Whole calls: 28.0 us with two
-// threads per row, 26.1 now (10 us of it launch and wait), 2048 x 2048 97.5 -> 88.3, 4 x 2048 x 2048 without a mask
+// steps; clock stamps of the longest, inputs in HBM: barriers and tensor memory ready at 3500, Q in shared memory 5400,
+// first scores 6800; 3100 a step - scores and maximum 1000 to 1250, exponentials 1000, the wait for P V, rescaling and
+// storing P 850, the wait for the next scores 270 - in which 1060 clocks of P V and 530 of Q K^T hide; 1500 for the last
+// P V, 2400 for O (1500 of them through shared memory); 23,100 in all.  Whole calls: 28.2 us with two
+// threads per row, 25.8 now (10 us of it launch and wait), 2048 x 2048 97.5 -> 88.3, 4 x 2048 x 2048 without a mask
 // 500 -> 467; 38 us on the mma.sync kernel, whose tensor instructions run at an eighth of the rate, 388 us as a
-// streaming pass per query row.
+// streaming pass per query row.  The instance of head_dim 128 spills 40 bytes (96 registers, what 18 warps leave).
 #include "attention_math.cuh"
 #include "kernels.h"
 #include "sm100_prims.cuh"

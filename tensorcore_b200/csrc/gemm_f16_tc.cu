@@ -6,9 +6,11 @@
 //   * One CTA per SM walks the tiles of C (128 or 256 rows x 64 to 256 columns), each over the whole K, 64
 //     at a time, through a ring of stages that keeps running across tiles; two sets of accumulators in
 //     tensor memory where they fit, so that one tile is read out and stored while the next one's MMAs
-//     run.  What bounds it is shared-memory bandwidth: a K step of a 256 x 160 tile writes 52 KB and its
-//     MMAs read 72 KB (B once per 128 rows), 970 clocks at 128 bytes each against 640 of tensor work.  With few
-//     rows of A the waits and the issue of a K step are the bound, so a stage then holds several.
+//     run.  What bounds the K loop is what an SM takes in from L2, 64 bytes a clock.  Clock stamps of a CTA, clocks per
+//     64 of K (bytes it copies / tensor work): 256 x 160 860 (53 KB, 832 clocks / 640), 128 x 64 382 (24.6 KB, 384 / 216),
+//     256 x 256 1023 (65.5 KB, 1024 / 1024).  With few rows of A the waits and the issue of a K step are the bound, so a
+//     stage then holds several.  512 x 11008 x 4096 (256 x 160), inputs in HBM: 5500 clocks to the first operands, 54,800
+//     for 64 steps, 3700 for the last MMAs and the read-out, which nothing hides.
 //   * The issuing lane runs its loop alone, and the rows of a tile are a constant of the instance: a wait of the
 //     whole warp at each stage and a branch between MMAs cost 70 clocks a stage and more (whole calls,
 //     512 x 4096 x 11008 78.4 -> 55.8 us, 1024 x 4096 x 4096 47.9 -> 37.6, 512 x 11008 x 4096 51.5 -> 48.9).
@@ -415,8 +417,8 @@ cudaError_t launch_gemm_f16_tc(const void* A, const void* B, void* C, int M, int
     p.a_mnmajor = transpose_a ? 1 : 0;
     // Tile: the one whose rounds over the SMs take least, by a model of a 64-wide K step and of what a tile costs
     // beside its steps.  A step is four MMAs of N / 2 clocks per 128 rows, each at least 54 (the measured floor with
-    // both operands in shared memory), or the shared-memory traffic - the stage's bytes written once, A read
-    // once and B once per 128 rows - at 120 bytes per clock.  256 rows need less traffic per flop; their two
+    // both operands in shared memory), or its traffic, counted as the stage's bytes written once, A read
+    // once and B once per 128 rows, at 120 bytes per clock (a form that was fitted; the header says what the traffic is).  256 rows need less traffic per flop; their two
     // accumulators leave room for a second set only up to 128 columns, so a wider tile's read-out is not hidden:
     // 10000 clocks a round, against 1500 per 128 rows where it is (3000 to 7000 choose worse tiles: 256 x 14336 x 4096
     // 47 us instead of 44.5, 2048^3 30 instead of 28.7).  Fitted to whole calls of 144 shapes (M 64 to
