@@ -119,7 +119,12 @@ __device__ __forceinline__ void transpose_pieces(uint32_t (&h)[4][4], int lane) 
 // KS: 64-wide K slices per stage.  MT: rows of a tile in units of 128; fixed for each instance, because a branch
 // between two MMAs costs the issuing thread more than the MMA (4096^3 in 128 x 256 tiles 134 us with MT a run-time
 // value, 121 with a constant).
-template <int KS, int MT>
+// WIDE: results leave by 64-byte pieces of rows.  Up to kNarrowRows rows most lanes of a store have no row anyway, and an
+// instance without that code (36 to 62 registers, not 63) is faster: raw norm + GEMM calls back to back, wide / narrow, 8 x
+// 4592 x 4000 20.2 / 18.7 us, 27 x 8096 x 640 26.7 / 24.7; on average narrow takes 0.980 / 0.993 / 0.985 / 0.990 / 0.998 of
+// the time up to 8 / 16 / 32 / 48 / 64 rows (200 shapes), 0.998 from 65 to 128.
+constexpr int kNarrowRows = 64;
+template <int KS, int MT, bool WIDE>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap bmap) {
     const int BN = p.bn;
@@ -273,7 +278,7 @@ gemm_f16_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap,
             tc_fence_after_sync();
             const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>((acc * MT + half) * BN);
             int c0 = 0;
-            if (vec) {
+            if (WIDE && vec) {
                 // 32 columns at a time: a thread has 64 bytes of its row, and groups of four threads exchange 16-byte pieces
                 // so that each store writes 64 bytes of eight rows, not 16 of 32.
                 const int group_row = row - (lane & 3), piece = lane & 3;
@@ -383,8 +388,10 @@ cudaError_t launch_tile(const GemmParams& p, const void* A, const void* B, int l
     const long tiles = static_cast<long>((p.N + BN - 1) / BN) * ((p.M + tile_rows - 1) / tile_rows);
     const long sms = env.sm_count > 0 ? env.sm_count : 148;
     const dim3 grid(static_cast<unsigned>(tiles < sms ? tiles : sms));     // one CTA per SM walks the tiles
-    auto* kernel = p.mt == 1 ? (ks == 4 ? gemm_f16_tc_kernel<4, 1> : ks == 2 ? gemm_f16_tc_kernel<2, 1> : gemm_f16_tc_kernel<1, 1>)
-                             : (ks == 4 ? gemm_f16_tc_kernel<4, 2> : ks == 2 ? gemm_f16_tc_kernel<2, 2> : gemm_f16_tc_kernel<1, 2>);
+    const bool wide = p.mt == 2 || p.M > kNarrowRows;
+    auto* kernel = p.mt == 2 ? (ks == 4 ? gemm_f16_tc_kernel<4, 2, true> : ks == 2 ? gemm_f16_tc_kernel<2, 2, true> : gemm_f16_tc_kernel<1, 2, true>)
+                   : wide    ? (ks == 4 ? gemm_f16_tc_kernel<4, 1, true> : ks == 2 ? gemm_f16_tc_kernel<2, 1, true> : gemm_f16_tc_kernel<1, 1, true>)
+                             : (ks == 4 ? gemm_f16_tc_kernel<4, 1, false> : ks == 2 ? gemm_f16_tc_kernel<2, 1, false> : gemm_f16_tc_kernel<1, 1, false>);
     kernel<<<grid, (2 + 4 * p.mt) * 32, smem, stream>>>(q, amap, bmap);
     return cudaGetLastError();
 }
@@ -392,8 +399,9 @@ cudaError_t launch_tile(const GemmParams& p, const void* A, const void* B, int l
 }  // namespace
 
 cudaError_t init_gemm_tc_kernel(int smem_optin) {
-    for (auto* k : {gemm_f16_tc_kernel<1, 1>, gemm_f16_tc_kernel<2, 1>, gemm_f16_tc_kernel<4, 1>, gemm_f16_tc_kernel<1, 2>, gemm_f16_tc_kernel<2, 2>,
-                    gemm_f16_tc_kernel<4, 2>}) {
+    for (auto* k : {gemm_f16_tc_kernel<1, 1, true>, gemm_f16_tc_kernel<2, 1, true>, gemm_f16_tc_kernel<4, 1, true>, gemm_f16_tc_kernel<1, 1, false>,
+                    gemm_f16_tc_kernel<2, 1, false>, gemm_f16_tc_kernel<4, 1, false>, gemm_f16_tc_kernel<1, 2, true>, gemm_f16_tc_kernel<2, 2, true>,
+                    gemm_f16_tc_kernel<4, 2, true>}) {
         const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin);
         if (e != cudaSuccess) return e;
     }

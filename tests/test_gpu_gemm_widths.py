@@ -76,3 +76,28 @@ def test_rows_and_columns_past_the_result_stay(tc, ctx, M, N, ldc, dtype):
     assert err <= 1.05 * (2.0 ** -11 if dtype == "f16" else 2.0 ** -8) / np.sqrt(3.0)
     assert (C[M:] == 7.0).all() and (C[:, N:] == 7.0).all()
     assert tc.take_device_error(ctx) == 0
+
+
+@pytest.mark.parametrize("M", [1, 33, 63, 64, 65, 96, 128])
+@pytest.mark.parametrize("N,K", [(40, 64), (264, 128), (1000, 1024)])
+@pytest.mark.parametrize("tb", [True, False])
+def test_both_forms_of_the_read_out(tc, ctx, M, N, K, tb):
+    """Around the number of rows from which results leave by pieces of rows, one to four slices of K a stage; rows of the result
+    before and behind it stay.  (One row takes the row kernel: the bar is the same.)"""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M + N + K)
+    A, B = torch.randn(M, K, generator=g, device="cuda").half(), torch.randn((N, K) if tb else (K, N), generator=g, device="cuda").half()
+    room = torch.full((M + 16, N), 7.0, device="cuda").half()
+    C = room[8:8 + M]
+    bufs = [ctx.buffer_from_ptr(t.data_ptr(), t.numel() * 2) for t in (A, B, C)]
+    torch.cuda.synchronize()
+    tc.gemm(ctx, *bufs, M, N, K, transpose_b=tb)
+    for b in bufs:
+        b.close()
+    want = A.double() @ (B.double().t() if tb else B.double())
+    # of few results the rms scatters: three times 1 / sqrt(2 n)
+    bar = 1.05 * 2.0 ** -11 / np.sqrt(3.0) * (1 + 3 / np.sqrt(2 * M * N))
+    assert ((C.double() - want).square().mean() / want.square().mean()).sqrt().item() <= bar
+    assert (room[:8] == 7.0).all() and (room[8 + M:] == 7.0).all()
+    assert tc.take_device_error(ctx) == 0
