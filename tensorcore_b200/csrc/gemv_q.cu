@@ -205,8 +205,9 @@ gemv_q_box_kernel(const StreamParams p, const __grid_constant__ CUtensorMap wmap
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nwarps = blockDim.x >> 5, nthreads = blockDim.x;
     const int ns = p.ns, gpr = p.gpr;
-    // Two rows keep the divisions, with which Q8_0 does not spill (24 to 36 bytes otherwise: 11023 x 11008 34.7 -> 36.9 us a call).
-    constexpr bool kDivide = MB == 2;
+    // Two rows of Q8_0 keep the divisions, with which they do not spill (24 to 36 bytes otherwise: 11023 x 11008 34.7 -> 36.9 us
+    // a call; Q4_0 does not in either form, 30530 x 26368 144 us with divisions, 138 without).
+    constexpr bool kDivide = MB == 2 && FMT == FMT_Q8_0;
     const int r0 = kDivide ? static_cast<int>(static_cast<long long>(p.N) * blockIdx.x / gridDim.x) : p.rows_of.first(blockIdx.x);
     const int r1 = kDivide ? static_cast<int>(static_cast<long long>(p.N) * (blockIdx.x + 1) / gridDim.x) : p.rows_of.first(blockIdx.x + 1);
     const int rows = r1 - r0;
